@@ -235,6 +235,12 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, force_skinny: bo
   if M == 0:
     return
   lib = common_lib()
+  if (x.dtype == torch.float32 and x.is_cuda and x.stride(1) == 1 and (x.stride(0) >= K or M == 1)
+      and (x.is_contiguous() or (w.dtype == out.dtype == torch.float32 and w.is_contiguous() and out.is_contiguous()))):
+    # packed rows or a column range of wider ones: one kernel, so a row's value does not depend on how many rows there are
+    _check(lib, lib.mi_gemm_f32(_ptr(out, torch.float32), ctypes.c_void_p(x.data_ptr()), _ptr(w, torch.float32), M, N, K,
+                                max(int(x.stride(0)), K), N, _stream()))
+    return
   if not x.is_contiguous() or (x.dtype == torch.bfloat16 and (K % 8 != 0 or x.data_ptr() % 16 != 0 or w.data_ptr() % 16 != 0)):
     # x is a column range of wider rows, or its rows cannot be read 16 bytes at a time: the library product for many
     # bfloat16 rows, else the product that takes any strides and sizes
@@ -255,7 +261,7 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, force_skinny: bo
     linear_batched(out.unsqueeze(1), x.unsqueeze(1), w.unsqueeze(0))
     return
   if x.dtype == torch.float32:
-    _check(lib, lib.mi_gemm_f32(_ptr(out, torch.float32), _ptr(x), _ptr(w, torch.float32), M, N, K, N, _stream()))
+    _check(lib, lib.mi_gemm_f32(_ptr(out, torch.float32), _ptr(x), _ptr(w, torch.float32), M, N, K, K, N, _stream()))
     return
   if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
     raise KernelError(f"linear: operands must both be float32 or both bfloat16, got {x.dtype} and {w.dtype}")
