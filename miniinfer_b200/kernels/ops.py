@@ -1360,6 +1360,17 @@ def attention(out: torch.Tensor, qkv: torch.Tensor, kv_layer: torch.Tensor, bloc
     _attention_bf16(out, qkv, kv_layer, block_table, batch, num_heads, num_kv_heads, head_dim, scale, win, page_size, opts)
     return
   lib = common_lib()
+  if (qkv.dtype == torch.float32 and not force_generic and T <= 65535 and head_dim % 4 == 0 and head_dim <= 256 and num_heads <= 32 * num_kv_heads
+      and opts.softcap == 0 and score_bias is None and distance is None and qkv.data_ptr() % 16 == 0 and kv_layer.data_ptr() % 16 == 0
+      and qkv.shape[1] % 4 == 0 and batch.decode_items is not None and batch.prefill_tiles is not None):
+    # by the model's options alone, never by the step: a row takes the same kernel, and the same order of sums, in every step
+    _check(lib, lib.mi_attention_f32(
+      _ptr(out), _ptr(qkv), qkv.shape[1], _ptr(kv_layer), _ptr(block_table, torch.int32), block_table.shape[1],
+      _ptr(batch.prefill_tiles, torch.int32), batch.num_prefill_tiles, PREFILL_TILE, _ptr(batch.decode_items, torch.int32), batch.num_decode,
+      _ptr(batch.q_start, torch.int32), _ptr(batch.q_len, torch.int32), _ptr(batch.ctx_len, torch.int32), _ptr(batch.seq_slot, torch.int32),
+      num_heads, num_kv_heads, head_dim, page_size, ctypes.c_float(scale), win, opts.sink_ptr(), opts.gate_ptr(), gate_stride, ohd,
+      opts.keep_first, int(opts.gate_per_head), _stream()), kernels=int(batch.num_prefill_tiles > 0) + int(batch.num_decode > 0))
+    return
   _check(lib, lib.mi_attention_generic(
     _ptr(out), _ptr(qkv), qkv.shape[1], _dt(qkv), _ptr(kv_layer), _ptr(block_table, torch.int32),
     block_table.shape[1], _ptr(batch.token_item, torch.int32), _ptr(batch.positions, torch.int32),

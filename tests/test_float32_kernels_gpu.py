@@ -29,3 +29,58 @@ def test_linear_float32_forms_agree(N, K, lead):
   packed = torch.empty(130, N, device=DEV)
   ops.linear(packed, x.contiguous(), w)
   assert torch.equal(packed, first), "nor on where its operand lies"
+
+
+def _batch_of(slot, ctx, new):
+  from miniinfer_b200.kernels.ops import AttentionBatch
+  dev = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+  tiles = [(0, o) for o in range(0, new, 64)] if new > 1 else []
+  return AttentionBatch(token_item=dev([0] * new), positions=dev(list(range(ctx - new, ctx))), seq_slot=dev([slot]), q_start=dev([0]),
+                        q_len=dev([new]), ctx_len=dev([ctx]), num_tokens=new, num_items=1, prefill_tiles=dev(tiles).view(-1, 2),
+                        num_prefill_tiles=len(tiles), decode_items=dev([0] if new == 1 else []), num_decode=int(new == 1),
+                        max_ctx_len=ctx, scratch=None)
+
+
+# (items (context, new), query heads, kv heads, head size, page size, options): segments of 256 keys just full, one key over, and many
+# for a cluster; tiles of 64 tokens cut by groups that do not divide 32; windows and kept keys that share a segment
+F32_CASES = [
+  ([(256, 1), (257, 1), (2600, 1), (1, 1)], 16, 8, 128, 64, {}),
+  ([(300, 300), (700, 65), (513, 2)], 16, 8, 128, 64, dict(sink=True)),
+  ([(520, 130), (90, 1)], 6, 2, 20, 16, dict(window=100, keep_first=7)),
+  ([(900, 70), (777, 1)], 12, 1, 256, 48, dict(window=300, keep_first=290, sink=True, out_hd=200, gate="head")),
+  ([(1300, 33), (1025, 1)], 32, 1, 224, 64, dict(out_hd=192, gate="head")),
+  ([(610, 40), (512, 1)], 5, 5, 68, 16, dict(chunk=256, gate="value")),
+]
+
+
+@pytest.mark.parametrize("case", range(len(F32_CASES)))
+def test_attention_float32_against_the_generic_kernel_and_cut_by_cut(case):
+  from gpu_helpers import make_attention_case
+  from miniinfer_b200.kernels import ops
+  items, nh, nkv, hd, P, opt = F32_CASES[case]
+  qkv, kv, bt, batch = make_attention_case(items, nh, nkv, hd, P, torch.float32, seed=case)
+  T, ohd = qkv.shape[0], opt.get("out_hd", hd)
+  g = torch.Generator().manual_seed(case)
+  sink = torch.randn(nh, generator=g).to(DEV) if opt.get("sink") else None
+  per_head = opt.get("gate") == "head"
+  gate = torch.randn(T, nh * (1 if per_head else ohd), generator=g).to(DEV) if opt.get("gate") else None
+
+  def run(rows, b, generic=False):
+    out = torch.full((rows.stop - rows.start, nh * ohd), float("nan"), device=DEV)
+    ops.attention(out, qkv[rows], kv, bt, b, nh, nkv, hd, hd ** -0.5, opt.get("window"), force_generic=generic, sink=sink,
+                  gate=gate[rows].contiguous() if gate is not None else None, out_hd=ohd, keep_first=opt.get("keep_first", 0),
+                  chunk=opt.get("chunk"), gate_per_head=per_head)
+    return out
+
+  got, want = run(slice(0, T), batch), run(slice(0, T), batch, generic=True)
+  # both sum at most 2600 weighted values of unit size in float32: each errs by a few 1e-6, as test_attention_over_pages allows
+  assert (got - want).abs().max() < 2e-5
+  if DEV == "cpu":
+    return
+  at = 0
+  for b, (ctx, new) in enumerate(items):      # alone, and in portions of other sizes down to single tokens
+    slot = int(batch.seq_slot[b])
+    portions = [(0, new)] + ([(0, new // 3), (new // 3, new // 3 + 1), (new // 3 + 1, new - 1), (new - 1, new)] if new > 3 else [])
+    for lo, hi in portions:
+      assert torch.equal(run(slice(at + lo, at + hi), _batch_of(slot, ctx - new + hi, hi - lo)), got[at + lo:at + hi]), (b, lo, hi)
+    at += new
