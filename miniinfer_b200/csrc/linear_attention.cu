@@ -20,7 +20,7 @@
 //
 // Everything between the projections and the gate is float32: angles (a table made on the host), decays and their
 // logarithms, the state and the sums over it, the norm.
-#include "common.cuh"
+#include "chunked_state.cuh"
 
 namespace {
 
@@ -117,6 +117,7 @@ struct LinArgs {
   float* state; long long state_stride;  // [slot][heads][dim][vdim]
   const int* q_start; const int* q_len; const int* seq_slot;
   int heads, dim, vdim, R;
+  int skip_from;                         // > 0: items of at least so many new tokens are somebody else's (MODE 0)
   // stretches side by side (MODE 1, 2)
   float* seg_state;                      // [item, stretch][heads][dim][vdim]: a stretch's end state from a zero start (MODE 1
                                          // writes), then - after the carry kernel - the state it starts from (MODE 2 reads)
@@ -138,6 +139,7 @@ linear_recurrence_kernel(LinArgs a) {
   const int item = MODE == 0 ? blockIdx.y : blockIdx.y / LIN_SEGMENTS, head = blockIdx.x;
   const int seg = MODE == 0 ? 0 : blockIdx.y % LIN_SEGMENTS;
   int row0 = a.q_start[item], n_new = a.q_len[item];
+  if (MODE == 0 && a.skip_from > 0 && n_new >= a.skip_from) return;
   const int slot = a.seq_slot[item];
   const float hd = CHANNEL ? 1.f : a.head_decay[head];     // a constant of the model
   if (MODE != 0) {
@@ -421,7 +423,10 @@ MI_API int mi_linear_attention(void* out, int ldo, const void* q, int ldq, const
                                const float* head_decay, const float* rope, const int* positions, int rot_dims, float q_scale,
                                float k_scale, const float* norm_w, float eps, int gate_silu, float* state, long long state_stride,
                                const int* q_start, const int* q_len, const int* seq_slot, int T, int items, int heads, int dim,
-                               int vdim, float* scratch, float* segments, cudaStream_t stream) {
+                               int vdim, float* scratch, float* segments, float* chunks, int chunk_min, cudaStream_t stream) {
+  // chunks: null, or mi_chunked_state_floats of scratch - then items of at least chunk_min new tokens are walked a chunk of tokens at
+  // a time (bfloat16 only; excludes segments), the others token by token
+  MI_REQUIRE(chunks == nullptr || (dtype == MI_BF16 && segments == nullptr && chunk_min > 1), "linear_attention: chunks are for bfloat16 activations");
   MI_REQUIRE(T >= 0 && items >= 0 && items <= 65535 && heads > 0 && heads <= 65535, "linear_attention: bad counts T=%d items=%d heads=%d", T, items, heads);
   MI_REQUIRE(dim > 0 && vdim > 0 && dim <= 4096, "linear_attention: bad sizes dim=%d vdim=%d", dim, vdim);
   MI_REQUIRE((a_in != nullptr) != (head_decay != nullptr), "linear_attention: decays come per channel (logits) or per head (constants), one of the two");
@@ -453,6 +458,7 @@ MI_API int mi_linear_attention(void* out, int ldo, const void* q, int ldq, const
   d.raw = raw; d.qn = qn; d.kn = kn; d.g = g; d.head_decay = head_decay;
   d.state = state; d.state_stride = state_stride; d.q_start = q_start; d.q_len = q_len; d.seq_slot = seq_slot;
   d.heads = heads; d.dim = dim; d.vdim = vdim; d.R = R;
+  d.skip_from = chunks ? chunk_min : 0;
   d.seg_state = segments;
   d.seg_decay = segments ? segments + (size_t)items * LIN_SEGMENTS * heads * dim * vdim : nullptr;
 #define MI_LIN_REC(DKV, CPTV, CH)                                                                                          \
@@ -488,8 +494,14 @@ MI_API int mi_linear_attention(void* out, int ldo, const void* q, int ldq, const
     p.rot_dims = rot_dims; p.q_scale = q_scale; p.k_scale = k_scale; p.qn = qn; p.kn = kn; p.g = g; p.raw = raw;     \
     p.heads = heads; p.dim = dim; p.vdim = vdim;                                                                     \
     mi::launch(linear_prepare_kernel<TT, float>, pgrid, dim3(128), 0, stream, p);                                    \
-    if (channel) MI_LIN_DK(true);                                                                                    \
+    if (chunks && items == 1 && T >= chunk_min) ;                                                                    \
+    else if (channel) MI_LIN_DK(true);                                                                               \
     else MI_LIN_DK(false);                                                                                           \
+    if (chunks) {                                                                                                    \
+      mi::ChunkedStateArgs c{qn, kn, channel ? g : head_decay, channel ? mi::CHUNK_DECAY_CHANNEL : mi::CHUNK_DECAY_CONSTANT, nullptr, raw, state, \
+                             state_stride, q_start, q_len, seq_slot, items, heads, heads, dim, vdim, chunk_min};      \
+      if (int e = mi::chunked_state_run(c, T, chunks, stream)) return e;                                             \
+    }                                                                                                                \
     mi::launch(linear_output_kernel<TT>, ogrid, dim3(128), 0, stream, (TT*)out, ldo, (const float*)raw, (const TT*)gate, ldg, \
                norm_w, heads, vdim, eps, gate_silu);                                                                 \
   } while (0)

@@ -12,7 +12,7 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "delta_chunk.cuh"
+#include "chunked_state.cuh"
 
 namespace {
 
@@ -305,7 +305,6 @@ struct DeltaPrepArgs {
   float* qn; float* kn;                  // [tokens, kv_heads * dim]
   float* g;                              // [tokens, heads * dim], or [tokens, heads] with one decay a head
   float* qk;                             // [tokens, kv_heads]: qh . kh (one decay a head only)
-  float* lg;                             // [tokens, heads]: ln g (one decay a head only)
   int head_decay;
   float* beta;                           // [tokens, heads]
   const T* v; int ldv;                   // values, head h at column h * vdim
@@ -349,11 +348,7 @@ delta_prepare_kernel(DeltaPrepArgs<T> a) {
       const int h = u - a.kv_heads;
       const float neg_rate = -expf(a.A_log[h]);
       if (a.head_decay) {
-        if (lane == 0) {
-          const float lg = fmaxf(neg_rate * softplus_f(mi::to_float(a.a[(size_t)t * a.lda + h]) + a.dt_bias[h]), -1e30f);
-          a.lg[(size_t)t * a.heads + h] = lg;
-          a.g[(size_t)t * a.heads + h] = expf(lg);
-        }
+        if (lane == 0) a.g[(size_t)t * a.heads + h] = expf(neg_rate * softplus_f(mi::to_float(a.a[(size_t)t * a.lda + h]) + a.dt_bias[h]));
       } else for (int i = lane; i < a.dim; i += 32) {
         const float z = mi::to_float(a.a[(size_t)t * a.lda + (size_t)h * a.dim + i]) + a.dt_bias[h * a.dim + i];
         a.g[((size_t)t * a.heads + h) * a.dim + i] = expf(neg_rate * softplus_f(z));
@@ -717,20 +712,19 @@ MI_API int mi_selective_scan(void* y, int ldy, const void* u, int ldu, const voi
   return 0;
 }
 
-// scratch: float32 - unit q and k, decays, q . k, the decays' logarithms, beta, values / read-outs, each starting on a 16-byte boundary
+// scratch: float32 - unit q and k, decays, q . k, beta, values / read-outs, each starting on a 16-byte boundary
 MI_API long long mi_gated_delta_scratch_floats(int T, int heads, int kv_heads, int dim, int vdim, int head_decay) {
-  return (long long)T * ((long long)2 * kv_heads * dim + (long long)heads * (head_decay ? 2 : dim) + kv_heads + heads + (long long)heads * vdim) + 6 * 4;
+  return (long long)T * ((long long)2 * kv_heads * dim + (long long)heads * (head_decay ? 1 : dim) + kv_heads + heads + (long long)heads * vdim) + 5 * 4;
 }
 
 MI_API int mi_gated_delta_segments() { return DELTA_SEGMENTS; }
 
-// Floats of scratch of the walk by chunks, or 0 where it does not take the sizes (one decay a head only).
-MI_API long long mi_gated_delta_chunk_floats(int T, int items, int heads, int dim, int vdim) {
-  if (dim > mi::DELTA_CHUNK_MAX_DIM || dim % 4 != 0 || vdim % 4 != 0) return 0;
-  return mi::delta_chunk_scratch_floats(T, items, heads, dim, vdim);
+// Floats of scratch of the walk by chunks, or 0 where it does not take the sizes; delta 0: linear attention's.
+MI_API long long mi_chunked_state_floats(int T, int items, int heads, int dim, int vdim, int delta) {
+  return mi::chunked_state_takes(dim, vdim) ? mi::chunked_state_scratch_floats(T, items, heads, dim, vdim, delta != 0) : 0;
 }
 
-MI_API int mi_gated_delta_chunk_slabs(int T, int items, int heads) { return mi::delta_chunk_slabs(T, items, heads); }
+MI_API int mi_chunked_state_slabs(int T, int items, int heads) { return mi::chunked_state_slabs(T, items, heads); }
 
 // Blocks that walk one request's tokens in order (heads x groups of value columns): what a long prompt portion keeps
 // busy without stretches side by side.
@@ -750,10 +744,9 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
                           const float* norm_w, float eps, float* state, long long state_stride, const int* q_start, const int* q_len,
                           const int* seq_slot, int T, int items, int heads, int kv_heads, int dim, int vdim, float* scratch,
                           float* segments, int head_decay, int gate_silu, float* chunks, int chunk_min, cudaStream_t stream) {
-  // chunks: null, or mi_gated_delta_chunk_floats of scratch - then items of at least chunk_min new tokens are walked a chunk of
-  // tokens at a time (bfloat16 with one decay a head; excludes segments), the others token by token
-  MI_REQUIRE(chunks == nullptr || (dtype == MI_BF16 && head_decay && segments == nullptr && chunk_min > 1),
-             "gated_delta: chunks are for bfloat16 activations and one decay a head");
+  // chunks: null, or mi_chunked_state_floats of scratch - then items of at least chunk_min new tokens are walked a chunk of
+  // tokens at a time (bfloat16 only; excludes segments), the others token by token
+  MI_REQUIRE(chunks == nullptr || (dtype == MI_BF16 && segments == nullptr && chunk_min > 1), "gated_delta: chunks are for bfloat16 activations");
   // head_decay: a_in [T, heads] and dt_bias [heads], one decay a head, instead of [T, heads * dim] and [heads * dim]
   // segments: null, or items * DELTA_SEGMENTS * heads * dim * (vdim + dim) floats of scratch - then the items' tokens run
   // in stretches side by side (bfloat16 only: the sums then depend on where a portion starts; dim up to 256)
@@ -781,8 +774,7 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
   float* kn = qn + up4((size_t)T * kv_heads * dim);
   float* g = kn + up4((size_t)T * kv_heads * dim);
   float* qk = g + up4((size_t)T * heads * (head_decay ? 1 : dim));
-  float* lg = qk + up4((size_t)T * kv_heads);
-  float* beta = lg + (head_decay ? up4((size_t)T * heads) : 0);
+  float* beta = qk + up4((size_t)T * kv_heads);
   float* raw = beta + up4((size_t)T * heads);
   dim3 pgrid(T, (heads + kv_heads + 3) / 4 > 16 ? 16 : (heads + kv_heads + 3) / 4);
   dim3 ogrid(T, (heads + 3) / 4 > 16 ? 16 : (heads + 3) / 4);
@@ -822,7 +814,7 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
     DeltaPrepArgs<TT> p;                                                                                          \
     p.q = (const TT*)q; p.k = (const TT*)k; p.ldqk = ldqk; p.a = (const TT*)a_in; p.lda = lda; p.b = (const TT*)b_in; p.ldb = ldb; \
     p.dt_bias = dt_bias; p.A_log = A_log; p.qn = qn; p.kn = kn; p.g = g; p.beta = beta; p.T_ = T; p.heads = heads;  \
-    p.qk = qk; p.lg = lg; p.head_decay = head_decay;                                                                         \
+    p.qk = qk; p.head_decay = head_decay;                                                                         \
     p.kv_heads = kv_heads; p.dim = dim; p.v = (const TT*)v; p.ldv = ldv; p.raw = raw; p.vdim = vdim;                  \
     mi::launch(delta_prepare_kernel<TT>, pgrid, dim3(128), 0, stream, p);                                         \
     if (DK == 16) MI_DELTA(TT, 16);                                                                               \
@@ -830,8 +822,9 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
     else if (DK == 64) MI_DELTA(TT, 64);                                                                          \
     else MI_DELTA(TT, 128);                                                                                       \
     if (chunks) {                                                                                                 \
-      mi::DeltaChunkArgs c{qn, kn, lg, beta, raw, state, state_stride, q_start, q_len, seq_slot, items, heads, kv_heads, dim, vdim, chunk_min}; \
-      if (int e = mi::delta_chunk_run(c, T, chunks, stream)) return e;                                            \
+      mi::ChunkedStateArgs c{qn, kn, g, head_decay ? mi::CHUNK_DECAY_HEAD : mi::CHUNK_DECAY_CHANNEL, beta, raw, state, state_stride, q_start, q_len, \
+                             seq_slot, items, heads, kv_heads, dim, vdim, chunk_min};                              \
+      if (int e = mi::chunked_state_run(c, T, chunks, stream)) return e;                                            \
     }                                                                                                             \
     mi::launch(delta_output_kernel<TT>, ogrid, dim3(128), 0, stream, (TT*)out, ldo, (const float*)raw, (const TT*)gate, ldg, norm_w, heads, vdim, eps, gate_silu); \
   } while (0)

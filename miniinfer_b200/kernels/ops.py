@@ -610,10 +610,10 @@ DELTA_SEGMENTED_MAX_ITEMS = 4      # the same bound for the delta rule, whose sc
 # B200, 2048 tokens of one request, heads of 128 x 128: 8 heads (64 blocks in order) 5.18 -> 4.57 ms a step of six layers,
 # 16 heads (128 blocks) 7.23 -> 8.11 ms
 DELTA_SEGMENTED_MAX_BLOCKS = 96
-# New tokens a request from which a bfloat16 delta rule with one decay a head goes a chunk at a time.  Measured on B200, heads
-# of 128 x 128, the whole operation, chunks / in order in microseconds: 8 heads 78 / 85 at 128 tokens and 85 / 154 at 256; 16
-# heads 96 / 87 and 106 / 155; 32 heads 104 / 89 and 126 / 163
-DELTA_CHUNK_MIN_TOKENS = 160
+# New tokens a request from which a bfloat16 delta rule goes a chunk at a time (csrc/chunked_state.cu).  Measured on B200, a whole layer of
+# 8 / 16 / 32 heads of 128 x 128 with one decay a key channel, chunks against the walk in order, in microseconds: 96 tokens
+# 86, 94, 123 against 87, 93, 112; 128 tokens 86, 96, 126 against 104, 111, 137; 256 tokens 95, 109, 155 against 179, 189, 226
+DELTA_CHUNK_MIN_TOKENS = 112
 
 
 def selective_scan(y: torch.Tensor, u: torch.Tensor, dt_in: torch.Tensor, bc: torch.Tensor, b_off: int, c_off: int, z: torch.Tensor,
@@ -680,17 +680,12 @@ def gated_delta(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Te
   n = int(lib.mi_gated_delta_scratch_floats(T, heads, kv_heads, dim, vdim, int(head_decay))) + 8
   scratch = workspace.buffer("gated_delta_scratch", (n,), torch.float32) if workspace is not None else \
     torch.empty(n, dtype=torch.float32, device=v.device)
-  # long prompt portions in bfloat16: with one decay a head a chunk of tokens at a time (csrc/delta_chunk.cu); with one a key
-  # channel, or heads too wide for that, each request's tokens in up to 16 stretches side by side (five launches instead of three)
-  segments, chunks, launches = None, None, 3
-  lib.mi_gated_delta_chunk_floats.restype = ctypes.c_longlong
-  if (head_decay and v.dtype == torch.bfloat16 and T - ctx.num_items + 1 >= DELTA_CHUNK_MIN_TOKENS
-      and os.environ.get("MINIINFER_B200_DELTA_CHUNKS", "1") != "0"):
-    m = int(lib.mi_gated_delta_chunk_floats(T, ctx.num_items, heads, dim, vdim))
-    if m > 0:
-      chunks = workspace.buffer("gated_delta_chunks", (m,), torch.float32) if workspace is not None else \
-        torch.empty(m, dtype=torch.float32, device=v.device)
-      launches = (3 if ctx.num_items > 1 else 2) + 3 * int(lib.mi_gated_delta_chunk_slabs(T, ctx.num_items, heads))
+  # long prompt portions in bfloat16: a chunk of tokens at a time (csrc/chunked_state.cu); with heads too wide for that each
+  # request's tokens in up to 16 stretches side by side (five launches instead of three)
+  segments, launches = None, 3
+  chunks, more = _state_chunks(lib, v, ctx, heads, dim, vdim, workspace, DELTA_CHUNK_MIN_TOKENS, True)
+  if chunks is not None:
+    launches = (3 if ctx.num_items > 1 else 2) + more
   if (chunks is None and v.dtype == torch.bfloat16 and ctx.num_items <= DELTA_SEGMENTED_MAX_ITEMS and T >= SCAN_SEGMENTED_MIN_TOKENS * ctx.num_items
       and dim <= 256 and ctx.num_items * int(lib.mi_gated_delta_blocks(heads, dim, vdim)) <= DELTA_SEGMENTED_MAX_BLOCKS
       and os.environ.get("MINIINFER_B200_DELTA_SEGMENTS", "1") != "0"):
@@ -707,11 +702,28 @@ def gated_delta(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Te
                                  DELTA_CHUNK_MIN_TOKENS, _stream()), kernels=launches)
 
 
+# The same for linear attention: 48 tokens 53, 66, 94 against 57, 64, 100; 64 tokens 53, 67, 101 against 61, 74, 108; 256 tokens 66,
+# 81, 129 against 173, 177, 234
+LINEAR_CHUNK_MIN_TOKENS = 64
 LINEAR_SEGMENTED_MAX_ITEMS = 8     # steps of at most this many requests run long bfloat16 portions in stretches side by side
 # ... and only while the walk in order would leave SMs idle (blocks in order, all requests; an SM holds three, and
 # stretches cost twice the arithmetic).  Measured on B200, 8192 tokens of one request beside seven single tokens, 16 heads
 # of 128 x 128 (8 x 32 blocks in order): 4.7 ms in order.
 LINEAR_SEGMENTED_MAX_BLOCKS = 256
+
+
+def _state_chunks(lib, v: torch.Tensor, ctx, heads: int, dim: int, vdim: int, workspace, min_tokens: int, delta: bool):
+  """(scratch, launches) of the walk by chunks of tokens of a step that may bring a request ``min_tokens`` new tokens, or
+  (None, 0): a float32 step, a step of short portions, sizes that the chunks do not take."""
+  if v.dtype != torch.bfloat16 or v.shape[0] - ctx.num_items + 1 < min_tokens or os.environ.get("MINIINFER_B200_DELTA_CHUNKS", "1") == "0":
+    return None, 0
+  lib.mi_chunked_state_floats.restype = ctypes.c_longlong
+  m = int(lib.mi_chunked_state_floats(v.shape[0], ctx.num_items, heads, dim, vdim, int(delta)))
+  if m == 0:
+    return None, 0
+  chunks = workspace.buffer("state_chunks", (m,), torch.float32) if workspace is not None else \
+    torch.empty(m, dtype=torch.float32, device=v.device)
+  return chunks, 3 * int(lib.mi_chunked_state_slabs(v.shape[0], ctx.num_items, heads))
 
 
 def linear_attention(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Tensor, state: torch.Tensor, ctx,
@@ -751,7 +763,10 @@ def linear_attention(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: tor
   scratch = workspace.buffer("linear_attention_scratch", (n,), torch.float32) if workspace is not None else \
     torch.empty(n, dtype=torch.float32, device=v.device)
   segments, launches = None, 3
-  if (v.dtype == torch.bfloat16 and ctx.num_items <= LINEAR_SEGMENTED_MAX_ITEMS and T >= SCAN_SEGMENTED_MIN_TOKENS * ctx.num_items
+  chunks, more = _state_chunks(lib, v, ctx, heads, dim, vdim, workspace, LINEAR_CHUNK_MIN_TOKENS, False)
+  if chunks is not None:
+    launches = (3 if ctx.num_items > 1 else 2) + more
+  if (chunks is None and v.dtype == torch.bfloat16 and ctx.num_items <= LINEAR_SEGMENTED_MAX_ITEMS and T >= SCAN_SEGMENTED_MIN_TOKENS * ctx.num_items
       and ctx.num_items * int(lib.mi_linear_attention_blocks(heads, dim, vdim)) <= LINEAR_SEGMENTED_MAX_BLOCKS
       and os.environ.get("MINIINFER_B200_LINEAR_SEGMENTS", "1") != "0"):
     m = ctx.num_items * int(lib.mi_linear_attention_segments()) * heads * dim * (vdim + 1)
@@ -768,7 +783,8 @@ def linear_attention(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: tor
     _ptr(norm_weight, torch.float32) if norm_weight is not None else none, ctypes.c_float(eps), int(bool(gate_silu)),
     ctypes.c_void_p(state.data_ptr()), ctypes.c_longlong(state.stride(0)), _ptr(ctx.q_start, torch.int32), _ptr(ctx.q_len, torch.int32),
     _ptr(ctx.seq_slot, torch.int32), T, ctx.num_items, heads, dim, vdim, _ptr(scratch, torch.float32),
-    _ptr(segments, torch.float32) if segments is not None else none, _stream()), kernels=launches)
+    _ptr(segments, torch.float32) if segments is not None else none, _ptr(chunks, torch.float32) if chunks is not None else none,
+    LINEAR_CHUNK_MIN_TOKENS, _stream()), kernels=launches)
 
 
 def token_shift(out: torch.Tensor, resid: torch.Tensor, shift: Optional[torch.Tensor], state: Optional[torch.Tensor], ctx) -> None:

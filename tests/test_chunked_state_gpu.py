@@ -1,0 +1,117 @@
+"""Long portions of the matrix-state recurrences a chunk of 64 tokens at a time, at the sizes where chunks, blocks of eight tokens and
+tiles of channels end, against the recurrence in float64 on the same rounded inputs - read-outs and, in 32 bits, the state."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from gpu_helpers import DEV
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(DEV == "cpu", reason="the chunks are a form of the CUDA kernels")]
+
+
+def _ctx(lengths, positions=False):
+  dev = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+  starts = [sum(lengths[:i]) for i in range(len(lengths))]
+  return SimpleNamespace(q_start=dev(starts), q_len=dev(lengths), seq_slot=dev([len(lengths) - i for i in range(len(lengths))]),
+                         num_items=len(lengths), num_tokens=sum(lengths), token_item=dev([i for i, n in enumerate(lengths) for _ in range(n)]),
+                         positions=dev([t for n in lengths for t in range(n)]))
+
+
+def _walk(q, k, v, g, beta, S):
+  """q, k, g [T, H, D], v [T, H, Dv], beta [T, H] or None, S [H, D, Dv], all float64 -> read-outs, end state."""
+  out = []
+  for t in range(q.shape[0]):
+    S = g[t][:, :, None] * S
+    u = v[t] if beta is None else beta[t][:, None] * (v[t] - torch.einsum("hd,hdv->hv", k[t], S))
+    S = S + k[t][:, :, None] * u[:, None, :]
+    out.append(torch.einsum("hd,hdv->hv", q[t], S))
+  return torch.stack(out), S
+
+
+def _rms(x, eps):
+  return x / torch.sqrt((x * x).mean(-1, keepdim=True) + eps)
+
+
+# (tokens of every request, heads, query/key heads, key channels, value columns, what the decays are like)
+CASES = [
+  ((112,), 2, 1, 128, 128, "long"), ((128,), 3, 3, 40, 4, "mixed"), ((129, 5, 112), 2, 2, 64, 136, "mixed"), ((200,), 1, 1, 8, 200, "none"),
+  ((319, 192), 2, 1, 100, 64, "all"), ((257,), 4, 2, 32, 32, "mixed"),
+]
+# Two tf32 parts hold 22 bits of an operand and three of four products are taken, so a product errs by up to 3 * 2^-22; the sums of up to 128
+# of them and the triangular system add a few more: 1e-5 of the state's norm leaves a factor of ten.  (The walk in order: about 1e-6.)
+STATE_BOUND = 1e-5
+
+
+def _decays(kind, shape, g):
+  """Logits of a decay's step: everything kept, nothing kept, both within a block of tokens."""
+  z = torch.randn(shape, generator=g)
+  return {"long": z - 6.0, "none": z * 0.0 - 30.0, "all": z * 0.0 + 60.0, "mixed": torch.where(torch.rand(shape, generator=g) < 0.1, z + 25.0, z - 4.0)}[kind]
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_delta_rule_by_chunks(case, per_head):
+  from miniinfer_b200.kernels import ops
+  lengths, H, G, D, Dv, kind = CASES[case]
+  T, eps = sum(lengths), 1e-5
+  r = torch.Generator().manual_seed(100 + case)
+  bf = lambda *s: torch.randn(s, generator=r).to(torch.bfloat16)  # noqa: E731
+  q, k, v, b, gate = bf(T, G * D), bf(T, G * D), bf(T, H * Dv), bf(T, H), bf(T, H * Dv)
+  shape = (T, H) if per_head else (T, H * D)
+  a = _decays(kind, shape, r).to(torch.bfloat16)
+  dt_bias, A_log, norm = 0.1 * torch.randn(shape[1], generator=r), torch.randn(H, generator=r) * 0.3, 1 + 0.1 * torch.randn(Dv, generator=r)
+  start = torch.randn((len(lengths) + 1, H * D * Dv + 4), generator=r)
+  state, out = start.to(DEV), torch.empty((T, H * Dv), dtype=torch.bfloat16, device=DEV)
+  ctx = _ctx(lengths)
+  dev = lambda t: t.to(DEV)  # noqa: E731
+  ops.gated_delta(out, dev(q), dev(k), dev(v), dev(a), dev(b), dev(gate), dev(dt_bias), dev(A_log), dev(norm), eps, state,
+                  ctx, H, G, D, Dv)
+  unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+  step = torch.nn.functional.softplus(a.double() + dt_bias.double()).view(T, H, -1)
+  decay = torch.exp(-torch.exp(A_log.double())[None, :, None] * step).expand(T, H, D)
+  qq = (unit(q.double().view(T, G, D)) * D ** -0.5).repeat_interleave(H // G, 1)
+  kk = unit(k.double().view(T, G, D)).repeat_interleave(H // G, 1)
+  at = 0
+  for i, n in enumerate(lengths):
+    slot, rows = len(lengths) - i, slice(at, at + n)
+    o, S = _walk(qq[rows], kk[rows], v.double().view(T, H, Dv)[rows], decay[rows], torch.sigmoid(b.double())[rows],
+                 start[slot, :H * D * Dv].double().view(H, D, Dv))
+    got = state[slot, :H * D * Dv].double().cpu().view(H, D, Dv)
+    assert (got - S).norm() <= STATE_BOUND * S.norm(), i
+    want = _rms(o, eps) * norm.double() * torch.sigmoid(gate.double().view(T, H, Dv)[rows])
+    # rounded to bfloat16 once: 2^-8 of a value, and what a row's smallest read-outs lose against its root mean square
+    assert (out[rows].double().cpu().view(n, H, Dv) - want).abs().max() <= 2.0 ** -8 * max(1.0, want.abs().max()) + 1e-4
+    at += n
+  assert torch.equal(state[:, H * D * Dv:].cpu(), start[:, H * D * Dv:])
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_linear_attention_by_chunks(case, per_head):
+  from miniinfer_b200.kernels import ops
+  lengths, H, _, D, Dv, kind = CASES[case]
+  T, eps, tau = sum(lengths), 1e-5, 4.0
+  r = torch.Generator().manual_seed(200 + case)
+  bf = lambda *s: torch.randn(s, generator=r).to(torch.bfloat16)  # noqa: E731
+  q, k, v, gate = bf(T, H * D), bf(T, H * D), bf(T, H * Dv), bf(T, H * Dv)
+  logits = -_decays(kind, (T, H * D), r)
+  const = torch.tensor([0.0, 1.0, 0.999, 0.5][:H])
+  start = torch.randn((len(lengths) + 1, H * D * Dv), generator=r)
+  state, out = start.to(DEV), torch.empty((T, H * Dv), dtype=torch.bfloat16, device=DEV)
+  ops.linear_attention(out, q.to(DEV), k.to(DEV), v.to(DEV), gate.to(DEV), state, _ctx(lengths), H, D, Dv, eps,
+                       decay_logits=None if per_head else logits.to(DEV), tau=tau, head_decay=const.to(DEV) if per_head else None, q_scale=D ** -0.5)
+  if per_head:
+    decay = const.double()[None, :, None].expand(T, H, D)
+  else:
+    decay = torch.exp(torch.nn.functional.logsigmoid(logits.double()) / tau).view(T, H, D)
+  at = 0
+  for i, n in enumerate(lengths):
+    slot, rows = len(lengths) - i, slice(at, at + n)
+    o, S = _walk(q.double().view(T, H, D)[rows] * D ** -0.5, k.double().view(T, H, D)[rows], v.double().view(T, H, Dv)[rows], decay[rows], None,
+                 start[slot].double().view(H, D, Dv))
+    assert (state[slot].double().cpu().view(H, D, Dv) - S).norm() <= STATE_BOUND * S.norm(), i
+    gl = gate.double().view(T, H, Dv)[rows]
+    want = _rms(o, eps) * gl * torch.sigmoid(gl)
+    assert (out[rows].double().cpu().view(n, H, Dv) - want).abs().max() <= 2.0 ** -8 * max(1.0, want.abs().max()) + 1e-4
+    at += n
