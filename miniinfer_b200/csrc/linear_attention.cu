@@ -21,6 +21,7 @@
 // Everything between the projections and the gate is float32: angles (a table made on the host), decays and their
 // logarithms, the state and the sums over it, the norm.
 #include "chunked_state.cuh"
+#include "head_rows.cuh"
 
 namespace {
 
@@ -82,6 +83,46 @@ linear_prepare_kernel(LinPrepArgs<T, TA> a) {
     }
     for (int j = lane; j < a.vdim; j += 32)
       a.raw[((size_t)t * a.heads + h) * a.vdim + j] = mi::to_float(a.v[(size_t)t * a.ldv + (size_t)h * a.vdim + j]);
+  }
+}
+
+// The same four values at a time (head_rows.cuh); the two halves of a head's rotated values are a multiple of four apart.
+__global__ void __launch_bounds__(256)
+linear_prepare_rows_kernel(LinPrepArgs<__nv_bfloat16, float> a, int T) {
+  const int lane = threadIdx.x & 31, units = T * a.heads, step = gridDim.x * 8, half = a.rot_dims / 2;
+  mi::grid_dependency_sync();
+#pragma unroll 2
+  for (int u = blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += step) {
+    const int t = u / a.heads, h = u - t * a.heads;
+    const __nv_bfloat16* q = a.q + (size_t)t * a.ldq + (size_t)h * a.dim;
+    const __nv_bfloat16* k = a.k + (size_t)t * a.ldk + (size_t)h * a.dim;
+    const float* cs = a.rope ? a.rope + (size_t)a.positions[t] * a.rot_dims : nullptr;
+    const size_t at = (size_t)u * a.dim;
+    for (int i = 4 * lane; i < a.dim; i += 128) {
+      float4 x = mi::load_row4(q + i), y = mi::load_row4(k + i);
+      if (cs && i < a.rot_dims) {
+        const bool first = i < half;
+        const int pi = first ? i : i - half, partner = first ? i + half : i - half;
+        const float4 c = mi::load_row4(cs + pi), xo = mi::load_row4(q + partner), yo = mi::load_row4(k + partner);
+        float4 s = mi::load_row4(cs + half + pi);
+        if (first) s = mi::scaled4(s, -1.f);
+        x = make_float4(x.x * c.x + xo.x * s.x, x.y * c.y + xo.y * s.y, x.z * c.z + xo.z * s.z, x.w * c.w + xo.w * s.w);
+        y = make_float4(y.x * c.x + yo.x * s.x, y.y * c.y + yo.y * s.y, y.z * c.z + yo.z * s.z, y.w * c.w + yo.w * s.w);
+      }
+      *reinterpret_cast<float4*>(a.qn + at + i) = mi::scaled4(x, a.q_scale);
+      *reinterpret_cast<float4*>(a.kn + at + i) = mi::scaled4(y, a.k_scale);
+      if (a.a) {
+        float4 z = mi::load_row4(a.a + (size_t)t * a.lda + (size_t)h * a.dim + i);
+        if (a.a_bias) {
+          const float4 b = mi::load_row4(a.a_bias + h * a.dim + i);
+          z.x += b.x; z.y += b.y; z.z += b.z; z.w += b.w;
+        }
+        *reinterpret_cast<float4*>(a.g + at + i) = make_float4(expf(lin_log_sigmoid(z.x) * a.inv_tau), expf(lin_log_sigmoid(z.y) * a.inv_tau),
+                                                               expf(lin_log_sigmoid(z.z) * a.inv_tau), expf(lin_log_sigmoid(z.w) * a.inv_tau));
+      }
+    }
+    for (int j = 4 * lane; j < a.vdim; j += 128)
+      *reinterpret_cast<float4*>(a.raw + (size_t)u * a.vdim + j) = mi::load_row4(a.v + (size_t)t * a.ldv + (size_t)h * a.vdim + j);
   }
 }
 
@@ -461,6 +502,11 @@ MI_API int mi_linear_attention(void* out, int ldo, const void* q, int ldq, const
   d.skip_from = chunks ? chunk_min : 0;
   d.seg_state = segments;
   d.seg_decay = segments ? segments + (size_t)items * LIN_SEGMENTS * heads * dim * vdim : nullptr;
+  // rows of many tokens four values at a time (a step of few tokens is as fast either way, and keeps its order of sums)
+  using BF = const __nv_bfloat16;
+  const bool vec = dtype == MI_BF16 && T >= 64 && mi::rows4((BF*)q, dim, ldq) && mi::rows4((BF*)k, dim, ldk) && mi::rows4((BF*)v, vdim, ldv) &&
+                   mi::rows4((BF*)gate, vdim, ldg) && mi::rows4((BF*)out, vdim, ldo) && mi::rows4(norm_w, vdim, vdim) && mi::rows4(a_in, dim, lda) &&
+                   mi::rows4(a_bias, dim, dim) && (rope == nullptr || (rot_dims % 8 == 0 && ((uintptr_t)rope % 16) == 0)) && ((uintptr_t)raw % 16) == 0;
 #define MI_LIN_REC(DKV, CPTV, CH)                                                                                          \
   do {                                                                                                               \
     if (!segments) {                                                                                                 \
@@ -493,7 +539,12 @@ MI_API int mi_linear_attention(void* out, int ldo, const void* q, int ldq, const
     p.a = a_in; p.lda = lda; p.a_bias = a_bias; p.inv_tau = inv_tau; p.rope = rope; p.positions = positions;         \
     p.rot_dims = rot_dims; p.q_scale = q_scale; p.k_scale = k_scale; p.qn = qn; p.kn = kn; p.g = g; p.raw = raw;     \
     p.heads = heads; p.dim = dim; p.vdim = vdim;                                                                     \
-    mi::launch(linear_prepare_kernel<TT, float>, pgrid, dim3(128), 0, stream, p);                                    \
+    if constexpr (sizeof(TT) == 2) {                                                                                 \
+      if (vec) mi::launch(linear_prepare_rows_kernel, mi::head_rows_grid((long long)T * heads), dim3(256), 0, stream, p, T); \
+      else mi::launch(linear_prepare_kernel<TT, float>, pgrid, dim3(128), 0, stream, p);                             \
+    } else {                                                                                                         \
+      mi::launch(linear_prepare_kernel<TT, float>, pgrid, dim3(128), 0, stream, p);                                  \
+    }                                                                                                                \
     if (chunks && items == 1 && T >= chunk_min) ;                                                                    \
     else if (channel) MI_LIN_DK(true);                                                                               \
     else MI_LIN_DK(false);                                                                                           \
@@ -502,7 +553,10 @@ MI_API int mi_linear_attention(void* out, int ldo, const void* q, int ldq, const
                              state_stride, q_start, q_len, seq_slot, items, heads, heads, dim, vdim, chunk_min};      \
       if (int e = mi::chunked_state_run(c, T, chunks, stream)) return e;                                             \
     }                                                                                                                \
-    mi::launch(linear_output_kernel<TT>, ogrid, dim3(128), 0, stream, (TT*)out, ldo, (const float*)raw, (const TT*)gate, ldg, \
+    if (vec)                                                                                                         \
+      mi::launch(mi::head_output_kernel, mi::head_rows_grid((long long)T * heads), dim3(256), 0, stream, (__nv_bfloat16*)out, ldo, (const float*)raw, \
+                 (const __nv_bfloat16*)gate, ldg, norm_w, T, heads, vdim, eps, gate_silu);                            \
+    else mi::launch(linear_output_kernel<TT>, ogrid, dim3(128), 0, stream, (TT*)out, ldo, (const float*)raw, (const TT*)gate, ldg, \
                norm_w, heads, vdim, eps, gate_silu);                                                                 \
   } while (0)
   if (dtype == MI_BF16) MI_LIN_ALL(__nv_bfloat16);

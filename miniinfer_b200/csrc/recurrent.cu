@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "chunked_state.cuh"
+#include "head_rows.cuh"
 
 namespace {
 
@@ -50,6 +51,103 @@ causal_conv_kernel(T* __restrict__ out, int ldo, const T* __restrict__ x, int ld
   }
   if (silu) acc = silu_f(acc);
   out[(size_t)t * ldo + c] = mi::from_float<T>(acc);
+}
+
+// The same for bfloat16 rows that can be read 16 bytes at a time: a thread has eight channels of CONV_TOKENS tokens, so an input is
+// fetched for several taps, and all of the thread's inputs are asked for before any is used (2048 tokens of 2048 channels, four taps:
+// 32 us a value a thread, here 17.8; 8192 channels 122 and 56; the activation's exponential and division are most of that).
+constexpr int CONV_TOKENS = 4;
+
+template <int TAPS>
+__global__ void __launch_bounds__(128)
+causal_conv_vec_kernel(__nv_bfloat16* __restrict__ out, int ldo, const __nv_bfloat16* __restrict__ x, int ldx, const float* __restrict__ w,
+                       const float* __restrict__ bias, const float* __restrict__ in_bias, const float* __restrict__ state, long long state_stride,
+                       const int* __restrict__ token_item, const int* __restrict__ q_start, const int* __restrict__ seq_slot,
+                       int T, int C, int silu) {
+  const int c = 8 * (blockIdx.x * blockDim.x + threadIdx.x), t0 = blockIdx.y * CONV_TOKENS;
+  if (c >= C) {
+    mi::grid_dependency_sync();
+    return;
+  }
+  int items[CONV_TOKENS];
+#pragma unroll
+  for (int n = 0; n < CONV_TOKENS; ++n) items[n] = t0 + n < T ? token_item[t0 + n] : -1;
+  float wt[8 * TAPS], b[8], ib[8];      // the weights of a channel lie side by side
+#pragma unroll
+  for (int i = 0; i < 8 * TAPS; i += 2) {
+    const float2 p = *reinterpret_cast<const float2*>(w + (size_t)c * TAPS + i);
+    wt[i] = p.x;
+    wt[i + 1] = p.y;
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    b[i] = bias ? bias[c + i] : 0.f;
+    ib[i] = in_bias ? in_bias[c + i] : 0.f;
+  }
+  int item = items[0], j = t0 - q_start[item];
+  mi::grid_dependency_sync();
+  uint4 raw[CONV_TOKENS + TAPS - 1];      // rows t0 - (TAPS - 1) ..: those before the item's first row are not its inputs, and replaced
+#pragma unroll
+  for (int n = 0; n < CONV_TOKENS + TAPS - 1; ++n) {
+    const int row = min(max(t0 + n - (TAPS - 1), 0), T - 1);
+    raw[n] = *reinterpret_cast<const uint4*>(x + (size_t)row * ldx + c);
+  }
+  float in[TAPS][8];      // in[k]: the input k tokens back
+  auto take = [&](float (&to)[8], uint4 from) {
+    const uint32_t part[4] = {from.x, from.y, from.z, from.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&part[i]));
+      to[2 * i] = f.x + ib[2 * i];
+      to[2 * i + 1] = f.y + ib[2 * i + 1];
+    }
+  };
+  auto kept = [&]() {      // the inputs before the item's new tokens, as far as they reach
+    const float* st = state + (size_t)seq_slot[item] * state_stride + c;
+#pragma unroll
+    for (int k = 1; k < TAPS; ++k)
+      if (j < k) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) in[k - 1][i] = st[(size_t)(TAPS - 1 + j - k) * C + i];
+      }
+  };
+#pragma unroll
+  for (int k = 1; k < TAPS; ++k) take(in[k - 1], raw[TAPS - 1 - k]);
+  if (j < TAPS - 1) kept();
+#pragma unroll
+  for (int n = 0; n < CONV_TOKENS; ++n) {
+    const int t = t0 + n;
+    if (t >= T) return;
+    if (n > 0) {
+      ++j;
+      if (items[n] != item) {
+        item = items[n];
+        j = 0;
+        kept();
+      }
+    }
+#pragma unroll
+    for (int k = TAPS - 1; k > 0; --k)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) in[k][i] = in[k - 1][i];
+    take(in[0], raw[n + TAPS - 1]);
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float y[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int ch = 2 * i + e;
+        float acc = b[ch];
+#pragma unroll
+        for (int k = TAPS - 1; k >= 0; --k) acc = fmaf(wt[ch * TAPS + TAPS - 1 - k], in[k][ch], acc);      // oldest input first
+        y[e] = silu ? silu_f(acc) : acc;
+      }
+      const __nv_bfloat162 p = __floats2bfloat162_rn(y[0], y[1]);
+      o[i] = *reinterpret_cast<const uint32_t*>(&p);
+    }
+    *reinterpret_cast<uint4*>(out + (size_t)t * ldo + c) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
 }
 
 // After the convolution has run: the state becomes the last taps - 1 inputs of the request.  A thread per (item, channel).
@@ -360,6 +458,57 @@ delta_prepare_kernel(DeltaPrepArgs<T> a) {
   }
 }
 
+// The same four values at a time (head_rows.cuh).
+__global__ void __launch_bounds__(256)
+delta_prepare_rows_kernel(DeltaPrepArgs<__nv_bfloat16> a) {
+  mi::grid_dependency_sync();
+  const int lane = threadIdx.x & 31, per_token = a.kv_heads + a.heads, units = a.T_ * per_token, step = gridDim.x * 8;
+  for (int n = blockIdx.x * 8 + (threadIdx.x >> 5); n < units; n += step) {
+    const int t = n / per_token, u = n - t * per_token;
+    if (u < a.kv_heads) {
+      const __nv_bfloat16* q = a.q + (size_t)t * a.ldqk + (size_t)u * a.dim;
+      const __nv_bfloat16* k = a.k + (size_t)t * a.ldqk + (size_t)u * a.dim;
+      float sq = 0.f, sk = 0.f;
+      for (int i = 4 * lane; i < a.dim; i += 128) {
+        const float4 x = mi::load_row4(q + i), y = mi::load_row4(k + i);
+        sq = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, sq))));
+        sk = fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, fmaf(y.w, y.w, sk))));
+      }
+      sq = mi::warp_sum(sq);
+      sk = mi::warp_sum(sk);
+      const float fq = rsqrtf((float)a.dim) / sqrtf(sq + 1e-6f), fk = 1.f / sqrtf(sk + 1e-6f);
+      const size_t at = ((size_t)t * a.kv_heads + u) * a.dim;
+      float qk = 0.f;
+      for (int i = 4 * lane; i < a.dim; i += 128) {
+        const float4 x = mi::scaled4(mi::load_row4(q + i), fq), y = mi::scaled4(mi::load_row4(k + i), fk);
+        *reinterpret_cast<float4*>(a.qn + at + i) = x;
+        *reinterpret_cast<float4*>(a.kn + at + i) = y;
+        qk = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, qk))));
+      }
+      if (a.head_decay) {
+        qk = mi::warp_sum(qk);
+        if (lane == 0) a.qk[(size_t)t * a.kv_heads + u] = qk;
+      }
+    } else {
+      const int h = u - a.kv_heads;
+      const float neg_rate = -expf(a.A_log[h]);
+      if (a.head_decay) {
+        if (lane == 0) a.g[(size_t)t * a.heads + h] = expf(neg_rate * softplus_f(mi::to_float(a.a[(size_t)t * a.lda + h]) + a.dt_bias[h]));
+      } else {
+        for (int i = 4 * lane; i < a.dim; i += 128) {
+          const float4 z = mi::load_row4(a.a + (size_t)t * a.lda + (size_t)h * a.dim + i), b = mi::load_row4(a.dt_bias + h * a.dim + i);
+          *reinterpret_cast<float4*>(a.g + ((size_t)t * a.heads + h) * a.dim + i) =
+            make_float4(expf(neg_rate * softplus_f(z.x + b.x)), expf(neg_rate * softplus_f(z.y + b.y)),
+                        expf(neg_rate * softplus_f(z.z + b.z)), expf(neg_rate * softplus_f(z.w + b.w)));
+        }
+      }
+      if (lane == 0) a.beta[(size_t)t * a.heads + h] = sigmoid_f(mi::to_float(a.b[(size_t)t * a.ldb + h]));
+      for (int j = 4 * lane; j < a.vdim; j += 128)
+        *reinterpret_cast<float4*>(a.raw + ((size_t)t * a.heads + h) * a.vdim + j) = mi::load_row4(a.v + (size_t)t * a.ldv + (size_t)h * a.vdim + j);
+    }
+  }
+}
+
 // 4 bytes from global to shared memory without a register in between; zeros if not `take`
 __device__ __forceinline__ void copy4(float* dst, const float* src, bool take) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -652,7 +801,17 @@ MI_API int mi_causal_conv(void* out, int ldo, const void* x, int ldx, int dtype,
   MI_REQUIRE(state_stride >= (long long)(taps - 1) * C, "causal_conv: the state rows are too short");
   if (T == 0) return 0;
   dim3 grid((C + 255) / 256, T), sgrid((C + 255) / 256, items);
-  if (dtype == MI_BF16) {
+  // eight channels and four tokens a thread where rows start on 16-byte boundaries and there are a million values: 70 tokens of 2048
+  // channels take 3 us a value a thread and 6 this way (a thread's weights alone are 128 bytes)
+  const bool vec = dtype == MI_BF16 && (long long)T * C >= 1 << 20 && taps >= 2 && taps <= 4 && C % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 &&
+                   ((uintptr_t)x % 16) == 0 && ((uintptr_t)out % 16) == 0 && ((uintptr_t)w % 8) == 0;
+  if (vec) {
+    auto kernel = taps == 2 ? causal_conv_vec_kernel<2> : taps == 3 ? causal_conv_vec_kernel<3> : causal_conv_vec_kernel<4>;
+    mi::launch(kernel, dim3((C / 8 + 127) / 128, (T + CONV_TOKENS - 1) / CONV_TOKENS), dim3(128), 0, stream, (__nv_bfloat16*)out, ldo,
+               (const __nv_bfloat16*)x, ldx, w, bias, in_bias, (const float*)state, state_stride, token_item, q_start, seq_slot, T, C, silu);
+    mi::launch(conv_state_kernel<__nv_bfloat16>, sgrid, dim3(256), 0, stream, state, state_stride, (const __nv_bfloat16*)x, ldx, in_bias,
+               q_start, q_len, seq_slot, C, taps);
+  } else if (dtype == MI_BF16) {
     mi::launch(causal_conv_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)x, ldx, w, bias, in_bias,
                (const float*)state, state_stride, token_item, q_start, seq_slot, C, taps, silu);
     if (taps > 1) mi::launch(conv_state_kernel<__nv_bfloat16>, sgrid, dim3(256), 0, stream, state, state_stride, (const __nv_bfloat16*)x, ldx, in_bias,
@@ -779,6 +938,11 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
   dim3 pgrid(T, (heads + kv_heads + 3) / 4 > 16 ? 16 : (heads + kv_heads + 3) / 4);
   dim3 ogrid(T, (heads + 3) / 4 > 16 ? 16 : (heads + 3) / 4);
   dim3 rgrid(heads, items, (vdim + cols - 1) / cols);
+  // rows of many tokens four values at a time (a step of few tokens is as fast either way, and keeps its order of sums)
+  using BF = const __nv_bfloat16;
+  const bool vec = dtype == MI_BF16 && T >= 64 && mi::rows4((BF*)q, dim, ldqk) && mi::rows4((BF*)k, dim, ldqk) && mi::rows4((BF*)v, vdim, ldv) &&
+                   (head_decay || (mi::rows4((BF*)a_in, dim, lda) && mi::rows4(dt_bias, dim, dim))) && mi::rows4((BF*)gate, vdim, ldg) &&
+                   mi::rows4((BF*)out, vdim, ldo) && mi::rows4(norm_w, vdim, vdim);
 #define MI_DELTA(TT, DKV)                                                                                         \
   do { if (head_decay) MI_DELTA_FORM(TT, DKV, true); else MI_DELTA_FORM(TT, DKV, false); } while (0)
 #define MI_DELTA_FORM(TT, DKV, HD)                                                                                \
@@ -816,7 +980,12 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
     p.dt_bias = dt_bias; p.A_log = A_log; p.qn = qn; p.kn = kn; p.g = g; p.beta = beta; p.T_ = T; p.heads = heads;  \
     p.qk = qk; p.head_decay = head_decay;                                                                         \
     p.kv_heads = kv_heads; p.dim = dim; p.v = (const TT*)v; p.ldv = ldv; p.raw = raw; p.vdim = vdim;                  \
-    mi::launch(delta_prepare_kernel<TT>, pgrid, dim3(128), 0, stream, p);                                         \
+    if constexpr (sizeof(TT) == 2) {                                                                              \
+      if (vec) mi::launch(delta_prepare_rows_kernel, mi::head_rows_grid((long long)T * (heads + kv_heads)), dim3(256), 0, stream, p); \
+      else mi::launch(delta_prepare_kernel<TT>, pgrid, dim3(128), 0, stream, p);                                  \
+    } else {                                                                                                      \
+      mi::launch(delta_prepare_kernel<TT>, pgrid, dim3(128), 0, stream, p);                                       \
+    }                                                                                                             \
     if (DK == 16) MI_DELTA(TT, 16);                                                                               \
     else if (DK == 32) MI_DELTA(TT, 32);                                                                          \
     else if (DK == 64) MI_DELTA(TT, 64);                                                                          \
@@ -826,7 +995,11 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
                              seq_slot, items, heads, kv_heads, dim, vdim, chunk_min};                              \
       if (int e = mi::chunked_state_run(c, T, chunks, stream)) return e;                                            \
     }                                                                                                             \
-    mi::launch(delta_output_kernel<TT>, ogrid, dim3(128), 0, stream, (TT*)out, ldo, (const float*)raw, (const TT*)gate, ldg, norm_w, heads, vdim, eps, gate_silu); \
+    if (vec)                                                                                                      \
+      mi::launch(mi::head_output_kernel, mi::head_rows_grid((long long)T * heads), dim3(256), 0, stream, (__nv_bfloat16*)out, ldo, (const float*)raw, \
+                 (const __nv_bfloat16*)gate, ldg, norm_w, T, heads, vdim, eps, gate_silu);                         \
+    else                                                                                                          \
+      mi::launch(delta_output_kernel<TT>, ogrid, dim3(128), 0, stream, (TT*)out, ldo, (const float*)raw, (const TT*)gate, ldg, norm_w, heads, vdim, eps, gate_silu); \
   } while (0)
   if (dtype == MI_BF16) MI_DELTA_ALL(__nv_bfloat16);
   else if (dtype == MI_F32) MI_DELTA_ALL(float);

@@ -115,3 +115,25 @@ def test_linear_attention_by_chunks(case, per_head):
     want = _rms(o, eps) * gl * torch.sigmoid(gl)
     assert (out[rows].double().cpu().view(n, H, Dv) - want).abs().max() <= 2.0 ** -8 * max(1.0, want.abs().max()) + 1e-4
     at += n
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("lengths,C,lead", [((1025,), 1024, 0), ((1, 2, 700, 3, 1), 1496, 8), ((9, 1018), 1032, 16)])      # items end inside the four tokens of a thread
+def test_causal_convolution_eight_channels_a_thread(taps, lengths, C, lead):
+  from miniinfer_b200.kernels import ops
+  T = sum(lengths)
+  r = torch.Generator().manual_seed(taps * T + C)
+  rows = torch.randn((T, lead + C + 8), generator=r).to(torch.bfloat16)
+  w, bias, in_bias = torch.randn((C, taps), generator=r), torch.randn(C, generator=r), torch.randn(C, generator=r)
+  start = torch.randn((len(lengths) + 1, (taps - 1) * C + 4), generator=r)
+  state, out = start.to(DEV), torch.empty((T, C), dtype=torch.bfloat16, device=DEV)
+  ops.causal_conv(out, rows.to(DEV)[:, lead:lead + C], w.to(DEV), bias.to(DEV), state, _ctx(lengths), silu=True, in_bias=in_bias.to(DEV))
+  at = 0
+  for i, n in enumerate(lengths):
+    slot = len(lengths) - i
+    u = torch.cat([start[slot, :(taps - 1) * C].double().view(taps - 1, C), rows[at:at + n, lead:lead + C].double() + in_bias.double()])
+    want = torch.nn.functional.silu(sum(u[k:k + n] * w[:, k].double() for k in range(taps)) + bias.double())
+    got = out[at:at + n].double().cpu()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all(), i      # one rounding to bfloat16; sums of a few float32 products
+    assert torch.allclose(state[slot, :(taps - 1) * C].double().cpu().view(taps - 1, C), u[n:], atol=1e-6)
+    at += n
