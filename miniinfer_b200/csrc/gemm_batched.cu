@@ -11,7 +11,7 @@
 // logit per output value instead, at value_gate[m * gate_stride + b * N + n].
 //
 // This is the product of the 32-bit path for strided operands, of per-head up- and down-projections of a latent
-// attention, and the fallback of the bfloat16 path for inner sizes that are no multiple of 8.  Tiles of 64 x 64
+// attention, and the fallback of the bfloat16 path for inner sizes that are no multiple of 8.  The general kernel: tiles of 64 x 64
 // through shared memory, 16 values of k at a time, 4 x 4 outputs a thread.
 #include "common.cuh"
 
@@ -172,6 +172,101 @@ gemm_batched_mma_few_rows_kernel(BatchedArgs a) {
   }
 }
 
+// Many rows in bfloat16 on the tensor cores (mma.sync), for operands whose rows can be fetched 16 bytes at a time: tiles of 64 x 64, a
+// warp 32 x 32, K in stages of 64 by cp.async.  These products are small and read their rows once - 2048 rows of 16 heads,
+// 64 x 192 each, move 17 MB - so the memory bounds them, where the FMA kernel above was bound by its arithmetic (50.6 us,
+// 13.8 here); a tcgen05 tile of 128 rows would wait for the same bytes.
+constexpr int TK = 64, LDS = TK + 8, TSTAGES = 3;
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+template <typename TO>
+__global__ void __launch_bounds__(128)
+gemm_batched_mma_kernel(BatchedArgs a) {
+  extern __shared__ __align__(16) __nv_bfloat16 tiles[];      // [TSTAGES][x rows, w rows][64][LDS]
+  const int b = blockIdx.z, m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
+  const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + (size_t)b * a.x_batch;
+  const __nv_bfloat16* w = (const __nv_bfloat16*)a.w + (size_t)b * a.w_batch;
+  const int steps = (a.K + TK - 1) / TK;
+  auto stage = [&](int s, bool weights) {
+    if (s < steps) {
+      __nv_bfloat16* dst = tiles + ((s % TSTAGES) * 2 + (weights ? 1 : 0)) * 64 * LDS;
+#pragma unroll
+      for (int i = threadIdx.x; i < 64 * TK / 8; i += 128) {
+        const int r = i / (TK / 8), k = s * TK + i % (TK / 8) * 8, row = (weights ? n0 : m0) + r;
+        const bool in = row < (weights ? a.N : a.M) && k < a.K;
+        const __nv_bfloat16* src = weights ? w + (in ? (size_t)row * a.ldw + k : 0) : x + (in ? (size_t)row * a.lda + k : 0);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * LDS + i % (TK / 8) * 8)),
+                     "l"(src), "r"(in ? 16 : 0) : "memory");
+      }
+    }
+    if (!weights) asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int s = 0; s < TSTAGES - 1; ++s) stage(s, true);      // the weights are written by no kernel: fetched before the wait
+  mi::grid_dependency_sync();
+  for (int s = 0; s < TSTAGES - 1; ++s) stage(s, false);
+  float c[2][4][4] = {};
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(TSTAGES - 2) : "memory");
+    __syncthreads();
+    stage(s + TSTAGES - 1, true);
+    stage(s + TSTAGES - 1, false);
+    const __nv_bfloat16 *xs = tiles + (s % TSTAGES) * 2 * 64 * LDS, *ws = xs + 64 * LDS;
+#pragma unroll
+    for (int k = 0; k < TK; k += 16) {
+      uint32_t xa[2][4], wb[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ldmatrix4(xa[i], xs + (wm + 16 * i + (lane & 15)) * LDS + k + (lane >> 4) * 8);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) ldmatrix4(wb[j], ws + (wn + 16 * j + (lane & 7) + (lane >> 4) * 8) * LDS + k + ((lane >> 3) & 1) * 8);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                       : "+f"(c[i][j][0]), "+f"(c[i][j][1]), "+f"(c[i][j][2]), "+f"(c[i][j][3])
+                       : "r"(xa[i][0]), "r"(xa[i][1]), "r"(xa[i][2]), "r"(xa[i][3]), "r"(wb[j >> 1][(j & 1) * 2]), "r"(wb[j >> 1][(j & 1) * 2 + 1]));
+    }
+  }
+  TO* out = (TO*)a.out + (size_t)b * a.o_batch;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = m0 + wm + 16 * i + (lane >> 2) + 8 * h;
+      if (m >= a.M) continue;
+      float gate = 1.f;
+      if (a.row_gate) gate = 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.row_gate)[(size_t)m * a.gate_stride + b])));
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int n = n0 + wn + 8 * j + (lane & 3) * 2;
+        float y[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          y[e] = c[i][j][2 * h + e];
+          if (n + e >= a.N) continue;
+          if (a.bias) y[e] += a.bias[n + e];
+          if (a.act == 1) y[e] = y[e] > 20.f ? y[e] : log1pf(expf(y[e]));
+          if (a.value_gate)
+            y[e] *= 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.value_gate)[(size_t)m * a.gate_stride + (size_t)b * a.N + n + e])));
+          y[e] *= gate;
+        }
+        TO* o = out + (size_t)m * a.ldo + n;
+        if (n + 1 < a.N && ((uintptr_t)o % (2 * sizeof(TO))) == 0) {
+          if constexpr (sizeof(TO) == 2) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(y[0], y[1]);
+          else *reinterpret_cast<float2*>(o) = make_float2(y[0], y[1]);
+        } else {
+          if (n < a.N) o[0] = mi::from_float<TO>(y[0]);
+          if (n + 1 < a.N) o[1] = mi::from_float<TO>(y[1]);
+        }
+      }
+    }
+}
+
 }  // namespace
 
 MI_API int mi_gemm_batched_few_rows(void* out, int out_dtype, const void* x, const void* w, int dtype, int batch, int M, int N, int K,
@@ -214,6 +309,18 @@ MI_API int mi_gemm_batched(void* out, int out_dtype, const void* x, const void* 
   a.row_gate = row_gate; a.gate_stride = gate_stride; a.value_gate = value_gate;
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
   MI_REQUIRE(grid.y <= 65535, "gemm_batched: M=%d is too large for one launch", M);
+  // rows that start on 16-byte boundaries and hold whole 16 bytes; the others keep the FMA kernel
+  const bool whole = dtype == MI_BF16 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && x_batch % 8 == 0 && w_batch % 8 == 0 &&
+                     ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0;
+  if (whole && (out_dtype == MI_BF16 || out_dtype == MI_F32)) {
+    constexpr size_t smem = (size_t)TSTAGES * 2 * 64 * LDS * sizeof(__nv_bfloat16);
+    auto kernel = out_dtype == MI_BF16 ? gemm_batched_mma_kernel<__nv_bfloat16> : gemm_batched_mma_kernel<float>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return mi_fail("gemm_batched: %zu bytes of shared memory were refused", smem);
+    mi::launch(kernel, grid, dim3(128), smem, stream, a);
+    MI_LAUNCH_OK("gemm_batched");
+    return 0;
+  }
   if (dtype == MI_F32 && out_dtype == MI_F32) mi::launch(gemm_batched_kernel<float, float>, grid, dim3(256), 0, stream, a);
   else if (dtype == MI_BF16 && out_dtype == MI_BF16) mi::launch(gemm_batched_kernel<__nv_bfloat16, __nv_bfloat16>, grid, dim3(256), 0, stream, a);
   else if (dtype == MI_BF16 && out_dtype == MI_F32) mi::launch(gemm_batched_kernel<__nv_bfloat16, float>, grid, dim3(256), 0, stream, a);

@@ -1322,6 +1322,12 @@ class AttentionBatch:
     for k in self.__slots__:
       setattr(self, k, kw.get(k))
 
+  def decode_only(self) -> "AttentionBatch":
+    """The same step without its prompt portions, for a launcher that has dealt with those."""
+    rest = AttentionBatch(**{k: getattr(self, k) for k in self.__slots__})
+    rest.num_prefill_tiles = 0
+    return rest
+
 
 def attention(out: torch.Tensor, qkv: torch.Tensor, kv_layer: torch.Tensor, block_table: torch.Tensor,
               batch: AttentionBatch, num_heads: int, num_kv_heads: int, head_dim: int, scale: float,
@@ -1393,6 +1399,36 @@ def attention(out: torch.Tensor, qkv: torch.Tensor, kv_layer: torch.Tensor, bloc
     _ptr(batch.seq_slot, torch.int32), T, num_heads, num_kv_heads, head_dim, page_size,
     ctypes.c_float(scale), win, opts.sink_ptr(), opts.gate_ptr(), gate_stride, ohd, opts.keep_first, ctypes.c_float(opts.softcap),
     opts.score_bias_ptr(), int(opts.gate_per_head), opts.distance_ptr(), _stream()))
+
+
+def latent_attention(out: torch.Tensor, q: torch.Tensor, kv_layer: torch.Tensor, block_table: torch.Tensor, batch: AttentionBatch,
+                     num_heads: int, head_dim: int, scale: float, window: Optional[int], sink: Optional[torch.Tensor], out_hd: int) -> None:
+  """``attention`` of ``num_heads`` query heads over one key/value head whose cached value rows are the first ``out_hd`` values of
+  its key rows (attention through a latent, as ``latent_down`` stores it): what knows that reads a row once.  ``q
+  [tokens, num_heads * head_dim]``, ``out [tokens, num_heads * out_hd]``."""
+  page_size = kv_layer.shape[3]
+  if (q.is_cuda and q.dtype == torch.bfloat16 and batch.num_prefill_tiles and batch.prefill_tiles is not None and q.shape[1] == num_heads * head_dim
+      and head_dim % 16 == 0 and 64 <= head_dim <= 256 and out_hd % 8 == 0 and page_size % 64 == 0 and q.is_contiguous() and q.data_ptr() % 16 == 0
+      and out.data_ptr() % 16 == 0 and kv_layer.data_ptr() % 16 == 0 and os.environ.get("MINIINFER_B200_PREFILL_TC", "1") != "0"):
+    if (out.shape != (q.shape[0], num_heads * out_hd) or out.dtype != q.dtype or kv_layer.dtype != q.dtype or not 0 < out_hd <= head_dim
+        or kv_layer.shape[1:] != (2, 1, page_size, head_dim)):
+      raise KernelError("latent_attention: shapes or dtypes do not match")
+    lib = common_lib()
+    if batch.scratch is not None:
+      status = batch.scratch.zeros("attention_prefill_status", 1, torch.int32)
+    else:
+      status = torch.zeros(1, dtype=torch.int32, device=q.device)
+    _check(lib, lib.mi_attention_prefill_latent(
+      _ptr(out), _rows_tensor_map(lib, q, head_dim), _rows_tensor_map(lib, kv_layer, head_dim), _ptr(block_table, torch.int32), block_table.shape[1],
+      _ptr(batch.prefill_tiles, torch.int32), batch.num_prefill_tiles, _ptr(batch.q_start, torch.int32), _ptr(batch.q_len, torch.int32),
+      _ptr(batch.ctx_len, torch.int32), _ptr(batch.seq_slot, torch.int32), _ptr(status, torch.int32), num_heads, head_dim, out_hd, page_size,
+      ctypes.c_float(scale), int(window) if window else 0, _ptr(sink, torch.float32) if sink is not None else _ptr(None), _stream()))
+    if batch.scratch is None and int(status[0]) != 0:
+      raise KernelError("attention_prefill_latent: a bounded wait on a barrier ran out")
+    if not batch.num_decode:
+      return
+    batch = batch.decode_only()
+  attention(out, q, kv_layer, block_table, batch, num_heads, 1, head_dim, scale, window, sink=sink, out_hd=out_hd)
 
 
 class _AttentionOptions:
@@ -1665,6 +1701,21 @@ def _qkv_tensor_map(lib, qkv: torch.Tensor):
       _tensor_maps.clear()
     m = ctypes.create_string_buffer(128)
     code = lib.mi_qkv_tensor_map(m, _ptr(qkv), ctypes.c_longlong(qkv.shape[0]), ctypes.c_longlong(qkv.shape[1]))
+    if code != 0:
+      raise KernelError(lib.mi_last_error().decode())
+    _tensor_maps[key] = m
+  return m
+
+
+def _rows_tensor_map(lib, t: torch.Tensor, width: int):
+  """The TMA descriptor of a contiguous tensor as rows of ``width`` values (kept per address and shape)."""
+  key = ("rows", t.data_ptr(), t.numel(), width)
+  m = _tensor_maps.get(key)
+  if m is None:
+    if len(_tensor_maps) > 4096:
+      _tensor_maps.clear()
+    m = ctypes.create_string_buffer(128)
+    code = lib.mi_rows_tensor_map(m, _ptr(t), ctypes.c_longlong(t.numel() // width), ctypes.c_longlong(width))
     if code != 0:
       raise KernelError(lib.mi_last_error().decode())
     _tensor_maps[key] = m

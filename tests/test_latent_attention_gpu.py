@@ -1,0 +1,59 @@
+"""Attention over one shared key/value head whose values are the first columns of its keys, against the generic kernel on the same
+cache: works of 128 rows that end inside a token's heads, tiles of 128 keys just full and one key over, windows, sinks."""
+import pytest
+import torch
+
+from gpu_helpers import DEV, make_attention_case
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(DEV == "cpu", reason="the kernels against one another")]
+
+
+# (items (context, new), heads, key size, value size, page size, window, sink)
+CASES = [
+  ([(128, 128), (129, 2), (300, 300)], 16, 224, 192, 64, None, True),
+  ([(700, 65), (64, 64), (513, 1)], 32, 256, 192, 64, None, False),
+  ([(1000, 257), (90, 90)], 5, 64, 64, 128, 100, True),
+  ([(640, 33), (1500, 9), (40, 1)], 12, 112, 104, 64, 128, False),
+  ([(2, 2), (700, 640)], 1, 256, 256, 64, 333, True),
+  ([(260, 200)], 40, 176, 128, 192, None, True),
+]
+
+
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_latent_attention(case):
+  from miniinfer_b200.kernels import ops
+  items, nh, hd, ohd, P, window, with_sink = CASES[case]
+  qkv, kv, bt, batch = make_attention_case(items, nh, 1, hd, P, torch.bfloat16, seed=case, scale_q=2.0)
+  q = qkv[:, :nh * hd].contiguous()
+  kv[:, 1, :, :, :ohd] = kv[:, 0, :, :, :ohd]
+  sink = torch.randn(nh, generator=torch.Generator().manual_seed(case)).to(DEV) if with_sink else None
+  T = q.shape[0]
+  got = torch.full((T, nh * ohd), float("nan"), dtype=torch.bfloat16, device=DEV)
+  want = torch.empty_like(got)
+  ops.latent_attention(got, q, kv, bt, batch, nh, hd, hd ** -0.5, window, sink, ohd)
+  ops.attention(want, q, kv, bt, batch, nh, 1, hd, hd ** -0.5, window, force_generic=True, sink=sink, out_hd=ohd)
+  # weights rounded to bfloat16 (2^-9 of each, of values of unit size) and one rounding of the result, as test_attention_over_pages allows
+  assert (got.float() - want.float()).abs().max() < 2e-2
+
+
+@pytest.mark.parametrize("M,N,K,B", [(17, 1, 8, 3), (64, 64, 192, 2), (65, 70, 200, 5), (300, 128, 64, 1)])      # edges of the 64 x 64 tiles and of K's stages
+@pytest.mark.parametrize("gate", ["row", "value", "bias"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_per_head_products_of_many_rows(M, N, K, B, gate, dtype):
+  from miniinfer_b200.kernels import ops
+  g = torch.Generator().manual_seed(M + N + K)
+  r = lambda *s: torch.randn(s, generator=g).to(torch.bfloat16)  # noqa: E731
+  x, w, logits, bias = r(M, B, K), r(B, N, K), r(M, B * N), torch.randn(N, generator=g)
+  out = torch.empty((M, B, N), dtype=dtype, device=DEV)
+  ops.linear_batched(out, x.to(DEV), w.to(DEV), bias=bias.to(DEV) if gate == "bias" else None, softplus=gate == "bias",
+                     row_gate=logits.to(DEV) if gate == "row" else None, value_gate=logits.to(DEV) if gate == "value" else None)
+  z = torch.einsum("mbk,bnk->mbn", x.double(), w.double())
+  size = torch.einsum("mbk,bnk->mbn", x.double().abs(), w.double().abs())
+  if gate == "bias":
+    want = torch.nn.functional.softplus(z + bias.double())
+  else:
+    want = z * torch.sigmoid(logits.double()[:, :B].unsqueeze(2) if gate == "row" else logits.double().view(M, B, N))
+  # products are exact in float32; K additions of truncated float32 and, in bfloat16, one rounding of the result - two where the library's
+  # product is gated by a pass of its own
+  bound = K * 2.0 ** -23 * size + (2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -20) * want.abs() + 1e-6
+  assert ((out.double().cpu() - want).abs() <= bound).all()
