@@ -1,4 +1,4 @@
-// Prefill attention of many query heads over ONE shared key/value head whose values are the first columns of its keys - attention
+// Attention of many query heads over ONE shared key/value head whose values are the first columns of its keys - attention
 // through a latent - in bf16 on the fifth-generation tensor cores (tcgen05), for key rows of 64 to 256 values.
 //
 // The query rows of the step lie behind one another, [token, head], so a piece of work is any 128 of them that belong to one
@@ -19,6 +19,13 @@
 // of 128 x 64 x 16 takes 81 cycles where one of 128 x 128 x 16 takes 95.  Neither the exponentials nor the copies from L2 matter (left
 // out in turn: no change).  Measured on B200, 2048 tokens, latent 192 + 32: 16 heads 51 us, 232 by the mma.sync kernel; 1000 tokens
 // of 32 heads of 192 + 64 with a window of 1024 33 us, 149 by that
+//
+// Decode tokens run through the same tiles: a work is one request's up to 128 heads and a piece of its keys, counted from key 0, and
+// leaves sums that are not normalised for latent_merge_kernel.  Most of the 128 rows are padding, which costs nothing: a piece is bound
+// by the latency of its one or two tiles and by bytes, and every key row is fetched once for all heads, as key and as value
+// at once.  Measured on B200, 8 tokens of 32 heads of 192 + 64 over 2048 keys each: the layer around them 87.7 us with the
+// mma.sync kernel of attention_decode.cu (16 heads a pass, keys and values fetched apart: 40.6 us, its merge 6.3), 55.9 so.
+//
 // (the mma.sync kernel of attention_prefill.cu takes the other forms: keys and values of their own, pages that are no multiple
 // of 64, sizes of other alignment).
 #include <cuda.h>
@@ -47,6 +54,10 @@ struct Args {
   int boxes, steps, n_out, out_hd;      // boxes and 16s of columns of a row, columns of P V (whole boxes), of which out_hd are stored
   float scale_log2;              // scale * log2(e)
   const float* sink;             // [nh] or null
+  // decode tokens: a piece of chunk keys (counted from key 0) of one request and up to 128 of its heads is a work
+  const int* decode_items;       // [n_dec]: item of each decode entry
+  float *part_o, *part_ml;       // [n_dec, max_splits, nh, out_hd] not normalised; [n_dec, max_splits, nh, 2]: base-2 maximum, sum
+  int n_dec, chunk, max_splits;
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -143,6 +154,7 @@ struct Work {
   int rows;                      // of the 128 that exist; 0: none
   int row0, first;               // first row in the step's [token, head] rows; the same counted from the item's first new token's
   int start, p_first, p_last, lo_last, t_begin, n;
+  int slot;                      // decode: entry and piece, entry * max_splits + piece
   const int* bt;
 };
 
@@ -161,6 +173,24 @@ __device__ __forceinline__ Work work_of(const Args& a, int w, int per_tile) {
   k.lo_last = mi::first_visible(k.p_last, a.window);
   k.t_begin = mi::first_visible(k.p_first, a.window) / BN;
   k.n = k.p_last / BN - k.t_begin + 1;
+  k.slot = 0;
+  k.bt = a.block_table + (size_t)a.seq_slot[item] * a.bt_stride;
+  return k;
+}
+// Of decode tokens: the first piece of every request, then the second, ...
+__device__ __forceinline__ Work decode_work_of(const Args& a, int w, int parts) {
+  Work k;
+  const int part = w % parts, entry = w / parts % a.n_dec, split = w / parts / a.n_dec;
+  const int item = a.decode_items[entry];
+  const int p = a.ctx_len[item] - 1, lo = mi::first_visible(p, a.window), piece = lo / a.chunk + split;
+  k.rows = p >= 0 && piece * a.chunk <= p ? min(BM, a.nh - part * BM) : 0;
+  k.first = part * BM;
+  k.row0 = a.q_start[item] * a.nh + k.first;
+  k.start = k.p_first = k.p_last = p;
+  k.lo_last = lo;
+  k.t_begin = max(lo, piece * a.chunk) / BN;
+  k.n = min(p, (piece + 1) * a.chunk - 1) / BN - k.t_begin + 1;
+  k.slot = entry * a.max_splits + split;
   k.bt = a.block_table + (size_t)a.seq_slot[item] * a.bt_stride;
   return k;
 }
@@ -171,9 +201,11 @@ __device__ __forceinline__ int nth_work(int i, int b, int blocks, int total) {
   return w < total ? w : -1;
 }
 
+template <bool DECODE>
 __global__ void __launch_bounds__(THREADS, 1)
-attention_prefill_latent_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, Args a) {
-  const int per_tile = (64 * a.nh + BM - 1) / BM, total = per_tile * a.n_tiles, blocks = gridDim.x, me = blockIdx.x;
+attention_latent_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, Args a) {
+  const int per_tile = ((DECODE ? 1 : 64) * a.nh + BM - 1) / BM, total = per_tile * (DECODE ? a.n_dec * a.max_splits : a.n_tiles);
+  const int blocks = gridDim.x, me = blockIdx.x;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int q_bytes = a.boxes * Q_COL_BYTES, tile_bytes = a.boxes * K_COL_BYTES;
@@ -218,7 +250,7 @@ attention_prefill_latent_kernel(const __grid_constant__ CUtensorMap q_map, const
       for (int i = 0;; ++i) {
         const int w = nth_work(i, me, blocks, total);
         if (w < 0 || *abort) break;
-        const Work k = work_of(a, w, per_tile);
+        const Work k = DECODE ? decode_work_of(a, w, per_tile) : work_of(a, w, per_tile);
         if (k.rows <= 0) continue;
         mbar_wait(q_empty, (it & 1) ^ 1, abort, a.status);
         mbar_expect_tx(q_full, (uint32_t)q_bytes);
@@ -248,7 +280,7 @@ attention_prefill_latent_kernel(const __grid_constant__ CUtensorMap q_map, const
       for (int i = 0;; ++i) {
         const int w = nth_work(i, me, blocks, total);
         if (w < 0 || *abort) break;
-        const Work k = work_of(a, w, per_tile);
+        const Work k = DECODE ? decode_work_of(a, w, per_tile) : work_of(a, w, per_tile);
         if (k.rows <= 0) continue;
         auto scores = [&](int j) {
           const int g = g0 + j, b = g % STAGES;
@@ -306,7 +338,7 @@ attention_prefill_latent_kernel(const __grid_constant__ CUtensorMap q_map, const
     for (int i = 0;; ++i) {
       const int w = nth_work(i, me, blocks, total);
       if (w < 0) break;
-      const Work k = work_of(a, w, per_tile);
+      const Work k = DECODE ? decode_work_of(a, w, per_tile) : work_of(a, w, per_tile);
       if (k.rows <= 0) continue;
       const bool valid = r < k.rows;
       const int f = k.first + r, pos = valid ? k.start + f / a.nh : k.p_last, lo = mi::first_visible(pos, a.window);
@@ -375,6 +407,28 @@ attention_prefill_latent_kernel(const __grid_constant__ CUtensorMap q_map, const
         if (g >= back) wait_o(g - back);
       row_sum[half * BM + r] = l_run;
       meet();
+      if constexpr (DECODE) {
+        const size_t at = (size_t)k.slot * a.nh + f;      // (of a head that exists)
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          const int c = 2 * n + half;
+          if (32 * c < a.n_out && quarter * 32 < k.rows) {
+            float o[32];
+            tmem_ld(o, t_lane + O_COL + 32 * c);
+            if (valid && !*abort) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                if (32 * c + 4 * q < a.out_hd)
+                  *reinterpret_cast<float4*>(a.part_o + at * a.out_hd + 32 * c + 4 * q) = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+            }
+          }
+        }
+        if (valid && half == 0 && !*abort) *reinterpret_cast<float2*>(a.part_ml + 2 * at) = make_float2(m_run, row_sum[r] + row_sum[BM + r]);
+        tc_fence_before();
+        meet();      // (the sums are read too: the next work may leave its own)
+        if (lane == 0) mbar_arrive(o_free);
+        continue;
+      }
       const float sink2 = a.sink ? a.sink[f % a.nh] * 1.4426950408889634f : -INFINITY;      // base 2, like the scores
       const float m_all = fmaxf(m_run, sink2), weight = exp2f(m_run - m_all);
       const float factor = weight / ((row_sum[r] + row_sum[BM + r]) * weight + (a.sink ? exp2f(sink2 - m_all) : 0.f));
@@ -414,6 +468,41 @@ attention_prefill_latent_kernel(const __grid_constant__ CUtensorMap q_map, const
   }
 }
 
+// The pieces of a decode token added up, a block per (request, query head) and a thread per value; pieces in ascending order.
+// An entry without keys (a padded one) gets zeros.
+constexpr int MERGE_PIECES = 256;      // whose factors are made a thread each, at a time
+__global__ void __launch_bounds__(256)
+latent_merge_kernel(Args a) {
+  __shared__ float s_f[MERGE_PIECES], s_l[MERGE_PIECES];
+  const int head = blockIdx.x, entry = blockIdx.y, item = a.decode_items[entry];
+  const int p = a.ctx_len[item] - 1, n = p < 0 ? 0 : p / a.chunk - mi::first_visible(p, a.window) / a.chunk + 1;
+  const float sink2 = a.sink ? a.sink[head] * 1.4426950408889634f : -INFINITY;      // base 2, like the scores
+  mi::grid_dependency_sync();
+  const float* ml = a.part_ml + 2 * ((size_t)entry * a.max_splits * a.nh + head);
+  const float* po = a.part_o + ((size_t)entry * a.max_splits * a.nh + head) * a.out_hd;
+  float m = sink2;
+  for (int s = threadIdx.x & 31; s < n; s += 32) m = fmaxf(m, ml[(size_t)2 * s * a.nh]);
+  m = mi::warp_max(m);
+  float l = a.sink ? exp2f(sink2 - m) : 0.f, acc = 0.f;
+  for (int s0 = 0; s0 < n; s0 += MERGE_PIECES) {
+    const int near = min(n - s0, MERGE_PIECES);
+    __syncthreads();
+    for (int s = threadIdx.x; s < near; s += blockDim.x) {
+      const float2 v = *reinterpret_cast<const float2*>(ml + (size_t)2 * (s0 + s) * a.nh);
+      s_f[s] = exp2f(v.x - m);
+      s_l[s] = v.y;
+    }
+    __syncthreads();
+    for (int s = 0; s < near; ++s) l = fmaf(s_l[s], s_f[s], l);
+    if (threadIdx.x < a.out_hd) {
+#pragma unroll 16
+      for (int s = 0; s < near; ++s) acc = fmaf(po[(size_t)(s0 + s) * a.nh * a.out_hd + threadIdx.x], s_f[s], acc);
+    }
+  }
+  if (threadIdx.x < a.out_hd)
+    a.out[((size_t)a.q_start[item] * a.nh + head) * a.out_hd + threadIdx.x] = __float2bfloat16_rn(n > 0 ? acc * (1.f / l) : 0.f);
+}
+
 size_t smem_bytes(int boxes) { return 1024 + (size_t)boxes * (Q_COL_BYTES + STAGES * K_COL_BYTES) + 32 * 8 + 6 * BM * sizeof(float); }
 
 }  // namespace
@@ -441,31 +530,61 @@ MI_API int mi_rows_tensor_map(void* out_map, const void* base, long long rows, l
 
 // q_map, kv_map: mi_rows_tensor_map of the queries [T * nh, hd] and of the layer's cache [pages * 2 * page_size, hd] (one key/value head).
 // out [T * nh, out_hd].  status: one word, set to 2 if a bounded wait ran out.
-MI_API int mi_attention_prefill_latent(void* out, const void* q_map, const void* kv_map, const int* block_table, int bt_stride, const int* tiles,
-                                       int n_tiles, const int* q_start, const int* q_len, const int* ctx_len, const int* seq_slot, int* status,
-                                       int nh, int hd, int out_hd, int page_size, float scale, int window, const float* sink, cudaStream_t stream) {
-  MI_REQUIRE(hd >= 64 && hd <= 256 && hd % 16 == 0 && out_hd > 0 && out_hd <= hd && out_hd % 8 == 0, "attention_prefill_latent: bad head sizes %d, %d", hd, out_hd);
-  MI_REQUIRE(n_tiles >= 0 && nh > 0 && page_size > 0 && page_size % 64 == 0 && scale > 0.f && ((uintptr_t)out % 16) == 0,
-             "attention_prefill_latent: nh=%d, page_size=%d, the scale or the output do not fit", nh, page_size);
-  if (n_tiles == 0) return 0;
-  const long long works = (64ll * nh + BM - 1) / BM * n_tiles;
-  MI_REQUIRE(works <= 1 << 30, "attention_prefill_latent: %d tiles of %d heads are too many for one launch", n_tiles, nh);
-  Args a{(__nv_bfloat16*)out, block_table, bt_stride, tiles, q_start, q_len, ctx_len, seq_slot, status, n_tiles, nh, page_size, window,
-         (hd + BOX - 1) / BOX, hd / 16, (out_hd + BOX - 1) / BOX * BOX, out_hd, scale * 1.4426950408889634f, sink};
-  static bool ready[64] = {};
+static int latent_launch(Args& a, const void* q_map, const void* kv_map, int hd, long long works, cudaStream_t stream) {
+  a.boxes = (hd + BOX - 1) / BOX;
+  a.steps = hd / 16;
+  a.n_out = (a.out_hd + BOX - 1) / BOX * BOX;
+  MI_REQUIRE(hd >= 64 && hd <= 256 && hd % 16 == 0 && a.out_hd > 0 && a.out_hd <= hd && a.out_hd % 8 == 0, "attention_latent: bad head sizes %d, %d", hd, a.out_hd);
+  MI_REQUIRE(a.nh > 0 && a.page_size > 0 && a.page_size % 64 == 0 && a.scale_log2 > 0.f && ((uintptr_t)a.out % 16) == 0,
+             "attention_latent: nh=%d, page_size=%d, the scale or the output do not fit", a.nh, a.page_size);
+  MI_REQUIRE(works <= 1 << 30, "attention_latent: %lld works of %d heads are too many for one launch", works, a.nh);
+  auto kernel = a.n_dec ? attention_latent_kernel<true> : attention_latent_kernel<false>;
+  static bool ready[64][2] = {};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !ready[dev]) {
-    if (cudaFuncSetAttribute(attention_prefill_latent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(4)) != cudaSuccess)
-      return mi_fail("attention_prefill_latent: %zu bytes of shared memory were refused", smem_bytes(4));
-    if (dev >= 0 && dev < 64) ready[dev] = true;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !ready[dev][a.n_dec > 0]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(4)) != cudaSuccess)
+      return mi_fail("attention_latent: %zu bytes of shared memory were refused", smem_bytes(4));
+    if (dev >= 0 && dev < 64) ready[dev][a.n_dec > 0] = true;
   }
   CUtensorMap qm, km;
   memcpy(&qm, q_map, sizeof(qm));
   memcpy(&km, kv_map, sizeof(km));
   const int blocks = (int)(works < mi::sm_count() ? works : mi::sm_count());
   // the shared memory of four boxes at any size: a block then has its SM's tensor memory to itself
-  if (mi::launch(attention_prefill_latent_kernel, dim3(blocks), dim3(THREADS), smem_bytes(4), stream, qm, km, a) != cudaSuccess)
-    return mi_fail("attention_prefill_latent: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+  if (mi::launch(kernel, dim3(blocks), dim3(THREADS), smem_bytes(4), stream, qm, km, a) != cudaSuccess)
+    return mi_fail("attention_latent: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+  return 0;
+}
+
+MI_API int mi_attention_prefill_latent(void* out, const void* q_map, const void* kv_map, const int* block_table, int bt_stride, const int* tiles,
+                                       int n_tiles, const int* q_start, const int* q_len, const int* ctx_len, const int* seq_slot, int* status,
+                                       int nh, int hd, int out_hd, int page_size, float scale, int window, const float* sink, cudaStream_t stream) {
+  MI_REQUIRE(n_tiles >= 0, "attention_prefill_latent: n_tiles=%d", n_tiles);
+  if (n_tiles == 0) return 0;
+  Args a{(__nv_bfloat16*)out, block_table, bt_stride, tiles, q_start, q_len, ctx_len, seq_slot, status, n_tiles, nh, page_size, window,
+         0, 0, 0, out_hd, scale * 1.4426950408889634f, sink, nullptr, nullptr, nullptr, 0, 0, 0};
+  const int code = latent_launch(a, q_map, kv_map, hd, (64ll * nh + BM - 1) / BM * n_tiles, stream);
+  if (code != 0) return code;
   MI_LAUNCH_OK("attention_prefill_latent");
+  return 0;
+}
+
+// One new token of each of the items decode_items[n_dec].  chunk: keys of a piece, a multiple of 128; max_splits: at least the pieces of any
+// entry.  scratch: n_dec * max_splits * nh * (out_hd + 2) floats, 16-byte aligned.
+MI_API int mi_attention_decode_latent(void* out, const void* q_map, const void* kv_map, const int* block_table, int bt_stride, const int* decode_items,
+                                      int n_dec, const int* q_start, const int* ctx_len, const int* seq_slot, int* status, float* scratch, int nh,
+                                      int hd, int out_hd, int page_size, float scale, int window, const float* sink, int chunk, int max_splits,
+                                      cudaStream_t stream) {
+  MI_REQUIRE(n_dec >= 0 && n_dec <= 65535 && max_splits > 0 && chunk > 0 && chunk % BN == 0 && ((uintptr_t)scratch % 16) == 0,
+             "attention_decode_latent: %d entries, chunk %d, %d pieces or the scratch do not fit", n_dec, chunk, max_splits);
+  if (n_dec == 0) return 0;
+  Args a{(__nv_bfloat16*)out, block_table, bt_stride, nullptr, q_start, nullptr, ctx_len, seq_slot, status, 0, nh, page_size, window,
+         0, 0, 0, out_hd, scale * 1.4426950408889634f, sink, decode_items, scratch, scratch + (size_t)n_dec * max_splits * nh * out_hd,
+         n_dec, chunk, max_splits};
+  const int code = latent_launch(a, q_map, kv_map, hd, (long long)(nh + BM - 1) / BM * n_dec * max_splits, stream);
+  if (code != 0) return code;
+  if (mi::launch(latent_merge_kernel, dim3(nh, n_dec), dim3((out_hd + 31) / 32 * 32), 0, stream, a) != cudaSuccess)
+    return mi_fail("attention_decode_latent: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+  MI_LAUNCH_OK("attention_decode_latent");
   return 0;
 }

@@ -30,7 +30,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-r
               "-Xptxas", "-v"]
 
 COMMON_SOURCES = ["common.cu", "embedding.cu", "norm.cu", "gemm_f32.cu", "gemm_skinny.cu", "gemm_skinny_fused.cu",
-                  "qk_norm_rope.cu", "attention_generic.cu", "attention_f32.cu", "attention_prefill_latent.cu", "activation.cu", "sampling.cu", "gemm_cublas.cu", "gemm_tc.cu",
+                  "qk_norm_rope.cu", "attention_generic.cu", "attention_f32.cu", "attention_latent.cu", "activation.cu", "sampling.cu", "gemm_cublas.cu", "gemm_tc.cu",
                   "gemm_stream_tc.cu", "qkv_prepare.cu", "moe.cu", "gemm_batched.cu", "recurrent.cu", "chunked_state.cu", "latent_prepare.cu",
                   "hyper.cu", "linear_attention.cu", "gated_recurrence.cu", "depth.cu"]
 COMMON_LIBS = ["cublas"]

@@ -1322,10 +1322,13 @@ class AttentionBatch:
     for k in self.__slots__:
       setattr(self, k, kw.get(k))
 
-  def decode_only(self) -> "AttentionBatch":
-    """The same step without its prompt portions, for a launcher that has dealt with those."""
+  def without(self, prefill, decode) -> "AttentionBatch":
+    """The same step without its prompt portions or without its decode tokens, for a launcher that has dealt with those."""
     rest = AttentionBatch(**{k: getattr(self, k) for k in self.__slots__})
-    rest.num_prefill_tiles = 0
+    if prefill:
+      rest.num_prefill_tiles = 0
+    if decode:
+      rest.num_decode = 0
     return rest
 
 
@@ -1401,34 +1404,74 @@ def attention(out: torch.Tensor, qkv: torch.Tensor, kv_layer: torch.Tensor, bloc
     opts.score_bias_ptr(), int(opts.gate_per_head), opts.distance_ptr(), _stream()))
 
 
+def latent_decode_chunk(units: int, span: int, sms: int) -> int:
+  """Keys of a piece for ``units`` (request, 128 heads) pairs of up to ``span`` keys: of 128, 256, ... the one whose busiest
+  block has the least to do, a piece costing its tiles of 128 keys and about two more for its queries, its partial sums and
+  their merge.  (8 requests of 2048 keys: 128 pieces of one tile on 148 SMs; 64 requests: 128 pieces of 1024 keys.)"""
+  best, chunk = None, 128
+  while True:
+    cost = -(-units * -(-span // chunk) // sms) * (chunk // 128 + 2)
+    if best is None or cost < best[0]:
+      best = (cost, chunk)
+    if chunk >= span or chunk >= 1 << 20:
+      return best[1]
+    chunk *= 2
+
+
 def latent_attention(out: torch.Tensor, q: torch.Tensor, kv_layer: torch.Tensor, block_table: torch.Tensor, batch: AttentionBatch,
                      num_heads: int, head_dim: int, scale: float, window: Optional[int], sink: Optional[torch.Tensor], out_hd: int) -> None:
   """``attention`` of ``num_heads`` query heads over one key/value head whose cached value rows are the first ``out_hd`` values of
   its key rows (attention through a latent, as ``latent_down`` stores it): what knows that reads a row once.  ``q
   [tokens, num_heads * head_dim]``, ``out [tokens, num_heads * out_hd]``."""
   page_size = kv_layer.shape[3]
-  if (q.is_cuda and q.dtype == torch.bfloat16 and batch.num_prefill_tiles and batch.prefill_tiles is not None and q.shape[1] == num_heads * head_dim
-      and head_dim % 16 == 0 and 64 <= head_dim <= 256 and out_hd % 8 == 0 and page_size % 64 == 0 and q.is_contiguous() and q.data_ptr() % 16 == 0
-      and out.data_ptr() % 16 == 0 and kv_layer.data_ptr() % 16 == 0 and os.environ.get("MINIINFER_B200_PREFILL_TC", "1") != "0"):
-    if (out.shape != (q.shape[0], num_heads * out_hd) or out.dtype != q.dtype or kv_layer.dtype != q.dtype or not 0 < out_hd <= head_dim
-        or kv_layer.shape[1:] != (2, 1, page_size, head_dim)):
-      raise KernelError("latent_attention: shapes or dtypes do not match")
-    lib = common_lib()
+  if not (q.is_cuda and q.dtype == torch.bfloat16 and q.shape[1] == num_heads * head_dim and head_dim % 16 == 0 and 64 <= head_dim <= 256
+          and out_hd % 8 == 0 and page_size % 64 == 0 and q.is_contiguous() and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
+          and kv_layer.data_ptr() % 16 == 0):
+    attention(out, q, kv_layer, block_table, batch, num_heads, 1, head_dim, scale, window, sink=sink, out_hd=out_hd)
+    return
+  if (out.shape != (q.shape[0], num_heads * out_hd) or out.dtype != q.dtype or kv_layer.dtype != q.dtype or not 0 < out_hd <= head_dim
+      or kv_layer.shape[1:] != (2, 1, page_size, head_dim)):
+    raise KernelError("latent_attention: shapes or dtypes do not match")
+  win, sinks = int(window) if window else 0, _ptr(sink, torch.float32) if sink is not None else _ptr(None)
+  prefill = batch.num_prefill_tiles and batch.prefill_tiles is not None and os.environ.get("MINIINFER_B200_PREFILL_TC", "1") != "0"
+  decode = batch.num_decode and os.environ.get("MINIINFER_B200_DECODE_TMA", "1") != "0"
+  lib = common_lib()
+  if prefill or decode:
+    maps = _rows_tensor_map(lib, q, head_dim), _rows_tensor_map(lib, kv_layer, head_dim)
+  if prefill:
     if batch.scratch is not None:
       status = batch.scratch.zeros("attention_prefill_status", 1, torch.int32)
     else:
       status = torch.zeros(1, dtype=torch.int32, device=q.device)
     _check(lib, lib.mi_attention_prefill_latent(
-      _ptr(out), _rows_tensor_map(lib, q, head_dim), _rows_tensor_map(lib, kv_layer, head_dim), _ptr(block_table, torch.int32), block_table.shape[1],
+      _ptr(out), *maps, _ptr(block_table, torch.int32), block_table.shape[1],
       _ptr(batch.prefill_tiles, torch.int32), batch.num_prefill_tiles, _ptr(batch.q_start, torch.int32), _ptr(batch.q_len, torch.int32),
       _ptr(batch.ctx_len, torch.int32), _ptr(batch.seq_slot, torch.int32), _ptr(status, torch.int32), num_heads, head_dim, out_hd, page_size,
-      ctypes.c_float(scale), int(window) if window else 0, _ptr(sink, torch.float32) if sink is not None else _ptr(None), _stream()))
+      ctypes.c_float(scale), win, sinks, _stream()))
     if batch.scratch is None and int(status[0]) != 0:
       raise KernelError("attention_prefill_latent: a bounded wait on a barrier ran out")
-    if not batch.num_decode:
-      return
-    batch = batch.decode_only()
-  attention(out, q, kv_layer, block_table, batch, num_heads, 1, head_dim, scale, window, sink=sink, out_hd=out_hd)
+  if decode:
+    span = min(batch.max_ctx_len, win) if win else batch.max_ctx_len
+    chunk = latent_decode_chunk(batch.num_decode * -(-num_heads // 128), span, _num_sms(q.device))
+    max_splits = -(-span // chunk) + 1
+    n = batch.num_decode * max_splits * num_heads * (out_hd + 2)
+    if batch.scratch is not None:
+      scratch = batch.scratch.buffer("attention_decode_partials", (n,), torch.float32)
+      status = batch.scratch.zeros("attention_decode_counters", batch.num_decode + 1, torch.int32)[:1]
+    else:
+      scratch = torch.empty(n, dtype=torch.float32, device=q.device)
+      status = torch.zeros(1, dtype=torch.int32, device=q.device)
+    _check(lib, lib.mi_attention_decode_latent(
+      _ptr(out), *maps, _ptr(block_table, torch.int32), block_table.shape[1], _ptr(batch.decode_items, torch.int32), batch.num_decode,
+      _ptr(batch.q_start, torch.int32), _ptr(batch.ctx_len, torch.int32), _ptr(batch.seq_slot, torch.int32), _ptr(status, torch.int32),
+      _ptr(scratch, torch.float32), num_heads, head_dim, out_hd, page_size, ctypes.c_float(scale), win, sinks, chunk, max_splits, _stream()),
+      kernels=2)
+    if batch.scratch is None and int(status[0]) != 0:
+      raise KernelError("attention_decode_latent: a bounded wait on a barrier ran out")
+  if (prefill or not batch.num_prefill_tiles) and (decode or not batch.num_decode):
+    return
+  rest = batch.without(prefill, decode)
+  attention(out, q, kv_layer, block_table, rest, num_heads, 1, head_dim, scale, window, sink=sink, out_hd=out_hd)
 
 
 class _AttentionOptions:

@@ -16,6 +16,11 @@ CASES = [
   ([(640, 33), (1500, 9), (40, 1)], 12, 112, 104, 64, 128, False),
   ([(2, 2), (700, 640)], 1, 256, 256, 64, 333, True),
   ([(260, 200)], 40, 176, 128, 192, None, True),
+  # decode tokens: pieces of one tile and of several, more heads than a work has rows, a window that begins inside a piece
+  ([(1, 1), (128, 1), (129, 1), (2048, 1)], 32, 256, 192, 64, None, True),
+  ([(1000, 1), (3, 1)], 130, 224, 192, 64, 333, False),
+  ([(40 + 7 * i, 1) for i in range(100)], 16, 112, 104, 128, None, True),
+  ([(1 + 11 * i, 1) for i in range(80)], 3, 64, 64, 64, 300, False),
 ]
 
 
@@ -23,7 +28,7 @@ CASES = [
 def test_latent_attention(case):
   from miniinfer_b200.kernels import ops
   items, nh, hd, ohd, P, window, with_sink = CASES[case]
-  qkv, kv, bt, batch = make_attention_case(items, nh, 1, hd, P, torch.bfloat16, seed=case, scale_q=2.0)
+  qkv, kv, bt, batch = make_attention_case(items, nh, 1, hd, P, torch.bfloat16, seed=case, num_slots=max(8, len(items)), scale_q=2.0)
   q = qkv[:, :nh * hd].contiguous()
   kv[:, 1, :, :, :ohd] = kv[:, 0, :, :, :ohd]
   sink = torch.randn(nh, generator=torch.Generator().manual_seed(case)).to(DEV) if with_sink else None
