@@ -483,17 +483,118 @@ moe_combine_kernel(TOut* __restrict__ out, const TY* __restrict__ y, const int* 
   }
 }
 
+// Eight consecutive values as float32, as they lie in memory until they are needed.
+template <typename T> struct Eight;
+template <> struct Eight<__nv_bfloat16> {
+  uint4 a;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { a = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ float at(int i) const {
+    const uint32_t w = i < 2 ? a.x : (i < 4 ? a.y : (i < 6 ? a.z : a.w));
+    return __uint_as_float((i & 1) ? w & 0xffff0000u : w << 16);
+  }
+};
+template <> struct Eight<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* p) { a = reinterpret_cast<const float4*>(p)[0]; b = reinterpret_cast<const float4*>(p)[1]; }
+  __device__ __forceinline__ float at(int i) const {
+    const float4 v = i < 4 ? a : b;
+    return (i & 3) == 0 ? v.x : ((i & 3) == 1 ? v.y : ((i & 3) == 2 ? v.z : v.w));
+  }
+};
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&v)[8]) {
+  uint4 o;
+  uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 x = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    w[i] = *reinterpret_cast<const uint32_t*>(&x);
+  }
+  *reinterpret_cast<uint4*>(p) = o;
+}
+__device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+
+// The same sums in the same order for rows of 8k aligned values: eight values a thread, the rows of four choices on their way at
+// once, a token's columns dealt to several blocks.  Bound by latency for few tokens, by the rows' bytes for many; a value a thread and a
+// choice at a time waited for every choice in turn (1500 tokens, four of 16
+// experts, 2048 columns: 15 us, 6.3 so).
+constexpr int COMBINE_THREADS = 128;
+
+template <typename TOut, typename TY>
+__global__ void __launch_bounds__(COMBINE_THREADS)
+moe_combine8_kernel(TOut* __restrict__ out, const TY* __restrict__ y, const int* __restrict__ pos_of, const float* __restrict__ w, int top, int N,
+                    const TOut* __restrict__ shared, const float* __restrict__ shared_logit, int logit_stride) {
+  const int t = blockIdx.x, n = (blockIdx.y * COMBINE_THREADS + threadIdx.x) * 8;
+  mi::grid_dependency_sync();
+  if (n >= N) return;
+  pos_of += (size_t)t * top;
+  w += (size_t)t * top;
+  float acc[8] = {};
+  for (int k0 = 0; k0 < top; k0 += 4) {
+    Eight<TY> v[4];
+    float f[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (k0 + j < top) {
+        f[j] = w[k0 + j];
+        v[j].load(y + (size_t)pos_of[k0 + j] * N + n);
+      }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (k0 + j < top) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = fmaf(f[j], v[j].at(i), acc[i]);
+      }
+  }
+  if (shared) {
+    const float sw = shared_logit ? 1.f / (1.f + expf(-shared_logit[(size_t)t * logit_stride])) : 1.f;
+    Eight<TOut> v;
+    v.load(shared + (size_t)t * N + n);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = fmaf(sw, v.at(i), acc[i]);
+  }
+  store8(out + (size_t)t * N + n, acc);
+}
+
+template <typename TOut, typename TY>
+void launch_combine(void* out, const void* y, const int* pos_of, const float* weights, int T, int top, int N, const void* shared,
+                    const float* shared_logit, int logit_stride, cudaStream_t stream) {
+  const int columns = (N / 8 + COMBINE_THREADS - 1) / COMBINE_THREADS;
+  if (N % 8 == 0 && (((uintptr_t)out | (uintptr_t)y | (uintptr_t)shared) % 16) == 0 && columns <= 65535)
+    mi::launch(moe_combine8_kernel<TOut, TY>, dim3(T, columns), dim3(COMBINE_THREADS), 0, stream, (TOut*)out, (const TY*)y, pos_of, weights, top, N,
+               (const TOut*)shared, shared_logit, logit_stride);
+  else
+    mi::launch(moe_combine_kernel<TOut, TY>, dim3(T), dim3(256), 0, stream, (TOut*)out, (const TY*)y, pos_of, weights, top, N,
+               (const TOut*)shared, shared_logit, logit_stride);
+}
+
 // The tokens' rows put in the order of the experts' rows: xs[pos] = x[pair / top] for the rows that a pair owns, zeros
-// for the others; 16 bytes a thread.  (The tcgen05 product reads its rows by TMA, which wants them side by side.)
+// for the others; 16 bytes a thread and row, four of them on their way at once (6000 rows of 2048 values: 11 us a row a block, 8.4 so).  (The
+// tcgen05 product reads its rows by TMA, which wants them side by side.)
+constexpr int GATHER_ROWS = 4;
+
 __global__ void __launch_bounds__(256)
-moe_gather_kernel(__nv_bfloat16* __restrict__ xs, const __nv_bfloat16* __restrict__ x, const int* __restrict__ sorted_pair,
+moe_gather_kernel(__nv_bfloat16* __restrict__ xs, const __nv_bfloat16* __restrict__ x, const int* __restrict__ sorted_pair, int rows,
                   int top, int H8) {
   mi::grid_dependency_sync();
-  const int pos = blockIdx.x;
-  const int pair = sorted_pair[pos];
+  const int pos = blockIdx.x * GATHER_ROWS, n = min(GATHER_ROWS, rows - pos);
+  const uint4* src[GATHER_ROWS];
+#pragma unroll
+  for (int r = 0; r < GATHER_ROWS; ++r) {
+    const int pair = r < n ? sorted_pair[pos + r] : -1;
+    src[r] = pair >= 0 ? reinterpret_cast<const uint4*>(x) + (size_t)(pair / top) * H8 : nullptr;
+  }
   uint4* dst = reinterpret_cast<uint4*>(xs) + (size_t)pos * H8;
-  const uint4* src = pair >= 0 ? reinterpret_cast<const uint4*>(x) + (size_t)(pair / top) * H8 : nullptr;
-  for (int i = threadIdx.x; i < H8; i += blockDim.x) dst[i] = src ? src[i] : make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < H8; i += blockDim.x) {
+    uint4 v[GATHER_ROWS];
+#pragma unroll
+    for (int r = 0; r < GATHER_ROWS; ++r) v[r] = src[r] ? src[r][i] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int r = 0; r < GATHER_ROWS; ++r)
+      if (r < n) dst[(size_t)r * H8 + i] = v[r];
+  }
 }
 
 template <int WM, int WN, int MODE, int STAGES>
@@ -602,7 +703,8 @@ MI_API int mi_moe_gather(void* xs, const void* x, const int* sorted_pair, int ro
   MI_REQUIRE(rows >= 0 && top > 0 && H > 0 && H % 8 == 0, "moe_gather: rows of %d values (a multiple of 8 in bfloat16)", H);
   MI_REQUIRE(((uintptr_t)xs % 16) == 0 && ((uintptr_t)x % 16) == 0, "moe_gather: operands must be 16-byte aligned");
   if (rows == 0) return 0;
-  mi::launch(moe_gather_kernel, dim3(rows), dim3(256), 0, stream, (__nv_bfloat16*)xs, (const __nv_bfloat16*)x, sorted_pair, top, H / 8);
+  mi::launch(moe_gather_kernel, dim3((rows + GATHER_ROWS - 1) / GATHER_ROWS), dim3(H / 8 > 128 ? 256 : 128), 0, stream, (__nv_bfloat16*)xs,
+             (const __nv_bfloat16*)x, sorted_pair, rows, top, H / 8);
   MI_LAUNCH_OK("moe_gather");
   return 0;
 }
@@ -614,11 +716,11 @@ MI_API int mi_moe_combine(void* out, int out_dtype, const void* y, int y_dtype, 
   MI_REQUIRE(T >= 0 && top > 0 && N > 0, "moe_combine: bad sizes");
   if (T == 0) return 0;
   if (out_dtype == MI_BF16 && y_dtype == MI_F32)
-    mi::launch(moe_combine_kernel<__nv_bfloat16, float>, dim3(T), dim3(256), 0, stream, (__nv_bfloat16*)out, (const float*)y, pos_of, weights, top, N, (const __nv_bfloat16*)shared, shared_logit, logit_stride);
+    launch_combine<__nv_bfloat16, float>(out, y, pos_of, weights, T, top, N, shared, shared_logit, logit_stride, stream);
   else if (out_dtype == MI_BF16 && y_dtype == MI_BF16)
-    mi::launch(moe_combine_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(T), dim3(256), 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)y, pos_of, weights, top, N, (const __nv_bfloat16*)shared, shared_logit, logit_stride);
+    launch_combine<__nv_bfloat16, __nv_bfloat16>(out, y, pos_of, weights, T, top, N, shared, shared_logit, logit_stride, stream);
   else if (out_dtype == MI_F32 && y_dtype == MI_F32)
-    mi::launch(moe_combine_kernel<float, float>, dim3(T), dim3(256), 0, stream, (float*)out, (const float*)y, pos_of, weights, top, N, (const float*)shared, shared_logit, logit_stride);
+    launch_combine<float, float>(out, y, pos_of, weights, T, top, N, shared, shared_logit, logit_stride, stream);
   else
     return mi_fail("moe_combine: unknown dtypes %d, %d", out_dtype, y_dtype);
   MI_LAUNCH_OK("moe_combine");
