@@ -42,7 +42,9 @@ __device__ __forceinline__ float2 block_sum2(float2 v, float2* scratch /* >= 33 
 
 // Latency is all there is to a decode step's few rows: both sums of squares at once, all loads of a row on their way together
 // (8 tokens, query latent of 1536: 10.0 us with one sum after the other in 128 threads, 6.5 so).  Where tokens are more than the
-// multiprocessors hold at once, the bigger block only keeps others out (2048 tokens: 9.4 us at 256 threads, 6.8 at 128).
+// multiprocessors hold at once, the bigger block only keeps others out (2048 tokens: 9.4 us at 256 threads, 6.8 at 128).  The block's
+// size is part of the order in which a row's squares are added: float32 rows, whose bits must not depend on how many tokens share
+// their step, have the same block in every step.
 constexpr int DOWN_THREADS = 256, DOWN_FEW_TOKENS = 1024;
 
 template <typename T>
@@ -135,7 +137,7 @@ MI_API int mi_latent_down(const void* down, int dtype, int ld, int q_off, int kv
   MI_REQUIRE(R * sizeof(float) <= 32 * 1024, "latent_down: rotated part of %d values is too long", R);
   if (T == 0) return 0;
   const size_t smem = (size_t)R * sizeof(float);
-  const dim3 block(T <= DOWN_FEW_TOKENS ? DOWN_THREADS : DOWN_THREADS / 2);
+  const dim3 block(dtype == MI_F32 || T <= DOWN_FEW_TOKENS ? DOWN_THREADS : DOWN_THREADS / 2);
   if (dtype == MI_BF16)
     mi::launch(latent_down_kernel<__nv_bfloat16>, dim3(T), block, smem, stream, (const __nv_bfloat16*)down, ld, q_off, kv_off, Q, C, R, hdp,
                q_w, kv_w, eps, (__nv_bfloat16*)cq_out, rope, positions, interleaved, slot_mapping, (__nv_bfloat16*)kv_layer, page_size);

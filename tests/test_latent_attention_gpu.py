@@ -62,3 +62,22 @@ def test_per_head_products_of_many_rows(M, N, K, B, gate, dtype):
   # product is gated by a pass of its own
   bound = K * 2.0 ** -23 * size + (2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -20) * want.abs() + 1e-6
   assert ((out.double().cpu() - want).abs() <= bound).all()
+
+
+def test_float32_norms_do_not_depend_on_how_many_tokens_share_the_step():
+  from miniinfer_b200.kernels import ops
+  T, Q, C, R, P = 1500, 700, 192, 32, 64
+  g = torch.Generator().manual_seed(3)
+  down, q_w, kv_w = torch.randn((T, Q + C + R), generator=g).to(DEV), torch.randn(Q, generator=g).to(DEV), torch.randn(C, generator=g).to(DEV)
+  rope, pos = torch.randn((T, R), generator=g).to(DEV), torch.arange(T, dtype=torch.int32, device=DEV)
+  runs = []
+  for step in (T, 1025, 1024, 512, 1):      # whole and in portions
+    cq, kv = torch.empty((T, Q), device=DEV), torch.zeros((-(-T // P), 2, 1, P, C + R), device=DEV)
+    for a in range(0, T, step) if step > 1 else range(0, T, 97):
+      rows = slice(a, min(a + step, T))
+      ops.latent_down(down[rows].contiguous(), 0, Q, Q, C, R, q_w, kv_w, 1e-6, cq[rows], rope, pos[rows].contiguous(), False, pos[rows].contiguous(), kv)
+    runs.append((cq, kv.transpose(1, 3).reshape(-1, 2 * (C + R))[:T]))
+  for step, (cq, kv) in zip((1025, 1024, 512), runs[1:]):
+    assert torch.equal(cq, runs[0][0]) and torch.equal(kv, runs[0][1]), step
+  some = slice(0, T, 97)
+  assert torch.equal(runs[-1][0][some], runs[0][0][some]) and torch.equal(runs[-1][1][some], runs[0][1][some])
