@@ -78,17 +78,29 @@ __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_grou
 
 // ------------------------------------------------------------------------------------------------------------ products
 
-// A float32 number as the sum of two tf32 ones, rounded to nearest in the integer unit: four plain instructions, where two
-// conversions cost the state kernel twice the instructions (of 1600 a warp and chunk, 110 us for 32 chunks).  The lower part
-// keeps bits that the tensor core does not look at.
+// A float32 number as the sum of two tf32 ones, the upper rounded to nearest in the integer unit: three plain instructions, where
+// two conversions cost the state kernel twice the instructions (of 1600 a warp and chunk, 110 us for 32 chunks).  The lower part
+// keeps bits that the tensor core does not look at: at most one of its twelve, so cutting it off errs as much as rounding it.
+// Rounding it in the integer unit is not open: the sum would carry a NaN of all ones, which is what arithmetic returns, into a
+// zero - as it does in the upper part, where the lower one remains a NaN.
 struct Two {
   uint32_t hi, lo;
   __device__ __forceinline__ Two() {}
   __device__ __forceinline__ explicit Two(float x) {
     hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
+    lo = __float_as_uint(x - __uint_as_float(hi));
   }
 };
+// Whether some lane of the warp holds a number that is not finite.  A tile's product with a triangular matrix multiplies the zeros
+// behind the diagonal too, and zero times such a number is a NaN in rows of earlier tokens: the warp then adds up its elements
+// one by one, up to the diagonal.
+template <int N>
+__device__ __forceinline__ bool any_not_finite(const float (&v)[N]) {
+  bool bad = false;
+#pragma unroll
+  for (int i = 0; i < N; ++i) bad |= !(fabsf(v[i]) <= 3.402823466e38f);
+  return __any_sync(0xffffffffu, bad);
+}
 __device__ __forceinline__ void mma1(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -407,6 +419,14 @@ chunk_build_kernel(Args a) {
       load_b(r, inv + (HALF + k) * LDT + c, LDT, g, t4);
       mma3(x, l, r);
     }
+    if (any_not_finite(x)) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = m + g + 8 * (e >> 1), col = c + 2 * t4 + (e & 1);
+        x[e] = 0.f;
+        for (int k = 0; k <= row; ++k) x[e] = fmaf(inv[(HALF + row) * LDT + HALF + k], inv[(HALF + k) * LDT + col], x[e]);
+      }
+    }
     __syncthreads();
     st2(inv + (HALF + m + g) * LDT + c + 2 * t4, -x[0], -x[1]);
     st2(inv + (HALF + m + g + 8) * LDT + c + 2 * t4, -x[2], -x[3]);
@@ -436,6 +456,14 @@ chunk_build_kernel(Args a) {
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
+        if (any_not_finite(c[j])) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int t = m0 + g + 8 * (e >> 1), col = n0 + 8 * j + 2 * t4 + (e & 1);
+            c[j][e] = 0.f;
+            for (int k = 0; k <= t; ++k) c[j][e] = fmaf(inv[t * LDT + k], right[k * ldr + col] * (scale ? scale[k] : 1.f), c[j][e]);
+          }
+        }
         st2(out + (size_t)(m0 + g) * ldo + n0 + 8 * j + 2 * t4, c[j][0], c[j][1]);
         st2(out + (size_t)(m0 + g + 8) * ldo + n0 + 8 * j + 2 * t4, c[j][2], c[j][3]);
       }
@@ -711,6 +739,20 @@ chunk_out_kernel(Args a) {
   __syncthreads();
 #pragma unroll 2
   for (int k = 0; k < m0 + 32; k += 8) multiply(aa, LDA, us, k);      // A U: nothing behind the diagonal
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (any_not_finite(acc[i][j])) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = m0 + 16 * i + g + 8 * (e >> 1), c = n0 + 8 * j + 2 * t4 + (e & 1);
+          float y = 0.f, z = 0.f;
+          for (int d = 0; d < a.dim; ++d) y = fmaf(qt[t * ldq + d], s0[d * LDV + c], y);
+          for (int s = 0; s <= t; ++s) z = fmaf(aa[t * LDA + s], us[s * LDV + c], z);
+          acc[i][j][e] = fabsf(z) <= 3.402823466e38f ? y + z : NAN;      // an infinite value: the recurrence adds it up over channels of both signs
+        }
+      }
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll

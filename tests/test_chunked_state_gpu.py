@@ -137,3 +137,86 @@ def test_causal_convolution_eight_channels_a_thread(taps, lengths, C, lead):
     assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all(), i      # one rounding to bfloat16; sums of a few float32 products
     assert torch.allclose(state[slot, :(taps - 1) * C].double().cpu().view(taps - 1, C), u[n:], atol=1e-6)
     at += n
+
+
+# Where a number that is not finite shows: exactly where the recurrence, token after token, takes it - from its token on, in its
+# column or channel -, never before it, in another request or in another head.  Tokens of the first chunk, of the first
+# and second half of a later one, and the portion's last; 130 tokens of another request behind.
+BAD_AT = [5, 70, 101, 199]
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["q", "k", "v", "a", "b", "state"])
+@pytest.mark.parametrize("per_head", [False, True])
+def test_delta_rule_of_numbers_that_are_not_finite(where, per_head, bad):
+  from miniinfer_b200.kernels import ops
+  lengths, H, G, D, Dv, eps = (200, 130), 2, 2, 40, 72, 1e-5
+  T = sum(lengths)
+  for token in BAD_AT:
+    r = torch.Generator().manual_seed(7)
+    bf = lambda *s: torch.randn(s, generator=r).to(torch.bfloat16)  # noqa: E731
+    x = {"q": bf(T, G * D), "k": bf(T, G * D), "v": bf(T, H * Dv), "b": bf(T, H), "a": bf(T, H if per_head else H * D)}
+    gate, start = bf(T, H * Dv), torch.randn((3, H * D * Dv), generator=r)
+    dt_bias, A_log, norm = torch.zeros(x["a"].shape[1]), torch.zeros(H), torch.ones(Dv)
+    if where == "state":
+      start.view(3, H, D, Dv)[2, 0, 17, 9] = bad
+    else:
+      x[where][token, 0 if per_head and where == "a" else min(9, x[where].shape[1] // H - 1)] = bad      # head 0
+    state, out = start.to(DEV), torch.empty((T, H * Dv), dtype=torch.bfloat16, device=DEV)
+    d = lambda t: t.to(DEV)  # noqa: E731
+    ops.gated_delta(out, d(x["q"]), d(x["k"]), d(x["v"]), d(x["a"]), d(x["b"]), d(gate), d(dt_bias), d(A_log), d(norm), eps, state, _ctx(lengths), H, G, D, Dv)
+    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+    decay = torch.exp(-torch.nn.functional.softplus(x["a"].double()).view(T, H, -1)).expand(T, H, D)
+    qq, kk, at = unit(x["q"].double().view(T, G, D)) * D ** -0.5, unit(x["k"].double().view(T, G, D)), 0
+    for i, n in enumerate(lengths):
+      slot, rows = len(lengths) - i, slice(at, at + n)
+      o, S = _walk(qq[rows], kk[rows], x["v"].double().view(T, H, Dv)[rows], decay[rows], torch.sigmoid(x["b"].double())[rows], start[slot].double().view(H, D, Dv))
+      _same_where_finite(state[slot].cpu().view(H, D, Dv), S, STATE_BOUND * S[S.isfinite()].norm(), (token, i, "state"))
+      want = _rms(o, eps) * torch.sigmoid(gate.double().view(T, H, Dv)[rows])
+      _same_where_finite(out[rows].cpu().view(n, H, Dv), want, None, (token, i, "read-outs"))
+      at += n
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["q", "k", "v", "a", "state"])
+@pytest.mark.parametrize("per_head", [False, True])
+def test_linear_attention_of_numbers_that_are_not_finite(where, per_head, bad):
+  from miniinfer_b200.kernels import ops
+  lengths, H, D, Dv, eps, tau = (200, 130), 2, 40, 72, 1e-5, 4.0
+  T = sum(lengths)
+  if per_head and where == "a":
+    return      # constants of the model
+  for token in BAD_AT:
+    r = torch.Generator().manual_seed(8)
+    bf = lambda *s: torch.randn(s, generator=r).to(torch.bfloat16)  # noqa: E731
+    x = {"q": bf(T, H * D), "k": bf(T, H * D), "v": bf(T, H * Dv), "a": torch.randn((T, H * D), generator=r) + 2.0}
+    gate, start, const = bf(T, H * Dv), torch.randn((3, H * D * Dv), generator=r), torch.tensor([0.97, 0.8])
+    if where == "state":
+      start.view(3, H, D, Dv)[2, 0, 17, 9] = bad
+    else:
+      x[where][token, 9] = bad
+    state, out = start.to(DEV), torch.empty((T, H * Dv), dtype=torch.bfloat16, device=DEV)
+    d = lambda t: t.to(DEV)  # noqa: E731
+    ops.linear_attention(out, d(x["q"]), d(x["k"]), d(x["v"]), d(gate), state, _ctx(lengths), H, D, Dv, eps, decay_logits=None if per_head else d(x["a"]),
+                         tau=tau, head_decay=d(const) if per_head else None, q_scale=D ** -0.5)
+    decay = const.double()[None, :, None].expand(T, H, D) if per_head else torch.exp(torch.nn.functional.logsigmoid(x["a"].double()) / tau).view(T, H, D)
+    at = 0
+    for i, n in enumerate(lengths):
+      slot, rows = len(lengths) - i, slice(at, at + n)
+      o, S = _walk(x["q"].double().view(T, H, D)[rows] * D ** -0.5, x["k"].double().view(T, H, D)[rows], x["v"].double().view(T, H, Dv)[rows], decay[rows], None,
+                   start[slot].double().view(H, D, Dv))
+      _same_where_finite(state[slot].cpu().view(H, D, Dv), S, STATE_BOUND * S[S.isfinite()].norm(), (token, i, "state"))
+      gl = gate.double().view(T, H, Dv)[rows]
+      _same_where_finite(out[rows].cpu().view(n, H, Dv), _rms(o, eps) * gl * torch.sigmoid(gl), None, (token, i, "read-outs"))
+      at += n
+
+
+def _same_where_finite(got, want, norm, what):
+  """The same places finite, and those equal: in their norm, or within one rounding to bfloat16."""
+  fine = want.isfinite()
+  assert torch.equal(got.isfinite(), fine), what
+  off, w = (got.double() - want)[fine], want[fine]
+  if norm is not None:
+    assert off.norm() <= norm, what
+  elif w.numel():
+    assert (off.abs() <= 2.0 ** -8 * w.abs().clamp(min=1.0) + 1e-4).all(), what
