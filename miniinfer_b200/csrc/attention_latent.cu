@@ -14,6 +14,13 @@
 // share a row of scores, 64 each, and agree on its maximum through shared memory; the output row is rescaled only when the
 // maximum has moved by more than a factor of 2^8.
 //
+// Rows that no row of a work may see - behind its last key, before its window: another request's, or never written - must not be
+// multiplied, for a weight of zero times an infinity is a NaN: P V leaves out whole sixteens of such keys, and the softmax warps zero
+// what is left of them in shared memory (at most 30 rows, in a work's first and last tile), once their registers are free: 51.2 us
+// for 2048 tokens where reading them all took 50.6; before the exponentials the same lines took 53.0, in a warp of its own 52.8.
+// Keys that some rows of a work see and others do not are multiplied for all: a number that is not finite there reaches up to 127
+// rows before its own, as it reached the other rows of a tile of 64 tokens in the mma.sync kernel.
+//
 // What bounds it: a tile's stage is given back by its P V, so the copy of the tile after next and its S lie on a chain of about 6800
 // cycles for two tiles, of which the products are 4600 (clock stamps).  Tiles of 64 keys in four stages are no faster: a product
 // of 128 x 64 x 16 takes 81 cycles where one of 128 x 128 x 16 takes 95.  Neither the exponentials nor the copies from L2 matter (left
@@ -153,7 +160,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 struct Work {
   int rows;                      // of the 128 that exist; 0: none
   int row0, first;               // first row in the step's [token, head] rows; the same counted from the item's first new token's
-  int start, p_first, p_last, lo_last, t_begin, n;
+  int start, p_first, p_last, lo_first, lo_last, t_begin, n;
   int slot;                      // decode: entry and piece, entry * max_splits + piece
   const int* bt;
 };
@@ -171,7 +178,8 @@ __device__ __forceinline__ Work work_of(const Args& a, int w, int per_tile) {
   k.p_first = k.start + k.first / a.nh;
   k.p_last = k.start + (k.first + max(k.rows, 1) - 1) / a.nh;
   k.lo_last = mi::first_visible(k.p_last, a.window);
-  k.t_begin = mi::first_visible(k.p_first, a.window) / BN;
+  k.lo_first = mi::first_visible(k.p_first, a.window);
+  k.t_begin = k.lo_first / BN;
   k.n = k.p_last / BN - k.t_begin + 1;
   k.slot = 0;
   k.bt = a.block_table + (size_t)a.seq_slot[item] * a.bt_stride;
@@ -187,13 +195,15 @@ __device__ __forceinline__ Work decode_work_of(const Args& a, int w, int parts) 
   k.first = part * BM;
   k.row0 = a.q_start[item] * a.nh + k.first;
   k.start = k.p_first = k.p_last = p;
-  k.lo_last = lo;
+  k.lo_first = k.lo_last = lo;
   k.t_begin = max(lo, piece * a.chunk) / BN;
   k.n = min(p, (piece + 1) * a.chunk - 1) / BN - k.t_begin + 1;
   k.slot = entry * a.max_splits + split;
   k.bt = a.block_table + (size_t)a.seq_slot[item] * a.bt_stride;
   return k;
 }
+// The keys of the tile from key0 on that some row of the work sees: the first, and one past the last.
+__device__ __forceinline__ int2 seen_keys(const Work& k, int key0) { return make_int2(max(k.lo_first - key0, 0), min(k.p_last + 1 - key0, BN)); }
 // The i-th work of block b: rounds that go back and forth, so that the block with the longest work of one round gets the
 // shortest of the next.  -1 past the end.
 __device__ __forceinline__ int nth_work(int i, int b, int blocks, int total) {
@@ -213,7 +223,7 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
   uint64_t* bars = reinterpret_cast<uint64_t*>(k_s + STAGES * tile_bytes);
   uint64_t *q_full = bars, *q_empty = bars + 1, *o_free = bars + 2;
   uint64_t *k_full = bars + 3, *k_empty = k_full + STAGES;  // of a tile: copied; read by S and by P V
-  uint64_t *s_full = k_empty + STAGES, *p_full = s_full + STAGES, *o_full = p_full + STAGES;      // of a tile: S computed, weights written, P V added
+  uint64_t *s_full = k_empty + STAGES, *p_full = s_full + STAGES, *o_full = p_full + STAGES;      // of a tile: S computed, weights written and rows zeroed, P V added
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + STAGES);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* row_max = reinterpret_cast<float*>(bars + 32);     // [2 tiles][2 halves][BM]; at a work's end the halves' sums in [half][BM] behind
@@ -305,8 +315,16 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
           if (*abort) break;
           tc_fence_after();
           const uint64_t v_desc = smem_desc(smem_u32(k_s + b * tile_bytes), K_COL_BYTES, 1024);
-          for (int s = 0; s < BN / 16; ++s)      // 16 keys further: 2048 bytes of every box
-            tc_mma_ts(tmem + O_COL, tmem + S_COL + BN * b + 8 * s, v_desc + (uint64_t)(s * (2048 >> 4)), idesc_pv, (j > 0 || s > 0) ? 1u : 0u);
+          auto add = [&](int s, bool onto) {      // 16 keys further: 2048 bytes of every box
+            tc_mma_ts(tmem + O_COL, tmem + S_COL + BN * b + 8 * s, v_desc + (uint64_t)(s * (2048 >> 4)), idesc_pv, onto ? 1u : 0u);
+          };
+          if (j == 0 || j == k.n - 1) {
+            const int2 keys = seen_keys(k, (k.t_begin + j) * BN);
+#pragma unroll 1
+            for (int s = keys.x / 16; 16 * s < keys.y; ++s) add(s, j > 0 || s > keys.x / 16);
+          } else {
+            for (int s = 0; s < BN / 16; ++s) add(s, true);
+          }
           tc_commit(&o_full[b]);
           tc_commit(&k_empty[b]);
           if (j + STAGES < k.n) scores(j + STAGES);
@@ -395,6 +413,17 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
 #pragma unroll
         for (int e = 0; e < BN / 4; ++e) packed[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
         tmem_st(s_addr + BN / 4 * half, packed);      // two keys to a column
+        if (j == 0 || j == k.n - 1) {      // the rows that nobody sees in the sixteens at the edges (S has read them): zeros before P V reads them
+          const int2 keys = seen_keys(k, key0);
+          if ((keys.x | keys.y) & 15) {
+            if (8 * lane < a.n_out) {
+              unsigned char* column = k_s + b * tile_bytes + (lane >> 3) * K_COL_BYTES + (lane & 7) * 16;
+              for (int row = (keys.x & ~15) + warp; row < keys.x; row += SOFTMAX_WARPS) *reinterpret_cast<uint4*>(column + row * 128) = make_uint4(0, 0, 0, 0);
+              for (int row = keys.y + warp; row < ((keys.y + 15) & ~15); row += SOFTMAX_WARPS) *reinterpret_cast<uint4*>(column + row * 128) = make_uint4(0, 0, 0, 0);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          }
+        }
         l_run += (part[0] + part[1]) + (part[2] + part[3]);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         if (g >= STAGES) wait_o(g - STAGES);      // long done - S of this tile came behind it -: keeps this thread in step with the barrier

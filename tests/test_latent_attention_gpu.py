@@ -81,3 +81,43 @@ def test_float32_norms_do_not_depend_on_how_many_tokens_share_the_step():
     assert torch.equal(cq, runs[0][0]) and torch.equal(kv, runs[0][1]), step
   some = slice(0, T, 97)
   assert torch.equal(runs[-1][0][some], runs[0][0][some]) and torch.equal(runs[-1][1][some], runs[0][1][some])
+
+
+# (items, heads, key size, value size, page size, window): contexts that end inside a tile, a page and sixteen keys
+UNSEEN = [
+  ([(300, 300), (65, 1), (129, 2)], 16, 224, 192, 64, None),
+  ([(1000, 257), (513, 1), (2047, 1)], 32, 256, 192, 64, 300),
+  ([(333, 40), (200, 1)], 5, 112, 104, 128, 100),
+  ([(700, 9), (641, 1)], 130, 64, 64, 192, 33),
+]
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("case", range(len(UNSEEN)))
+def test_rows_that_no_token_may_see_change_nothing(case, bad):
+  from miniinfer_b200.kernels import ops
+  items, nh, hd, ohd, P, window = UNSEEN[case]
+  qkv, kv, bt, batch = make_attention_case(items, nh, 1, hd, P, torch.bfloat16, seed=case)
+  q = qkv[:, :nh * hd].contiguous()
+  kv[:, 1, :, :, :ohd] = kv[:, 0, :, :, :ohd]
+  seen = torch.zeros((kv.shape[0], P), dtype=torch.bool, device=DEV)
+  for b, (c, n) in enumerate(items):
+    slot = int(batch.seq_slot[b])
+    for j in range(max(0, c - n - window + 1) if window else 0, c):
+      seen[bt[slot, j // P].long(), j % P] = True
+
+  def run():
+    out = torch.full((q.shape[0], nh * ohd), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.latent_attention(out, q, kv, bt, batch, nh, hd, hd ** -0.5, window, None, ohd)
+    return out
+
+  want = run()
+  kv[~seen.view(-1, 1, 1, P, 1).expand_as(kv)] = bad
+  assert torch.isfinite(want).all() and torch.equal(run(), want)
+  # a bad row of a prompt's later token: nothing in the works of 128 rows before its own
+  c, n = items[0]
+  at = n - 3
+  kv[bt[int(batch.seq_slot[0]), (c - n + at) // P].long(), :, :, (c - n + at) % P] = bad
+  untouched = at * nh // 128 * 128 // nh
+  got = run()
+  assert torch.equal(got[:untouched], want[:untouched]) and not torch.isfinite(got[at:n].float()).all()
