@@ -18,6 +18,8 @@
 // tokens behind 2000 each 1484 -> 78.
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "attention_scores.cuh"
 #include "common.cuh"
 
@@ -167,11 +169,12 @@ attention_f32_kernel(const F32Args a) {
         __syncthreads();
         // a row's key is visible in this stretch; a warp none of whose rows sees any key of the chunk has nothing to do
         const int j = c + lane;
-        bool seen[RW], any = false;
+        bool seen[RW], any = false, every = true;
 #pragma unroll
         for (int i = 0; i < RW; ++i) {
           seen[i] = first_keys ? j < kept[i] : j >= lo[i] && j <= p[i];
           any |= seen[i];
+          every &= seen[i] || p[i] < 0;      // (a row that does not exist)
         }
         if (__any_sync(0xffffffffu, any)) {
           uint64_t acc[RW];
@@ -195,8 +198,9 @@ attention_f32_kernel(const F32Args a) {
             asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(acc[i]));
             const float sc = seen[i] ? a.scale * (x + y) : -INFINITY;
             const float m_new = fmaxf(m[i], mi::warp_max(sc));
-            const float alpha = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);      // (no key of this segment seen yet)
-            pe[i] = seen[i] ? expf(sc - m_new) : 0.f;
+            const bool none = m_new == -INFINITY;      // no key of this segment seen yet, or none whose score weighs anything
+            const float alpha = none ? 1.f : expf(m[i] - m_new);
+            pe[i] = seen[i] ? expf(sc - (none ? 0.f : m_new)) : 0.f;
             l[i] = l[i] * alpha + mi::warp_sum(pe[i]);
             m[i] = m_new;
 #pragma unroll
@@ -207,30 +211,40 @@ attention_f32_kernel(const F32Args a) {
           for (int i = 0; i < RW; i += 2) *reinterpret_cast<float2*>(pw + lane * 8 + i) = make_float2(pe[i], pe[i + 1]);
           __syncwarp();
           const float* vr = sm + at.values(s);
-#pragma unroll 4
-          for (int jj = 0; jj < CHUNK; ++jj) {
-            float w[RW];
+          // MASKED: a row takes nothing from a key that it may not see, not even zero times its value, which may be no number
+          auto weigh = [&](auto masked) {
+            constexpr bool MASKED = decltype(masked)::value;
+            unsigned mask[RW];
 #pragma unroll
-            for (int i = 0; i < RW; i += 2) {
-              const float2 t = *reinterpret_cast<const float2*>(pw + jj * 8 + i);
-              w[i] = t.x;
-              w[i + 1] = t.y;
-            }
+            for (int i = 0; i < RW; ++i) mask[i] = MASKED ? __ballot_sync(0xffffffffu, seen[i]) : 0u;
+#pragma unroll(MASKED ? 1 : 4)
+            for (int jj = 0; jj < CHUNK; ++jj) {
+              float w[RW];
 #pragma unroll
-            for (int n = 0; n < NV; ++n) {
-              const int d = 128 * n + 4 * lane;
-              if (d < hd) {
-                const float4 v = *reinterpret_cast<const float4*>(vr + jj * hd + d);
+              for (int i = 0; i < RW; i += 2) {
+                const float2 t = *reinterpret_cast<const float2*>(pw + jj * 8 + i);
+                w[i] = t.x;
+                w[i + 1] = t.y;
+              }
 #pragma unroll
-                for (int i = 0; i < RW; ++i) {
-                  o[i][4 * n] = fmaf(w[i], v.x, o[i][4 * n]);
-                  o[i][4 * n + 1] = fmaf(w[i], v.y, o[i][4 * n + 1]);
-                  o[i][4 * n + 2] = fmaf(w[i], v.z, o[i][4 * n + 2]);
-                  o[i][4 * n + 3] = fmaf(w[i], v.w, o[i][4 * n + 3]);
+              for (int n = 0; n < NV; ++n) {
+                const int d = 128 * n + 4 * lane;
+                if (d < hd) {
+                  const float4 v = *reinterpret_cast<const float4*>(vr + jj * hd + d);
+#pragma unroll
+                  for (int i = 0; i < RW; ++i) {
+                    if (MASKED && !(mask[i] >> jj & 1)) continue;
+                    o[i][4 * n] = fmaf(w[i], v.x, o[i][4 * n]);
+                    o[i][4 * n + 1] = fmaf(w[i], v.y, o[i][4 * n + 1]);
+                    o[i][4 * n + 2] = fmaf(w[i], v.z, o[i][4 * n + 2]);
+                    o[i][4 * n + 3] = fmaf(w[i], v.w, o[i][4 * n + 3]);
+                  }
                 }
               }
             }
-          }
+          };
+          if (WARPS == 1 || __all_sync(0xffffffffu, every)) weigh(std::false_type());      // (one token's rows see the same keys, and the others are staged as zeros)
+          else if constexpr (WARPS > 1) weigh(std::true_type());
         }
         __syncthreads();      // the stage may be filled again
       }
@@ -259,9 +273,8 @@ attention_f32_kernel(const F32Args a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) oo[4 * n + e] = 128 * n + 4 * lane < hd ? run_o[r * hd + 128 * n + 4 * lane + e] : 0.f;
       for (int b = 0; b < a.cluster && round + b < segs; ++b) {
-        const float pm = *cluster.map_shared_rank(part_m + r, b);
-        if (pm == -INFINITY) continue;      // no key of that segment is visible
-        const float pl = *cluster.map_shared_rank(part_l + r, b);
+        const float pm = *cluster.map_shared_rank(part_m + r, b), pl = *cluster.map_shared_rank(part_l + r, b);
+        if (pm == -INFINITY && pl == 0.f) continue;      // no key of that segment is visible (scores that are no numbers leave a sum that is none)
         const float m_new = fmaxf(mm, pm), fa = expf(mm - m_new), fb = expf(pm - m_new);
         ll = ll * fa + pl * fb;
         mm = m_new;

@@ -84,3 +84,61 @@ def test_attention_float32_against_the_generic_kernel_and_cut_by_cut(case):
     for lo, hi in portions:
       assert torch.equal(run(slice(at + lo, at + hi), _batch_of(slot, ctx - new + hi, hi - lo)), got[at + lo:at + hi]), (b, lo, hi)
     at += new
+
+
+@pytest.mark.skipif(DEV == "cpu", reason="what the CUDA kernels read")
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("case", range(len(F32_CASES)))
+def test_attention_float32_rows_take_nothing_from_keys_they_may_not_see(case, bad):
+  from gpu_helpers import make_attention_case
+  from miniinfer_b200.kernels import ops
+  items, nh, nkv, hd, P, opt = F32_CASES[case]
+  qkv, kv, bt, batch = make_attention_case(items, nh, nkv, hd, P, torch.float32, seed=case)
+  T, ohd = qkv.shape[0], opt.get("out_hd", hd)
+
+  def run(generic=False):
+    out = torch.full((T, nh * ohd), 7.0, device=DEV)
+    ops.attention(out, qkv, kv, bt, batch, nh, nkv, hd, hd ** -0.5, opt.get("window"), force_generic=generic, out_hd=ohd, keep_first=opt.get("keep_first", 0),
+                  chunk=opt.get("chunk"))
+    return out
+
+  want = run()
+  seen = torch.zeros((kv.shape[0], P), dtype=torch.bool, device=DEV)
+  for b, (c, n) in enumerate(items):
+    slot, w, ch, kept = int(batch.seq_slot[b]), opt.get("window"), opt.get("chunk"), opt.get("keep_first", 0)
+    lo = max(0, c - n - w + 1) if w else ((c - n) // ch * ch if ch else 0)
+    for j in range(c):
+      if j >= lo or j < kept:
+        seen[bt[slot, j // P].long(), j % P] = True
+  kv[~seen.view(-1, 1, 1, P, 1).expand_as(kv)] = bad
+  assert torch.isfinite(want).all() and torch.equal(run(), want)
+  at = 0
+  for b, (c, n) in enumerate(items):      # the row of a later token of the same prompt: nothing before it, everything from it on
+    if n > 2:
+      j = c - 2
+      kv[bt[int(batch.seq_slot[b]), j // P].long(), :, :, j % P] = bad
+      got = run()
+      assert torch.equal(got[at:at + n - 2], want[at:at + n - 2]), b
+      assert not torch.isfinite(got[at + n - 2:at + n]).view(2, nh, ohd).any(-1).any(), b
+    at += n
+
+
+@pytest.mark.skipif(DEV == "cpu", reason="the kernels against one another")
+@pytest.mark.parametrize("score", [float("nan"), float("-inf")])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_attention_float32_segments_of_scores_that_are_no_numbers(score, with_sink):
+  from gpu_helpers import make_attention_case
+  from miniinfer_b200.kernels import ops
+  nh, nkv, hd, P = 4, 2, 64, 64
+  qkv, kv, bt, batch = make_attention_case([(700, 30), (520, 1)], nh, nkv, hd, P, torch.float32, seed=5)
+  qkv = qkv.abs()
+  for b in range(2):      # the segment of keys 256 .. 511: every score of it is not a number, or overflows downwards
+    for j in range(256, 512):
+      kv[bt[int(batch.seq_slot[b]), j // P].long(), 0, :, j % P] = float("nan") if score != score else -3e38
+  sink = torch.tensor([0.5, -1.0, 2.0, 0.0], device=DEV) if with_sink else None
+  outs = []
+  for generic in (False, True):
+    outs.append(torch.full((qkv.shape[0], nh * hd), 7.0, device=DEV))
+    ops.attention(outs[-1], qkv, kv, bt, batch, nh, nkv, hd, hd ** -0.5, None, force_generic=generic, sink=sink)
+  assert torch.equal(torch.isnan(outs[0]), torch.isnan(outs[1])) and bool(torch.isnan(outs[0]).all()) == (score != score)
+  assert torch.allclose(outs[0], outs[1], atol=2e-5, equal_nan=True)
