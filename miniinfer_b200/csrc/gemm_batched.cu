@@ -5,14 +5,14 @@
 // x[b] starts at x + b * x_batch with rows lda apart, w[b] at w + b * w_batch with rows ldw apart, out[b] at
 // out + b * o_batch with rows ldo apart - so the heads of a token's row (a batch stride of one head, a row stride of
 // the whole row) are multiplied with a matrix per head without being repacked, and a column range of a row can be
-// an operand.  Products and sums in float32, k ascending, whatever the storage type: a row's result does not depend
-// on the other rows.  act: 0 none, 1 softplus (log(1 + exp(z)), z itself above 20).  row_gate: one logit per
+// an operand.  Products and sums in float32, whatever the storage type - k ascending but for bfloat16 results on the tensor
+// cores, which add up sixteen products at a time -: a row's result does not depend on the other rows.  act: 0 none, 1 softplus (log(1 + exp(z)), z itself above 20).  row_gate: one logit per
 // (row, batch) at row_gate[m * gate_stride + b]; the output rows of batch b are multiplied with its sigmoid.  value_gate: one
 // logit per output value instead, at value_gate[m * gate_stride + b * N + n].
 //
-// This is the product of the 32-bit path for strided operands, of per-head up- and down-projections of a latent
-// attention, and the fallback of the bfloat16 path for inner sizes that are no multiple of 8.  The general kernel: tiles of 64 x 64
-// through shared memory, 16 values of k at a time, 4 x 4 outputs a thread.
+// This is the product of per-head up- and down-projections of a latent attention, of the 32-bit path for batches of them and
+// for rows whose values do not lie side by side, and the fallback of the bfloat16 path for inner sizes that are no multiple of 8.
+// The general kernel: tiles of 64 x 64 through shared memory, 16 values of k at a time, 4 x 4 outputs a thread.
 #include "common.cuh"
 
 namespace {
@@ -175,7 +175,10 @@ gemm_batched_mma_few_rows_kernel(BatchedArgs a) {
 // Many rows in bfloat16 on the tensor cores (mma.sync), for operands whose rows can be fetched 16 bytes at a time: tiles of 64 x 64, a
 // warp 32 x 32, K in stages of 64 by cp.async.  These products are small and read their rows once - 2048 rows of 16 heads,
 // 64 x 192 each, move 17 MB - so the memory bounds them, where the FMA kernel above was bound by its arithmetic (50.6 us,
-// 13.8 here); a tcgen05 tile of 128 rows would wait for the same bytes.
+// 13.8 here); a tcgen05 tile of 128 rows would wait for the same bytes.  The tensor core cuts off what its accumulator does not
+// hold, always towards zero: every sixteen products start from zero and are added to the sum in a rounded addition.  bfloat16
+// results only: in float32 the sums of sixteen would still err by more than the chain of FMAs (K = 4096, carried on in the
+// accumulator: 4.4e-6 of the norm, by FMAs 6.1e-7).
 constexpr int TK = 64, LDS = TK + 8, TSTAGES = 3;
 
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __nv_bfloat16* p) {
@@ -183,7 +186,6 @@ __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __nv_bfloat16*
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
 
-template <typename TO>
 __global__ void __launch_bounds__(128)
 gemm_batched_mma_kernel(BatchedArgs a) {
   extern __shared__ __align__(16) __nv_bfloat16 tiles[];      // [TSTAGES][x rows, w rows][64][LDS]
@@ -226,13 +228,18 @@ gemm_batched_mma_kernel(BatchedArgs a) {
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                       : "+f"(c[i][j][0]), "+f"(c[i][j][1]), "+f"(c[i][j][2]), "+f"(c[i][j][3])
-                       : "r"(xa[i][0]), "r"(xa[i][1]), "r"(xa[i][2]), "r"(xa[i][3]), "r"(wb[j >> 1][(j & 1) * 2]), "r"(wb[j >> 1][(j & 1) * 2 + 1]));
+        for (int j = 0; j < 4; ++j) {
+          float p[4];
+          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                       : "=f"(p[0]), "=f"(p[1]), "=f"(p[2]), "=f"(p[3])
+                       : "r"(xa[i][0]), "r"(xa[i][1]), "r"(xa[i][2]), "r"(xa[i][3]), "r"(wb[j >> 1][(j & 1) * 2]), "r"(wb[j >> 1][(j & 1) * 2 + 1]),
+                         "f"(0.f));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) c[i][j][e] += p[e];
+        }
     }
   }
-  TO* out = (TO*)a.out + (size_t)b * a.o_batch;
+  __nv_bfloat16* out = (__nv_bfloat16*)a.out + (size_t)b * a.o_batch;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -255,13 +262,12 @@ gemm_batched_mma_kernel(BatchedArgs a) {
             y[e] *= 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.value_gate)[(size_t)m * a.gate_stride + (size_t)b * a.N + n + e])));
           y[e] *= gate;
         }
-        TO* o = out + (size_t)m * a.ldo + n;
-        if (n + 1 < a.N && ((uintptr_t)o % (2 * sizeof(TO))) == 0) {
-          if constexpr (sizeof(TO) == 2) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(y[0], y[1]);
-          else *reinterpret_cast<float2*>(o) = make_float2(y[0], y[1]);
+        __nv_bfloat16* o = out + (size_t)m * a.ldo + n;
+        if (n + 1 < a.N && ((uintptr_t)o % 4) == 0) {
+          *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(y[0], y[1]);
         } else {
-          if (n < a.N) o[0] = mi::from_float<TO>(y[0]);
-          if (n + 1 < a.N) o[1] = mi::from_float<TO>(y[1]);
+          if (n < a.N) o[0] = __float2bfloat16_rn(y[0]);
+          if (n + 1 < a.N) o[1] = __float2bfloat16_rn(y[1]);
         }
       }
     }
@@ -310,14 +316,13 @@ MI_API int mi_gemm_batched(void* out, int out_dtype, const void* x, const void* 
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
   MI_REQUIRE(grid.y <= 65535, "gemm_batched: M=%d is too large for one launch", M);
   // rows that start on 16-byte boundaries and hold whole 16 bytes; the others keep the FMA kernel
-  const bool whole = dtype == MI_BF16 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && x_batch % 8 == 0 && w_batch % 8 == 0 &&
+  const bool whole = dtype == MI_BF16 && out_dtype == MI_BF16 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && x_batch % 8 == 0 && w_batch % 8 == 0 &&
                      ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0;
-  if (whole && (out_dtype == MI_BF16 || out_dtype == MI_F32)) {
+  if (whole) {
     constexpr size_t smem = (size_t)TSTAGES * 2 * 64 * LDS * sizeof(__nv_bfloat16);
-    auto kernel = out_dtype == MI_BF16 ? gemm_batched_mma_kernel<__nv_bfloat16> : gemm_batched_mma_kernel<float>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_batched_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return mi_fail("gemm_batched: %zu bytes of shared memory were refused", smem);
-    mi::launch(kernel, grid, dim3(128), smem, stream, a);
+    mi::launch(gemm_batched_mma_kernel, grid, dim3(128), smem, stream, a);
     MI_LAUNCH_OK("gemm_batched");
     return 0;
   }

@@ -504,8 +504,8 @@ def linear_batched(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, bias: Op
                    row_gate: Optional[torch.Tensor] = None, value_gate: Optional[torch.Tensor] = None) -> None:
   """out[:, b, :] = x[:, b, :] @ w[b]^T for ``x [M, batch, K]``, ``w [batch, N, K]``, ``out [M, batch, N]`` - views whose
   strides may be anything as long as the last axis is contiguous (the heads of a token's row, a column range of a
-  row); float32 sums, k ascending.  bfloat16 with more than 16 rows and nothing but a gate a value behind the product: one
-  strided batched library product, the gate in a kernel behind it.
+  row); float32 sums, k ascending except on the tensor cores (bfloat16 rows that can be read 16 bytes at a time).  bfloat16 with more
+  than 16 rows and nothing but a gate a value behind the product: one strided batched library product, the gate in a kernel behind it.
   ``bias [N]`` float32 is added, ``softplus`` applied, and with ``row_gate [M, >= batch]``
   (one logit per row and batch) or ``value_gate [M, batch * N]`` (one per output value) the result is multiplied with its sigmoid."""
   lib = common_lib()

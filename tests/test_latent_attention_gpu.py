@@ -58,10 +58,27 @@ def test_per_head_products_of_many_rows(M, N, K, B, gate, dtype):
     want = torch.nn.functional.softplus(z + bias.double())
   else:
     want = z * torch.sigmoid(logits.double()[:, :B].unsqueeze(2) if gate == "row" else logits.double().view(M, B, N))
-  # products are exact in float32; K additions of truncated float32 and, in bfloat16, one rounding of the result - two where the library's
+  # products are exact in float32; K additions and, in bfloat16, one rounding of the result - two where the library's
   # product is gated by a pass of its own
   bound = K * 2.0 ** -23 * size + (2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -20) * want.abs() + 1e-6
   assert ((out.double().cpu() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("M,N,K,B", [(64, 64, 192, 2), (65, 70, 4096, 1)])
+def test_per_head_products_into_float32_add_in_order(M, N, K, B):
+  from miniinfer_b200.kernels import ops
+  g = torch.Generator().manual_seed(K)
+  x, w = torch.randn((M, B, K + 8), generator=g).to(torch.bfloat16).to(DEV), torch.randn((B, N, K), generator=g).to(torch.bfloat16).to(DEV)
+  outs = []
+  for lead in (0, 1):      # rows on 16-byte boundaries, and rows that can only be read a value at a time
+    store = torch.zeros((M, B, K + 8), dtype=torch.bfloat16, device=DEV)
+    store[:, :, lead:lead + K] = x[:, :, :K]
+    outs.append(torch.empty((M, B, N), device=DEV))
+    ops.linear_batched(outs[-1], store[:, :, lead:lead + K], w)
+  assert torch.equal(outs[0], outs[1])
+  want = torch.einsum("mbk,bnk->mbn", x[:, :, :K].double(), w.double())
+  # a chain of K rounded additions: half an ulp each, of partial sums that grow like a random walk: below sqrt(K) 2^-24 of the norm
+  assert (outs[0].double() - want).norm() <= K ** 0.5 * 2.0 ** -24 * want.norm()
 
 
 def test_float32_norms_do_not_depend_on_how_many_tokens_share_the_step():
