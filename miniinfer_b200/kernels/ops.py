@@ -1425,7 +1425,7 @@ def latent_attention(out: torch.Tensor, q: torch.Tensor, kv_layer: torch.Tensor,
   [tokens, num_heads * head_dim]``, ``out [tokens, num_heads * out_hd]``."""
   page_size = kv_layer.shape[3]
   if not (q.is_cuda and q.dtype == torch.bfloat16 and q.shape[1] == num_heads * head_dim and head_dim % 16 == 0 and 64 <= head_dim <= 256
-          and out_hd % 8 == 0 and page_size % 64 == 0 and q.is_contiguous() and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
+          and scale > 0 and out_hd % 8 == 0 and page_size % 64 == 0 and q.is_contiguous() and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
           and kv_layer.data_ptr() % 16 == 0):
     attention(out, q, kv_layer, block_table, batch, num_heads, 1, head_dim, scale, window, sink=sink, out_hd=out_hd)
     return
@@ -1443,6 +1443,8 @@ def latent_attention(out: torch.Tensor, q: torch.Tensor, kv_layer: torch.Tensor,
       status = batch.scratch.zeros("attention_prefill_status", 1, torch.int32)
     else:
       status = torch.zeros(1, dtype=torch.int32, device=q.device)
+  if sink is not None and (sink.shape != (num_heads,) or sink.dtype != torch.float32):
+    raise KernelError("latent_attention: the sinks must be one float32 per query head")
     _check(lib, lib.mi_attention_prefill_latent(
       _ptr(out), *maps, _ptr(block_table, torch.int32), block_table.shape[1],
       _ptr(batch.prefill_tiles, torch.int32), batch.num_prefill_tiles, _ptr(batch.q_start, torch.int32), _ptr(batch.q_len, torch.int32),
@@ -1451,7 +1453,7 @@ def latent_attention(out: torch.Tensor, q: torch.Tensor, kv_layer: torch.Tensor,
     if batch.scratch is None and int(status[0]) != 0:
       raise KernelError("attention_prefill_latent: a bounded wait on a barrier ran out")
   if decode:
-    span = min(batch.max_ctx_len, win) if win else batch.max_ctx_len
+    span = min(batch.max_ctx_len, abs(win)) if win else batch.max_ctx_len
     chunk = latent_decode_chunk(batch.num_decode * -(-num_heads // 128), span, _num_sms(q.device))
     max_splits = -(-span // chunk) + 1
     n = batch.num_decode * max_splits * num_heads * (out_hd + 2)

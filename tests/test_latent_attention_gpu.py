@@ -140,6 +140,19 @@ def test_rows_that_no_token_may_see_change_nothing(case, bad):
   assert torch.equal(got[:untouched], want[:untouched]) and not torch.isfinite(got[at:n].float()).all()
 
 
+def test_what_latent_attention_does_not_take_goes_to_attention_or_is_refused():
+  from miniinfer_b200.kernels import ops
+  qkv, kv, bt, batch = make_attention_case([(300, 40), (129, 1)], 16, 1, 224, 64, torch.bfloat16, seed=2)
+  q = qkv[:, :16 * 224].contiguous()
+  kv[:, 1] = kv[:, 0]
+  got, want = torch.empty((2, q.shape[0], 16 * 192), dtype=torch.bfloat16, device=DEV)
+  ops.latent_attention(got, q, kv, bt, batch, 16, 224, -0.05, None, None, 192)      # a scale that turns the maximum around
+  ops.attention(want, q, kv, bt, batch, 16, 1, 224, -0.05, None, out_hd=192)
+  assert torch.equal(got, want)
+  with pytest.raises(ops.KernelError, match="sinks"):
+    ops.latent_attention(got, q, kv, bt, batch, 16, 224, 0.05, None, torch.zeros(3, device=DEV), 192)
+
+
 # The result's own rounding to bfloat16 leaves 1.66e-3 of the norm.  Prompts: weights rounded relative to their row's maximum, divided by
 # their own sum, leave 1.72e-3 in all where scores have a standard deviation of 4 (relative to a lagging maximum and divided by
 # the sum of unrounded weights: 2.07e-3).  Decode tokens: weights in two parts leave 1.66e-3 (in one part 1.80e-3).
