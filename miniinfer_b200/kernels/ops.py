@@ -1385,7 +1385,7 @@ def attention(out: torch.Tensor, qkv: torch.Tensor, kv_layer: torch.Tensor, bloc
     _attention_bf16(out, qkv, kv_layer, block_table, batch, num_heads, num_kv_heads, head_dim, scale, win, page_size, opts)
     return
   lib = common_lib()
-  if (qkv.dtype == torch.float32 and not force_generic and T <= 65535 and head_dim % 4 == 0 and head_dim <= 256 and num_heads <= 32 * num_kv_heads
+  if (qkv.dtype == torch.float32 and not force_generic and head_dim % 4 == 0 and head_dim <= 256 and num_heads <= 32 * num_kv_heads
       and opts.softcap == 0 and score_bias is None and distance is None and qkv.data_ptr() % 16 == 0 and kv_layer.data_ptr() % 16 == 0
       and qkv.shape[1] % 4 == 0 and batch.decode_items is not None and batch.prefill_tiles is not None):
     # by the model's options alone, never by the step: a row takes the same kernel, and the same order of sums, in every step

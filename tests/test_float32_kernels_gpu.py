@@ -142,3 +142,16 @@ def test_attention_float32_segments_of_scores_that_are_no_numbers(score, with_si
     ops.attention(outs[-1], qkv, kv, bt, batch, nh, nkv, hd, hd ** -0.5, None, force_generic=generic, sink=sink)
   assert torch.equal(torch.isnan(outs[0]), torch.isnan(outs[1])) and bool(torch.isnan(outs[0]).all()) == (score != score)
   assert torch.allclose(outs[0], outs[1], atol=2e-5, equal_nan=True)
+
+
+@pytest.mark.skipif(DEV == "cpu", reason="a step too long for the general kernel's grid")
+def test_attention_float32_of_more_tokens_than_a_grid_dimension():
+  from gpu_helpers import make_attention_case
+  from miniinfer_b200.kernels import ops
+  T, nh, hd, P = 65600, 2, 8, 64
+  qkv, kv, bt, batch = make_attention_case([(T, T)], nh, 1, hd, P, torch.float32, seed=4)
+  out = torch.empty(T, nh * hd, device=DEV)
+  ops.attention(out, qkv, kv, bt, batch, nh, 1, hd, hd ** -0.5, 40)
+  tail = torch.empty(150, nh * hd, device=DEV)      # the same rows as the last portion of the request
+  ops.attention(tail, qkv[T - 150:], kv, bt, _batch_of(int(batch.seq_slot[0]), T, 150), nh, 1, hd, hd ** -0.5, 40)
+  assert torch.isfinite(out).all() and torch.equal(out[T - 150:], tail)
