@@ -235,7 +235,9 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, force_skinny: bo
   if M == 0:
     return
   lib = common_lib()
-  if (x.dtype == torch.float32 and x.is_cuda and x.stride(1) == 1 and (x.stride(0) >= K or M == 1)
+  if x.dtype == torch.float32 and not x.is_cuda:
+    _ptr(x)      # says so
+  if (x.dtype == torch.float32 and x.stride(1) == 1 and (x.stride(0) >= K or M == 1)
       and (x.is_contiguous() or (w.dtype == out.dtype == torch.float32 and w.is_contiguous() and out.is_contiguous()))):
     # packed rows or a column range of wider ones: one kernel, so a row's value does not depend on how many rows there are
     _check(lib, lib.mi_gemm_f32(_ptr(out, torch.float32), ctypes.c_void_p(x.data_ptr()), _ptr(w, torch.float32), M, N, K,
@@ -259,9 +261,6 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, force_skinny: bo
         torch.mm(x, _transposed(w), out_dtype=torch.float32, out=out)
         return
     linear_batched(out.unsqueeze(1), x.unsqueeze(1), w.unsqueeze(0))
-    return
-  if x.dtype == torch.float32:
-    _check(lib, lib.mi_gemm_f32(_ptr(out, torch.float32), _ptr(x), _ptr(w, torch.float32), M, N, K, K, N, _stream()))
     return
   if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
     raise KernelError(f"linear: operands must both be float32 or both bfloat16, got {x.dtype} and {w.dtype}")
