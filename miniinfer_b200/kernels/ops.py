@@ -1431,6 +1431,8 @@ def latent_attention(out: torch.Tensor, q: torch.Tensor, kv_layer: torch.Tensor,
   if (out.shape != (q.shape[0], num_heads * out_hd) or out.dtype != q.dtype or kv_layer.dtype != q.dtype or not 0 < out_hd <= head_dim
       or kv_layer.shape[1:] != (2, 1, page_size, head_dim)):
     raise KernelError("latent_attention: shapes or dtypes do not match")
+  if sink is not None and (sink.shape != (num_heads,) or sink.dtype != torch.float32):
+    raise KernelError("latent_attention: the sinks must be one float32 per query head")
   win, sinks = int(window) if window else 0, _ptr(sink, torch.float32) if sink is not None else _ptr(None)
   prefill = batch.num_prefill_tiles and batch.prefill_tiles is not None and os.environ.get("MINIINFER_B200_PREFILL_TC", "1") != "0"
   decode = batch.num_decode and os.environ.get("MINIINFER_B200_DECODE_TMA", "1") != "0"
@@ -1442,8 +1444,6 @@ def latent_attention(out: torch.Tensor, q: torch.Tensor, kv_layer: torch.Tensor,
       status = batch.scratch.zeros("attention_prefill_status", 1, torch.int32)
     else:
       status = torch.zeros(1, dtype=torch.int32, device=q.device)
-  if sink is not None and (sink.shape != (num_heads,) or sink.dtype != torch.float32):
-    raise KernelError("latent_attention: the sinks must be one float32 per query head")
     _check(lib, lib.mi_attention_prefill_latent(
       _ptr(out), *maps, _ptr(block_table, torch.int32), block_table.shape[1],
       _ptr(batch.prefill_tiles, torch.int32), batch.num_prefill_tiles, _ptr(batch.q_start, torch.int32), _ptr(batch.q_len, torch.int32),
