@@ -659,8 +659,8 @@ def gated_delta(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Te
   one decay a head.  All operands may be column ranges of wider rows.  Three launches: what
   does not depend on the state for all tokens at once, the recurrence, the read-outs' norm and gate; float32 scratch
   between them from ``workspace`` (a ``Workspace``; made here if absent).  A bfloat16 step of long prompt portions walks
-  each request's tokens in stretches side by side (``csrc/recurrent.cu``); a float32 step walks them in order, so that its
-  sums do not depend on how a request was cut."""
+  each request's tokens a chunk at a time (``csrc/chunked_state.cu``) or, with heads that the chunks do not take, in stretches side
+  by side (``csrc/recurrent.cu``); a float32 step walks them in order, so that its sums do not depend on how a request was cut."""
   lib = common_lib()
   T = v.shape[0]
   head_decay = dt_bias.shape == (heads,)
@@ -711,10 +711,21 @@ LINEAR_SEGMENTED_MAX_ITEMS = 8     # steps of at most this many requests run lon
 LINEAR_SEGMENTED_MAX_BLOCKS = 256
 
 
+LONGEST_PORTION = "longest_portion"      # the entry of a step's work keys that holds the class of its longest portion
+
+
+def longest_portion_class(longest: int) -> int:
+  """The most new tokens of a step's requests, as far as launches depend on them: the greatest of the bounds from which a
+  recurrence goes by chunks that it reaches, or 0."""
+  return max((b for b in (LINEAR_CHUNK_MIN_TOKENS, DELTA_CHUNK_MIN_TOKENS) if longest >= b), default=0)
+
+
 def _state_chunks(lib, v: torch.Tensor, ctx, heads: int, dim: int, vdim: int, workspace, min_tokens: int, delta: bool):
-  """(scratch, launches) of the walk by chunks of tokens of a step that may bring a request ``min_tokens`` new tokens, or
-  (None, 0): a float32 step, a step of short portions, sizes that the chunks do not take."""
-  if v.dtype != torch.bfloat16 or v.shape[0] - ctx.num_items + 1 < min_tokens or os.environ.get("MINIINFER_B200_DELTA_CHUNKS", "1") == "0":
+  """(scratch, launches) of the walk by chunks of tokens of a step that brings a request ``min_tokens`` new tokens - or may bring
+  them, where the step's keys do not tell -, or (None, 0): a float32 step, a step of short portions, sizes that the chunks do not take."""
+  known = getattr(ctx, "work_key", {}).get(LONGEST_PORTION)
+  longest = known[0] if known else v.shape[0] - ctx.num_items + 1
+  if v.dtype != torch.bfloat16 or longest < min_tokens or os.environ.get("MINIINFER_B200_DELTA_CHUNKS", "1") == "0":
     return None, 0
   lib.mi_chunked_state_floats.restype = ctypes.c_longlong
   m = int(lib.mi_chunked_state_floats(v.shape[0], ctx.num_items, heads, dim, vdim, int(delta)))
@@ -737,7 +748,8 @@ def linear_attention(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: tor
   silu or sigmoid, ``norm_weight [vdim]`` optional.  ``q``, ``k`` ``[T, heads * dim]`` are first rotated by the token's position
   (``rope [positions, rot_dims]``, cos then sin; value i with value i + rot_dims / 2) and scaled.  ``q``, ``k``, ``v``, ``gate``
   and ``out`` may be column ranges of wider rows.  Three launches; a bfloat16 step of long prompt portions walks each
-  request's tokens in stretches side by side (five launches), a float32 step always in order."""
+  request's tokens a chunk at a time or, with heads that the chunks do not take, in stretches side by side (five launches), a
+  float32 step always in order."""
   lib = common_lib()
   T = v.shape[0]
   if (q.shape != (T, heads * dim) or k.shape != q.shape or v.shape != (T, heads * vdim) or gate.shape != v.shape or out.shape != v.shape

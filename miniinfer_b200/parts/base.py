@@ -87,6 +87,10 @@ class HostStep:
     """Indices of the items that bring exactly one token."""
     return np.flatnonzero(self.q_len == 1).astype(np.int32)
 
+  def longest_portion(self) -> int:
+    """The most new tokens of an item."""
+    return int(self.q_len.max()) if len(self.q_len) else 0
+
   def longest_decode_context(self) -> int:
     """The largest length, this step's token included, among the items that bring one token (0: none)."""
     one = self.q_len == 1

@@ -20,14 +20,14 @@ their logarithms, the state, the sums over it and the norm are float32 whatever 
 
 from __future__ import annotations
 
-from typing import Dict, Optional, Sequence
+from typing import Dict, List, Optional, Sequence
 
 import torch
 
 from ..cache.specs import CacheSpec, FixedStateSpec
 from ..kernels import ops
-from .base import Mixer, ParamSpec, Piece, PositionEncoding, whole
-from .recurrent import _state_rows
+from .base import Mixer, ParamSpec, Piece, PositionEncoding, StepWork, whole
+from .recurrent import LongestPortion, _state_rows
 
 
 class LinearAttentionMixer(Mixer):
@@ -98,6 +98,9 @@ class LinearAttentionMixer(Mixer):
       raise ValueError(f"{self.name}: the rotary encoding covers {rotary} values, more than dim={self.dim}")
     if dtype == torch.bfloat16 and self.hidden_size % 8:
       raise ValueError(f"{self.name}: width={self.hidden_size} must be a multiple of 8 in bfloat16 (rows are read 16 bytes at a time)")
+
+  def step_work(self) -> List[StepWork]:
+    return [LongestPortion()]
 
   def forward(self, x: torch.Tensor, ctx, cache) -> torch.Tensor:
     T = x.shape[0]

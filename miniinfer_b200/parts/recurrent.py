@@ -7,19 +7,33 @@ so steps of these mixers are replayed from CUDA graphs like steps of attention.
 
 from __future__ import annotations
 
-from typing import Dict, Optional
+from typing import Dict, List, Optional
 
+import numpy as np
 import torch
 
 from ..cache.specs import CacheSpec, FixedStateSpec
 from ..kernels import ops
-from .base import Mixer, ParamSpec, Piece, whole
+from .base import HostStep, Mixer, ParamSpec, Piece, StepWork, whole
 
 
 def _state_rows(cache, name: str) -> torch.Tensor:
   if cache.kind != "state":
     raise RuntimeError(f"{name}: a recurrent mixer needs a per-request state, got a cache of kind {cache.kind!r}")
   return cache.tensor
+
+
+class LongestPortion(StepWork):
+  """No list, only a key: whether some request of the step brings enough tokens for a recurrence to go by chunks.  A step of many
+  short portions would else launch the chunks' kernels for nothing (30 requests of 20 tokens: three launches a layer)."""
+
+  name = ops.LONGEST_PORTION
+
+  def build(self, step: HostStep) -> np.ndarray:
+    return np.zeros(0, dtype=np.int32)
+
+  def key(self, step: HostStep) -> tuple:
+    return (ops.longest_portion_class(step.longest_portion()),)
 
 
 class SelectiveScanMixer(Mixer):
@@ -175,6 +189,9 @@ class GatedDeltaMixer(Mixer):
       raise ValueError(f"{self.name}: the convolution takes up to 16 taps, got {self.taps}")
     if self.dim > 4096:
       raise ValueError(f"{self.name}: the delta-rule kernel keeps up to 4096 key channels a head, got dim={self.dim}")
+
+  def step_work(self) -> List[StepWork]:
+    return [LongestPortion()]
 
   def forward(self, x: torch.Tensor, ctx, cache) -> torch.Tensor:
     T = x.shape[0]

@@ -273,3 +273,14 @@ def test_the_attention_work_lists_of_a_step():
   # a step of decode tokens only has neither kind of tile
   only = HostStep(np.ones(3, dtype=np.int32), np.array([5, 6, 7], dtype=np.int32), 4096)
   assert PrefillTiles().build(only).size == 0 and PrefillWideTiles().key(only) == (0,)
+
+
+def test_a_step_of_short_portions_is_told_from_one_with_a_long_portion():
+  """The key by which recurrences go by chunks: the greatest of their bounds that the step's longest portion reaches."""
+  from miniinfer_b200.kernels import ops
+  from miniinfer_b200.parts.base import HostStep
+  from miniinfer_b200.parts.recurrent import LongestPortion
+  low, high = sorted((ops.LINEAR_CHUNK_MIN_TOKENS, ops.DELTA_CHUNK_MIN_TOKENS))
+  for portions, want in (([20] * 30, 0), ([1, low - 1], 0), ([1, low], low), ([high - 1] * 9, low), ([high, 3], high), ([5000], high)):
+    step = HostStep(np.array(portions, dtype=np.int32), np.zeros(len(portions), dtype=np.int32), 8192)
+    assert LongestPortion().key(step) == (want,) and len(LongestPortion().build(step)) == 0, portions
