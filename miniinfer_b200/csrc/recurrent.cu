@@ -801,9 +801,10 @@ MI_API int mi_causal_conv(void* out, int ldo, const void* x, int ldx, int dtype,
   MI_REQUIRE(state_stride >= (long long)(taps - 1) * C, "causal_conv: the state rows are too short");
   if (T == 0) return 0;
   dim3 grid((C + 255) / 256, T), sgrid((C + 255) / 256, items);
-  // eight channels and four tokens a thread where rows start on 16-byte boundaries and there are a million values: 70 tokens of 2048
-  // channels take 3 us a value a thread and 6 this way (a thread's weights alone are 128 bytes)
-  const bool vec = dtype == MI_BF16 && (long long)T * C >= 1 << 20 && taps >= 2 && taps <= 4 && C % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 &&
+  // eight channels and four tokens a thread where rows start on 16-byte boundaries and there are more than half a million values (a
+  // thread's weights alone are 128 bytes).  Four taps, this way / a value a thread, in microseconds: 64 x 2048 6.4 / 4.1, 256 x 2048
+  // 6.5 / 6.5, 64 x 8192 6.7 / 6.5, 384 x 2048 7.7 / 8.3, 192 x 4096 7.7 / 8.3, 128 x 8192 7.7 / 10.2, 2048 x 2048 16.3 / 29.8
+  const bool vec = dtype == MI_BF16 && (long long)T * C > 1 << 19 && taps >= 2 && taps <= 4 && C % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 &&
                    ((uintptr_t)x % 16) == 0 && ((uintptr_t)out % 16) == 0 && ((uintptr_t)w % 8) == 0;
   if (vec) {
     auto kernel = taps == 2 ? causal_conv_vec_kernel<2> : taps == 3 ? causal_conv_vec_kernel<3> : causal_conv_vec_kernel<4>;
