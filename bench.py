@@ -535,7 +535,7 @@ def kernel_case(name: str, reps: int = 3) -> str:
       what = f"{T} tokens ({cuts[0]} of one request), {H} heads of {Dk} x {Dv} on {G} q/k heads"
   elif name == "linear_attention":
     # as the delta rule's case: one prompt portion of 8192 tokens beside seven decode tokens, 16 heads of 128 x 128, a decay per
-    # token and key channel (the walk in order: MINIINFER_B200_LINEAR_SEGMENTS=0 in the environment; else stretches side by side)
+    # token and key channel (MINIINFER_B200_DELTA_CHUNKS=0 in the environment: stretches side by side; MINIINFER_B200_LINEAR_SEGMENTS=0 too: the walk in order)
     from types import SimpleNamespace
     cuts = [8192] + [1] * 7
     T = sum(cuts)

@@ -153,9 +153,9 @@ def test_a_key_far_back_is_read_through_the_state(dtype, channel):
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,D,Dv,channel", [(2, 24, 40, True), (1, 128, 64, True), (3, 64, 32, False)])
 def test_linear_attention_of_long_portions(dtype, H, D, Dv, channel):
-  """Portions of hundreds of tokens: in bfloat16 a request's tokens run in stretches side by side, each from a zero
-  state, and are chained afterwards by the products of their decays; the result is the recurrence's, and the state
-  left behind lets the request go on token by token."""
+  """Portions of hundreds of tokens: in bfloat16 a request's tokens go a chunk of 64 at a time; the result is the
+  recurrence's, and the state left behind lets the request go on token by token.  (Heads that the chunks do not take:
+  ``test_long_portions_of_heads_that_chunks_do_not_take``.)"""
   g = torch.Generator().manual_seed(D + Dv)
   T, eps = 1300, 1e-5
   r = lambda *s: torch.randn(s, generator=g)

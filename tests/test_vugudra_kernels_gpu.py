@@ -173,9 +173,9 @@ def test_gated_delta_rule_against_the_plain_recurrence(dtype, H, G, D, Dv):
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,G,D,Dv", [(2, 1, 24, 40), (1, 1, 128, 64)])
 def test_gated_delta_rule_of_long_portions(dtype, H, G, D, Dv):
-  """Portions of hundreds of tokens: in bfloat16 a request's tokens run in stretches side by side - each from a zero state
-  and, in further columns that start as the identity, as the map of the state it starts from - which are chained
-  afterwards; the result is the recurrence's, and the state left behind lets the request go on token by token."""
+  """Portions of hundreds of tokens: in bfloat16 a request's tokens go a chunk of 64 at a time; the result is the
+  recurrence's, and the state left behind lets the request go on token by token.  (Heads that the chunks do not take:
+  ``test_long_portions_of_heads_that_chunks_do_not_take``.)"""
   from miniinfer_b200.kernels import ops
   g = torch.Generator().manual_seed(D + Dv)
   T, eps = 1300, 1e-5
