@@ -13,11 +13,11 @@
 // M): rows are staged as they lie in memory, K fastest, so that cp.async brings them without a transposition and a 16-byte
 // read of shared memory gives two packed operands; rows of 36 floats keep the eight rows that a warp reads at a time in
 // different banks.  Two forms, both in three stages of 32 columns:
-//   * more than 32 rows: four warps share a tile of 64 x 64 and walk the parts of a group one after the other;
+//   * more than 32 rows: four warps share a tile of 64 x 64 and walk the parts of a group, or of all four, one after the other;
 //   * up to 32 rows: every warp has a tile of its rows x 32 and parts of its own, staged by itself, so that the weights come
 //     in at many places at once; the warps' sums are added up in shared memory.
 // The groups go to the four blocks of a cluster, whose sums are added up in each other's shared memory, in the order that
-// one block would - for few rows only where the tiles alone leave SMs idle.
+// one block would - for few rows only where the tiles alone leave SMs idle, for many from some hundred columns on.
 // Measured on B200, weights in L2, in microseconds, against one form of 64 x 64 tiles, 4 x 4 elements a thread, staged one
 // step at a time: 8 x 4096 x 1024 74 -> 9.4, 16 x 1024 x 2048 146 -> 6.8, 40 x 6144 x 1024 75 -> 28, 302 x 4096 x 1024 174 -> 86,
 // 302 x 1024 x 2048 149 -> 52, 2048 x 4096 x 1024 583 -> 484 (35 of the 70 TFLOP/s that a loop of FMAs alone reaches),
@@ -77,7 +77,7 @@ struct Tile {
 };
 
 // CLUSTER: the block's group is its rank in a cluster of GROUPS blocks.
-template <int TM, bool SHARED, bool CLUSTER, bool VEC>      // (a shared tile's groups always go to a cluster)
+template <int TM, bool SHARED, bool CLUSTER, bool VEC>
 __device__ __forceinline__ void product(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w,
                                         int M, int N, int K, int ldx, int ldo, int m_tile, int n_tile, int rank) {
   using T = Tile<TM, SHARED>;
@@ -89,10 +89,12 @@ __device__ __forceinline__ void product(float* __restrict__ out, const float* __
   float* stages = sm + (SHARED ? 0 : warp * STAGES * T::STAGE);
   const int len = ((K + GROUPS * PARTS - 1) / (GROUPS * PARTS) + BK - 1) / BK * BK;       // columns of a part
   const int per_part = len / BK;
-  // parts that this warp walks: its block's group, or one part of that, or a group
-  const int parts = SHARED || !CLUSTER ? PARTS : 1;
-  const int first = SHARED ? rank * PARTS : (CLUSTER ? rank * PARTS + warp : warp * PARTS);
-  const int begin = first * len, steps = per_part * parts;      // (columns beyond K are staged as zeros)
+  // parts that this warp walks: its block's group, or one part of that, or a group, or all
+  constexpr bool ALL = SHARED && !CLUSTER;
+  const int parts = ALL ? GROUPS * PARTS : SHARED || !CLUSTER ? PARTS : 1;
+  const int first = ALL ? 0 : SHARED ? rank * PARTS : (CLUSTER ? rank * PARTS + warp : warp * PARTS);
+  // a part without columns is +0 and left out (in another, columns beyond K are staged as zeros)
+  const int begin = first * len, steps = per_part * min(parts, max(0, (K - begin + len - 1) / len));
 
   auto stage_w = [&](int s) {
     if (s < steps) stage_rows<BN, MOVERS, VEC>(stages + (s % STAGES) * T::STAGE + BM * LDS, w, n0, N, K, begin + s * BK, K, thread);
@@ -108,11 +110,15 @@ __device__ __forceinline__ void product(float* __restrict__ out, const float* __
   for (int s = 0; s < STAGES - 1; ++s) stage_x(s);
 
   uint64_t acc[TM][TN];
-  float group[TM][TN];
+  float group[TM][TN], total[ALL ? TM : 1][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) { acc[i][j] = 0; group[i][j] = 0.f; }
+    for (int j = 0; j < TN; ++j) {
+      acc[i][j] = 0;
+      group[i][j] = 0.f;
+      if (ALL) total[ALL ? i : 0][j] = 0.f;
+    }
 
   int in_part = 0, part = 0;
   for (int s = 0; s < steps; ++s) {
@@ -142,7 +148,8 @@ __device__ __forceinline__ void product(float* __restrict__ out, const float* __
         for (int j = 0; j < TN; ++j) {
           const float sum = halves(acc[i][j]);
           acc[i][j] = 0;
-          group[i][j] = part == 0 ? sum : group[i][j] + sum;
+          group[i][j] = (ALL ? part % PARTS : part) == 0 ? sum : group[i][j] + sum;
+          if (ALL && (part % PARTS == PARTS - 1 || s + 1 == steps)) total[ALL ? i : 0][j] = part < PARTS ? group[i][j] : total[ALL ? i : 0][j] + group[i][j];
         }
       ++part;
     }
@@ -155,7 +162,15 @@ __device__ __forceinline__ void product(float* __restrict__ out, const float* __
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) mine[(row + 4 * i) * T::LDP + col + 8 * j] = group[i][j];
+    for (int j = 0; j < TN; ++j) mine[(row + 4 * i) * T::LDP + col + 8 * j] = ALL ? total[ALL ? i : 0][j] + 0.f : group[i][j];      // (+ 0: as groups without columns do)
+  if (ALL) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < BM * BN; i += 128) {
+      const int r = i / BN, c = i % BN;
+      if (m0 + r < M && n0 + c < N) out[(size_t)(m0 + r) * ldo + n0 + c] = sm[r * T::LDP + c];
+    }
+    return;
+  }
   if (!CLUSTER) {      // a group a warp
     __syncthreads();
     for (int i = threadIdx.x; i < BM * BN; i += 128) {
@@ -191,10 +206,10 @@ __device__ __forceinline__ void product(float* __restrict__ out, const float* __
   cluster.sync();      // nobody leaves while its sums are read
 }
 
-template <int TM, bool VEC>
+template <int TM, bool SHARED, bool VEC>
 __global__ void __launch_bounds__(128)
 gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w, int M, int N, int K, int ldx, int ldo) {
-  product<TM, false, false, VEC>(out, x, w, M, N, K, ldx, ldo, blockIdx.y, blockIdx.x, 0);
+  product<TM, SHARED, false, VEC>(out, x, w, M, N, K, ldx, ldo, blockIdx.y, blockIdx.x, 0);
 }
 
 template <int TM, bool SHARED, bool VEC>
@@ -208,20 +223,27 @@ int launch_tiles(float* out, const float* x, const float* w, int M, int N, int K
   using T = Tile<TM, SHARED>;
   const int m_tiles = (M + T::BM - 1) / T::BM, n_tiles = (N + T::BN - 1) / T::BN;
   MI_REQUIRE(m_tiles <= 65535, "gemm_f32: M=%d is too large for one launch", M);
-  auto whole = gemm_f32_kernel<TM, VEC>;
+  auto whole = gemm_f32_kernel<TM, SHARED, VEC>;
   auto groups = gemm_f32_groups_kernel<TM, SHARED, VEC>;
   static bool ready[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !ready[dev]) {
-    if ((!SHARED && cudaFuncSetAttribute(whole, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM) != cudaSuccess) ||
+    if (cudaFuncSetAttribute(whole, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(groups, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM) != cudaSuccess)
       return mi_fail("gemm_f32: %zu bytes of shared memory were refused", T::SMEM);
     if (dev >= 0 && dev < 64) ready[dev] = true;
   }
+  // Few columns: a block walks all parts of a shared tile itself, for a cluster's blocks would wait longer for one another than
+  // they work (`alone`, below).  In microseconds, walked / in clusters: 40 x 1024 x 128 7.6 / 8.8, x 192 10.7 / 8.8; 300 x 1024
+  // x 64 4.6 / 9.7, x 256 14.0 / 15.9, x 384 20.1 / 16.3; 40 x 4096 x 256 13.9 / 15.4; 300 x 4096 x 384 46 / 49, x 512 60 / 50; 2048 x
+  // 1024 x 384 58 / 73, x 512 75 / 73; 2048 x 4096 x 64 41 / 144, x 384 196 / 273.  (64 x 64 tiles before: 300 x 1024 x 64 5.9, 2048 x
+  // 4096 x 64 41.5, x 384 222.)
   // Few rows: from a tile for every SM on, a block walks a tile's groups itself (24 x 6144 x 1024, 192 tiles: 21.5 us against
   // 22.4 with clusters; 8 x 151936 x 1024: 120 against 206).  Shared tiles are better off in clusters at any size (2048 x 4096 x
   // 1024: 484 against 499; 302 x 4096 x 1024: 86 against 121), whose smaller blocks fill the SMs more evenly.
-  if (!SHARED && n_tiles >= mi::sm_count())
+  const long long tiles = (long long)m_tiles * n_tiles;
+  const bool alone = K <= 128 || (K <= 256 && tiles >= 64) || (K <= 384 && tiles >= 320);
+  if (SHARED ? alone : n_tiles >= mi::sm_count())
     mi::launch(whole, dim3(n_tiles, m_tiles), dim3(128), T::SMEM, stream, out, x, w, M, N, K, ldx, ldo);
   else
     mi::launch(groups, dim3(GROUPS * n_tiles, m_tiles), dim3(128), T::SMEM, stream, out, x, w, M, N, K, ldx, ldo);
@@ -231,6 +253,9 @@ int launch_tiles(float* out, const float* x, const float* w, int M, int N, int K
 
 template <bool VEC>
 int launch_rows(float* out, const float* x, const float* w, int M, int N, int K, int ldx, int ldo, cudaStream_t stream) {
+  // Few rows of few columns against many weights go by shared tiles too: 8 x 4096 x 64 4.6 us so and 5.8 by tiles of few rows, 24 x 4096
+  // x 128 8.0 and 10.5 (8 x 4096 x 128 8.0 and 6.0; 8 x 1024 x 64 4.4 and 2.9, 24 x 1024 x 64 4.4 and 4.3)
+  if (N >= 4096 && K <= (M > 16 ? 128 : 64)) return launch_tiles<8, true, VEC>(out, x, w, M, N, K, ldx, ldo, stream);
   if (M <= 8) return launch_tiles<2, false, VEC>(out, x, w, M, N, K, ldx, ldo, stream);
   if (M <= 16) return launch_tiles<4, false, VEC>(out, x, w, M, N, K, ldx, ldo, stream);
   if (M <= 32) return launch_tiles<8, false, VEC>(out, x, w, M, N, K, ldx, ldo, stream);

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.skipif(DEV == "cpu", reason="the order of a CUDA kernel's sums")
-@pytest.mark.parametrize("N,K", [(31, 5), (33, 64), (160, 513), (4800, 36), (70, 2052)])      # 4800 columns: a tile for every SM
+@pytest.mark.parametrize("N,K", [(31, 5), (33, 64), (160, 513), (4800, 36), (70, 2052), (96, 128), (64, 200), (40, 1000)])      # 4800 columns: a tile for every SM
 @pytest.mark.parametrize("lead", [0, 3])      # columns of a wider row in front of the operand: rows that do not start on 16 bytes
 def test_linear_float32_forms_agree(N, K, lead):
   from miniinfer_b200.kernels import ops
