@@ -22,11 +22,15 @@
 // scratch than SLAB_UNITS (chunk, head) pairs is worked through in slabs, the state row carrying over.
 //
 // Every product runs on the tensor cores (mma.sync m16n8k8) with each float32 operand as the sum of two tf32 numbers and
-// three of the four partial products, 22 bits of every operand: as FMAs they were bound by the reads of shared memory that
+// three of the four partial products, added up in float32: as FMAs they were bound by the reads of shared memory that
 // feed them.  tcgen05 has no use here: the chain of chunks is latency, and its operands are made in registers.  Against
-// float64 the state errs by 1.6e-7 to 5.6e-7 of its norm after 700 and 2048 tokens; walked in order, by 1.2e-7 to 8.2e-7.
-// Measured on B200, one request of 2048 tokens, 8 heads of 128 x 128, one decay a key channel: 159 us (build 41, state 95, out
-// 22) where stretches side by side took 1041; 16 heads with one decay a head 215 us, 251 by FMA kernels.
+// float64 the state errs, in parts of its norm, after 2048 tokens of 8 heads of 128 x 128 (in brackets what did these steps before:
+// the walk in stretches, and for the delta rule with one decay a head chunks of FMAs): delta rule, decays a channel about 1 / 50 a
+// token 1.9e-7 (3.5e-7), 1 / 3000 3.2e-7 (3.4e-6), stronger than 1 / 2 1.4e-7 (0.7e-7); a head 1.6e-7 (2.4e-7), 2.3e-7 (4.2e-7), 1.3e-7
+// (0.9e-7); linear attention 1.3e-7 (1.7e-7), 4.7e-7 (1.3e-5), 0.65e-7 (0.3e-7).
+// Measured on B200, one request of 2048 tokens, 8 / 16 / 32 heads of 128 x 128, the whole operation in microseconds: delta rule with
+// one decay a key channel 193, 284, 494 (in stretches 1017, 1204, 1254), one a head 188, 270, 473 (chunks of FMAs 208, 296, 586), linear
+// attention 126, 188, 345 (in stretches 173, 281, 476).
 #include "chunked_state.cuh"
 
 namespace mi {
@@ -43,13 +47,13 @@ __host__ __device__ inline int pad(int x, int m) { return (x + m - 1) / m * m; }
 
 struct Args : ChunkedStateArgs {
   int dp, vp;                          // dim padded to 32, vdim padded to 32
-  // per (chunk, head): W [C][dp] and U0 / U [C][vp] (delta rule), A [C][C], K^ and Q~ [C][dp], S_0 [dp][vp], P_C [dp]
+  // per (chunk, head): W [C][dp] and U0 / U [C][vp] (delta rule), A [C][C], K^ and Q~ [C][dp], S_0 [dp][vp], P_C and what its rounding leaves [2][dp]
   float *w, *u, *at, *kh, *qt, *s0, *pc;
   int c0, c1;                          // the slab's chunks
 };
 
 __host__ __device__ inline long long unit_floats(int dp, int vp, bool delta) {
-  return (delta ? (long long)C * (dp + vp) : 0) + C * C + 2ll * C * dp + (long long)dp * vp + dp;
+  return (delta ? (long long)C * (dp + vp) : 0) + C * C + 2ll * C * dp + (long long)dp * vp + 2 * dp;
 }
 
 // The item that chunk number c (over the items that are long enough) belongs to and the chunk's place in it; item -1: none.
@@ -101,23 +105,35 @@ __device__ __forceinline__ bool any_not_finite(const float (&v)[N]) {
   for (int i = 0; i < N; ++i) bad |= !(fabsf(v[i]) <= 3.402823466e38f);
   return __any_sync(0xffffffffu, bad);
 }
-__device__ __forceinline__ void mma1(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+__device__ __forceinline__ void mma1(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, const float (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %12, %13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
-// c += a b for a 16 x 8 operand (rows g and g + 8, columns t and t + 4) and an 8 x 8 one (rows t and t + 4, column g), g = lane / 4,
-// t = lane % 4; c: row g columns 2 t and 2 t + 1, then row g + 8.  The small partial products first.
-__device__ __forceinline__ void mma3(float (&c)[4], const Two (&a)[4], const Two (&b)[2]) {
-  mma1(c, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
-  mma1(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
-  mma1(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
-}
-// The same with the small partial products in sums of their own, so that a chain of products is half as long.
-__device__ __forceinline__ void mma3(float (&c)[4], float (&small)[4], const Two (&a)[4], const Two (&b)[2]) {
-  mma1(small, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
-  mma1(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
-  mma1(small, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
+// A sum of products in two parts: the products of the upper parts of the operands, and those with a lower part, which are 2^-11 of them.
+struct Sum {
+  float c[4], small[4];
+  __device__ __forceinline__ Sum() {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[e] = small[e] = 0.f;
+  }
+  __device__ __forceinline__ float at(int e) const { return c[e] + small[e]; }
+};
+// s += a b for a 16 x 8 operand (rows g and g + 8, columns t and t + 4) and an 8 x 8 one (rows t and t + 4, column g), g = lane / 4,
+// t = lane % 4; s: row g columns 2 t and 2 t + 1, then row g + 8.  The tensor core cuts its accumulator off towards zero at every
+// product, so only the small products are carried on in it: eight products of upper parts - 22 bits each, exact - start from zero and
+// join the sum in a rounded addition.  (All carried on, read-outs of 2048 tokens erred by 1.1e-6 of their norm; so by 2.6e-7, and the walk
+// in order by 2.5e-7.  The fourth product costs 10 % and takes 2 % off that.)
+__device__ __forceinline__ void mma3(Sum& s, const Two (&a)[4], const Two (&b)[2]) {
+  const float zero[4] = {0.f, 0.f, 0.f, 0.f};
+  float p[4];
+  mma1(s.small, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi, s.small);
+  mma1(s.small, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo, s.small);
+  mma1(p, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi, zero);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    s.c[e] += p[e];
+  }
 }
 // The 16 x 8 operand of a row-major tile.
 __device__ __forceinline__ void load_a(Two (&a)[4], const float* p, int ld, int g, int t) {
@@ -157,7 +173,7 @@ __device__ __forceinline__ void load_b(Two (&b)[2], const uint2* p, int ld, int 
 
 constexpr int LDT = C + 4;             // a row of the inverse
 struct BuildLayout {                   // float offsets
-  int ld, k, q, g, total, diag, beta, floats;
+  int ld, k, q, g, total, diag, beta, rest, f, floats;
   __host__ __device__ explicit BuildLayout(int dp) {
     ld = dp + 4;
     k = 0;                                                            // [C][ld] keys; E k; then the values, VT columns at a time
@@ -166,7 +182,9 @@ struct BuildLayout {                   // float offsets
     total = g + C * ld;                                               // [NB][dp] a block's whole product
     diag = total + NB * dp;                                           // [NB][64] products inside a block: 36 of q, 28 of k
     beta = diag + NB * 64;                                            // [C]
-    floats = beta + C;
+    rest = beta + C;                                                  // [NB][dp] one decay a channel: what the rounding of the block's product leaves
+    f = rest + NB * dp;                                               // one decay a head: F [C], E [C], a block's product [NB], as doubles [NB]
+    floats = f + 2 * C + 3 * NB;
   }
 };
 
@@ -214,7 +232,7 @@ chunk_build_kernel(Args a) {
         if (a.decay == CHUNK_DECAY_CHANNEL) {
           x = ld4(a.g + ((size_t)(row0 + t) * a.heads + head) * a.dim + d);
         } else {
-          const float y = a.decay == CHUNK_DECAY_HEAD ? a.g[(size_t)(row0 + t) * a.heads + head] : a.g[head];
+          const float y = a.decay == CHUNK_DECAY_HEAD ? expf(a.g[(size_t)(row0 + t) * a.heads + head]) : a.g[head];
           x = make_float4(y, y, y, y);
         }
       }
@@ -223,6 +241,32 @@ chunk_build_kernel(Args a) {
     if (DELTA && tid < C) bt[tid] = tid < n ? a.beta[(size_t)(row0 + tid) * a.heads + head] : 0.f;
   }
   copies_begun();
+  // One decay a head: F, E and the blocks' products are sums of logarithms (a constant's: products) in double, rounded once.  A constant's
+  // float products err alike in every chunk, and logarithms of decays near one hold digits that the decays do not.
+  const bool per_head = a.decay != CHUNK_DECAY_CHANNEL, logs = a.decay == CHUNK_DECAY_HEAD;
+  float* fs = sm + at.f;
+  double* whole = reinterpret_cast<double*>(fs + 2 * C + NB);
+  if (per_head && tid < NB) {
+    double x[8], sum = logs ? 0. : 1.;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int t = 8 * tid + j;
+      x[j] = t >= n ? sum : (double)a.g[logs ? (size_t)(row0 + t) * a.heads + head : head];
+    }
+    double f = sum;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      f = logs ? f + x[j] : f * x[j];
+      fs[8 * tid + j] = logs ? expf((float)f) : (float)f;
+    }
+    whole[tid] = f;
+    fs[2 * C + tid] = logs ? expf((float)f) : (float)f;
+#pragma unroll
+    for (int j = 7; j >= 0; --j) {
+      fs[C + 8 * tid + j] = logs ? expf((float)sum) : (float)sum;
+      sum = logs ? sum + x[j] : sum * x[j];
+    }
+  }
   copies_done<0>();
   __syncthreads();
 
@@ -258,16 +302,29 @@ chunk_build_kernel(Args a) {
   // E k, F q and F k over the keys, queries and decays, a thread eight tokens of a block in a channel
   for (int i = tid; i < NB * dp; i += THREADS) {
     const int b = i / dp, d = i % dp;
-    float gv[8], kv[8], f = 1.f;
+    float gv[8], kv[8], f = 1.f, rest = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) { gv[j] = gs[(8 * b + j) * ld + d]; kv[j] = ks[(8 * b + j) * ld + d]; }
+    if (per_head) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        qs[(8 * b + j) * ld + d] *= fs[8 * b + j];
+        gs[(8 * b + j) * ld + d] = fs[8 * b + j] * kv[j];
+        ks[(8 * b + j) * ld + d] = fs[C + 8 * b + j] * kv[j];
+      }
+      total[b * dp + d] = fs[2 * C + b];
+      continue;
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+      const float before = f;
       f *= gv[j];
+      rest = fmaf(rest, gv[j], fmaf(before, gv[j], -f));
       qs[(8 * b + j) * ld + d] *= f;
       gs[(8 * b + j) * ld + d] = f * kv[j];
     }
     total[b * dp + d] = f;
+    sm[at.rest + b * dp + d] = rest;
     f = 1.f;
 #pragma unroll
     for (int j = 7; j >= 0; --j) {
@@ -278,11 +335,18 @@ chunk_build_kernel(Args a) {
   __syncthreads();
   // Between blocks: warp I has the rows of its block - eight of F k above eight of F q - and every earlier block's E k, times the
   // products of the blocks between
-  float acc[NB - 1][4];
+  Sum acc[NB - 1];
+  if (warp == 0 && per_head) {      // P_C and what its rounding leaves
+    double p = logs ? 0. : 1.;
 #pragma unroll
-  for (int j = 0; j < NB - 1; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+    for (int b = 0; b < NB; ++b) p = logs ? p + whole[b] : p * whole[b];
+    if (logs) p = exp(p);
+    const float high = (float)p, low = (float)(p - (double)high);
+    for (int d = lane; d < dp; d += 32) {
+      a.pc[unit * 2 * dp + d] = high;
+      a.pc[unit * 2 * dp + dp + d] = low;
+    }
+  }
   if (warp > 0) {
     const float *fk = gs + (8 * warp + g) * ld, *fq = qs + (8 * warp + g) * ld;
     for (int d = 0; d < dp; d += 8) {
@@ -312,7 +376,7 @@ chunk_build_kernel(Args a) {
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
       float x = 0.f, y = 0.f;
-      if (j < warp) { x = acc[j < NB - 1 ? j : 0][2]; y = acc[j < NB - 1 ? j : 0][3]; }
+      if (j < warp) { x = acc[j < NB - 1 ? j : 0].at(2); y = acc[j < NB - 1 ? j : 0].at(3); }
       if (j == warp) {
         x = 2 * t4 <= g ? dq[2 * t4] : 0.f;
         y = 2 * t4 + 1 <= g ? dq[2 * t4 + 1] : 0.f;
@@ -332,7 +396,12 @@ chunk_build_kernel(Args a) {
       a.kh[(unit * C + t) * dp + d] = ks[t * ld + d] * behind;
       a.qt[(unit * C + t) * dp + d] = qs[t * ld + d] * before;
     }
-    if (b == NB - 1) a.pc[unit * dp + d] = before * total[b * dp + d];
+    if (b == NB - 1 && !per_head) {
+      double p = 1.;
+      for (int j = 0; j < NB; ++j) p *= (double)total[j * dp + d] + (double)sm[at.rest + j * dp + d];
+      a.pc[unit * 2 * dp + d] = (float)p;
+      a.pc[unit * 2 * dp + dp + d] = (float)(p - (double)(float)p);
+    }
   }
   if (!DELTA) return;
   __syncthreads();
@@ -359,8 +428,8 @@ chunk_build_kernel(Args a) {
 #pragma unroll
     for (int j = 0; j < NB - 1; ++j) {
       if (j < warp) {
-        lt[(8 * j + 2 * t4) * C + t] = bt[t] * acc[j][0];
-        lt[(8 * j + 2 * t4 + 1) * C + t] = bt[t] * acc[j][1];
+        lt[(8 * j + 2 * t4) * C + t] = bt[t] * acc[j].at(0);
+        lt[(8 * j + 2 * t4 + 1) * C + t] = bt[t] * acc[j].at(1);
       }
     }
     if (2 * t4 < g) lt[(8 * warp + 2 * t4) * C + t] = bt[t] * dk[2 * t4];
@@ -396,7 +465,7 @@ chunk_build_kernel(Args a) {
   __syncthreads();
   {
     const int m = (warp & 1) * 16, c = (warp >> 1) * 8;      // a warp 16 rows x 8 columns of the 32 x 32
-    float x[4] = {0.f, 0.f, 0.f, 0.f};
+    Sum ba;
 #pragma unroll
     for (int k = 0; k < HALF; k += 8) {      // B A^-1, B being L's lower half (kept transposed)
       Two l[4], r[2];
@@ -406,19 +475,20 @@ chunk_build_kernel(Args a) {
       l[2] = Two(p[4 * C]);
       l[3] = Two(p[4 * C + 8]);
       load_b(r, inv + k * LDT + c, LDT, g, t4);
-      mma3(x, l, r);
+      mma3(ba, l, r);
     }
-    st2(inv + (HALF + m + g) * LDT + c + 2 * t4, x[0], x[1]);
-    st2(inv + (HALF + m + g + 8) * LDT + c + 2 * t4, x[2], x[3]);
+    st2(inv + (HALF + m + g) * LDT + c + 2 * t4, ba.at(0), ba.at(1));
+    st2(inv + (HALF + m + g + 8) * LDT + c + 2 * t4, ba.at(2), ba.at(3));
     __syncthreads();
-    x[0] = x[1] = x[2] = x[3] = 0.f;
+    Sum dba;
 #pragma unroll
     for (int k = 0; k < HALF; k += 8) {
       Two l[4], r[2];
       load_a(l, inv + (HALF + m) * LDT + HALF + k, LDT, g, t4);
       load_b(r, inv + (HALF + k) * LDT + c, LDT, g, t4);
-      mma3(x, l, r);
+      mma3(dba, l, r);
     }
+    float x[4] = {dba.at(0), dba.at(1), dba.at(2), dba.at(3)};
     if (any_not_finite(x)) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -437,11 +507,7 @@ chunk_build_kernel(Args a) {
   auto multiply = [&](const float* right, int ldr, int columns, const float* scale, float* out, int ldo) {
     const int m0 = (warp & 3) * 16;
     for (int n0 = (warp >> 2) * 32; n0 < columns; n0 += 64) {
-      float c[4][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
+      Sum sum[4];
       for (int k = 0; k < m0 + 16; k += 8) {      // (the inverse is zero behind its diagonal)
         Two x[4];
         load_a(x, inv + m0 * LDT + k, LDT, g, t4);
@@ -451,21 +517,22 @@ chunk_build_kernel(Args a) {
           Two y[2];
           y[0] = Two(right[(k + t4) * ldr + n0 + 8 * j + g] * s0);
           y[1] = Two(right[(k + t4 + 4) * ldr + n0 + 8 * j + g] * s1);
-          mma3(c[j], x, y);
+          mma3(sum[j], x, y);
         }
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (any_not_finite(c[j])) {
+        float c[4] = {sum[j].at(0), sum[j].at(1), sum[j].at(2), sum[j].at(3)};
+        if (any_not_finite(c)) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int t = m0 + g + 8 * (e >> 1), col = n0 + 8 * j + 2 * t4 + (e & 1);
-            c[j][e] = 0.f;
-            for (int k = 0; k <= t; ++k) c[j][e] = fmaf(inv[t * LDT + k], right[k * ldr + col] * (scale ? scale[k] : 1.f), c[j][e]);
+            c[e] = 0.f;
+            for (int k = 0; k <= t; ++k) c[e] = fmaf(inv[t * LDT + k], right[k * ldr + col] * (scale ? scale[k] : 1.f), c[e]);
           }
         }
-        st2(out + (size_t)(m0 + g) * ldo + n0 + 8 * j + 2 * t4, c[j][0], c[j][1]);
-        st2(out + (size_t)(m0 + g + 8) * ldo + n0 + 8 * j + 2 * t4, c[j][2], c[j][3]);
+        st2(out + (size_t)(m0 + g) * ldo + n0 + 8 * j + 2 * t4, c[0], c[1]);
+        st2(out + (size_t)(m0 + g + 8) * ldo + n0 + 8 * j + 2 * t4, c[2], c[3]);
       }
     }
   };
@@ -490,10 +557,10 @@ struct StateLayout {                   // float offsets
   int ld, k, u, p, stage, s2, u2, floats;
   __host__ __device__ StateLayout(int dp, bool delta) {
     ld = dp + 8;
-    k = delta ? C * ld : 0;            // a stage: W [C][ld], K^ [C][ld], U0 or V [C][LDU], P_C [dp]
+    k = delta ? C * ld : 0;            // a stage: W [C][ld], K^ [C][ld], U0 or V [C][LDU], P_C [2][dp]
     u = k + C * ld;
     p = u + C * LDU;
-    stage = p + dp;
+    stage = p + 2 * dp;
     s2 = 2 * stage;                    // [dp][LDS2] pairs, [C][LDU2] pairs
     u2 = s2 + (delta ? 2 * dp * LDS2 : 0);
     floats = u2 + 2 * C * LDU2;
@@ -541,7 +608,7 @@ chunk_state_kernel(Args a) {
         copy16(buf + at.u + t * LDU + col, a.raw + (in ? (size_t)(row0 + first + t) * (a.heads * a.vdim) + head * a.vdim + v0 + col : 0), in);
       }
     }
-    if (tid < dp / 4) copy16(buf + at.p + 4 * tid, a.pc + unit * dp + 4 * tid, true);
+    if (tid < dp / 2) copy16(buf + at.p + 4 * tid, a.pc + unit * 2 * dp + 4 * tid, true);
     copies_begun();
   };
   fetch(from, sm);
@@ -588,11 +655,7 @@ chunk_state_kernel(Args a) {
     if (DELTA) {      // U = U0 - W S_0: a warp 16 tokens, half of the columns
       constexpr int HT = NT / 2;
       const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * (CB / 2);
-      float x[HT][4], small[HT][4];
-#pragma unroll
-      for (int j = 0; j < HT; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) x[j][e] = small[j][e] = 0.f;
+      Sum x[HT];
 #pragma unroll 4
       for (int k = 0; k < dp; k += 8) {
         Two w[4];
@@ -601,7 +664,7 @@ chunk_state_kernel(Args a) {
         for (int j = 0; j < HT; ++j) {
           Two s[2];
           load_b(s, s2 + k * LDS2 + n0 + 8 * j, LDS2, g, 2 * t4, 2 * t4 + 1);
-          mma3(x[j], small[j], w, s);
+          mma3(x[j], w, s);
         }
       }
 #pragma unroll
@@ -610,7 +673,7 @@ chunk_state_kernel(Args a) {
         for (int h = 0; h < 2; ++h) {
           const int t = m0 + g + 8 * h, col = n0 + 8 * j + 2 * t4;
           const float2 u0 = *reinterpret_cast<const float2*>(cur + at.u + t * LDU + col);
-          const float y0 = u0.x - (x[j][2 * h] + small[j][2 * h]), y1 = u0.y - (x[j][2 * h + 1] + small[j][2 * h + 1]);
+          const float y0 = u0.x - x[j].at(2 * h), y1 = u0.y - x[j].at(2 * h + 1);
           st2(a.u + (unit * C + t) * a.vp + v0 + col, y0, y1);
           const Two p(y0), q(y1);
           *reinterpret_cast<uint4*>(u2 + t * LDU2 + col) = make_uint4(p.hi, p.lo, q.hi, q.lo);
@@ -624,13 +687,7 @@ chunk_state_kernel(Args a) {
     }
     __syncthreads();
     if (holds) {      // S = diag(P_C) S_0 + K^^T U
-      const float p0 = cur[at.p + d0], p1 = cur[at.p + d0 + 1];
-      float small[NT][4];
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        S[j][0] *= p0; S[j][1] *= p0; S[j][2] *= p1; S[j][3] *= p1;
-        small[j][0] = small[j][1] = small[j][2] = small[j][3] = 0.f;
-      }
+      Sum more[NT];
 #pragma unroll
       for (int k = 0; k < C; k += 8) {
         Two x[4];
@@ -639,13 +696,20 @@ chunk_state_kernel(Args a) {
         for (int j = 0; j < NT; ++j) {
           Two y[2];
           load_b(y, u2 + k * LDU2 + 8 * j, LDU2, g, t4, t4 + 4);
-          mma3(S[j], small[j], x, y);
+          mma3(more[j], x, y);
         }
       }
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
+      for (int h = 0; h < 2; ++h) {      // (P_C in two parts: products of decays near one are all rounded to the same side, a constant's to the same value)
+        const float p = cur[at.p + d0 + h], p_low = cur[at.p + dp + d0 + h];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[j][e] += small[j][e];
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int e = 2 * h; e < 2 * h + 2; ++e) {
+            const float low = S[j][e] * p_low;
+            S[j][e] = fmaf(S[j][e], p, more[j].at(e) + (fabsf(low) <= 3.402823466e38f ? low : 0.f));      // (an infinite state stays one)
+          }
+      }
       keep();
     }
     __syncthreads();      // everyone is done with this stage before the fetch after next fills it
@@ -710,13 +774,7 @@ chunk_out_kernel(Args a) {
   }
   copies_begun();
   const int m0 = (warp & 1) * 32, n0 = (warp >> 1) * 32;
-  float acc[2][4][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+  Sum sum[2][4];
   auto multiply = [&](const float* left, int ldl, const float* right, int k) {      // eight inner values, in the order 0 2 4 6 1 3 5 7
     Two x[2][4];
 #pragma unroll
@@ -728,7 +786,7 @@ chunk_out_kernel(Args a) {
       y[0] = Two(r[0]);
       y[1] = Two(r[LDV]);
 #pragma unroll
-      for (int i = 0; i < 2; ++i) mma3(acc[i][j], x[i], y);
+      for (int i = 0; i < 2; ++i) mma3(sum[i][j], x[i], y);
     }
   };
   copies_done<1>();
@@ -739,10 +797,13 @@ chunk_out_kernel(Args a) {
   __syncthreads();
 #pragma unroll 2
   for (int k = 0; k < m0 + 32; k += 8) multiply(aa, LDA, us, k);      // A U: nothing behind the diagonal
+  float acc[2][4][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = sum[i][j].at(e);
       if (any_not_finite(acc[i][j])) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -753,6 +814,7 @@ chunk_out_kernel(Args a) {
           acc[i][j][e] = fabsf(z) <= 3.402823466e38f ? y + z : NAN;      // an infinite value: the recurrence adds it up over channels of both signs
         }
       }
+    }
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll

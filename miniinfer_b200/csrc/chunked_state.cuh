@@ -12,7 +12,7 @@ enum ChunkDecay { CHUNK_DECAY_CHANNEL = 0, CHUNK_DECAY_HEAD = 1, CHUNK_DECAY_CON
 
 struct ChunkedStateArgs {
   const float* qn; const float* kn;           // [tokens, qk_heads * dim], head h reads head h / (heads / qk_heads)
-  const float* g;                             // decays in 0 .. 1: [tokens, heads * dim], [tokens, heads] or [heads] (ChunkDecay)
+  const float* g;                             // decays in 0 .. 1: [tokens, heads * dim], their logarithms [tokens, heads], or [heads] (ChunkDecay)
   int decay;
   const float* beta;                          // [tokens, heads] write strengths of the delta rule, or null: S <- diag(g) S + k v^T
   float* raw;                                 // [tokens, heads * vdim]: the values in, the read-outs out

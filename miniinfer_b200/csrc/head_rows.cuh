@@ -24,6 +24,9 @@ __device__ __forceinline__ void store_row4(__nv_bfloat16* p, float4 v) {
   raw.y = *reinterpret_cast<const uint32_t*>(&hi);
   *reinterpret_cast<uint2*>(p) = raw;
 }
+// exp(x) for x <= 0, near 1 from the difference to 1: expf errs there by parts of an ulp to one side, which thousands of tokens of
+// decays near 1 add up.
+__device__ __forceinline__ float decay_exp(float x) { return x > -0.5f ? 1.f + expm1f(x) : expf(x); }
 __device__ __forceinline__ float4 scaled4(float4 v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); }
 
 // Whether rows of `values` values a head, `stride` values a token, start on the boundaries of four values everywhere.

@@ -117,8 +117,8 @@ linear_prepare_rows_kernel(LinPrepArgs<__nv_bfloat16, float> a, int T) {
           const float4 b = mi::load_row4(a.a_bias + h * a.dim + i);
           z.x += b.x; z.y += b.y; z.z += b.z; z.w += b.w;
         }
-        *reinterpret_cast<float4*>(a.g + at + i) = make_float4(expf(lin_log_sigmoid(z.x) * a.inv_tau), expf(lin_log_sigmoid(z.y) * a.inv_tau),
-                                                               expf(lin_log_sigmoid(z.z) * a.inv_tau), expf(lin_log_sigmoid(z.w) * a.inv_tau));
+        *reinterpret_cast<float4*>(a.g + at + i) = make_float4(mi::decay_exp(lin_log_sigmoid(z.x) * a.inv_tau), mi::decay_exp(lin_log_sigmoid(z.y) * a.inv_tau),
+                                                               mi::decay_exp(lin_log_sigmoid(z.z) * a.inv_tau), mi::decay_exp(lin_log_sigmoid(z.w) * a.inv_tau));
       }
     }
     for (int j = 4 * lane; j < a.vdim; j += 128)

@@ -403,6 +403,7 @@ struct DeltaPrepArgs {
   float* qn; float* kn;                  // [tokens, kv_heads * dim]
   float* g;                              // [tokens, heads * dim], or [tokens, heads] with one decay a head
   float* qk;                             // [tokens, kv_heads]: qh . kh (one decay a head only)
+  float* lg;                             // [tokens, heads]: ln g (one decay a head only)
   int head_decay;
   float* beta;                           // [tokens, heads]
   const T* v; int ldv;                   // values, head h at column h * vdim
@@ -446,7 +447,11 @@ delta_prepare_kernel(DeltaPrepArgs<T> a) {
       const int h = u - a.kv_heads;
       const float neg_rate = -expf(a.A_log[h]);
       if (a.head_decay) {
-        if (lane == 0) a.g[(size_t)t * a.heads + h] = expf(neg_rate * softplus_f(mi::to_float(a.a[(size_t)t * a.lda + h]) + a.dt_bias[h]));
+        if (lane == 0) {
+          const float lg = neg_rate * softplus_f(mi::to_float(a.a[(size_t)t * a.lda + h]) + a.dt_bias[h]);
+          a.lg[(size_t)t * a.heads + h] = lg;
+          a.g[(size_t)t * a.heads + h] = expf(lg);
+        }
       } else for (int i = lane; i < a.dim; i += 32) {
         const float z = mi::to_float(a.a[(size_t)t * a.lda + (size_t)h * a.dim + i]) + a.dt_bias[h * a.dim + i];
         a.g[((size_t)t * a.heads + h) * a.dim + i] = expf(neg_rate * softplus_f(z));
@@ -493,13 +498,17 @@ delta_prepare_rows_kernel(DeltaPrepArgs<__nv_bfloat16> a) {
       const int h = u - a.kv_heads;
       const float neg_rate = -expf(a.A_log[h]);
       if (a.head_decay) {
-        if (lane == 0) a.g[(size_t)t * a.heads + h] = expf(neg_rate * softplus_f(mi::to_float(a.a[(size_t)t * a.lda + h]) + a.dt_bias[h]));
+        if (lane == 0) {
+          const float lg = neg_rate * softplus_f(mi::to_float(a.a[(size_t)t * a.lda + h]) + a.dt_bias[h]);
+          a.lg[(size_t)t * a.heads + h] = lg;
+          a.g[(size_t)t * a.heads + h] = expf(lg);
+        }
       } else {
         for (int i = 4 * lane; i < a.dim; i += 128) {
           const float4 z = mi::load_row4(a.a + (size_t)t * a.lda + (size_t)h * a.dim + i), b = mi::load_row4(a.dt_bias + h * a.dim + i);
           *reinterpret_cast<float4*>(a.g + ((size_t)t * a.heads + h) * a.dim + i) =
-            make_float4(expf(neg_rate * softplus_f(z.x + b.x)), expf(neg_rate * softplus_f(z.y + b.y)),
-                        expf(neg_rate * softplus_f(z.z + b.z)), expf(neg_rate * softplus_f(z.w + b.w)));
+            make_float4(mi::decay_exp(neg_rate * softplus_f(z.x + b.x)), mi::decay_exp(neg_rate * softplus_f(z.y + b.y)),
+                        mi::decay_exp(neg_rate * softplus_f(z.z + b.z)), mi::decay_exp(neg_rate * softplus_f(z.w + b.w)));
         }
       }
       if (lane == 0) a.beta[(size_t)t * a.heads + h] = sigmoid_f(mi::to_float(a.b[(size_t)t * a.ldb + h]));
@@ -872,9 +881,9 @@ MI_API int mi_selective_scan(void* y, int ldy, const void* u, int ldu, const voi
   return 0;
 }
 
-// scratch: float32 - unit q and k, decays, q . k, beta, values / read-outs, each starting on a 16-byte boundary
+// scratch: float32 - unit q and k, decays, q . k, the decays' logarithms, beta, values / read-outs, each starting on a 16-byte boundary
 MI_API long long mi_gated_delta_scratch_floats(int T, int heads, int kv_heads, int dim, int vdim, int head_decay) {
-  return (long long)T * ((long long)2 * kv_heads * dim + (long long)heads * (head_decay ? 1 : dim) + kv_heads + heads + (long long)heads * vdim) + 5 * 4;
+  return (long long)T * ((long long)2 * kv_heads * dim + (long long)heads * (head_decay ? 2 : dim) + kv_heads + heads + (long long)heads * vdim) + 6 * 4;
 }
 
 MI_API int mi_gated_delta_segments() { return DELTA_SEGMENTS; }
@@ -934,7 +943,8 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
   float* kn = qn + up4((size_t)T * kv_heads * dim);
   float* g = kn + up4((size_t)T * kv_heads * dim);
   float* qk = g + up4((size_t)T * heads * (head_decay ? 1 : dim));
-  float* beta = qk + up4((size_t)T * kv_heads);
+  float* lg = qk + up4((size_t)T * kv_heads);
+  float* beta = lg + (head_decay ? up4((size_t)T * heads) : 0);
   float* raw = beta + up4((size_t)T * heads);
   dim3 pgrid(T, (heads + kv_heads + 3) / 4 > 16 ? 16 : (heads + kv_heads + 3) / 4);
   dim3 ogrid(T, (heads + 3) / 4 > 16 ? 16 : (heads + 3) / 4);
@@ -979,7 +989,7 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
     DeltaPrepArgs<TT> p;                                                                                          \
     p.q = (const TT*)q; p.k = (const TT*)k; p.ldqk = ldqk; p.a = (const TT*)a_in; p.lda = lda; p.b = (const TT*)b_in; p.ldb = ldb; \
     p.dt_bias = dt_bias; p.A_log = A_log; p.qn = qn; p.kn = kn; p.g = g; p.beta = beta; p.T_ = T; p.heads = heads;  \
-    p.qk = qk; p.head_decay = head_decay;                                                                         \
+    p.qk = qk; p.lg = lg; p.head_decay = head_decay;                                                                         \
     p.kv_heads = kv_heads; p.dim = dim; p.v = (const TT*)v; p.ldv = ldv; p.raw = raw; p.vdim = vdim;                  \
     if constexpr (sizeof(TT) == 2) {                                                                              \
       if (vec) mi::launch(delta_prepare_rows_kernel, mi::head_rows_grid((long long)T * (heads + kv_heads)), dim3(256), 0, stream, p); \
@@ -992,7 +1002,7 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
     else if (DK == 64) MI_DELTA(TT, 64);                                                                          \
     else MI_DELTA(TT, 128);                                                                                       \
     if (chunks) {                                                                                                 \
-      mi::ChunkedStateArgs c{qn, kn, g, head_decay ? mi::CHUNK_DECAY_HEAD : mi::CHUNK_DECAY_CHANNEL, beta, raw, state, state_stride, q_start, q_len, \
+      mi::ChunkedStateArgs c{qn, kn, head_decay ? lg : g, head_decay ? mi::CHUNK_DECAY_HEAD : mi::CHUNK_DECAY_CHANNEL, beta, raw, state, state_stride, q_start, q_len, \
                              seq_slot, items, heads, kv_heads, dim, vdim, chunk_min};                              \
       if (int e = mi::chunked_state_run(c, T, chunks, stream)) return e;                                            \
     }                                                                                                             \

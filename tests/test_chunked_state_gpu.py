@@ -220,3 +220,31 @@ def _same_where_finite(got, want, norm, what):
     assert off.norm() <= norm, what
   elif w.numel():
     assert (off.abs() <= 2.0 ** -8 * w.abs().clamp(min=1.0) + 1e-4).all(), what
+
+
+# The sums of the chunks' products must not drift: 2048 tokens of decays of about 1 / 3000 a token.  Decays a channel and a head as the walk
+# in order and chunks of FMAs held them or better: it erred by 3.4e-6 and 4.2e-7 (delta rule), 1.3e-5 and 9.4e-7 (linear attention) of the
+# state's norm; sums carried on in the tensor core's accumulator, which is cut off towards zero, by 2.6e-6, 2.4e-6, 9.1e-6 and 5.5e-6.  Now seen:
+# 3.2e-7, 2.3e-7, 4.7e-7 and 1.6e-7.
+@pytest.mark.parametrize("kind,per_head,bound", [("delta", False, 1e-6), ("delta", True, 4.2e-7), ("linear", False, 1.5e-6), ("linear", True, 5e-7)])
+def test_states_of_long_memories_do_not_drift(kind, per_head, bound):
+  from miniinfer_b200.kernels import ops
+  T, H, D = 2048, 4, 128
+  r = torch.Generator().manual_seed(T + D)
+  bf = lambda *s: torch.randn(s, generator=r).to(torch.bfloat16).to(DEV)  # noqa: E731
+  q, k, v, b, gate = bf(T, H * D), bf(T, H * D), bf(T, H * D), bf(T, H), bf(T, H * D)
+  z = torch.randn((T, H if per_head else H * D), generator=r) - 8.0
+  state, out = torch.randn((2, H * D * D), generator=r).to(DEV), torch.empty((T, H * D), dtype=torch.bfloat16, device=DEV)
+  start, heads = state[1].double().view(H, D, D).clone(), lambda t: t.double().view(T, H, D)  # noqa: E731
+  if kind == "delta":
+    a, zero = z.to(torch.bfloat16).to(DEV), torch.zeros(z.shape[1], device=DEV)
+    ops.gated_delta(out, q, k, v, a, b, gate, zero, torch.zeros(H, device=DEV), torch.ones(D, device=DEV), 1e-5, state, _ctx([T]), H, H, D, D)
+    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+    decay = torch.exp(-torch.nn.functional.softplus(a.double())).view(T, H, -1).expand(T, H, D)
+    _, S = _walk(unit(heads(q)), unit(heads(k)), heads(v), decay, torch.sigmoid(b.double()), start)
+  else:
+    const, logits = torch.sigmoid(torch.linspace(7.0, 9.0, H)).to(DEV), (-z).to(DEV)
+    ops.linear_attention(out, q, k, v, gate, state, _ctx([T]), H, D, D, 1e-5, decay_logits=None if per_head else logits, head_decay=const if per_head else None)
+    decay = const.double()[None, :, None].expand(T, H, D) if per_head else torch.sigmoid(logits.double()).view(T, H, D)
+    _, S = _walk(heads(q), heads(k), heads(v), decay, None, start)
+  assert (state[1].double().view(H, D, D) - S).norm() <= bound * S.norm()
