@@ -19,7 +19,7 @@
 //                registers, leaves every chunk's S_0, U = U0 - W S_0 and the state behind the last chunk;
 //   chunk_out    a block per (chunk, head, 64 value columns), all at once: O, written over the values.
 // Chunks are counted over the items of at least min_tokens new tokens, in their order; a step whose chunks need more
-// scratch than SLAB_UNITS (chunk, head) pairs is worked through in slabs, the state row carrying over.
+// scratch than SLAB_FLOATS is worked through in slabs, the state row carrying over.
 //
 // Every product runs on the tensor cores (mma.sync m16n8k8) with each float32 operand as the sum of two tf32 numbers and
 // three of the four partial products, added up in float32: as FMAs they were bound by the reads of shared memory that
@@ -37,7 +37,7 @@ namespace mi {
 namespace {
 
 constexpr int C = CHUNK_TOKENS;
-constexpr int SLAB_UNITS = 2048;
+constexpr long long SLAB_FLOATS = 72ll << 20;      // 288 MiB: 87 chunks of 16 heads of 128 x 128 (delta rule)
 constexpr int THREADS = 256;
 constexpr int OB = 64;                 // value columns of a chunk_out block
 constexpr int VT = 128;                // value columns that chunk_build takes at a time
@@ -827,7 +827,10 @@ chunk_out_kernel(Args a) {
 }
 
 int most_chunks(int T, int items) { return T / C + items; }      // every item's last chunk may be a short one
-int slab_chunks(int heads) { return SLAB_UNITS / heads > 1 ? SLAB_UNITS / heads : 1; }
+int slab_chunks(int heads, int dim, int vdim, bool delta) {
+  const long long n = SLAB_FLOATS / (heads * unit_floats(pad(dim, 32), pad(vdim, 32), delta));
+  return n < 1 ? 1 : n < 65535 ? (int)n : 65535;
+}
 
 template <typename K>
 bool allow(K kernel, size_t smem) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess; }
@@ -835,11 +838,15 @@ bool allow(K kernel, size_t smem) { return cudaFuncSetAttribute(kernel, cudaFunc
 }  // namespace
 
 long long chunked_state_scratch_floats(int T, int items, int heads, int dim, int vdim, bool delta) {
-  const long long chunks = most_chunks(T, items) < slab_chunks(heads) ? most_chunks(T, items) : slab_chunks(heads);
+  const int slab = slab_chunks(heads, dim, vdim, delta);
+  const long long chunks = most_chunks(T, items) < slab ? most_chunks(T, items) : slab;
   return chunks * heads * unit_floats(pad(dim, 32), pad(vdim, 32), delta);
 }
 
-int chunked_state_slabs(int T, int items, int heads) { return (most_chunks(T, items) + slab_chunks(heads) - 1) / slab_chunks(heads); }
+int chunked_state_slabs(int T, int items, int heads, int dim, int vdim, bool delta) {
+  const int slab = slab_chunks(heads, dim, vdim, delta);
+  return (most_chunks(T, items) + slab - 1) / slab;
+}
 
 int chunked_state_run(const ChunkedStateArgs& in, int T, float* scratch, cudaStream_t stream) {
   MI_REQUIRE(chunked_state_takes(in.dim, in.vdim) && in.min_tokens > 0 && in.heads % in.qk_heads == 0,
@@ -851,7 +858,7 @@ int chunked_state_run(const ChunkedStateArgs& in, int T, float* scratch, cudaStr
   static_cast<ChunkedStateArgs&>(a) = in;
   a.dp = pad(in.dim, 32);
   a.vp = pad(in.vdim, 32);
-  const int total = most_chunks(T, in.items), slab = total < slab_chunks(in.heads) ? total : slab_chunks(in.heads);
+  const int total = most_chunks(T, in.items), most = slab_chunks(in.heads, in.dim, in.vdim, delta), slab = total < most ? total : most;
   const size_t units = (size_t)slab * in.heads;
   a.w = scratch;
   a.u = a.w + (delta ? units * C * a.dp : 0);

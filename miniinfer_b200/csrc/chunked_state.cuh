@@ -26,7 +26,7 @@ struct ChunkedStateArgs {
 inline bool chunked_state_takes(int dim, int vdim) { return dim > 0 && dim <= CHUNK_MAX_DIM && dim % 4 == 0 && vdim > 0 && vdim % 4 == 0; }
 // Floats of scratch for a step of T tokens in `items` items (some slabs of chunks at a time share it).
 long long chunked_state_scratch_floats(int T, int items, int heads, int dim, int vdim, bool delta);
-int chunked_state_slabs(int T, int items, int heads);      // three launches each
+int chunked_state_slabs(int T, int items, int heads, int dim, int vdim, bool delta);      // three launches each
 int chunked_state_run(const ChunkedStateArgs& a, int T, float* scratch, cudaStream_t stream);
 
 }  // namespace mi

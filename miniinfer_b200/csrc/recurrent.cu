@@ -893,7 +893,9 @@ MI_API long long mi_chunked_state_floats(int T, int items, int heads, int dim, i
   return mi::chunked_state_takes(dim, vdim) ? mi::chunked_state_scratch_floats(T, items, heads, dim, vdim, delta != 0) : 0;
 }
 
-MI_API int mi_chunked_state_slabs(int T, int items, int heads) { return mi::chunked_state_slabs(T, items, heads); }
+MI_API int mi_chunked_state_slabs(int T, int items, int heads, int dim, int vdim, int delta) {
+  return mi::chunked_state_slabs(T, items, heads, dim, vdim, delta != 0);
+}
 
 // Blocks that walk one request's tokens in order (heads x groups of value columns): what a long prompt portion keeps
 // busy without stretches side by side.

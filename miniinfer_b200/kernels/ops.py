@@ -733,7 +733,7 @@ def _state_chunks(lib, v: torch.Tensor, ctx, heads: int, dim: int, vdim: int, wo
     return None, 0
   chunks = workspace.buffer("state_chunks", (m,), torch.float32) if workspace is not None else \
     torch.empty(m, dtype=torch.float32, device=v.device)
-  return chunks, 3 * int(lib.mi_chunked_state_slabs(v.shape[0], ctx.num_items, heads))
+  return chunks, 3 * int(lib.mi_chunked_state_slabs(v.shape[0], ctx.num_items, heads, dim, vdim, int(delta)))
 
 
 def linear_attention(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Tensor, state: torch.Tensor, ctx,

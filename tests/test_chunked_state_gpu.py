@@ -248,3 +248,61 @@ def test_states_of_long_memories_do_not_drift(kind, per_head, bound):
     decay = const.double()[None, :, None].expand(T, H, D) if per_head else torch.sigmoid(logits.double()).view(T, H, D)
     _, S = _walk(heads(q), heads(k), heads(v), decay, None, start)
   assert (state[1].double().view(H, D, D) - S).norm() <= bound * S.norm()
+
+
+def _run(kind, per_head, lengths, H, D, Dv, seed, ws):
+  """A step of the operation ``kind`` and the recurrence in float64, on the GPU -> for every request (state, its reference, read-outs, theirs)."""
+  from miniinfer_b200.kernels import ops
+  T, eps = sum(lengths), 1e-5
+  r = torch.Generator().manual_seed(seed)
+  bf = lambda *s: torch.randn(s, generator=r).to(torch.bfloat16).to(DEV)  # noqa: E731
+  q, k, v, b, gate = bf(T, H * D), bf(T, H * D), bf(T, H * Dv), bf(T, H), bf(T, H * Dv)
+  start = torch.randn((len(lengths) + 1, H * D * Dv), generator=r)
+  state, out = start.to(DEV), torch.empty((T, H * Dv), dtype=torch.bfloat16, device=DEV)
+  heads = lambda t, n: t.double().view(T, H, n)  # noqa: E731
+  if kind == "delta":
+    a = (torch.randn((T, H if per_head else H * D), generator=r) - 3.0).to(torch.bfloat16).to(DEV)
+    zero = lambda n: torch.zeros(n, device=DEV)  # noqa: E731
+    ops.gated_delta(out, q, k, v, a, b, gate, zero(a.shape[1]), zero(H), torch.ones(Dv, device=DEV), eps, state, _ctx(lengths), H, H, D, Dv, workspace=ws)
+    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+    qq, kk, beta = unit(heads(q, D)) * D ** -0.5, unit(heads(k, D)), torch.sigmoid(b.double())
+    decay = torch.exp(-torch.nn.functional.softplus(a.double())).view(T, H, -1).expand(T, H, D)
+    act = torch.sigmoid(heads(gate, Dv))
+  else:
+    logits, const = (torch.randn((T, H * D), generator=r) + 3.0).to(DEV), torch.linspace(0.9, 0.99, H).to(DEV)
+    ops.linear_attention(out, q, k, v, gate, state, _ctx(lengths), H, D, Dv, eps, decay_logits=None if per_head else logits,
+                         head_decay=const if per_head else None, q_scale=D ** -0.5, workspace=ws)
+    qq, kk, beta = heads(q, D) * D ** -0.5, heads(k, D), None
+    decay = const.double()[None, :, None].expand(T, H, D) if per_head else torch.sigmoid(logits.double()).view(T, H, D)
+    act = torch.nn.functional.silu(heads(gate, Dv))
+  at = 0
+  for i, n in enumerate(lengths):
+    slot, rows = len(lengths) - i, slice(at, at + n)
+    o, S = _walk(qq[rows], kk[rows], heads(v, Dv)[rows], decay[rows], None if beta is None else beta[rows], start[slot].to(DEV).double().view(H, D, Dv))
+    yield state[slot].double().view(H, D, Dv), S, out[rows].double().view(n, H, Dv), _rms(o, eps) * act[rows]
+    at += n
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("kind", ["delta", "linear"])
+def test_chunks_in_more_than_one_slab(kind, per_head):
+  """240 heads: a slab of scratch holds 23 chunks (linear attention: 33) of the step's 24 + 15, so it ends inside a request."""
+  from miniinfer_b200.engine.context import Workspace
+  ws = Workspace(torch.device(DEV))
+  for i, (state, S, out, want) in enumerate(_run(kind, per_head, (1500, 900), 240, 8, 8, 11, ws)):
+    assert (state - S).norm() <= STATE_BOUND * S.norm(), i
+    assert ((out - want).abs() <= 2.0 ** -8 * want.abs().clamp(min=1.0) + 1e-4).all(), i
+  assert ws._bufs[("state_chunks", torch.float32)].numel() < (2400 // 64 + 2) * 240 * (64 * 64 + 2 * 64 * 32 + 32 * 32)      # not all chunks at once
+
+
+@pytest.mark.parametrize("D", [50, 136])      # channels that the chunks do not take: rows of no whole 16 bytes, more than 128
+@pytest.mark.parametrize("kind,per_head", [("delta", False), ("linear", False), ("linear", True)])
+def test_long_portions_of_heads_that_chunks_do_not_take(kind, per_head, D):
+  """Such a bfloat16 step runs each request's tokens in stretches side by side."""
+  from miniinfer_b200.engine.context import Workspace
+  ws = Workspace(torch.device(DEV))
+  for i, (state, S, out, want) in enumerate(_run(kind, per_head, (700, 515), 2, D, 40, 12 + D, ws)):
+    assert (state - S).norm() <= STATE_BOUND * S.norm(), i
+    assert ((out - want).abs() <= 2.0 ** -8 * want.abs().clamp(min=1.0) + 1e-4).all(), i
+  names = {name for name, _ in ws._bufs}
+  assert ("gated_delta_segments" if kind == "delta" else "linear_attention_segments") in names and "state_chunks" not in names
