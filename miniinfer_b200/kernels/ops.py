@@ -609,9 +609,11 @@ DELTA_SEGMENTED_MAX_ITEMS = 4      # the same bound for the delta rule, whose sc
 # B200, 2048 tokens of one request, heads of 128 x 128: 8 heads (64 blocks in order) 5.18 -> 4.57 ms a step of six layers,
 # 16 heads (128 blocks) 7.23 -> 8.11 ms
 DELTA_SEGMENTED_MAX_BLOCKS = 96
-# New tokens a request from which a bfloat16 delta rule goes a chunk at a time (csrc/chunked_state.cu).  Measured on B200, a whole layer of
-# 8 / 16 / 32 heads of 128 x 128 with one decay a key channel, chunks against the walk in order, in microseconds: 96 tokens
-# 86, 94, 123 against 87, 93, 112; 128 tokens 86, 96, 126 against 104, 111, 137; 256 tokens 95, 109, 155 against 179, 189, 226
+# New tokens a request from which a bfloat16 delta rule goes a chunk at a time (csrc/chunked_state.cu).  Measured on B200, the operation
+# for 8 / 16 / 32 heads of 128 x 128, chunks against the walk in order, in microseconds.  One decay a key channel: 96 tokens 64, 69, 75
+# against 62, 63, 65; 112 tokens 65, 69, 75 against 71, 73, 75; 128 tokens 65, 70, 75 against 80, 82, 85; 256 tokens 73, 78, 90 against 153,
+# 156, 162.  One decay a head: 96 tokens 65, 69, 75 against 60, 61, 63; 112 tokens 65, 69, 68 against 68, 70, 73; 128 tokens 66, 69, 75
+# against 77, 79, 82; 256 tokens 72, 78, 89 against 145, 149, 153
 DELTA_CHUNK_MIN_TOKENS = 112
 
 
@@ -701,8 +703,9 @@ def gated_delta(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Te
                                  DELTA_CHUNK_MIN_TOKENS, _stream()), kernels=launches)
 
 
-# The same for linear attention: 48 tokens 53, 66, 94 against 57, 64, 100; 64 tokens 53, 67, 101 against 61, 74, 108; 256 tokens 66,
-# 81, 129 against 173, 177, 234
+# The same for linear attention.  Decays a key channel: 48 tokens 36, 44, 47 against 38, 41, 41; 64 tokens 36, 42, 48 against 45, 49,
+# 50; 128 tokens 39, 47, 51 against 81, 84, 87.  A constant a head: 48 tokens 35, 43, 45 against 36, 37, 37; 64 tokens 34, 40, 45 against 42,
+# 44, 46; 128 tokens 36, 44, 49 against 76, 77, 80
 LINEAR_CHUNK_MIN_TOKENS = 64
 LINEAR_SEGMENTED_MAX_ITEMS = 8     # steps of at most this many requests run long bfloat16 portions in stretches side by side
 # ... and only while the walk in order would leave SMs idle (blocks in order, all requests; an SM holds three, and
