@@ -30,14 +30,15 @@
 // What bounds it: a tile's stage is given back by its P V, so the copy of the tile after next and its S lie on a chain of about 6800
 // cycles for two tiles, of which the products are 4600 (clock stamps).  Tiles of 64 keys in four stages are no faster: a product
 // of 128 x 64 x 16 takes 81 cycles where one of 128 x 128 x 16 takes 95.  Neither the exponentials nor the copies from L2 matter (left
-// out in turn: no change).  Measured on B200, 2048 tokens, latent 192 + 32: 16 heads 51 us, 232 by the mma.sync kernel; 1000 tokens
-// of 32 heads of 192 + 64 with a window of 1024 33 us, 149 by that
+// out in turn: no change).  (Stamps and trials, 51 us, are of the form whose maximum lagged and that read all rows.)  Measured on B200, 2048
+// tokens, latent 192 + 32: 16 heads 55 us, 232 by the mma.sync kernel; 1000 tokens of 32 heads of 192 + 64 with a window of 1024 35 us,
+// 149 by that.
 //
 // Decode tokens run through the same tiles: a work is one request's up to 128 heads and a piece of its keys, counted from key 0, and
 // leaves sums that are not normalised for latent_merge_kernel.  Most of the 128 rows are padding, which costs nothing: a piece is bound
 // by the latency of its one or two tiles and by bytes, and every key row is fetched once for all heads, as key and as value
 // at once.  Measured on B200, 8 tokens of 32 heads of 192 + 64 over 2048 keys each: the layer around them 87.7 us with the
-// mma.sync kernel of attention_decode.cu (16 heads a pass, keys and values fetched apart: 40.6 us, its merge 6.3), 55.9 so.
+// mma.sync kernel of attention_decode.cu (16 heads a pass, keys and values fetched apart: 40.6 us, its merge 6.3), 51.2 so.
 //
 // (the mma.sync kernel of attention_prefill.cu takes the other forms: keys and values of their own, pages that are no multiple
 // of 64, sizes of other alignment).
