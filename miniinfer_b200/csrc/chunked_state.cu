@@ -13,31 +13,37 @@
 // product of the decays between the two tokens, each in 0 .. 1, so nothing overflows and a decay of zero is just that.
 // Tokens go in blocks of eight.  With F_t the product from the start of t's block to t, E_s the one from behind s to the
 // end of its block and B_b a block's whole product, P_t / P_s = F_t B_(I-1) .. B_(J+1) E_s for t in block I and s in an earlier
-// block J; inside a block the product is walked.  Three kernels:
-//   chunk_build  a block per (chunk, head), all at once: A, L, the inverse of I + L, W, U0, K^ and Q~;
-//   chunk_state  a block per (request, head, group of value columns), the only one that walks the chunks in order: keeps S in
+// block J; inside a block the product is walked.  Kernels:
+//   chunk_build  a block per (chunk, head), all at once: A and Q~; for the delta rule L, the inverse of I + L, W, U0 and K^; for linear
+//                attention, where U = V, K^^T V;
+//   chunk_state  (delta rule) a block per (request, head, group of value columns), the only one that walks the chunks in order: keeps S in
 //                registers, leaves every chunk's S_0, U = U0 - W S_0 and the state behind the last chunk;
+//   chunk_scan   (linear attention) the same walk without products, a thread four elements of S;
 //   chunk_out    a block per (chunk, head, 64 value columns), all at once: O, written over the values.
 // Chunks are counted over the items of at least min_tokens new tokens, in their order; a step whose chunks need more
 // scratch than SLAB_FLOATS is worked through in slabs, the state row carrying over.
 //
 // Every product runs on the tensor cores (mma.sync m16n8k8) with each float32 operand as the sum of two tf32 numbers and
-// three of the four partial products, added up in float32: as FMAs they were bound by the reads of shared memory that
-// feed them.  tcgen05 has no use here: the chain of chunks is latency, and its operands are made in registers.  Against
-// float64 the state errs, in parts of its norm, after 2048 tokens of 8 heads of 128 x 128 (in brackets what did these steps before:
-// the walk in stretches, and for the delta rule with one decay a head chunks of FMAs): delta rule, decays a channel about 1 / 50 a
-// token 1.9e-7 (3.5e-7), 1 / 3000 3.2e-7 (3.4e-6), stronger than 1 / 2 1.4e-7 (0.7e-7); a head 1.6e-7 (2.4e-7), 2.3e-7 (4.2e-7), 1.3e-7
-// (0.9e-7); linear attention 1.3e-7 (1.7e-7), 4.7e-7 (1.3e-5), 0.65e-7 (0.3e-7).
+// three of the four partial products (two where one operand is the values, which come from bfloat16 and have no lower part), added up
+// in float32: as FMAs they were bound by the reads of shared memory that feed them.  tcgen05 has no use here: the chain of chunks is
+// latency, and its operands are made in registers.  Against float64 the state errs, in parts of its norm, after 2048 tokens of 8 heads of
+// 128 x 128 (in brackets what did these steps before: the walk in stretches, and for the delta rule with one decay a head chunks of
+// FMAs): delta rule, decays a channel about 1 / 50 a token 1.9e-7 (3.5e-7), 1 / 3000 3.2e-7 (3.4e-6), stronger than 1 / 2 1.2e-7
+// (0.7e-7); a head 1.6e-7 (2.4e-7), 2.3e-7 (4.2e-7), 1.2e-7 (0.9e-7); linear attention 1.4e-7 (1.7e-7), 4.7e-7 (1.3e-5), 0.65e-7 (0.3e-7).
 // Measured on B200, one request of 2048 tokens, 8 / 16 / 32 heads of 128 x 128, the whole operation in microseconds: delta rule with
-// one decay a key channel 193, 284, 494 (in stretches 1017, 1204, 1254), one a head 188, 270, 473 (chunks of FMAs 208, 296, 586), linear
-// attention 126, 188, 345 (in stretches 173, 281, 476).
+// one decay a key channel 129, 227, 412 (in stretches 1017, 1204, 1254), one a head 121, 208, 375, linear attention 82, 139, 248
+// (in stretches 173, 281, 476).  What bounds them: build and out run through some 50 and 20 KB of instructions once, which come from L2,
+// and their products at a third of the tensor cores' rate - splitting the operands takes as many issue slots as the products -; the walk
+// takes 2700 cycles a chunk with 8 columns a block, of which its two products' tensor cycles are 800.
 #include "chunked_state.cuh"
+
+#include <type_traits>
 
 namespace mi {
 namespace {
 
 constexpr int C = CHUNK_TOKENS;
-constexpr long long SLAB_FLOATS = 72ll << 20;      // 288 MiB: 87 chunks of 16 heads of 128 x 128 (delta rule)
+constexpr long long SLAB_FLOATS = 72ll << 20;      // 288 MiB: 86 chunks of 16 heads of 128 x 128 (delta rule)
 constexpr int THREADS = 256;
 constexpr int OB = 64;                 // value columns of a chunk_out block
 constexpr int VT = 128;                // value columns that chunk_build takes at a time
@@ -47,18 +53,21 @@ __host__ __device__ inline int pad(int x, int m) { return (x + m - 1) / m * m; }
 
 struct Args : ChunkedStateArgs {
   int dp, vp;                          // dim padded to 32, vdim padded to 32
-  // per (chunk, head): W [C][dp] and U0 / U [C][vp] (delta rule), A [C][C], K^ and Q~ [C][dp], S_0 [dp][vp], P_C and what its rounding leaves [2][dp]
+  // per (chunk, head): A [C][C], Q~ [C][dp], S_0 [dp][vp], P_C and what its rounding leaves [2][dp]; the delta rule's W and K^ [C][row_floats(dp)] and
+  // U0 / U [vp / 8][C][8], as chunk_state holds them in shared memory; linear attention's K^^T V in the place of S_0 at first
   float *w, *u, *at, *kh, *qt, *s0, *pc;
   int c0, c1;                          // the slab's chunks
 };
 
+__host__ __device__ inline int row_floats(int dp) { return dp + 8; }      // of W and K^: 8-byte reads of a quarter warp's rows fall into different banks
 __host__ __device__ inline long long unit_floats(int dp, int vp, bool delta) {
-  return (delta ? (long long)C * (dp + vp) : 0) + C * C + 2ll * C * dp + (long long)dp * vp + 2 * dp;
+  return (delta ? (long long)C * (2 * row_floats(dp) + vp) : 0) + C * C + (long long)C * dp + (long long)dp * vp + 2 * dp;
 }
 
 // The item that chunk number c (over the items that are long enough) belongs to and the chunk's place in it; item -1: none.
 __device__ __forceinline__ void find_chunk(const Args& a, int c, int& item, int& place) {
   item = -1;
+#pragma unroll 1
   for (int b = 0; b < a.items; ++b) {
     const int n = a.q_len[b];
     if (n < a.min_tokens) continue;
@@ -71,14 +80,28 @@ __device__ __forceinline__ void find_chunk(const Args& a, int c, int& item, int&
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 __device__ __forceinline__ void st2(float* p, float x, float y) { *reinterpret_cast<float2*>(p) = make_float2(x, y); }
-__device__ __forceinline__ void copy16(float* dst, const float* src, bool take) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const int bytes = take ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+// Rows come by bulk copies, a thread a row: as 16-byte copies of all threads, with their addresses, they took 4400 cycles to ask for.
+__device__ __forceinline__ unsigned shared_at(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(uint64_t* bar) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_at(bar)) : "memory"); }
+__device__ __forceinline__ void bars_ready() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void bar_expect(uint64_t* bar, int bytes) {      // by one thread; a copy may end before
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_at(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void copies_begun() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_copy(float* to, const float* from, int floats, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(shared_at(to)), "l"(from), "r"(floats * 4), "r"(shared_at(bar)) : "memory");
+}
+// before a barrier behind which bulk copies go where this thread has read or written
+__device__ __forceinline__ void bulk_may_follow() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// False if the block's own copies, the only thing ever waited for, have not come: what depends on them is then made NaN.
+constexpr int WAIT_LIMIT = 1 << 22;
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, int parity) {
+  unsigned done = 0;
+#pragma unroll 1
+  for (int i = 0; i < WAIT_LIMIT && !done; ++i)
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(shared_at(bar)), "r"(parity) : "memory");
+  return done;
+}
 
 // ------------------------------------------------------------------------------------------------------------ products
 
@@ -95,6 +118,17 @@ struct Two {
     lo = __float_as_uint(x - __uint_as_float(hi));
   }
 };
+// a += b, of two pairs in one instruction each: what limits these kernels is the number of instructions that can be issued
+__device__ __forceinline__ void add2(float& a0, float& a1, float b0, float b1) {
+  asm("{\n .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %3};\n add.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}\n" : "+f"(a0), "+f"(a1) : "f"(b0), "f"(b1));
+}
+// Two numbers at a time: the lower parts, x - hi, as one pair.
+__device__ __forceinline__ void split2(Two& a, Two& b, float x, float y) {
+  a.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  b.hi = (__float_as_uint(y) + 0x1000u) & 0xffffe000u;
+  asm("{\n .reg .b64 h, m, v;\n mov.b64 h, {%2, %3};\n mov.b64 m, {%6, %6};\n mov.b64 v, {%4, %5};\n fma.rn.f32x2 v, h, m, v;\n mov.b64 {%0, %1}, v;\n}\n"
+      : "=r"(a.lo), "=r"(b.lo) : "r"(a.hi), "r"(b.hi), "f"(x), "f"(y), "f"(-1.f));
+}
 // Whether some lane of the warp holds a number that is not finite.  A tile's product with a triangular matrix multiplies the zeros
 // behind the diagonal too, and zero times such a number is a NaN in rows of earlier tokens: the warp then adds up its elements
 // one by one, up to the diagonal.
@@ -130,17 +164,22 @@ __device__ __forceinline__ void mma3(Sum& s, const Two (&a)[4], const Two (&b)[2
   mma1(s.small, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi, s.small);
   mma1(s.small, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo, s.small);
   mma1(p, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi, zero);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    s.c[e] += p[e];
-  }
+  add2(s.c[0], s.c[1], p[0], p[1]);
+  add2(s.c[2], s.c[3], p[2], p[3]);
+}
+// The same for an 8 x 8 operand of numbers that tf32 holds, as the values are, which come from bfloat16: no lower part.
+__device__ __forceinline__ void mma2(Sum& s, const Two (&a)[4], float b0, float b1) {
+  const float zero[4] = {0.f, 0.f, 0.f, 0.f};
+  float p[4];
+  mma1(s.small, a[0].lo, a[1].lo, a[2].lo, a[3].lo, __float_as_uint(b0), __float_as_uint(b1), s.small);
+  mma1(p, a[0].hi, a[1].hi, a[2].hi, a[3].hi, __float_as_uint(b0), __float_as_uint(b1), zero);
+  add2(s.c[0], s.c[1], p[0], p[1]);
+  add2(s.c[2], s.c[3], p[2], p[3]);
 }
 // The 16 x 8 operand of a row-major tile.
-__device__ __forceinline__ void load_a(Two (&a)[4], const float* p, int ld, int g, int t) {
-  a[0] = Two(p[g * ld + t]);
-  a[1] = Two(p[(g + 8) * ld + t]);
-  a[2] = Two(p[g * ld + t + 4]);
-  a[3] = Two(p[(g + 8) * ld + t + 4]);
+__device__ __forceinline__ void load_a(Two (&a)[4], const float* p, int ld, int g, int t, float s0 = 1.f, float s1 = 1.f) {      // s0, s1: of its columns t and t + 4
+  split2(a[0], a[1], p[g * ld + t] * s0, p[(g + 8) * ld + t] * s0);
+  split2(a[2], a[3], p[g * ld + t + 4] * s1, p[(g + 8) * ld + t + 4] * s1);
 }
 // The same with two values a read: the inner index runs 0 2 4 6 1 3 5 7, so the 8 x 8 operand beside it has rows 2 t and 2 t + 1.
 __device__ __forceinline__ void load_a_pairs(Two (&a)[4], const float* p, int ld, int g, int t) {
@@ -153,40 +192,33 @@ __device__ __forceinline__ void load_a_pairs(Two (&a)[4], const float* p, int ld
 // The transpose of a row-major 8 x 16 tile, rows 2 g and 2 g + 1 in the places of g and g + 8.
 __device__ __forceinline__ void load_a_transposed(Two (&a)[4], const float* p, int ld, int g, int t) {
   const float2 x = *reinterpret_cast<const float2*>(p + t * ld + 2 * g), y = *reinterpret_cast<const float2*>(p + (t + 4) * ld + 2 * g);
-  a[0] = Two(x.x);
-  a[1] = Two(x.y);
-  a[2] = Two(y.x);
-  a[3] = Two(y.y);
+  split2(a[0], a[1], x.x, x.y);
+  split2(a[2], a[3], y.x, y.y);
 }
 __device__ __forceinline__ void load_b(Two (&b)[2], const float* p, int ld, int g, int t) {
-  b[0] = Two(p[t * ld + g]);
-  b[1] = Two(p[(t + 4) * ld + g]);
+  split2(b[0], b[1], p[t * ld + g], p[(t + 4) * ld + g]);
 }
-// Rows r0 and r1 of a tile of numbers already in two parts.
-__device__ __forceinline__ void load_b(Two (&b)[2], const uint2* p, int ld, int g, int r0, int r1) {
-  const uint2 x = p[r0 * ld + g], y = p[r1 * ld + g];
-  b[0].hi = x.x; b[0].lo = x.y;
-  b[1].hi = y.x; b[1].lo = y.y;
-}
-
 // -------------------------------------------------------------------------------------------------------------- build
 
 constexpr int LDT = C + 4;             // a row of the inverse
+constexpr int PAIRS = NB * (NB - 1) / 2;      // of blocks of eight tokens, an earlier one and a later one
 struct BuildLayout {                   // float offsets
   int ld, k, q, g, total, diag, beta, rest, f, floats;
   __host__ __device__ explicit BuildLayout(int dp) {
     ld = dp + 4;
-    k = 0;                                                            // [C][ld] keys; E k; then the values, VT columns at a time
-    q = k + C * (dp > VT ? ld : VT + 4);                              // [C][ld] queries; F q; then L^T [C][C] and the inverse [C][LDT]
-    g = q + (C * ld > C * C + C * LDT ? C * ld : C * C + C * LDT);    // [C][ld] decays; F k; then diag(beta) K~
-    total = g + C * ld;                                               // [NB][dp] a block's whole product
+    const int rows = C * (dp > VT ? ld : VT + 4);      // of channels, then of values, VT columns at a time
+    k = 0;                                                            // [C][ld] keys; E k; then delta: the values, linear: K^
+    q = k + rows;                                                     // [C][ld] queries; F q; then L^T [C][C] and behind it half of the tiles' sums, then the inverse [C][LDT]
+    g = q + (C * ld > C * C + C * LDT ? C * ld : C * C + C * LDT);    // [C][ld] decays; delta: F k, diag(beta) K~; linear: the values
+    total = g + rows;                                                 // [NB][dp] a block's whole product
     diag = total + NB * dp;                                           // [NB][64] products inside a block: 36 of q, 28 of k
     beta = diag + NB * 64;                                            // [C]
     rest = beta + C;                                                  // [NB][dp] one decay a channel: what the rounding of the block's product leaves
-    f = rest + NB * dp;                                               // one decay a head: F [C], E [C], a block's product [NB], as doubles [NB]
-    floats = f + 2 * C + 3 * NB;
+    f = rest + NB * dp;                                               // one decay a head: F [C], E [C], a block's product [NB], as doubles [NB], the decays [C], what they are of [C]
+    floats = f + 4 * C + 3 * NB;
   }
 };
+static_assert(PAIRS * 128 <= C * LDT, "half of the tiles' sums lie where the inverse will");
 
 // Sums 64 values over the 32 lanes; lane l ends with the sums number 2 l and 2 l + 1 in v[0] and v[1].
 __device__ __forceinline__ void reduce_scatter(float (&v)[64], int lane) {
@@ -202,6 +234,34 @@ __device__ __forceinline__ void reduce_scatter(float (&v)[64], int lane) {
   }
 }
 
+// Block I's rows - eight of F k above eight of F q - times every earlier block's E k and the products of the blocks between, over the
+// channels d0 .. d1 - 1.  I is known to the compiler, so the reads of a step's tiles stand before its products.
+template <int I, bool DELTA>
+__device__ __forceinline__ void between_blocks(Sum (&acc)[NB - 1], const float* ks, const float* qs, const float* gs, const float* total, int ld, int dp,
+                                               int d0, int d1, int g, int t4) {
+  const float *fk = gs + (8 * I + g) * ld + t4, *fq = qs + (8 * I + g) * ld + t4;
+#pragma unroll 1
+  for (int d = d0; d < d1; d += 8) {
+    float e0[I > 0 ? I : 1], e1[I > 0 ? I : 1], p0 = 1.f, p1 = 1.f;
+#pragma unroll
+    for (int j = I - 1; j >= 0; --j) {
+      if (j + 1 < I) { p0 *= total[(j + 1) * dp + d + t4]; p1 *= total[(j + 1) * dp + d + t4 + 4]; }
+      const float* ek = ks + (8 * j + g) * ld + d + t4;
+      e0[j] = ek[0] * p0;
+      e1[j] = ek[4] * p1;
+    }
+    Two x[4];
+    split2(x[0], x[2], DELTA ? fk[d] : 0.f, DELTA ? fk[d + 4] : 0.f);
+    split2(x[1], x[3], fq[d], fq[d + 4]);
+#pragma unroll
+    for (int j = I - 1; j >= 0; --j) {
+      Two y[2];
+      split2(y[0], y[1], e0[j], e1[j]);
+      mma3(acc[j], x, y);
+    }
+  }
+}
+
 template <bool DELTA>
 __global__ void __launch_bounds__(THREADS, 2)
 chunk_build_kernel(Args a) {
@@ -210,8 +270,14 @@ chunk_build_kernel(Args a) {
   const int ld = at.ld, dp = a.dp;
   float *ks = sm + at.k, *qs = sm + at.q, *gs = sm + at.g, *total = sm + at.total, *bt = sm + at.beta;
   __shared__ int found[2];
+  __shared__ __align__(8) uint64_t bars[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, head = blockIdx.y;
-  if (tid == 0) find_chunk(a, a.c0 + blockIdx.x, found[0], found[1]);
+  if (tid == 0) {
+    find_chunk(a, a.c0 + blockIdx.x, found[0], found[1]);
+    bar_init(bars);
+    bar_init(bars + 1);
+    bars_ready();
+  }
   mi::grid_dependency_sync();
   __syncthreads();
   const int item = found[0];
@@ -219,126 +285,149 @@ chunk_build_kernel(Args a) {
   const int first = found[1] * C, n = min(C, a.q_len[item] - first), row0 = a.q_start[item] + first;
   const int kvh = head / (a.heads / a.qk_heads);
   const size_t unit = (size_t)blockIdx.x * a.heads + head;
-  {      // tokens behind the last and channels behind the last: zero keys and queries, decays of one
-    const int per_row = dp / 4, rows = THREADS / per_row, t0 = tid / per_row, d = (tid - t0 * per_row) * 4;
-#pragma unroll 4
-    for (int t = t0; t < C && t0 < rows; t += rows) {
-      const bool in = t < n && d < a.dim;
-      const size_t from = in ? ((size_t)(row0 + t) * a.qk_heads + kvh) * a.dim + d : 0;
-      copy16(ks + t * ld + d, a.kn + from, in);
-      copy16(qs + t * ld + d, a.qn + from, in);
-      float4 x = make_float4(1.f, 1.f, 1.f, 1.f);
-      if (in) {
-        if (a.decay == CHUNK_DECAY_CHANNEL) {
-          x = ld4(a.g + ((size_t)(row0 + t) * a.heads + head) * a.dim + d);
-        } else {
-          const float y = a.decay == CHUNK_DECAY_HEAD ? expf(a.g[(size_t)(row0 + t) * a.heads + head]) : a.g[head];
-          x = make_float4(y, y, y, y);
-        }
+  const bool per_head = a.decay != CHUNK_DECAY_CHANNEL, logs = a.decay == CHUNK_DECAY_HEAD;
+  float *fs = sm + at.f, *of_token = fs + 2 * C + 3 * NB, *step_of = of_token + C;
+  double* whole = reinterpret_cast<double*>(fs + 2 * C + NB);
+  // Rows of keys, queries and decays, a thread a row; tokens behind the last and channels behind the last: zero keys and queries, decays of one
+  if (tid == 0) bar_expect(bars, n * (per_head ? 2 : 3) * a.dim * 4);
+  {
+    const int t = tid & (C - 1), which = tid / C;      // (a warp has one kind of rows)
+    if (which < (per_head ? 2 : 3)) {
+      float* to = (which == 0 ? ks : which == 1 ? qs : gs) + t * ld;
+      const float fill = which == 2 ? 1.f : 0.f;
+      if (t < n)
+        bulk_copy(to, which == 2 ? a.g + ((size_t)(row0 + t) * a.heads + head) * a.dim
+                                 : (which ? a.qn : a.kn) + ((size_t)(row0 + t) * a.qk_heads + kvh) * a.dim, a.dim, bars);
+#pragma unroll 1
+      for (int d = t < n ? a.dim : 0; d < dp; d += 4) st4(to + d, make_float4(fill, fill, fill, fill));
+    } else if (tid >= 3 * C) {
+      if (DELTA) bt[t] = t < n ? a.beta[(size_t)(row0 + t) * a.heads + head] : 0.f;
+      if (per_head) {
+        const float x = t < n ? a.g[logs ? (size_t)(row0 + t) * a.heads + head : head] : logs ? 0.f : 1.f;
+        step_of[t] = x;
+        of_token[t] = logs ? expf(x) : x;
       }
-      st4(gs + t * ld + d, x);
     }
-    if (DELTA && tid < C) bt[tid] = tid < n ? a.beta[(size_t)(row0 + tid) * a.heads + head] : 0.f;
   }
-  copies_begun();
   // One decay a head: F, E and the blocks' products are sums of logarithms (a constant's: products) in double, rounded once.  A constant's
   // float products err alike in every chunk, and logarithms of decays near one hold digits that the decays do not.
-  const bool per_head = a.decay != CHUNK_DECAY_CHANNEL, logs = a.decay == CHUNK_DECAY_HEAD;
-  float* fs = sm + at.f;
-  double* whole = reinterpret_cast<double*>(fs + 2 * C + NB);
-  if (per_head && tid < NB) {
-    double x[8], sum = logs ? 0. : 1.;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int t = 8 * tid + j;
-      x[j] = t >= n ? sum : (double)a.g[logs ? (size_t)(row0 + t) * a.heads + head : head];
-    }
-    double f = sum;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      f = logs ? f + x[j] : f * x[j];
-      fs[8 * tid + j] = logs ? expf((float)f) : (float)f;
-    }
-    whole[tid] = f;
-    fs[2 * C + tid] = logs ? expf((float)f) : (float)f;
-#pragma unroll
-    for (int j = 7; j >= 0; --j) {
-      fs[C + 8 * tid + j] = logs ? expf((float)sum) : (float)sum;
-      sum = logs ? sum + x[j] : sum * x[j];
+  if (per_head) {
+    __syncthreads();
+    if (tid < 2 * C) {      // F of a token, then E of one
+      const int t = tid & (C - 1), b = t & ~7;
+      const bool forward = tid < C;
+      double f = logs ? 0. : 1.;
+#pragma unroll 1
+      for (int j = forward ? b : b + 7; forward ? j <= t : j > t; j += forward ? 1 : -1) f = logs ? f + (double)step_of[j] : f * (double)step_of[j];
+      const float r = logs ? expf((float)f) : (float)f;
+      fs[tid] = r;
+      if (forward && (t & 7) == 7) {
+        whole[t >> 3] = f;
+        fs[2 * C + (t >> 3)] = r;
+      }
     }
   }
-  copies_done<0>();
+  bool late = !bar_wait(bars, 0);
   __syncthreads();
-
-  // Inside the blocks, a warp a block of eight tokens and a lane four key channels: products number p (p + 1) / 2 + s of q_p and
-  // k_s for s <= p, then 36 + p (p - 1) / 2 + s of k_p and k_s for s < p, the decays between s and p walked.
+  // Inside the blocks, a warp a block of eight tokens, a lane two key channels at a time: products number p (p + 1) / 2 + s of q_p and
+  // k_s for s <= p, then 36 + p (p - 1) / 2 + s of k_p and k_s for s < p, the decays between s and p walked.  A key that has
+  // walked to the block's end is E k; F q and F k are left beside it, each in the place of what it was made from.
   {
     float v[64];
 #pragma unroll
     for (int i = 0; i < 64; ++i) v[i] = 0.f;
-    if (4 * lane < dp) {
-      const float* kr = ks + warp * 8 * ld + 4 * lane;
-      const float *qr = qs + warp * 8 * ld + 4 * lane, *gr = gs + warp * 8 * ld + 4 * lane;
-      float4 key[8];      // key s times the decays from behind s to the token at hand
+    const float* table = fs + 8 * warp;      // (one decay a head)
+#pragma unroll 1
+    for (int d = 2 * lane; d < dp; d += 64) {
+      float *kr = ks + warp * 8 * ld + d, *qr = qs + warp * 8 * ld + d, *gr = gs + warp * 8 * ld + d;
+      const float* decays = per_head ? of_token + 8 * warp : gr;
+      const int to_next = per_head ? 1 : ld, to_second = per_head ? 0 : 1;
+      float2 key[8];      // key s times the decays from behind s to the token at hand
+      float2 f = make_float2(1.f, 1.f), rest = make_float2(0.f, 0.f);
 #pragma unroll
       for (int p = 0; p < 8; ++p) {
-        const float4 kp = ld4(kr + p * ld), qp = ld4(qr + p * ld), gp = ld4(gr + p * ld);
+        const float2 kp = *reinterpret_cast<const float2*>(kr + p * ld), qp = *reinterpret_cast<const float2*>(qr + p * ld);
+        const float2 gp = make_float2(decays[p * to_next], decays[p * to_next + to_second]);
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
           if (s < p) {
-            key[s].x *= gp.x; key[s].y *= gp.y; key[s].z *= gp.z; key[s].w *= gp.w;
-            v[36 + p * (p - 1) / 2 + s] = fmaf(kp.x, key[s].x, fmaf(kp.y, key[s].y, fmaf(kp.z, key[s].z, kp.w * key[s].w)));
-            v[p * (p + 1) / 2 + s] = fmaf(qp.x, key[s].x, fmaf(qp.y, key[s].y, fmaf(qp.z, key[s].z, qp.w * key[s].w)));
+            key[s].x *= gp.x; key[s].y *= gp.y;
+            const int i = p * (p + 1) / 2 + s;
+            v[i] = fmaf(qp.x, key[s].x, fmaf(qp.y, key[s].y, v[i]));
+            if (DELTA) {
+              const int l = 36 + p * (p - 1) / 2 + s;
+              v[l] = fmaf(kp.x, key[s].x, fmaf(kp.y, key[s].y, v[l]));
+            }
           }
         }
         key[p] = kp;
-        v[p * (p + 1) / 2 + p] = fmaf(qp.x, kp.x, fmaf(qp.y, kp.y, fmaf(qp.z, kp.z, qp.w * kp.w)));
+        const int i = p * (p + 1) / 2 + p;
+        v[i] = fmaf(qp.x, kp.x, fmaf(qp.y, kp.y, v[i]));
+        const float2 before = f;
+        f.x *= gp.x; f.y *= gp.y;
+        rest.x = fmaf(rest.x, gp.x, fmaf(before.x, gp.x, -f.x));
+        rest.y = fmaf(rest.y, gp.y, fmaf(before.y, gp.y, -f.y));
+        if (per_head) f.x = f.y = table[p];
+        st2(qr + p * ld, qp.x * f.x, qp.y * f.y);
+        if (DELTA) st2(gr + p * ld, kp.x * f.x, kp.y * f.y);
       }
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const float2 k = *reinterpret_cast<const float2*>(kr + s * ld);
+        const float e = table[C + s];
+        st2(kr + s * ld, per_head ? k.x * e : key[s].x, per_head ? k.y * e : key[s].y);
+      }
+      if (per_head) f.x = f.y = fs[2 * C + warp];
+      st2(total + warp * dp + d, f.x, f.y);
+      st2(sm + at.rest + warp * dp + d, rest.x, rest.y);
     }
     reduce_scatter(v, lane);
     st2(sm + at.diag + warp * 64 + 2 * lane, v[0], v[1]);
   }
+  bulk_may_follow();
   __syncthreads();
-  // E k, F q and F k over the keys, queries and decays, a thread eight tokens of a block in a channel
-  for (int i = tid; i < NB * dp; i += THREADS) {
-    const int b = i / dp, d = i % dp;
-    float gv[8], kv[8], f = 1.f, rest = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { gv[j] = gs[(8 * b + j) * ld + d]; kv[j] = ks[(8 * b + j) * ld + d]; }
-    if (per_head) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        qs[(8 * b + j) * ld + d] *= fs[8 * b + j];
-        gs[(8 * b + j) * ld + d] = fs[8 * b + j] * kv[j];
-        ks[(8 * b + j) * ld + d] = fs[C + 8 * b + j] * kv[j];
-      }
-      total[b * dp + d] = fs[2 * C + b];
-      continue;
+  int values_round = 0;
+  auto fetch_values = [&](float* to, int v0) {      // VT columns from v0 on, zeros behind the last token; what lies behind the last column reaches only columns there
+    const int columns = min(VT, a.vdim - v0);
+    if (tid == 0) bar_expect(bars + 1, n * columns * 4);
+    if (tid < C) {
+      float* row = to + tid * (VT + 4);
+      if (tid < n) bulk_copy(row, a.raw + (size_t)(row0 + tid) * (a.heads * a.vdim) + head * a.vdim + v0, columns, bars + 1);
+#pragma unroll 1
+      for (int c = tid < n ? columns : 0; c < VT; c += 4) st4(row + c, make_float4(0.f, 0.f, 0.f, 0.f));
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float before = f;
-      f *= gv[j];
-      rest = fmaf(rest, gv[j], fmaf(before, gv[j], -f));
-      qs[(8 * b + j) * ld + d] *= f;
-      gs[(8 * b + j) * ld + d] = f * kv[j];
-    }
-    total[b * dp + d] = f;
-    sm[at.rest + b * dp + d] = rest;
-    f = 1.f;
-#pragma unroll
-    for (int j = 7; j >= 0; --j) {
-      ks[(8 * b + j) * ld + d] = f * kv[j];
-      f *= gv[j];
-    }
+  };
+  auto values_there = [&]() {
+    late |= !bar_wait(bars + 1, values_round & 1);
+    ++values_round;
+  };
+  if (!DELTA) fetch_values(gs, 0);
+  // Between blocks: warp I has block I over the lower half of the channels and block 7 - I over the upper, seven tiles each (all channels of
+  // block I a warp, behind branches: 13000 cycles and more; so 7400).  The two warps of a pair share their code.  One body for all blocks, its
+  // tiles behind branches, is a quarter of the instructions and 15000 cycles: the reads of a step's tiles no longer stand before its products.
+  float own[NB - 1][4], other[NB - 1][4];
+  switch (min(warp, NB - 1 - warp)) {
+#define MI_BETWEEN(I)                                                                                                              \
+  case I: {                                                                                                                        \
+    constexpr int J = NB - 1 - I;                                                                                                  \
+    const bool first_of_pair = warp == I;                                                                                          \
+    Sum x[NB - 1], y[NB - 1];                                                                                                      \
+    between_blocks<I, DELTA>(x, ks, qs, gs, total, ld, dp, first_of_pair ? 0 : dp / 2, first_of_pair ? dp / 2 : dp, g, t4);        \
+    between_blocks<J, DELTA>(y, ks, qs, gs, total, ld, dp, first_of_pair ? dp / 2 : 0, first_of_pair ? dp : dp / 2, g, t4);        \
+    _Pragma("unroll") for (int j = 0; j < J; ++j)                                                                                  \
+      _Pragma("unroll") for (int e = 0; e < 4; ++e) {                                                                              \
+        const float v = j < I ? x[j].at(e) : 0.f, w = y[j].at(e);                                                                  \
+        own[j][e] = first_of_pair ? v : w;                                                                                         \
+        other[j][e] = first_of_pair ? w : v;                                                                                       \
+      }                                                                                                                            \
+    break;                                                                                                                         \
   }
-  __syncthreads();
-  // Between blocks: warp I has the rows of its block - eight of F k above eight of F q - and every earlier block's E k, times the
-  // products of the blocks between
-  Sum acc[NB - 1];
+    MI_BETWEEN(0) MI_BETWEEN(1) MI_BETWEEN(2) MI_BETWEEN(3)
+#undef MI_BETWEEN
+  }
   if (warp == 0 && per_head) {      // P_C and what its rounding leaves
     double p = logs ? 0. : 1.;
-#pragma unroll
+#pragma unroll 1
     for (int b = 0; b < NB; ++b) p = logs ? p + whole[b] : p * whole[b];
     if (logs) p = exp(p);
     const float high = (float)p, low = (float)(p - (double)high);
@@ -347,108 +436,141 @@ chunk_build_kernel(Args a) {
       a.pc[unit * 2 * dp + dp + d] = low;
     }
   }
-  if (warp > 0) {
-    const float *fk = gs + (8 * warp + g) * ld, *fq = qs + (8 * warp + g) * ld;
-    for (int d = 0; d < dp; d += 8) {
-      Two x[4];
-      x[0] = Two(fk[d + t4]);
-      x[1] = Two(fq[d + t4]);
-      x[2] = Two(fk[d + t4 + 4]);
-      x[3] = Two(fq[d + t4 + 4]);
-      float p0 = 1.f, p1 = 1.f;
-#pragma unroll
-      for (int j = NB - 2; j >= 0; --j) {
-        if (j < warp) {
-          if (j + 1 < warp) { p0 *= total[(j + 1) * dp + d + t4]; p1 *= total[(j + 1) * dp + d + t4 + 4]; }
-          const float* ek = ks + (8 * j + g) * ld + d + t4;
-          Two y[2];
-          y[0] = Two(ek[0] * p0);
-          y[1] = Two(ek[4] * p1);
-          mma3(acc[j], x, y);
-        }
-      }
+  // Q~ and K^, a thread the blocks b0, b0 + step, ... of a channel, with the products of the blocks before and behind
+  const int step = THREADS / dp, b0 = tid / dp, my_d = tid - b0 * dp, b_last = b0 + (NB - 1 - b0) / step * step;
+  auto forward = [&](auto use) {
+    float before = 1.f;
+    int at_b = 0;
+#pragma unroll 1
+    for (int b = b0; b < NB && b0 < step; b += step) {
+#pragma unroll 1
+      for (; at_b < b; ++at_b) before *= total[at_b * dp + my_d];
+      use(8 * b, before);
     }
+  };
+  auto backward = [&](auto use) {
+    float behind = 1.f;
+    int at_b = NB - 1;
+#pragma unroll 1
+    for (int b = b_last; b >= 0 && b0 < step; b -= step) {
+#pragma unroll 1
+      for (; at_b > b; --at_b) behind *= total[at_b * dp + my_d];
+      use(8 * b, behind);
+    }
+  };
+  forward([&](int row, float before) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a.qt[(unit * C + row + j) * dp + my_d] = qs[(row + j) * ld + my_d] * before;
+  });
+  if (DELTA)
+    backward([&](int row, float behind) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a.kh[(unit * C + row + j) * row_floats(dp) + my_d] = ks[(row + j) * ld + my_d] * behind;
+    });
+  if (b0 == step - 1 && !per_head) {
+    double p = 1.;
+#pragma unroll 1
+    for (int j = 0; j < NB; ++j) p *= (double)total[j * dp + my_d] + (double)sm[at.rest + j * dp + my_d];
+    a.pc[unit * 2 * dp + my_d] = (float)p;
+    a.pc[unit * 2 * dp + dp + my_d] = (float)(p - (double)(float)p);
   }
-  // A, a row a token: zeros behind the diagonal
+  bulk_may_follow();
+  __syncthreads();      // everyone is done with E k, F q and F k
+  float *lt = qs, *inv = qs + C * C;
+#pragma unroll
+  for (int j = 0; j < NB - 1; ++j)      // the other half of block 7 - warp's tiles, block I's from number I (I - 1) / 2 on
+    if (j < NB - 1 - warp) st4(inv + (((NB - 1 - warp) * (NB - 2 - warp) / 2 + j) * 32 + lane) * 4, make_float4(other[j][0], other[j][1], other[j][2], other[j][3]));
+  if (DELTA) {
+    fetch_values(ks, 0);
+    forward([&](int row, float before) {      // F k becomes K~
+#pragma unroll
+      for (int j = 0; j < 8; ++j) gs[(row + j) * ld + my_d] *= before;
+    });
+  } else {
+    backward([&](int row, float behind) {      // E k becomes K^
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ks[(row + j) * ld + my_d] *= behind;
+    });
+  }
+  if (!DELTA) values_there();
+  __syncthreads();
+  // A, a row a token: zeros behind the diagonal; and L^T, the part before the diagonal
   {
-    float* out = a.at + unit * C * C + (size_t)(8 * warp + g) * C + 2 * t4;
-    const float* dq = sm + at.diag + warp * 64 + g * (g + 1) / 2;
+    const int t = 8 * warp + g;
+    float* out = a.at + unit * C * C + (size_t)t * C + 2 * t4;
+    const float *dq = sm + at.diag + warp * 64 + g * (g + 1) / 2, *dk = sm + at.diag + warp * 64 + 36 + g * (g - 1) / 2;
+    const float* half = inv + (warp * (warp - 1) / 2 * 32 + lane) * 4;
+    const float b = DELTA ? bt[t] : 0.f;
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
       float x = 0.f, y = 0.f;
-      if (j < warp) { x = acc[j < NB - 1 ? j : 0].at(2); y = acc[j < NB - 1 ? j : 0].at(3); }
+      if (j < warp) {
+        const int i = j < NB - 1 ? j : 0;
+        const float4 h = ld4(half + j * 128);
+        x = own[i][2] + h.z;
+        y = own[i][3] + h.w;
+        if (DELTA) {
+          lt[(8 * j + 2 * t4) * C + t] = b * (own[i][0] + h.x);
+          lt[(8 * j + 2 * t4 + 1) * C + t] = b * (own[i][1] + h.y);
+        }
+      }
       if (j == warp) {
         x = 2 * t4 <= g ? dq[2 * t4] : 0.f;
         y = 2 * t4 + 1 <= g ? dq[2 * t4 + 1] : 0.f;
+        if (DELTA) {
+          if (2 * t4 < g) lt[(8 * warp + 2 * t4) * C + t] = b * dk[2 * t4];
+          if (2 * t4 + 1 < g) lt[(8 * warp + 2 * t4 + 1) * C + t] = b * dk[2 * t4 + 1];
+        }
       }
       st2(out + 8 * j, x, y);
     }
   }
-  // K^ and Q~, and F k becomes diag(beta) K~
-  for (int i = tid; i < NB * dp; i += THREADS) {
-    const int b = i / dp, d = i % dp;
-    float before = 1.f, behind = 1.f;
-    for (int j = 0; j < b; ++j) before *= total[j * dp + d];
-    for (int j = NB - 1; j > b; --j) behind *= total[j * dp + d];
+  if (!DELTA) {      // K^^T V: a warp 16 key channels - a lane those numbered 2 g and 2 g + 1 -, 32 value columns at a time
+    for (int v0 = 0; v0 < a.vp; v0 += VT) {
+      if (v0 > 0) {
+        bulk_may_follow();
+        __syncthreads();
+        fetch_values(gs, v0);
+        values_there();
+        __syncthreads();
+      }
+      if (16 * warp >= dp) continue;
+#pragma unroll 1
+      for (int c = 0; c < min(VT, a.vp - v0); c += 32) {
+        Sum more[4];
+#pragma unroll 1
+        for (int k = 0; k < C; k += 8) {
+          Two x[4];
+          load_a_transposed(x, ks + k * ld + 16 * warp, ld, g, t4);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int t = 8 * b + j;
-      a.kh[(unit * C + t) * dp + d] = ks[t * ld + d] * behind;
-      a.qt[(unit * C + t) * dp + d] = qs[t * ld + d] * before;
-    }
-    if (b == NB - 1 && !per_head) {
-      double p = 1.;
-      for (int j = 0; j < NB; ++j) p *= (double)total[j * dp + d] + (double)sm[at.rest + j * dp + d];
-      a.pc[unit * 2 * dp + d] = (float)p;
-      a.pc[unit * 2 * dp + dp + d] = (float)(p - (double)(float)p);
-    }
-  }
-  if (!DELTA) return;
-  __syncthreads();
-  for (int i = tid; i < NB * dp; i += THREADS) {      // (a loop of its own: the warps above still read F k)
-    const int b = i / dp, d = i % dp;
-    float before = 1.f;
-    for (int j = 0; j < b; ++j) before *= total[j * dp + d];
+          for (int j = 0; j < 4; ++j) {
+            const float* y = gs + (k + t4) * (VT + 4) + c + 8 * j + g;
+            mma2(more[j], x, y[0], y[4 * (VT + 4)]);
+          }
+        }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) gs[(8 * b + j) * ld + d] *= bt[8 * b + j] * before;
-  }
-  auto fetch_values = [&](int v0) {
-    for (int i = tid; i < C * VT / 4; i += THREADS) {
-      const int t = i / (VT / 4), c = v0 + (i % (VT / 4)) * 4;
-      const bool in = t < n && c < a.vdim;
-      copy16(ks + t * (VT + 4) + c - v0, a.raw + (in ? (size_t)(row0 + t) * (a.heads * a.vdim) + head * a.vdim + c : 0), in);
-    }
-    copies_begun();
-  };
-  fetch_values(0);
-  float *lt = qs, *inv = qs + C * C;
-  {      // L^T, the part before the diagonal
-    const int t = 8 * warp + g;
-    const float* dk = sm + at.diag + warp * 64 + 36 + g * (g - 1) / 2;
+        for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int j = 0; j < NB - 1; ++j) {
-      if (j < warp) {
-        lt[(8 * j + 2 * t4) * C + t] = bt[t] * acc[j].at(0);
-        lt[(8 * j + 2 * t4 + 1) * C + t] = bt[t] * acc[j].at(1);
+          for (int h = 0; h < 2; ++h)
+            st2(a.s0 + (unit * dp + 16 * warp + 2 * g + h) * a.vp + v0 + c + 8 * j + 2 * t4, late ? NAN : more[j].at(2 * h), late ? NAN : more[j].at(2 * h + 1));
       }
     }
-    if (2 * t4 < g) lt[(8 * warp + 2 * t4) * C + t] = bt[t] * dk[2 * t4];
-    if (2 * t4 + 1 < g) lt[(8 * warp + 2 * t4 + 1) * C + t] = bt[t] * dk[2 * t4 + 1];
+    return;
   }
   __syncthreads();
-  // The inverse of I + L in halves of 32 tokens, [[A, 0], [B, D]]^-1 = [[A^-1, 0], [-D^-1 (B A^-1), D^-1]]: A and D by substitution, a
-  // thread a column - an unknown that is final is taken off all later rows -, the rest as two products.  (One substitution over
-  // 64 rows kept two warps busy and six waiting for a quarter of the kernel.)
-  constexpr int HALF = C / 2;
+  // The inverse of I + L from blocks of 16 tokens on, [[A, 0], [B, D]]^-1 = [[A^-1, 0], [-D^-1 (B A^-1), D^-1]]: the blocks on the diagonal by
+  // substitution, a thread a column - an unknown that is final is taken off all later rows -, then 32 and 64 as two products each.
+  // (Substitution over 32 rows was 640 instructions in a row for two warps, 5700 cycles; so 1300 and 1100.)
+  constexpr int HALF = C / 2, SUB = C / 4;
   if (tid < C) {
-    const int h0 = tid & HALF, col = tid - h0;
-    float x[HALF];
+    const int h0 = tid & ~(SUB - 1), col = tid - h0;
+    float x[SUB];
 #pragma unroll
-    for (int t = 0; t < HALF; ++t) x[t] = t == col ? 1.f : 0.f;
+    for (int t = 0; t < SUB; ++t) x[t] = t == col ? 1.f : 0.f;
 #pragma unroll
-    for (int s = 0; s < HALF - 1; ++s) {
+    for (int s = 0; s < SUB - 1; ++s) {
 #pragma unroll
-      for (int q = (s + 1) / 4 * 4; q < HALF; q += 4) {
+      for (int q = (s + 1) / 4 * 4; q < SUB; q += 4) {
         const float4 l = ld4(lt + (h0 + s) * C + h0 + q);
         if (q > s) x[q] = fmaf(-l.x, x[s], x[q]);
         if (q + 1 > s) x[q + 1] = fmaf(-l.y, x[s], x[q + 1]);
@@ -457,258 +579,362 @@ chunk_build_kernel(Args a) {
       }
     }
 #pragma unroll
-    for (int t = 0; t < HALF; ++t) {
+    for (int t = 0; t < SUB; ++t) {
       inv[(h0 + t) * LDT + tid] = x[t];
-      if (h0 == 0) inv[t * LDT + HALF + tid] = 0.f;
+      if (h0 & SUB) inv[(h0 - SUB + t) * LDT + tid] = 0.f;
     }
   }
   __syncthreads();
-  {
-    const int m = (warp & 1) * 16, c = (warp >> 1) * 8;      // a warp 16 rows x 8 columns of the 32 x 32
+  {      // 16 -> 32, twice, a thread two values of a column: as many rounded sums as the substitution had
+    const int r0 = (tid >> 7) * HALF + SUB, row = r0 + (tid >> 3 & 15), c = r0 - SUB + 2 * (tid & 7);
+    auto dot = [&](const float* left, int step, int k0) {      // sum over 16 k: left[k step] inv[k0 + k][c], [c + 1]
+      float x = 0.f, y = 0.f;
+#pragma unroll 4
+      for (int k = 0; k < SUB; ++k) {
+        const float2 r = *reinterpret_cast<const float2*>(inv + (k0 + k) * LDT + c);
+        x = fmaf(left[k * step], r.x, x);
+        y = fmaf(left[k * step], r.y, y);
+      }
+      return make_float2(x, y);
+    };
+    const float2 ba = dot(lt + (r0 - SUB) * C + row, C, r0 - SUB);      // B A^-1 (L is kept transposed)
+    st2(inv + row * LDT + c, ba.x, ba.y);
+    __syncthreads();
+    float2 x = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int k = r0; k <= row; ++k) {
+      const float2 r = *reinterpret_cast<const float2*>(inv + k * LDT + c);
+      x.x = fmaf(inv[row * LDT + k], r.x, x.x);
+      x.y = fmaf(inv[row * LDT + k], r.y, x.y);
+    }
+    __syncthreads();
+    st2(inv + row * LDT + c, -x.x, -x.y);
+    __syncthreads();
+  }
+  {      // 32 -> 64: a warp 16 rows x 8 columns
+    const int m = HALF + (warp & 1) * 16, c = (warp >> 1) * 8;
+    float* block = inv + (m + g) * LDT + c + 2 * t4;
     Sum ba;
-#pragma unroll
-    for (int k = 0; k < HALF; k += 8) {      // B A^-1, B being L's lower half (kept transposed)
+#pragma unroll 1
+    for (int k = 0; k < HALF; k += 8) {
       Two l[4], r[2];
-      const float* p = lt + (k + t4) * C + HALF + m + g;
-      l[0] = Two(p[0]);
-      l[1] = Two(p[8]);
-      l[2] = Two(p[4 * C]);
-      l[3] = Two(p[4 * C + 8]);
+      const float* p = lt + (k + t4) * C + m + g;
+      split2(l[0], l[1], p[0], p[8]);
+      split2(l[2], l[3], p[4 * C], p[4 * C + 8]);
       load_b(r, inv + k * LDT + c, LDT, g, t4);
       mma3(ba, l, r);
     }
-    st2(inv + (HALF + m + g) * LDT + c + 2 * t4, ba.at(0), ba.at(1));
-    st2(inv + (HALF + m + g + 8) * LDT + c + 2 * t4, ba.at(2), ba.at(3));
+    st2(block, ba.at(0), ba.at(1));
+    st2(block + 8 * LDT, ba.at(2), ba.at(3));
     __syncthreads();
     Sum dba;
-#pragma unroll
-    for (int k = 0; k < HALF; k += 8) {
+#pragma unroll 1
+    for (int k = HALF; k < C; k += 8) {
       Two l[4], r[2];
-      load_a(l, inv + (HALF + m) * LDT + HALF + k, LDT, g, t4);
-      load_b(r, inv + (HALF + k) * LDT + c, LDT, g, t4);
+      load_a(l, inv + m * LDT + k, LDT, g, t4);
+      load_b(r, inv + k * LDT + c, LDT, g, t4);
       mma3(dba, l, r);
     }
     float x[4] = {dba.at(0), dba.at(1), dba.at(2), dba.at(3)};
-    if (any_not_finite(x)) {
+    if (any_not_finite(x)) {      // element by element, and only up to the diagonal
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int row = m + g + 8 * (e >> 1), col = c + 2 * t4 + (e & 1);
         x[e] = 0.f;
-        for (int k = 0; k <= row; ++k) x[e] = fmaf(inv[(HALF + row) * LDT + HALF + k], inv[(HALF + k) * LDT + col], x[e]);
+#pragma unroll 1
+        for (int k = HALF; k <= row; ++k) x[e] = fmaf(inv[row * LDT + k], inv[k * LDT + col], x[e]);
       }
     }
     __syncthreads();
-    st2(inv + (HALF + m + g) * LDT + c + 2 * t4, -x[0], -x[1]);
-    st2(inv + (HALF + m + g + 8) * LDT + c + 2 * t4, -x[2], -x[3]);
+    st2(block, -x[0], -x[1]);
+    st2(block + 8 * LDT, -x[2], -x[3]);
   }
-  copies_done<0>();
   __syncthreads();
-  // W and U0: a warp 16 rows (warp % 4) of every other group of 32 columns
-  auto multiply = [&](const float* right, int ldr, int columns, const float* scale, float* out, int ldo) {
-    const int m0 = (warp & 3) * 16;
-    for (int n0 = (warp >> 2) * 32; n0 < columns; n0 += 64) {
-      Sum sum[4];
-      for (int k = 0; k < m0 + 16; k += 8) {      // (the inverse is zero behind its diagonal)
-        Two x[4];
-        load_a(x, inv + m0 * LDT + k, LDT, g, t4);
-        const float s0 = scale ? scale[k + t4] : 1.f, s1 = scale ? scale[k + t4 + 4] : 1.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          Two y[2];
-          y[0] = Two(right[(k + t4) * ldr + n0 + 8 * j + g] * s0);
-          y[1] = Two(right[(k + t4 + 4) * ldr + n0 + 8 * j + g] * s1);
-          mma3(sum[j], x, y);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float c[4] = {sum[j].at(0), sum[j].at(1), sum[j].at(2), sum[j].at(3)};
-        if (any_not_finite(c)) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int t = m0 + g + 8 * (e >> 1), col = n0 + 8 * j + 2 * t4 + (e & 1);
-            c[e] = 0.f;
-            for (int k = 0; k <= t; ++k) c[e] = fmaf(inv[t * LDT + k], right[k * ldr + col] * (scale ? scale[k] : 1.f), c[e]);
-          }
-        }
-        st2(out + (size_t)(m0 + g) * ldo + n0 + 8 * j + 2 * t4, c[0], c[1]);
-        st2(out + (size_t)(m0 + g + 8) * ldo + n0 + 8 * j + 2 * t4, c[2], c[3]);
-      }
-    }
-  };
-  multiply(gs, ld, dp, nullptr, a.w + unit * C * dp, dp);
+  values_there();
+  // W and U0, the inverse times diag(beta) times K~ and times V side by side: a warp two tiles of 16 rows, one of the upper and one
+  // of the lower half so that all have as much of the inverse before the diagonal, in 32 columns
   for (int v0 = 0; v0 < a.vp; v0 += VT) {
     if (v0 > 0) {
+      bulk_may_follow();
       __syncthreads();
-      fetch_values(v0);
-      copies_done<0>();
+      fetch_values(ks, v0);
+      values_there();
       __syncthreads();
     }
-    multiply(ks, VT + 4, min(VT, a.vp - v0), bt, a.u + unit * C * a.vp + v0, a.vp);
+    const int columns = dp + min(VT, a.vp - v0);
+#pragma unroll 1
+    for (int n0 = (v0 ? dp : 0) + (warp >> 1) * 32; n0 < columns; n0 += 128) {
+      const bool keys = n0 < dp;
+      const float* right = keys ? gs + n0 : ks + n0 - dp;
+      const int ldr = keys ? ld : VT + 4;
+      float* out = keys ? a.w + unit * C * row_floats(dp) + n0 : a.u + unit * C * a.vp + (size_t)(v0 + n0 - dp) * C;
+      const int ldo = keys ? row_floats(dp) : 8, next = keys ? 8 : 8 * C;      // floats to the next token, to the next eight columns
+#pragma unroll 1
+      for (int side = 0; side < 2; ++side) {
+        const int m0 = 16 * (side ? 3 - (warp & 1) : warp & 1);
+        Sum sum[4];
+#pragma unroll 1
+        for (int k = 0; k < m0 + 16; k += 8) {      // (the inverse is zero behind its diagonal)
+          Two l[4];
+          load_a(l, inv + m0 * LDT + k, LDT, g, t4, bt[k + t4], bt[k + t4 + 4]);
+          const float* r = right + (k + t4) * ldr + g;
+          if (keys) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              Two y[2];
+              split2(y[0], y[1], r[8 * j], r[4 * ldr + 8 * j]);
+              mma3(sum[j], l, y);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) mma2(sum[j], l, r[8 * j], r[4 * ldr + 8 * j]);
+          }
+        }
+        float* o = out + (size_t)(m0 + g) * ldo + 2 * t4;
+        unsigned bad = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float c[4] = {sum[j].at(0), sum[j].at(1), sum[j].at(2), sum[j].at(3)};
+          st2(o + j * next, late ? NAN : c[0], late ? NAN : c[1]);
+          st2(o + j * next + 8 * ldo, c[2], c[3]);
+          bad |= any_not_finite(c) ? 15u << 4 * j : 0;
+        }
+#pragma unroll 1
+        for (; bad; bad &= bad - 1) {      // element by element, and only up to the diagonal
+          const int j = __ffs(bad) - 1 >> 2, e = __ffs(bad) - 1 & 3, t = m0 + g + 8 * (e >> 1), col = 8 * j + 2 * t4 + (e & 1);
+          float y = 0.f;
+#pragma unroll 1
+          for (int k = 0; k <= t; ++k) y = fmaf(inv[t * LDT + k] * bt[k], right[k * ldr + col], y);
+          o[j * next + (e >> 1) * 8 * ldo + (e & 1)] = y;
+        }
+      }
+    }
   }
 }
 
 // -------------------------------------------------------------------------------------------------------------- state
 
-template <int CB>                      // value columns of a block
-struct StateLayout {                   // float offsets
-  // rows of S and U in two parts: strides at which the reads of a half warp, two rows apart (S) or one (U), fall into different banks
-  static constexpr int LDU = CB + 8, LDS2 = CB + 2, LDU2 = CB + 4;
-  int ld, k, u, p, stage, s2, u2, floats;
-  __host__ __device__ StateLayout(int dp, bool delta) {
-    ld = dp + 8;
-    k = delta ? C * ld : 0;            // a stage: W [C][ld], K^ [C][ld], U0 or V [C][LDU], P_C [2][dp]
-    u = k + C * ld;
-    p = u + C * LDU;
-    stage = p + 2 * dp;
-    s2 = 2 * stage;                    // [dp][LDS2] pairs, [C][LDU2] pairs
-    u2 = s2 + (delta ? 2 * dp * LDS2 : 0);
-    floats = u2 + 2 * C * LDU2;
-  }
-};
-
-template <int CB, bool DELTA>
-__global__ void __launch_bounds__(THREADS, 1)
-chunk_state_kernel(Args a) {
-  using L = StateLayout<CB>;
-  constexpr int LDU = L::LDU, LDS2 = L::LDS2, LDU2 = L::LDU2, NT = CB / 8;
-  extern __shared__ __align__(16) float sm[];
-  const L at(a.dp, DELTA);
-  const int dp = a.dp, ld = at.ld, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
-  const int head = blockIdx.x, v0 = blockIdx.y * CB, item = blockIdx.z;
-  const int n_new = a.q_len[item], row0 = a.q_start[item], slot = a.seq_slot[item];
-  if (n_new < a.min_tokens) return;
-  int base = 0;                        // the number of this item's first chunk
+// The chunks that an item's walk of this slab covers, and the number of the item's first chunk; from >= to: none.
+__device__ __forceinline__ void walk_of(const Args& a, int item, int& base, int& from, int& to) {
+  base = from = to = 0;
+  if (a.q_len[item] < a.min_tokens) return;
+#pragma unroll 1
   for (int b = 0; b < item; ++b)
     if (a.q_len[b] >= a.min_tokens) base += (a.q_len[b] + C - 1) / C;
-  const int from = max(a.c0, base), to = min(a.c1, base + (n_new + C - 1) / C);
-  if (from >= to) return;
-  uint2 *s2 = reinterpret_cast<uint2*>(sm + at.s2), *u2 = reinterpret_cast<uint2*>(sm + at.u2);
+  from = max(a.c0, base);
+  to = min(a.c1, base + (a.q_len[item] + C - 1) / C);
+}
+// P_C S_0 + K^^T U, P_C in two parts: products of decays near one are all rounded to the same side, a constant's to the same value.
+__device__ __forceinline__ float decayed(float s, float p, float p_low, float more) {
+  const float low = s * p_low;
+  return fmaf(s, p, more + (fabsf(low) <= 3.402823466e38f ? low : 0.f));      // (an infinite state stays one)
+}
+
+// Linear attention: U = V does not need the state, so K^^T V of all chunks is there and only P_C S_0 + K^^T V is walked, a thread four
+// elements of the state, their chunks' S_0 written over K^^T V.  (29 chunks of 16 heads of 128 x 128: 48 us with the products inside the
+// walk; the scan takes 9, the products 16 more in chunk_build.)
+constexpr int SCAN_THREADS = 256, SCAN_AHEAD = 4;
+__global__ void __launch_bounds__(SCAN_THREADS)
+chunk_scan_kernel(Args a) {
+  const int dp = a.dp, head = blockIdx.y, item = blockIdx.z;
+  const int i = (blockIdx.x * SCAN_THREADS + threadIdx.x) * 4, d = i / a.vp, c = i - d * a.vp;
+  int base, from, to;
+  walk_of(a, item, base, from, to);
+  if (from >= to || d >= dp) return;
+  const bool in = d < a.dim && c < a.vdim;
+  float* st = a.state + (size_t)a.seq_slot[item] * a.state_stride + (size_t)head * a.dim * a.vdim + (size_t)d * a.vdim + c;
   mi::grid_dependency_sync();
-  // which 16 bytes of a row of W and K^ this thread copies, of every k_rows-th row
-  const int per_row = dp / 4, k_rows = THREADS / per_row, kt = tid / per_row, kd = (tid - kt * per_row) * 4;
-  auto fetch = [&](int c, float* buf) {
+  float S[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) S[e] = in ? st[e] : 0.f;      // (a state's row may start at any multiple of four bytes)
+  float4 more[SCAN_AHEAD];
+  float p[SCAN_AHEAD], low[SCAN_AHEAD];
+  for (int c0 = from; c0 < to; c0 += SCAN_AHEAD) {
+#pragma unroll
+    for (int k = 0; k < SCAN_AHEAD; ++k) {
+      if (c0 + k < to) {
+        const size_t unit = (size_t)(c0 + k - a.c0) * a.heads + head;
+        more[k] = ld4(a.s0 + unit * dp * a.vp + i);
+        p[k] = a.pc[unit * 2 * dp + d];
+        low[k] = a.pc[unit * 2 * dp + dp + d];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < SCAN_AHEAD; ++k) {
+      if (c0 + k < to) {
+        st4(a.s0 + ((size_t)(c0 + k - a.c0) * a.heads + head) * dp * a.vp + i, make_float4(S[0], S[1], S[2], S[3]));
+        S[0] = decayed(S[0], p[k], low[k], more[k].x);
+        S[1] = decayed(S[1], p[k], low[k], more[k].y);
+        S[2] = decayed(S[2], p[k], low[k], more[k].z);
+        S[3] = decayed(S[3], p[k], low[k], more[k].w);
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (in) st[e] = S[e];
+}
+
+// The delta rule's walk.  A chunk is two products in a chain, W S_0 over the channels and K^^T U over the tokens, with the state in registers
+// between them; sixteen warps split the first one's channels in quarters (of 32 columns: in halves) and add up the parts in shared memory, and
+// a chunk's W, K^ and U0 come by four bulk copies one chunk ahead.  (32 chunks of 8 heads of 128 x 128: 100 us by eight warps that split no
+// channels, 16 columns a block and 16-byte copies by all threads; so 50.)
+constexpr int STATE_THREADS = 512;
+template <int CB>                      // value columns of a block
+struct StateLayout {                   // float offsets
+  static constexpr int NT = CB / 8, PARTS = CB == 32 ? 2 : 4;
+  // rows of S, of U and of the partial sums: strides at which a warp's reads, two rows apart (S) or one (U), fall into different banks
+  static constexpr int LDS = CB + 4, LDU = CB == 8 ? 8 : CB + 8, LDX = CB + 2;
+  int k, u, p, stage, s, ut, x, bars, floats;
+  __host__ __device__ explicit StateLayout(int dp) {
+    k = C * row_floats(dp);            // a stage: W, K^ [C][row_floats(dp)], U0 [NT][C][8], P_C [2][dp]
+    u = 2 * k;
+    p = u + C * CB;
+    stage = p + 2 * dp;
+    s = 2 * stage;                     // [dp][LDS]
+    ut = s + dp * LDS;                 // [C][LDU]
+    x = ut + C * LDU;                  // [PARTS][C][LDX]
+    bars = x + PARTS * C * LDX;
+    floats = bars + 4;
+  }
+  size_t bytes() const { return (size_t)floats * sizeof(float); }
+};
+
+template <int CB>
+__global__ void __launch_bounds__(STATE_THREADS, 1)
+chunk_state_kernel(Args a) {
+  using L = StateLayout<CB>;
+  constexpr int LDS = L::LDS, LDU = L::LDU, LDX = L::LDX, NT = L::NT, PARTS = L::PARTS;
+  constexpr int ST = NT > 1 ? NT / 2 : 1;      // 8-column tiles of S that a warp holds
+  extern __shared__ __align__(16) float sm[];
+  const L at(a.dp);
+  const int dp = a.dp, ld = row_floats(dp), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int head = blockIdx.x, v0 = blockIdx.y * CB, item = blockIdx.z;
+  int base, from, to;
+  walk_of(a, item, base, from, to);
+  if (from >= to) return;
+  float *ss = sm + at.s, *us = sm + at.ut;
+  float* parts = sm + at.x;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm + at.bars);
+  if (tid == 0) {
+    bar_init(full);
+    bar_init(full + 1);
+    bars_ready();
+  }
+  mi::grid_dependency_sync();
+  __syncthreads();
+  auto fetch = [&](int c) {      // by one thread, into a stage that everyone has left
     const size_t unit = (size_t)(c - a.c0) * a.heads + head;
-    if (kt < k_rows) {
-      const size_t from_row = (unit * C + kt) * dp + kd;
-#pragma unroll 8
-      for (int t = kt; t < C; t += k_rows) {
-        if (DELTA) copy16(buf + t * ld + kd, a.w + from_row + (size_t)(t - kt) * dp, true);
-        copy16(buf + at.k + t * ld + kd, a.kh + from_row + (size_t)(t - kt) * dp, true);
-      }
-    }
-    const int first = (c - base) * C, n = min(C, n_new - first);
-#pragma unroll
-    for (int i = tid; i < C * CB / 4; i += THREADS) {
-      const int t = i / (CB / 4), col = (i % (CB / 4)) * 4;
-      if (DELTA) {
-        copy16(buf + at.u + t * LDU + col, a.u + (unit * C + t) * a.vp + v0 + col, true);
-      } else {
-        const bool in = t < n && v0 + col < a.vdim;
-        copy16(buf + at.u + t * LDU + col, a.raw + (in ? (size_t)(row0 + first + t) * (a.heads * a.vdim) + head * a.vdim + v0 + col : 0), in);
-      }
-    }
-    if (tid < dp / 2) copy16(buf + at.p + 4 * tid, a.pc + unit * 2 * dp + 4 * tid, true);
-    copies_begun();
+    float* buf = sm + ((c - from) & 1) * at.stage;
+    uint64_t* bar = full + ((c - from) & 1);
+    bar_expect(bar, at.stage * 4);
+    bulk_copy(buf, a.w + unit * C * ld, C * ld, bar);
+    bulk_copy(buf + at.u, a.u + unit * C * a.vp + (size_t)v0 * C, C * CB, bar);
+    bulk_copy(buf + at.k, a.kh + unit * C * ld, C * ld, bar);
+    bulk_copy(buf + at.p, a.pc + unit * 2 * dp, 2 * dp, bar);
   };
-  fetch(from, sm);
-  // this warp's rows of S: 16 key channels - a lane those numbered 2 g and 2 g + 1 -, all columns of the block
-  const int d0 = 16 * warp + 2 * g;
-  const bool holds = 16 * warp < dp;
-  float* st = a.state + (size_t)slot * a.state_stride + (size_t)head * a.dim * a.vdim;
-  float S[NT][4];
+  if (tid == 0) fetch(from);
+  // this warp's part of S: 16 key channels - a lane those numbered 2 g and 2 g + 1 -, ST tiles of columns from j0 on.  With one
+  // tile for all the upper eight warps hold none and have half of the tokens of K^^T U.
+  const int d0 = 16 * (warp & 7) + 2 * g, j0 = NT > 1 ? (warp >> 3) * ST : 0;
+  const bool adds = 16 * (warp & 7) < dp, holds = adds && (NT > 1 || warp < 8);
+  float* st = a.state + (size_t)a.seq_slot[item] * a.state_stride + (size_t)head * a.dim * a.vdim;
+  float S[ST][4];
   auto keep = [&]() {
-    if (DELTA && holds) {
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
+    for (int j = 0; j < ST; ++j)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const Two x(S[j][2 * h]), y(S[j][2 * h + 1]);
-          *reinterpret_cast<uint4*>(s2 + (d0 + h) * LDS2 + 8 * j + 2 * t4) = make_uint4(x.hi, x.lo, y.hi, y.lo);
-        }
-    }
+      for (int h = 0; h < 2; ++h) st2(ss + (d0 + h) * LDS + 8 * (j0 + j) + 2 * t4, S[j][2 * h], S[j][2 * h + 1]);
   };
 #pragma unroll
-  for (int j = 0; j < NT; ++j)
+  for (int j = 0; j < ST; ++j)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const int d = d0 + (e >> 1), c = v0 + 8 * j + 2 * t4 + (e & 1);
+      const int d = d0 + (e >> 1), c = v0 + 8 * (j0 + j) + 2 * t4 + (e & 1);
       S[j][e] = (holds && d < a.dim && c < a.vdim) ? st[(size_t)d * a.vdim + c] : 0.f;
     }
-  keep();
+  if (holds) keep();
+  __syncthreads();
+  bool late = false;      // a wait for this block's own copies ran out: the state becomes NaN
   for (int c = from; c < to; ++c) {
-    const float* cur = sm + ((c - from) & 1) * at.stage;
+    const int stage = (c - from) & 1;
+    const float* cur = sm + stage * at.stage;
     const size_t unit = (size_t)(c - a.c0) * a.heads + head;
-    if (c + 1 < to) {
-      fetch(c + 1, sm + ((c + 1 - from) & 1) * at.stage);
-      copies_done<1>();
-    } else {
-      copies_done<0>();
-    }
-    __syncthreads();
-    if (holds) {
-#pragma unroll
-      for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) st2(a.s0 + (unit * dp + d0 + h) * a.vp + v0 + 8 * j + 2 * t4, S[j][2 * h], S[j][2 * h + 1]);
-    }
-    if (DELTA) {      // U = U0 - W S_0: a warp 16 tokens, half of the columns
-      constexpr int HT = NT / 2;
-      const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * (CB / 2);
+    if (tid == 0 && c + 1 < to) fetch(c + 1);
+    late |= !bar_wait(full + stage, ((c - from) >> 1) & 1);
+    {      // W S_0: a warp 16 tokens and a part of the channels - all columns, or of 32 half
+      constexpr int HT = CB == 32 ? 2 : NT;
+      const int m0 = (warp & 3) * 16, part = (warp >> 2) % PARTS, n0 = CB == 32 ? (warp >> 3) * 16 : 0;
+      const int k0 = part * (dp / PARTS), k1 = k0 + dp / PARTS;
       Sum x[HT];
 #pragma unroll 4
-      for (int k = 0; k < dp; k += 8) {
+      for (int k = k0; k < k1; k += 8) {
         Two w[4];
         load_a_pairs(w, cur + m0 * ld + k, ld, g, t4);
 #pragma unroll
         for (int j = 0; j < HT; ++j) {
           Two s[2];
-          load_b(s, s2 + k * LDS2 + n0 + 8 * j, LDS2, g, 2 * t4, 2 * t4 + 1);
+          const float* row = ss + (k + 2 * t4) * LDS + n0 + 8 * j + g;
+          split2(s[0], s[1], row[0], row[LDS]);
           mma3(x[j], w, s);
         }
       }
 #pragma unroll
       for (int j = 0; j < HT; ++j)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int t = m0 + g + 8 * h, col = n0 + 8 * j + 2 * t4;
-          const float2 u0 = *reinterpret_cast<const float2*>(cur + at.u + t * LDU + col);
-          const float y0 = u0.x - x[j].at(2 * h), y1 = u0.y - x[j].at(2 * h + 1);
-          st2(a.u + (unit * C + t) * a.vp + v0 + col, y0, y1);
-          const Two p(y0), q(y1);
-          *reinterpret_cast<uint4*>(u2 + t * LDU2 + col) = make_uint4(p.hi, p.lo, q.hi, q.lo);
-        }
-    } else {
+        for (int h = 0; h < 2; ++h) st2(parts + (part * C + m0 + g + 8 * h) * LDX + n0 + 8 * j + 2 * t4, x[j].at(2 * h), x[j].at(2 * h + 1));
+    }
+    if (holds) {
 #pragma unroll
-      for (int i = tid; i < C * CB; i += THREADS) {
-        const Two p(cur[at.u + i / CB * LDU + i % CB]);
-        u2[i / CB * LDU2 + i % CB] = make_uint2(p.hi, p.lo);
-      }
+      for (int j = 0; j < ST; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) st2(a.s0 + (unit * dp + d0 + h) * a.vp + v0 + 8 * (j0 + j) + 2 * t4, S[j][2 * h], S[j][2 * h + 1]);
     }
     __syncthreads();
-    if (holds) {      // S = diag(P_C) S_0 + K^^T U
-      Sum more[NT];
 #pragma unroll
-      for (int k = 0; k < C; k += 8) {
+    for (int i = tid; i < C * CB; i += STATE_THREADS) {      // U = U0 - W S_0, element i of [NT][C][8]
+      const int t = (i >> 3) & (C - 1), col = (i / (8 * C)) * 8 + (i & 7);
+      float x = parts[t * LDX + col];
+#pragma unroll
+      for (int q = 1; q < PARTS; ++q) x += parts[(q * C + t) * LDX + col];
+      const float y = cur[at.u + i] - x;
+      a.u[unit * C * a.vp + (size_t)v0 * C + i] = y;
+      us[t * LDU + col] = y;
+    }
+    __syncthreads();
+    Sum more[ST];
+    if (adds) {      // S = diag(P_C) S_0 + K^^T U
+      constexpr int KU = NT > 1 ? C : C / 2;
+      const int k0 = NT > 1 ? 0 : (warp >> 3) * KU;
+#pragma unroll
+      for (int k = 0; k < KU; k += 8) {
         Two x[4];
-        load_a_transposed(x, cur + at.k + k * ld + 16 * warp, ld, g, t4);
+        load_a_transposed(x, cur + at.k + (k0 + k) * ld + 16 * (warp & 7), ld, g, t4);
 #pragma unroll
-        for (int j = 0; j < NT; ++j) {
+        for (int j = 0; j < ST; ++j) {
           Two y[2];
-          load_b(y, u2 + k * LDU2 + 8 * j, LDU2, g, t4, t4 + 4);
+          load_b(y, us + (k0 + k) * LDU + 8 * (j0 + j), LDU, g, t4);
           mma3(more[j], x, y);
         }
       }
+    }
+    if (NT == 1) {
+      if (warp >= 8) st4(parts + ((warp & 7) * 32 + lane) * 4, make_float4(more[0].at(0), more[0].at(1), more[0].at(2), more[0].at(3)));
+      __syncthreads();
+      if (warp < 8) {
+        const float4 x = ld4(parts + (warp * 32 + lane) * 4);
+        add2(more[0].c[0], more[0].c[1], x.x, x.y);
+        add2(more[0].c[2], more[0].c[3], x.z, x.w);
+      }
+    }
+    if (holds) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {      // (P_C in two parts: products of decays near one are all rounded to the same side, a constant's to the same value)
+      for (int h = 0; h < 2; ++h) {
         const float p = cur[at.p + d0 + h], p_low = cur[at.p + dp + d0 + h];
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
+        for (int j = 0; j < ST; ++j)
 #pragma unroll
-          for (int e = 2 * h; e < 2 * h + 2; ++e) {
-            const float low = S[j][e] * p_low;
-            S[j][e] = fmaf(S[j][e], p, more[j].at(e) + (fabsf(low) <= 3.402823466e38f ? low : 0.f));      // (an infinite state stays one)
-          }
+          for (int e = 2 * h; e < 2 * h + 2; ++e) S[j][e] = decayed(S[j][e], p, p_low, more[j].at(e));
       }
       keep();
     }
@@ -716,114 +942,133 @@ chunk_state_kernel(Args a) {
   }
   if (holds) {
 #pragma unroll
-    for (int j = 0; j < NT; ++j)
+    for (int j = 0; j < ST; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int d = d0 + (e >> 1), c = v0 + 8 * j + 2 * t4 + (e & 1);
-        if (d < a.dim && c < a.vdim) st[(size_t)d * a.vdim + c] = S[j][e];
+        const int d = d0 + (e >> 1), c = v0 + 8 * (j0 + j) + 2 * t4 + (e & 1);
+        if (d < a.dim && c < a.vdim) st[(size_t)d * a.vdim + c] = late ? NAN : S[j][e];
       }
   }
 }
 
 // -------------------------------------------------------------------------------------------------------------- out
 
-constexpr int LDA = C + 8, LDV = OB + 4, OUT_THREADS = 128;
-__host__ __device__ inline size_t out_smem(int dp) { return (size_t)(C * (dp + 8) + C * LDA + dp * LDV + C * LDV) * sizeof(float); }
+// Three sums of up to 64 inner values each, one after the other: Q~ S_0 over the lower half of the channels, over the upper, A U over the
+// tokens.  Their operands take turns in two buffers, so three blocks share an SM (with all operands there at once two blocks did: linear
+// attention, 29 chunks of 16 heads of 128 x 128, 37 us).
+constexpr int LDL = C + 8, LDV = OB + 4, OUT_THREADS = 128;
+constexpr int OUT_BUFFER = C * LDL + C * LDV;
+static_assert(CHUNK_MAX_DIM / 2 <= C, "half of the channels fit a buffer");
+constexpr size_t OUT_SMEM = 2 * OUT_BUFFER * sizeof(float);
 
 // A warp 32 tokens x 32 columns: four operand halves split in two parts serve 24 products; with 16 x 32 a warp the splitting took
 // half of the instructions.
 template <bool DELTA>
-__global__ void __launch_bounds__(OUT_THREADS)
+__global__ void __launch_bounds__(OUT_THREADS, 3)
 chunk_out_kernel(Args a) {
   extern __shared__ __align__(16) float sm[];
-  const int dp = a.dp, ldq = dp + 8;
-  float *qt = sm, *aa = qt + C * ldq, *s0 = aa + C * LDA, *us = s0 + dp * LDV;
+  const int dp = a.dp, half = dp / 2;
   __shared__ int found[2];
+  __shared__ __align__(8) uint64_t bars[3];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, head = blockIdx.y, v0 = blockIdx.z * OB;
-  if (tid == 0) find_chunk(a, a.c0 + blockIdx.x, found[0], found[1]);
+  if (tid == 0) {
+    find_chunk(a, a.c0 + blockIdx.x, found[0], found[1]);
+    for (int b = 0; b < 3; ++b) bar_init(bars + b);
+    bars_ready();
+  }
   mi::grid_dependency_sync();
   __syncthreads();
   const int item = found[0];
   if (item < 0) return;
   const int first = found[1] * C, n = min(C, a.q_len[item] - first), row0 = a.q_start[item] + first;
   const size_t unit = (size_t)blockIdx.x * a.heads + head;
-  {
-    const int per_row = dp / 4, rows = OUT_THREADS / per_row, t0 = tid / per_row, d = (tid - t0 * per_row) * 4;
-#pragma unroll 4
-    for (int t = t0; t < C && t0 < rows; t += rows) copy16(qt + t * ldq + d, a.qt + (unit * C + t) * dp + d, true);
-  }
-#pragma unroll 4
-  for (int i = tid; i < dp * (OB / 4); i += OUT_THREADS) {
-    const int d = i / (OB / 4), c = (i % (OB / 4)) * 4;
-    const bool in = v0 + c < a.vp;
-    copy16(s0 + d * LDV + c, a.s0 + (in ? (unit * dp + d) * a.vp + v0 + c : 0), in);
-  }
-  copies_begun();
-#pragma unroll 4
-  for (int i = tid; i < C * (C / 4); i += OUT_THREADS) {
-    const int t = i / (C / 4), s = (i % (C / 4)) * 4;
-    copy16(aa + t * LDA + s, a.at + (unit * C + t) * C + s, true);
-  }
-#pragma unroll 4
-  for (int i = tid; i < C * (OB / 4); i += OUT_THREADS) {
-    const int t = i / (OB / 4), c = (i % (OB / 4)) * 4;
-    const bool in = DELTA ? v0 + c < a.vp : t < n && v0 + c < a.vdim;
-    const float* from = DELTA ? a.u + (in ? (unit * C + t) * a.vp + v0 + c : 0)
-                              : a.raw + (in ? (size_t)(row0 + t) * (a.heads * a.vdim) + head * a.vdim + v0 + c : 0);
-    copy16(us + t * LDV + c, from, in);
-  }
-  copies_begun();
-  const int m0 = (warp & 1) * 32, n0 = (warp >> 1) * 32;
-  Sum sum[2][4];
-  auto multiply = [&](const float* left, int ldl, const float* right, int k) {      // eight inner values, in the order 0 2 4 6 1 3 5 7
-    Two x[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) load_a_pairs(x[i], left + (m0 + 16 * i) * ldl + k, ldl, g, t4);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float* r = right + (k + 2 * t4) * LDV + n0 + 8 * j + g;
-      Two y[2];
-      y[0] = Two(r[0]);
-      y[1] = Two(r[LDV]);
-#pragma unroll
-      for (int i = 0; i < 2; ++i) mma3(sum[i][j], x[i], y);
+  // Three rounds of 64 rows of the left side and up to 64 of the right, a thread a row of one of them; no values behind the last token
+  auto fetch = [&](int part) {
+    float* buf = sm + (part & 1) * OUT_BUFFER;
+    const int r = tid & (C - 1), columns = min(OB, (DELTA || part < 2 ? a.vp : a.vdim) - v0), rows = part < 2 ? half : DELTA ? C : n;
+    if (tid == 0) bar_expect(bars + part, (C * (part < 2 ? half : C) + rows * columns) * 4);
+    if (tid < C) {
+      if (part < 2) bulk_copy(buf + r * LDL, a.qt + (unit * C + r) * dp + part * half, half, bars + part);
+      else bulk_copy(buf + r * LDL, a.at + (unit * C + r) * C, C, bars + part);
+    } else {
+      float* to = buf + C * LDL + r * LDV;
+      if (r >= rows) {
+#pragma unroll 1
+        for (int c = 0; c < OB; c += 4) st4(to + c, make_float4(0.f, 0.f, 0.f, 0.f));
+      } else if (part < 2) {
+        bulk_copy(to, a.s0 + (unit * dp + part * half + r) * a.vp + v0, columns, bars + part);
+      } else if (!DELTA) {
+        bulk_copy(to, a.raw + (size_t)(row0 + r) * (a.heads * a.vdim) + head * a.vdim + v0, columns, bars + part);
+      } else if (8 * r < columns) {      // (groups of eight columns of all tokens)
+        bulk_copy(buf + C * LDL + r * 8 * C, a.u + unit * C * a.vp + (size_t)(v0 + 8 * r) * C, 8 * C, bars + part);
+      }
     }
   };
-  copies_done<1>();
-  __syncthreads();
-#pragma unroll 2
-  for (int k = 0; k < dp; k += 8) multiply(qt, ldq, s0, k);      // Q~ S_0
-  copies_done<0>();
-  __syncthreads();
-#pragma unroll 2
-  for (int k = 0; k < m0 + 32; k += 8) multiply(aa, LDA, us, k);      // A U: nothing behind the diagonal
-  float acc[2][4][4];
+  const int m0 = (warp & 1) * 32, n0 = (warp >> 1) * 32;
+  Sum sum[2][4];
+  auto multiply = [&](const float* buf, int k_end, int ldr, int next, auto plain) {      // plain: the right side is what tf32 holds
+#pragma unroll 1
+    for (int k = 0; k < k_end; k += 8) {      // eight inner values, in the order 0 2 4 6 1 3 5 7
+      Two x[2][4];
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < 2; ++i) load_a_pairs(x[i], buf + (m0 + 16 * i) * LDL + k, LDL, g, t4);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < 4; ++j) {
+        const float* r = buf + C * LDL + (k + 2 * t4) * ldr + (n0 / 8 + j) * next + g;
+        if (plain.value) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][j][e] = sum[i][j].at(e);
-      if (any_not_finite(acc[i][j])) {
+          for (int i = 0; i < 2; ++i) mma2(sum[i][j], x[i], r[0], r[ldr]);
+        } else {
+          Two y[2];
+          split2(y[0], y[1], r[0], r[ldr]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int t = m0 + 16 * i + g + 8 * (e >> 1), c = n0 + 8 * j + 2 * t4 + (e & 1);
-          float y = 0.f, z = 0.f;
-          for (int d = 0; d < a.dim; ++d) y = fmaf(qt[t * ldq + d], s0[d * LDV + c], y);
-          for (int s = 0; s <= t; ++s) z = fmaf(aa[t * LDA + s], us[s * LDV + c], z);
-          acc[i][j][e] = fabsf(z) <= 3.402823466e38f ? y + z : NAN;      // an infinite value: the recurrence adds it up over channels of both signs
+          for (int i = 0; i < 2; ++i) mma3(sum[i][j], x[i], y);
         }
       }
     }
+  };
+  fetch(0);
+  fetch(1);
+  bool late = false;
+#pragma unroll 1
+  for (int part = 0; part < 2; ++part) {
+    late |= !bar_wait(bars + part, 0);
+    multiply(sm + part * OUT_BUFFER, half, LDV, 8, std::false_type());
+    if (part == 0) {
+      bulk_may_follow();
+      __syncthreads();
+      fetch(2);
+    }
+  }
+  late |= !bar_wait(bars + 2, 0);
+  __syncthreads();      // (the zeros behind the last token)
+  multiply(sm, m0 + 32, DELTA ? 8 : LDV, DELTA ? 8 * C : 8, std::integral_constant<bool, !DELTA>());      // A U: nothing behind the diagonal; linear attention's U are the values
+  float* o = a.raw + (size_t)row0 * (a.heads * a.vdim) + head * a.vdim + v0;
+  unsigned bad = 0;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < 4; ++j) {
+      const float x[4] = {sum[i][j].at(0), sum[i][j].at(1), sum[i][j].at(2), sum[i][j].at(3)};
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int t = m0 + 16 * i + g + 8 * h, c = v0 + n0 + 8 * j + 2 * t4;
-        if (t < n && c < a.vdim) st2(a.raw + (size_t)(row0 + t) * (a.heads * a.vdim) + head * a.vdim + c, acc[i][j][2 * h], acc[i][j][2 * h + 1]);
+        const int t = m0 + 16 * i + g + 8 * h, c = n0 + 8 * j + 2 * t4;
+        if (t < n && v0 + c < a.vdim) st2(o + (size_t)t * (a.heads * a.vdim) + c, late ? NAN : x[2 * h], late ? NAN : x[2 * h + 1]);
       }
+      bad |= any_not_finite(x) ? 15u << 4 * (4 * i + j) : 0;
+    }
+  const float *aa = sm, *us = sm + C * LDL;
+#pragma unroll 1
+  for (; bad; bad &= bad - 1) {
+    const int b = __ffs(bad) - 1, e = b & 3, t = m0 + 16 * (b >> 4) + g + 8 * (e >> 1), c = n0 + 8 * (b >> 2 & 3) + 2 * t4 + (e & 1);
+    if (t >= n || v0 + c >= a.vdim) continue;
+    float y = 0.f, z = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < a.dim; ++d) y = fmaf(a.qt[(unit * C + t) * dp + d], a.s0[(unit * dp + d) * a.vp + v0 + c], y);
+#pragma unroll 1
+    for (int s = 0; s <= t; ++s) z = fmaf(aa[t * LDL + s], DELTA ? us[(c / 8 * C + s) * 8 + (c & 7)] : us[s * LDV + c], z);
+    o[(size_t)t * (a.heads * a.vdim) + c] = fabsf(z) <= 3.402823466e38f ? y + z : NAN;      // an infinite value: the recurrence adds it up over channels of both signs
+  }
 }
 
 int most_chunks(int T, int items) { return T / C + items; }      // every item's last chunk may be a short one
@@ -861,39 +1106,41 @@ int chunked_state_run(const ChunkedStateArgs& in, int T, float* scratch, cudaStr
   const int total = most_chunks(T, in.items), most = slab_chunks(in.heads, in.dim, in.vdim, delta), slab = total < most ? total : most;
   const size_t units = (size_t)slab * in.heads;
   a.w = scratch;
-  a.u = a.w + (delta ? units * C * a.dp : 0);
+  a.kh = a.w + (delta ? units * C * row_floats(a.dp) : 0);
+  a.u = a.kh + (delta ? units * C * row_floats(a.dp) : 0);
   a.at = a.u + (delta ? units * C * a.vp : 0);
-  a.kh = a.at + units * C * C;
-  a.qt = a.kh + units * C * a.dp;
+  a.qt = a.at + units * C * C;
   a.s0 = a.qt + units * C * a.dp;
   a.pc = a.s0 + units * a.dp * a.vp;
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !configured[dev]) {
-    const size_t build = BuildLayout(CHUNK_MAX_DIM).floats * sizeof(float), out = out_smem(CHUNK_MAX_DIM);
+    const size_t build = BuildLayout(CHUNK_MAX_DIM).floats * sizeof(float), out = OUT_SMEM;
     if (!allow(chunk_build_kernel<true>, build) || !allow(chunk_build_kernel<false>, build) || !allow(chunk_out_kernel<true>, out) ||
-        !allow(chunk_out_kernel<false>, out) || !allow(chunk_state_kernel<16, true>, StateLayout<16>(CHUNK_MAX_DIM, true).floats * sizeof(float)) ||
-        !allow(chunk_state_kernel<32, true>, StateLayout<32>(CHUNK_MAX_DIM, true).floats * sizeof(float)) ||
-        !allow(chunk_state_kernel<16, false>, StateLayout<16>(CHUNK_MAX_DIM, false).floats * sizeof(float)) ||
-        !allow(chunk_state_kernel<32, false>, StateLayout<32>(CHUNK_MAX_DIM, false).floats * sizeof(float)))
+        !allow(chunk_out_kernel<false>, out) || !allow(chunk_state_kernel<8>, StateLayout<8>(CHUNK_MAX_DIM).bytes()) ||
+        !allow(chunk_state_kernel<16>, StateLayout<16>(CHUNK_MAX_DIM).bytes()) || !allow(chunk_state_kernel<32>, StateLayout<32>(CHUNK_MAX_DIM).bytes()))
       return mi_fail("chunked_state: the shared memory was refused");
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  // 16 value columns a block while such blocks fit the SMs in one round, 32 beyond: half as many chains, each a little longer
-  const bool wide = (long long)in.heads * in.items * (a.vp / 16) > mi::sm_count();
+  // Value columns of a chunk_state block: as few as still put every block on an SM of its own, 32 where none does
+  auto blocks = [&](int cb) { return (long long)in.heads * in.items * (a.vp / cb); };
+  const int cb = blocks(8) <= mi::sm_count() ? 8 : blocks(16) <= mi::sm_count() ? 16 : 32;
   for (int c0 = 0; c0 < total; c0 += slab) {
     a.c0 = c0;
     a.c1 = c0 + slab < total ? c0 + slab : total;
     mi::launch(delta ? chunk_build_kernel<true> : chunk_build_kernel<false>, dim3(a.c1 - a.c0, in.heads), dim3(THREADS),
                BuildLayout(a.dp).floats * sizeof(float), stream, a);
-    if (wide)
-      mi::launch(delta ? chunk_state_kernel<32, true> : chunk_state_kernel<32, false>, dim3(in.heads, a.vp / 32, in.items), dim3(THREADS),
-                 StateLayout<32>(a.dp, delta).floats * sizeof(float), stream, a);
+    const dim3 grid(in.heads, a.vp / cb, in.items);
+    if (!delta)
+      mi::launch(chunk_scan_kernel, dim3((a.dp * a.vp / 4 + SCAN_THREADS - 1) / SCAN_THREADS, in.heads, in.items), dim3(SCAN_THREADS), 0, stream, a);
+    else if (cb == 8)
+      mi::launch(chunk_state_kernel<8>, grid, dim3(STATE_THREADS), StateLayout<8>(a.dp).bytes(), stream, a);
+    else if (cb == 16)
+      mi::launch(chunk_state_kernel<16>, grid, dim3(STATE_THREADS), StateLayout<16>(a.dp).bytes(), stream, a);
     else
-      mi::launch(delta ? chunk_state_kernel<16, true> : chunk_state_kernel<16, false>, dim3(in.heads, a.vp / 16, in.items), dim3(THREADS),
-                 StateLayout<16>(a.dp, delta).floats * sizeof(float), stream, a);
+      mi::launch(chunk_state_kernel<32>, grid, dim3(STATE_THREADS), StateLayout<32>(a.dp).bytes(), stream, a);
     mi::launch(delta ? chunk_out_kernel<true> : chunk_out_kernel<false>, dim3(a.c1 - a.c0, in.heads, (a.vp + OB - 1) / OB), dim3(OUT_THREADS),
-               out_smem(a.dp), stream, a);
+               OUT_SMEM, stream, a);
   }
   MI_LAUNCH_OK("chunked_state");
   return 0;

@@ -15,7 +15,7 @@ struct ChunkedStateArgs {
   const float* g;                             // decays in 0 .. 1: [tokens, heads * dim], their logarithms [tokens, heads], or [heads] (ChunkDecay)
   int decay;
   const float* beta;                          // [tokens, heads] write strengths of the delta rule, or null: S <- diag(g) S + k v^T
-  float* raw;                                 // [tokens, heads * vdim]: the values in, the read-outs out
+  float* raw;                                 // [tokens, heads * vdim]: the values in (numbers that tf32 holds, as bfloat16 ones are), the read-outs out
   float* state; long long state_stride;       // [slot][heads][dim][vdim]
   const int* q_start; const int* q_len; const int* seq_slot;
   int items, heads, qk_heads, dim, vdim;

@@ -295,6 +295,28 @@ def test_chunks_in_more_than_one_slab(kind, per_head):
   assert ws._bufs[("state_chunks", torch.float32)].numel() < (2400 // 64 + 2) * 240 * (64 * 64 + 2 * 64 * 32 + 32 * 32)      # not all chunks at once
 
 
+# Value columns a block of the walk, from how many blocks there are: 16 and 32 (few heads, as everywhere above: 8); channels and columns that fill no tile
+@pytest.mark.parametrize("H", [14, 40])
+def test_delta_rule_of_many_heads(H):
+  for i, (state, S, out, want) in enumerate(_run("delta", False, (130,), H, 40, 88, 13, None)):
+    assert (state - S).norm() <= STATE_BOUND * S.norm(), i
+    assert ((out - want).abs() <= 2.0 ** -8 * want.abs().clamp(min=1.0) + 1e-4).all(), i
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+def test_linear_attention_in_more_than_one_slab(per_head):
+  """300 heads: a slab of scratch holds 34 chunks of the step's 39."""
+  from miniinfer_b200.engine.context import Workspace
+  for i, (state, S, out, want) in enumerate(_run("linear", per_head, (1500, 900), 300, 8, 8, 14, Workspace(torch.device(DEV)))):
+    assert (state - S).norm() <= STATE_BOUND * S.norm(), i
+    assert ((out - want).abs() <= 2.0 ** -8 * want.abs().clamp(min=1.0) + 1e-4).all(), i
+
+
+@pytest.mark.parametrize("lengths", [(70,), (1, 2, 31, 33, 4)])      # a stretch of eight tokens a block, and items that end inside it
+def test_causal_convolution_of_short_stretches(lengths):
+  test_causal_convolution_eight_channels_a_thread(4, lengths, 2048, 8)
+
+
 @pytest.mark.parametrize("D", [50, 136])      # channels that the chunks do not take: rows of no whole 16 bytes, more than 128
 @pytest.mark.parametrize("kind,per_head", [("delta", False), ("linear", False), ("linear", True)])
 def test_long_portions_of_heads_that_chunks_do_not_take(kind, per_head, D):
