@@ -131,55 +131,95 @@ gemm_batched_few_rows_kernel(BatchedArgs a) {
 }
 
 // The same on the tensor cores (mma.sync), where the values of k can be fetched in pairs: a warp takes eight output columns
-// of a batch and the whole of K, straight from global memory, so all of its loads are in flight together.
+// of a batch and the whole of K, straight from global memory, so all of its loads are in flight together.  EIGHT: rows of whole 16
+// bytes are fetched so, a thread of a quad eight values of k that two products share, in the same order for both operands, and the
+// weights, which no kernel writes, before the wait for the kernel before.  GATES: with an activation or a gate a value; without them
+// their code is not there to be jumped across (8 rows of 32 heads, 192 x 128 and 128 x 192, behind other kernels: 4.0 us each, so 3.4).
 __device__ __forceinline__ uint32_t pair_at(const __nv_bfloat16* p, bool take) { return take ? *reinterpret_cast<const uint32_t*>(p) : 0u; }
+__device__ __forceinline__ uint4 eight_at(const __nv_bfloat16* p, bool take) { return take ? *reinterpret_cast<const uint4*>(p) : make_uint4(0u, 0u, 0u, 0u); }
+__device__ __forceinline__ void mma_onto(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t w0, uint32_t w1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(w0), "r"(w1));
+}
 
-template <typename TO>
+template <typename TO, bool EIGHT, bool GATES>
 __global__ void __launch_bounds__(128)
 gemm_batched_mma_few_rows_kernel(BatchedArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, q = (lane & 3) * 2;
+  const int g = lane >> 2, t = lane & 3, q = t * 2;
   const int n0 = (blockIdx.x * 4 + warp) * 8;
   const int b = blockIdx.y;
-  mi::grid_dependency_sync();
-  if (n0 >= a.N) return;
   const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + (size_t)b * a.x_batch;
   const __nv_bfloat16* w = (const __nv_bfloat16*)a.w + (size_t)b * a.w_batch + (size_t)min(n0 + g, a.N - 1) * a.ldw;
   const bool lo = g < a.M, hi = g + 8 < a.M;
   const __nv_bfloat16* x0 = x + (size_t)(lo ? g : 0) * a.lda;
   const __nv_bfloat16* x1 = x + (size_t)(hi ? g + 8 : 0) * a.lda;
   float c[4] = {0.f, 0.f, 0.f, 0.f};
+  if constexpr (EIGHT) {
+    constexpr int AHEAD = 8;      // 256 values of k
+    uint4 wv[AHEAD];
+    auto weights = [&](int k0) {
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) wv[i] = eight_at(w + k0 + 32 * i + 8 * t, k0 + 32 * i + 8 * t < a.K);
+    };
+    weights(0);
+    mi::grid_dependency_sync();
+#pragma unroll 1
+    for (int k0 = 0; k0 < a.K; k0 += 32 * AHEAD) {
+      if (k0 > 0) weights(k0);
+      uint4 xa[AHEAD], xb[AHEAD];
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+        const int k = k0 + 32 * i + 8 * t;
+        xa[i] = eight_at(x0 + k, lo && k < a.K);
+        xb[i] = eight_at(x1 + k, hi && k < a.K);
+      }
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+        mma_onto(c, xa[i].x, xb[i].x, xa[i].y, xb[i].y, wv[i].x, wv[i].y);
+        mma_onto(c, xa[i].z, xb[i].z, xa[i].w, xb[i].w, wv[i].z, wv[i].w);
+      }
+    }
+    if (n0 >= a.N) return;
+  } else {
+    mi::grid_dependency_sync();
+    if (n0 >= a.N) return;
 #pragma unroll 8
-  for (int k = 0; k < a.K; k += 16) {
-    const int ka = k + q, kb = ka + 8;
-    const bool ia = ka < a.K, ib = kb < a.K;
-    const uint32_t w0 = pair_at(w + ka, ia), w1 = pair_at(w + kb, ib);
-    const uint32_t a0 = pair_at(x0 + ka, ia && lo), a1 = pair_at(x1 + ka, ia && hi), a2 = pair_at(x0 + kb, ib && lo), a3 = pair_at(x1 + kb, ib && hi);
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(w0), "r"(w1));
+    for (int k = 0; k < a.K; k += 16) {
+      const int ka = k + q, kb = ka + 8;
+      const bool ia = ka < a.K, ib = kb < a.K;
+      mma_onto(c, pair_at(x0 + ka, ia && lo), pair_at(x1 + ka, ia && hi), pair_at(x0 + kb, ib && lo), pair_at(x1 + kb, ib && hi), pair_at(w + ka, ia), pair_at(w + kb, ib));
+    }
   }
   TO* out = (TO*)a.out + (size_t)b * a.o_batch;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = g + (i >> 1) * 8, n = n0 + q + (i & 1);
-    if (m >= a.M || n >= a.N) continue;
-    float y = c[i];
-    if (a.bias) y += a.bias[n];
-    if (a.act == 1) y = y > 20.f ? y : log1pf(expf(y));
-    if (a.row_gate) y *= 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.row_gate)[(size_t)m * a.gate_stride + b])));
-    if (a.value_gate) y *= 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.value_gate)[(size_t)m * a.gate_stride + (size_t)b * a.N + n])));
-    out[(size_t)m * a.ldo + n] = mi::from_float<TO>(y);
+  for (int h = 0; h < 2; ++h) {
+    const int m = g + 8 * h;
+    if (m >= a.M) break;
+    const float gate = a.row_gate ? 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.row_gate)[(size_t)m * a.gate_stride + b]))) : 1.f;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int n = n0 + q + e;
+      if (n >= a.N) continue;
+      float y = c[2 * h + e];
+      if (GATES) {
+        if (a.bias) y += a.bias[n];
+        if (a.act == 1) y = y > 20.f ? y : log1pf(expf(y));
+        if (a.value_gate) y *= 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.value_gate)[(size_t)m * a.gate_stride + (size_t)b * a.N + n])));
+      }
+      out[(size_t)m * a.ldo + n] = mi::from_float<TO>(y * gate);
+    }
   }
 }
 
 // Many rows in bfloat16 on the tensor cores (mma.sync), for operands whose rows can be fetched 16 bytes at a time: tiles of 64 x 64, a
 // warp 32 x 32, K in stages of 64 by cp.async.  These products are small and read their rows once - 2048 rows of 16 heads,
-// 64 x 192 each, move 17 MB - so the memory bounds them, where the FMA kernel above was bound by its arithmetic (50.6 us,
-// 13.8 here); a tcgen05 tile of 128 rows would wait for the same bytes.  The tensor core cuts off what its accumulator does not
+// 64 x 192 each, move 17 MB - so the memory bounds them, where the FMA kernel above was bound by its arithmetic (50.6 us);
+// a tcgen05 tile of 128 rows would wait for the same bytes.  The tensor core cuts off what its accumulator does not
 // hold, always towards zero: every sixteen products start from zero and are added to the sum in a rounded addition.  bfloat16
 // results only: in float32 the sums of sixteen would still err by more than the chain of FMAs (K = 4096, carried on in the
 // accumulator: 4.4e-6 of the norm, by FMAs 6.1e-7).
-constexpr int TK = 64, LDS = TK + 8, TSTAGES = 3;
+constexpr int TK = 64, LDS = TK + 8, TSTAGES = 3, LDC = 64 + 4;
 
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __nv_bfloat16* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -239,38 +279,51 @@ gemm_batched_mma_kernel(BatchedArgs a) {
         }
     }
   }
-  __nv_bfloat16* out = (__nv_bfloat16*)a.out + (size_t)b * a.o_batch;
+  // Through shared memory, so that one loop serves all values of a thread and rows are written 16 bytes at a time.  Value by value from the
+  // registers the activation and the gates stood there 32 times, 110 KB of instructions that nearly all calls only jump across, line by
+  // line from L2: 2048 rows of 16 heads, 64 x 192, behind another kernel 16.8 us, so 9.7; 500 rows of 32 heads, 128 x 192, 18 and 9.2.
+  float* cs = reinterpret_cast<float*>(tiles);      // [64][LDC]
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int m = m0 + wm + 16 * i + (lane >> 2) + 8 * h;
-      if (m >= a.M) continue;
-      float gate = 1.f;
-      if (a.row_gate) gate = 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.row_gate)[(size_t)m * a.gate_stride + b])));
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int n = n0 + wn + 8 * j + (lane & 3) * 2;
-        float y[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          y[e] = c[i][j][2 * h + e];
-          if (n + e >= a.N) continue;
-          if (a.bias) y[e] += a.bias[n + e];
-          if (a.act == 1) y[e] = y[e] > 20.f ? y[e] : log1pf(expf(y[e]));
-          if (a.value_gate)
-            y[e] *= 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.value_gate)[(size_t)m * a.gate_stride + (size_t)b * a.N + n + e])));
-          y[e] *= gate;
-        }
-        __nv_bfloat16* o = out + (size_t)m * a.ldo + n;
-        if (n + 1 < a.N && ((uintptr_t)o % 4) == 0) {
-          *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(y[0], y[1]);
-        } else {
-          if (n < a.N) o[0] = __float2bfloat16_rn(y[0]);
-          if (n + 1 < a.N) o[1] = __float2bfloat16_rn(y[1]);
-        }
-      }
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float2*>(cs + (wm + 16 * i + (lane >> 2) + 8 * h) * LDC + wn + 8 * j + (lane & 3) * 2) = make_float2(c[i][j][2 * h], c[i][j][2 * h + 1]);
+  __syncthreads();
+  if (a.bias || a.act || a.value_gate) {
+#pragma unroll 1
+    for (int i = threadIdx.x; i < 64 * 64; i += 128) {
+      const int r = i >> 6, m = m0 + r, n = n0 + (i & 63);
+      if (m >= a.M || n >= a.N) continue;
+      float y = cs[r * LDC + (i & 63)];
+      if (a.bias) y += a.bias[n];
+      if (a.act == 1) y = y > 20.f ? y : log1pf(expf(y));
+      if (a.value_gate) y *= 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.value_gate)[(size_t)m * a.gate_stride + (size_t)b * a.N + n])));
+      cs[r * LDC + (i & 63)] = y;
     }
+    __syncthreads();
+  }
+  __nv_bfloat16* out = (__nv_bfloat16*)a.out + (size_t)b * a.o_batch;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < 64 * 8; i += 128) {
+    const int r = i >> 3, m = m0 + r, n = n0 + (i & 7) * 8;
+    if (m >= a.M || n >= a.N) continue;
+    const float gate = a.row_gate ? 1.f / (1.f + expf(-__bfloat162float(((const __nv_bfloat16*)a.row_gate)[(size_t)m * a.gate_stride + b]))) : 1.f;
+    const float* y = cs + r * LDC + (i & 7) * 8;
+    __nv_bfloat16* o = out + (size_t)m * a.ldo + n;
+    if (n + 8 <= a.N && ((uintptr_t)o % 16) == 0) {
+      __nv_bfloat162 v[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = __floats2bfloat162_rn(y[2 * e] * gate, y[2 * e + 1] * gate);
+      *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(v);
+    } else {
+#pragma unroll 1
+      for (int e = 0; e < 8 && n + e < a.N; ++e) o[e] = __float2bfloat16_rn(y[e] * gate);
+    }
+  }
 }
 
 }  // namespace
@@ -288,8 +341,15 @@ MI_API int mi_gemm_batched_few_rows(void* out, int out_dtype, const void* x, con
   const bool pairs = K % 2 == 0 && lda % 2 == 0 && ldw % 2 == 0 && x_batch % 2 == 0 && w_batch % 2 == 0 && ((uintptr_t)x % 4) == 0 && ((uintptr_t)w % 4) == 0;
   if (pairs && (out_dtype == MI_BF16 || out_dtype == MI_F32)) {
     const dim3 mgrid((N + 31) / 32, batch);
-    if (out_dtype == MI_BF16) mi::launch(gemm_batched_mma_few_rows_kernel<__nv_bfloat16>, mgrid, dim3(128), 0, stream, a);
-    else mi::launch(gemm_batched_mma_few_rows_kernel<float>, mgrid, dim3(128), 0, stream, a);
+    const bool eight = K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && x_batch % 8 == 0 && w_batch % 8 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0;
+    const bool gates = bias || act || value_gate;
+#define MI_FEW(TO)                                                                                                                     \
+  mi::launch(eight ? gates ? gemm_batched_mma_few_rows_kernel<TO, true, true> : gemm_batched_mma_few_rows_kernel<TO, true, false>       \
+                   : gates ? gemm_batched_mma_few_rows_kernel<TO, false, true> : gemm_batched_mma_few_rows_kernel<TO, false, false>,    \
+             mgrid, dim3(128), 0, stream, a)
+    if (out_dtype == MI_BF16) MI_FEW(__nv_bfloat16);
+    else MI_FEW(float);
+#undef MI_FEW
     MI_LAUNCH_OK("gemm_batched_few_rows");
     return 0;
   }

@@ -64,6 +64,13 @@ def test_per_head_products_of_many_rows(M, N, K, B, gate, dtype):
   assert ((out.double().cpu() - want).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("M,N,K,B", [(1, 8, 8, 3), (8, 33, 192, 2), (16, 70, 264, 2), (9, 5, 520, 1)])      # K in rounds of 256, columns that fill no warp
+@pytest.mark.parametrize("gate", ["row", "value", "bias"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_per_head_products_of_few_rows(M, N, K, B, gate, dtype):
+  test_per_head_products_of_many_rows(M, N, K, B, gate, dtype)
+
+
 @pytest.mark.parametrize("M,N,K,B", [(64, 64, 192, 2), (65, 70, 4096, 1)])
 def test_per_head_products_into_float32_add_in_order(M, N, K, B):
   from miniinfer_b200.kernels import ops
