@@ -1,9 +1,9 @@
 // Passes over the heads of every token around the matrix-state recurrences, for bfloat16 rows that can be read four values at a
 // time: what feeds a recurrence in float32, and the norm and gate of its read-outs.  A warp takes (token, head) pairs a grid apart;
 // a block a token and four heads spent its time starting and ending
-// (2048 tokens of 8 heads of 128, one value a lane and read against four: read-outs 9.9 and 8.3 us, the delta rule's inputs 15.0 and
-// 13.1; linear attention's inputs with decays, 1800 tokens of 16 heads, 28.5 and 19.9 - the logarithms and exponentials of the
-// decays are most of it).
+// (2048 tokens of 8 heads of 128, one value a lane and read against four: the delta rule's inputs 15.0 and 13.1 us; linear attention's
+// inputs with decays, 1800 tokens of 16 heads, 28.5 and 19.9 - the logarithms and exponentials of the decays are most of it).  Read-outs,
+// behind another kernel, with exact activations, unrolled, and as below: 1800 tokens of 16 heads 13.1 and 9.7 us, 2048 of 32 28.6 and 18.2.
 #pragma once
 
 #include "common.cuh"
@@ -39,34 +39,76 @@ inline dim3 head_rows_grid(long long units) {
   return dim3((unsigned)(blocks < most ? blocks : most));
 }
 
-// out[t, h] = o / sqrt(mean(o^2) + eps) * norm_w * act(gate[t, h]), o = raw[t, h]: norm_w [vdim] and gate optional.
+// 1 / (1 + exp(-z)) and z times it by the hardware's exponential and reciprocal, for what is rounded to bfloat16 next (the reciprocal keeps
+// results below 2^-126): a handful of instructions where the exact ones are fifty, of which a kernel this short mostly waits for the fetching.
+__device__ __forceinline__ float near_sigmoid(float z) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-z)));
+  return r;
+}
+__device__ __forceinline__ float near_silu(float z) { return z * near_sigmoid(z); }
+
+// out[t, h] = o / sqrt(mean(o^2) + eps) * norm_w * act(gate[t, h]), o = raw[t, h]: norm_w [vdim] and gate optional.  A warp
+// asks for the rows of UNITS (token, head) pairs before it works on the first; heads of more than 128 values take its lanes several times.
+constexpr int OUTPUT_UNITS = 2;
+template <bool WIDE>      // heads of more than 128 values
 static __global__ void __launch_bounds__(256)
 head_output_kernel(__nv_bfloat16* __restrict__ out, int ldo, const float* __restrict__ raw, const __nv_bfloat16* __restrict__ gate, int ldg,
                    const float* __restrict__ norm_w, int T, int heads, int vdim, float eps, int gate_silu) {
-  const int lane = threadIdx.x & 31, units = T * heads, step = gridDim.x * 8;
+  const int lane = threadIdx.x & 31, units = T * heads, step = gridDim.x * 8, j0 = 4 * lane;
+  const bool first = j0 < vdim;
+  const float4 one = make_float4(1.f, 1.f, 1.f, 1.f), w0 = norm_w && first ? load_row4(norm_w + j0) : one;
   grid_dependency_sync();
-#pragma unroll 2
-  for (int u = blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += step) {
-    const int t = u / heads, h = u - t * heads;
-    const float* o = raw + (size_t)u * vdim;
-    float ss = 0.f;
-    for (int j = 4 * lane; j < vdim; j += 128) {
-      const float4 v = load_row4(o + j);
-      ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
+#pragma unroll 1
+  for (int u0 = blockIdx.x * 8 + (threadIdx.x >> 5); u0 < units; u0 += OUTPUT_UNITS * step) {
+    float4 o[OUTPUT_UNITS], g[OUTPUT_UNITS];
+#pragma unroll
+    for (int i = 0; i < OUTPUT_UNITS; ++i) {
+      const int u = u0 + i * step, t = u / heads, h = u - t * heads;
+      const bool in = first && u < units;
+      o[i] = in ? load_row4(raw + (size_t)u * vdim + j0) : make_float4(0.f, 0.f, 0.f, 0.f);
+      g[i] = in && gate ? load_row4(gate + (size_t)t * ldg + h * vdim + j0) : one;
     }
-    const float rstd = 1.f / sqrtf(warp_sum(ss) / (float)vdim + eps);
-    for (int j = 4 * lane; j < vdim; j += 128) {
-      float4 y = scaled4(load_row4(o + j), rstd);
-      if (norm_w) {
-        const float4 w = load_row4(norm_w + j);
-        y.x *= w.x; y.y *= w.y; y.z *= w.z; y.w *= w.w;
-      }
+    auto write = [&](int u, int j, float4 v, float4 z, float4 w, float rstd) {
+      const int t = u / heads, h = u - t * heads;
+      float4 y = scaled4(v, rstd);
+      y.x *= w.x; y.y *= w.y; y.z *= w.z; y.w *= w.w;
       if (gate) {
-        const float4 g = load_row4(gate + (size_t)t * ldg + h * vdim + j);
-        auto act = [&](float z) { const float s = 1.f / (1.f + expf(-z)); return gate_silu ? z * s : s; };
-        y.x *= act(g.x); y.y *= act(g.y); y.z *= act(g.z); y.w *= act(g.w);
+        const float4 s = make_float4(near_sigmoid(z.x), near_sigmoid(z.y), near_sigmoid(z.z), near_sigmoid(z.w));
+        y.x *= gate_silu ? z.x * s.x : s.x;
+        y.y *= gate_silu ? z.y * s.y : s.y;
+        y.z *= gate_silu ? z.z * s.z : s.z;
+        y.w *= gate_silu ? z.w * s.w : s.w;
       }
       store_row4(out + (size_t)t * ldo + h * vdim + j, y);
+    };
+    float ss[OUTPUT_UNITS];
+#pragma unroll
+    for (int i = 0; i < OUTPUT_UNITS; ++i) {
+      ss[i] = fmaf(o[i].x, o[i].x, fmaf(o[i].y, o[i].y, fmaf(o[i].z, o[i].z, o[i].w * o[i].w)));
+      if (WIDE && u0 + i * step < units) {
+#pragma unroll 1
+        for (int j = j0 + 128; j < vdim; j += 128) {
+          const float4 v = load_row4(raw + (size_t)(u0 + i * step) * vdim + j);
+          ss[i] = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss[i]))));
+        }
+      }
+    }
+#pragma unroll
+    for (int b = 16; b > 0; b >>= 1)
+#pragma unroll
+      for (int i = 0; i < OUTPUT_UNITS; ++i) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], b);
+#pragma unroll
+    for (int i = 0; i < OUTPUT_UNITS; ++i) {
+      const int u = u0 + i * step;
+      if (u >= units) break;
+      const float rstd = 1.f / sqrtf(ss[i] / (float)vdim + eps);
+      if (first) write(u, j0, o[i], g[i], w0, rstd);
+#pragma unroll 1
+      for (int j = j0 + 128; WIDE && j < vdim; j += 128) {
+        const int t = u / heads, h = u - t * heads;
+        write(u, j, load_row4(raw + (size_t)u * vdim + j), gate ? load_row4(gate + (size_t)t * ldg + h * vdim + j) : one, norm_w ? load_row4(norm_w + j) : one, rstd);
+      }
     }
   }
 }

@@ -86,18 +86,22 @@ linear_prepare_kernel(LinPrepArgs<T, TA> a) {
   }
 }
 
+// A decay of linear attention.  A call, and not four copies of its hundred instructions.
+__device__ __noinline__ float linear_decay(float z, float inv_tau) { return mi::decay_exp(lin_log_sigmoid(z) * inv_tau); }
+
 // The same four values at a time (head_rows.cuh); the two halves of a head's rotated values are a multiple of four apart.
 __global__ void __launch_bounds__(256)
 linear_prepare_rows_kernel(LinPrepArgs<__nv_bfloat16, float> a, int T) {
   const int lane = threadIdx.x & 31, units = T * a.heads, step = gridDim.x * 8, half = a.rot_dims / 2;
   mi::grid_dependency_sync();
-#pragma unroll 2
+#pragma unroll 1
   for (int u = blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += step) {
     const int t = u / a.heads, h = u - t * a.heads;
     const __nv_bfloat16* q = a.q + (size_t)t * a.ldq + (size_t)h * a.dim;
     const __nv_bfloat16* k = a.k + (size_t)t * a.ldk + (size_t)h * a.dim;
     const float* cs = a.rope ? a.rope + (size_t)a.positions[t] * a.rot_dims : nullptr;
     const size_t at = (size_t)u * a.dim;
+#pragma unroll 1
     for (int i = 4 * lane; i < a.dim; i += 128) {
       float4 x = mi::load_row4(q + i), y = mi::load_row4(k + i);
       if (cs && i < a.rot_dims) {
@@ -117,10 +121,10 @@ linear_prepare_rows_kernel(LinPrepArgs<__nv_bfloat16, float> a, int T) {
           const float4 b = mi::load_row4(a.a_bias + h * a.dim + i);
           z.x += b.x; z.y += b.y; z.z += b.z; z.w += b.w;
         }
-        *reinterpret_cast<float4*>(a.g + at + i) = make_float4(mi::decay_exp(lin_log_sigmoid(z.x) * a.inv_tau), mi::decay_exp(lin_log_sigmoid(z.y) * a.inv_tau),
-                                                               mi::decay_exp(lin_log_sigmoid(z.z) * a.inv_tau), mi::decay_exp(lin_log_sigmoid(z.w) * a.inv_tau));
+        *reinterpret_cast<float4*>(a.g + at + i) = make_float4(linear_decay(z.x, a.inv_tau), linear_decay(z.y, a.inv_tau), linear_decay(z.z, a.inv_tau), linear_decay(z.w, a.inv_tau));
       }
     }
+#pragma unroll 1
     for (int j = 4 * lane; j < a.vdim; j += 128)
       *reinterpret_cast<float4*>(a.raw + (size_t)u * a.vdim + j) = mi::load_row4(a.v + (size_t)t * a.ldv + (size_t)h * a.vdim + j);
   }
@@ -554,7 +558,7 @@ MI_API int mi_linear_attention(void* out, int ldo, const void* q, int ldq, const
       if (int e = mi::chunked_state_run(c, T, chunks, stream)) return e;                                             \
     }                                                                                                                \
     if (vec)                                                                                                         \
-      mi::launch(mi::head_output_kernel, mi::head_rows_grid((long long)T * heads), dim3(256), 0, stream, (__nv_bfloat16*)out, ldo, (const float*)raw, \
+      mi::launch(vdim > 128 ? mi::head_output_kernel<true> : mi::head_output_kernel<false>, mi::head_rows_grid((long long)T * heads), dim3(256), 0, stream, (__nv_bfloat16*)out, ldo, (const float*)raw, \
                  (const __nv_bfloat16*)gate, ldg, norm_w, T, heads, vdim, eps, gate_silu);                            \
     else mi::launch(linear_output_kernel<TT>, ogrid, dim3(128), 0, stream, (TT*)out, ldo, (const float*)raw, (const TT*)gate, ldg, \
                norm_w, heads, vdim, eps, gate_silu);                                                                 \

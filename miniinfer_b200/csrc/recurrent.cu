@@ -53,100 +53,67 @@ causal_conv_kernel(T* __restrict__ out, int ldo, const T* __restrict__ x, int ld
   out[(size_t)t * ldo + c] = mi::from_float<T>(acc);
 }
 
-// The same for bfloat16 rows that can be read 16 bytes at a time: a thread has eight channels of CONV_TOKENS tokens, so an input is
-// fetched for several taps, and all of the thread's inputs are asked for before any is used (2048 tokens of 2048 channels, four taps:
-// 32 us a value a thread, here 17.8; 8192 channels 122 and 56; the activation's exponential and division are most of that).
-constexpr int CONV_TOKENS = 4;
+// The same for bfloat16 rows that can be read four bytes at a time: a thread has two channels of a block's tokens, the inputs of CONV_AHEAD of them
+// on their way at a time, the last taps - 1 in registers.  Stretches of one request are walked one after the other.  (2048 tokens of
+// 2048 channels, four taps: a value a thread 32 us; eight channels and four tokens a thread 17.8, of which most was the way of 32 KB of
+// instructions from L2 - 32 exact activations -; so 8.7; 1000 tokens of 8192 channels 31.2 and 14.)
+constexpr int CONV_AHEAD = 8;
 
 template <int TAPS>
 __global__ void __launch_bounds__(128)
 causal_conv_vec_kernel(__nv_bfloat16* __restrict__ out, int ldo, const __nv_bfloat16* __restrict__ x, int ldx, const float* __restrict__ w,
                        const float* __restrict__ bias, const float* __restrict__ in_bias, const float* __restrict__ state, long long state_stride,
-                       const int* __restrict__ token_item, const int* __restrict__ q_start, const int* __restrict__ seq_slot,
-                       int T, int C, int silu) {
-  const int c = 8 * (blockIdx.x * blockDim.x + threadIdx.x), t0 = blockIdx.y * CONV_TOKENS;
-  if (c >= C) {
-    mi::grid_dependency_sync();
-    return;
-  }
-  int items[CONV_TOKENS];
+                       const int* __restrict__ token_item, const int* __restrict__ q_start, const int* __restrict__ q_len,
+                       const int* __restrict__ seq_slot, int T, int C, int silu, int tokens) {
+  const int c = 2 * (blockIdx.x * blockDim.x + threadIdx.x), t_end = min(T, (int)(blockIdx.y + 1) * tokens);
+  const bool live = c < C;
+  const int cc = live ? c : 0;
+  float wt[2][TAPS], b[2], ib[2];
 #pragma unroll
-  for (int n = 0; n < CONV_TOKENS; ++n) items[n] = t0 + n < T ? token_item[t0 + n] : -1;
-  float wt[8 * TAPS], b[8], ib[8];      // the weights of a channel lie side by side
+  for (int e = 0; e < 2; ++e) {
 #pragma unroll
-  for (int i = 0; i < 8 * TAPS; i += 2) {
-    const float2 p = *reinterpret_cast<const float2*>(w + (size_t)c * TAPS + i);
-    wt[i] = p.x;
-    wt[i + 1] = p.y;
+    for (int k = 0; k < TAPS; ++k) wt[e][k] = w[(size_t)(cc + e) * TAPS + k];
+    b[e] = bias ? bias[cc + e] : 0.f;
+    ib[e] = in_bias ? in_bias[cc + e] : 0.f;
   }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    b[i] = bias ? bias[c + i] : 0.f;
-    ib[i] = in_bias ? in_bias[c + i] : 0.f;
-  }
-  int item = items[0], j = t0 - q_start[item];
   mi::grid_dependency_sync();
-  uint4 raw[CONV_TOKENS + TAPS - 1];      // rows t0 - (TAPS - 1) ..: those before the item's first row are not its inputs, and replaced
-#pragma unroll
-  for (int n = 0; n < CONV_TOKENS + TAPS - 1; ++n) {
-    const int row = min(max(t0 + n - (TAPS - 1), 0), T - 1);
-    raw[n] = *reinterpret_cast<const uint4*>(x + (size_t)row * ldx + c);
-  }
-  float in[TAPS][8];      // in[k]: the input k tokens back
-  auto take = [&](float (&to)[8], uint4 from) {
-    const uint32_t part[4] = {from.x, from.y, from.z, from.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&part[i]));
-      to[2 * i] = f.x + ib[2 * i];
-      to[2 * i + 1] = f.y + ib[2 * i + 1];
-    }
+  if (!live) return;
+  const __nv_bfloat16* xc = x + c;
+  auto input = [&](__nv_bfloat162 v) {
+    const float2 f = __bfloat1622float2(v);
+    return make_float2(f.x + ib[0], f.y + ib[1]);
   };
-  auto kept = [&]() {      // the inputs before the item's new tokens, as far as they reach
+#pragma unroll 1
+  for (int t = blockIdx.y * tokens; t < t_end;) {
+    const int item = token_item[t], start = q_start[item], j = t - start, end = min(t_end, start + q_len[item]);
     const float* st = state + (size_t)seq_slot[item] * state_stride + c;
+    float2 in[TAPS];      // in[k]: the input k tokens back
 #pragma unroll
-    for (int k = 1; k < TAPS; ++k)
-      if (j < k) {
+    for (int k = 1; k < TAPS; ++k) {      // (those before the item's new tokens are the state's)
+      if (j >= k) in[k - 1] = input(*reinterpret_cast<const __nv_bfloat162*>(xc + (size_t)(t - k) * ldx));
+      else in[k - 1] = make_float2(st[(size_t)(TAPS - 1 + j - k) * C], st[(size_t)(TAPS - 1 + j - k) * C + 1]);
+    }
+#pragma unroll 1
+    for (; t < end; t += CONV_AHEAD) {
+      __nv_bfloat162 raw[CONV_AHEAD];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) in[k - 1][i] = st[(size_t)(TAPS - 1 + j - k) * C + i];
-      }
-  };
+      for (int n = 0; n < CONV_AHEAD; ++n) raw[n] = *reinterpret_cast<const __nv_bfloat162*>(xc + (size_t)min(t + n, end - 1) * ldx);
 #pragma unroll
-  for (int k = 1; k < TAPS; ++k) take(in[k - 1], raw[TAPS - 1 - k]);
-  if (j < TAPS - 1) kept();
+      for (int n = 0; n < CONV_AHEAD; ++n) {
 #pragma unroll
-  for (int n = 0; n < CONV_TOKENS; ++n) {
-    const int t = t0 + n;
-    if (t >= T) return;
-    if (n > 0) {
-      ++j;
-      if (items[n] != item) {
-        item = items[n];
-        j = 0;
-        kept();
+        for (int k = TAPS - 1; k > 0; --k) in[k] = in[k - 1];
+        in[0] = input(raw[n]);
+        float2 acc = make_float2(b[0], b[1]);
+#pragma unroll
+        for (int k = TAPS - 1; k >= 0; --k) {      // oldest input first
+          acc.x = fmaf(wt[0][TAPS - 1 - k], in[k].x, acc.x);
+          acc.y = fmaf(wt[1][TAPS - 1 - k], in[k].y, acc.y);
+        }
+        if (silu) acc = make_float2(mi::near_silu(acc.x), mi::near_silu(acc.y));
+        if (t + n < end) *reinterpret_cast<__nv_bfloat162*>(out + (size_t)(t + n) * ldo + c) = __floats2bfloat162_rn(acc.x, acc.y);
       }
     }
-#pragma unroll
-    for (int k = TAPS - 1; k > 0; --k)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) in[k][i] = in[k - 1][i];
-    take(in[0], raw[n + TAPS - 1]);
-    uint32_t o[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float y[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int ch = 2 * i + e;
-        float acc = b[ch];
-#pragma unroll
-        for (int k = TAPS - 1; k >= 0; --k) acc = fmaf(wt[ch * TAPS + TAPS - 1 - k], in[k][ch], acc);      // oldest input first
-        y[e] = silu ? silu_f(acc) : acc;
-      }
-      const __nv_bfloat162 p = __floats2bfloat162_rn(y[0], y[1]);
-      o[i] = *reinterpret_cast<const uint32_t*>(&p);
-    }
-    *reinterpret_cast<uint4*>(out + (size_t)t * ldo + c) = make_uint4(o[0], o[1], o[2], o[3]);
+    t = end;
   }
 }
 
@@ -463,6 +430,9 @@ delta_prepare_kernel(DeltaPrepArgs<T> a) {
   }
 }
 
+// A decay of the delta rule.  A call, and not four copies of its hundred instructions.
+__device__ __noinline__ float delta_decay(float z, float neg_rate) { return mi::decay_exp(neg_rate * softplus_f(z)); }
+
 // The same four values at a time (head_rows.cuh).
 __global__ void __launch_bounds__(256)
 delta_prepare_rows_kernel(DeltaPrepArgs<__nv_bfloat16> a) {
@@ -474,6 +444,7 @@ delta_prepare_rows_kernel(DeltaPrepArgs<__nv_bfloat16> a) {
       const __nv_bfloat16* q = a.q + (size_t)t * a.ldqk + (size_t)u * a.dim;
       const __nv_bfloat16* k = a.k + (size_t)t * a.ldqk + (size_t)u * a.dim;
       float sq = 0.f, sk = 0.f;
+#pragma unroll 1
       for (int i = 4 * lane; i < a.dim; i += 128) {
         const float4 x = mi::load_row4(q + i), y = mi::load_row4(k + i);
         sq = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, sq))));
@@ -484,6 +455,7 @@ delta_prepare_rows_kernel(DeltaPrepArgs<__nv_bfloat16> a) {
       const float fq = rsqrtf((float)a.dim) / sqrtf(sq + 1e-6f), fk = 1.f / sqrtf(sk + 1e-6f);
       const size_t at = ((size_t)t * a.kv_heads + u) * a.dim;
       float qk = 0.f;
+#pragma unroll 1
       for (int i = 4 * lane; i < a.dim; i += 128) {
         const float4 x = mi::scaled4(mi::load_row4(q + i), fq), y = mi::scaled4(mi::load_row4(k + i), fk);
         *reinterpret_cast<float4*>(a.qn + at + i) = x;
@@ -504,14 +476,15 @@ delta_prepare_rows_kernel(DeltaPrepArgs<__nv_bfloat16> a) {
           a.g[(size_t)t * a.heads + h] = expf(lg);
         }
       } else {
-        for (int i = 4 * lane; i < a.dim; i += 128) {
+  #pragma unroll 1
+      for (int i = 4 * lane; i < a.dim; i += 128) {
           const float4 z = mi::load_row4(a.a + (size_t)t * a.lda + (size_t)h * a.dim + i), b = mi::load_row4(a.dt_bias + h * a.dim + i);
           *reinterpret_cast<float4*>(a.g + ((size_t)t * a.heads + h) * a.dim + i) =
-            make_float4(mi::decay_exp(neg_rate * softplus_f(z.x + b.x)), mi::decay_exp(neg_rate * softplus_f(z.y + b.y)),
-                        mi::decay_exp(neg_rate * softplus_f(z.z + b.z)), mi::decay_exp(neg_rate * softplus_f(z.w + b.w)));
+            make_float4(delta_decay(z.x + b.x, neg_rate), delta_decay(z.y + b.y, neg_rate), delta_decay(z.z + b.z, neg_rate), delta_decay(z.w + b.w, neg_rate));
         }
       }
       if (lane == 0) a.beta[(size_t)t * a.heads + h] = sigmoid_f(mi::to_float(a.b[(size_t)t * a.ldb + h]));
+#pragma unroll 1
       for (int j = 4 * lane; j < a.vdim; j += 128)
         *reinterpret_cast<float4*>(a.raw + ((size_t)t * a.heads + h) * a.vdim + j) = mi::load_row4(a.v + (size_t)t * a.ldv + (size_t)h * a.vdim + j);
     }
@@ -810,15 +783,19 @@ MI_API int mi_causal_conv(void* out, int ldo, const void* x, int ldx, int dtype,
   MI_REQUIRE(state_stride >= (long long)(taps - 1) * C, "causal_conv: the state rows are too short");
   if (T == 0) return 0;
   dim3 grid((C + 255) / 256, T), sgrid((C + 255) / 256, items);
-  // eight channels and four tokens a thread where rows start on 16-byte boundaries and there are more than half a million values (a
-  // thread's weights alone are 128 bytes).  Four taps, this way / a value a thread, in microseconds: 64 x 2048 6.4 / 4.1, 256 x 2048
-  // 6.5 / 6.5, 64 x 8192 6.7 / 6.5, 384 x 2048 7.7 / 8.3, 192 x 4096 7.7 / 8.3, 128 x 8192 7.7 / 10.2, 2048 x 2048 16.3 / 29.8
-  const bool vec = dtype == MI_BF16 && (long long)T * C > 1 << 19 && taps >= 2 && taps <= 4 && C % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 &&
+  // two channels and a stretch of tokens a thread where there are more than 2^17 values, rows start on 16-byte boundaries
+  // and hold whole 16 bytes.  Four taps, this way / a value a thread, in microseconds: 32 x 2048 4.0 / 3.8,
+  // 64 x 2048 4.1 / 4.1, 128 x 2048 4.1 / 4.9, 256 x 2048 4.3 / 6.5, 64 x 8192 4.3 / 6.6, 2048 x 2048 8.7 / 29.8
+  const bool vec = dtype == MI_BF16 && (long long)T * C > 1 << 17 && taps >= 2 && taps <= 4 && C % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 &&
                    ((uintptr_t)x % 16) == 0 && ((uintptr_t)out % 16) == 0 && ((uintptr_t)w % 8) == 0;
   if (vec) {
     auto kernel = taps == 2 ? causal_conv_vec_kernel<2> : taps == 3 ? causal_conv_vec_kernel<3> : causal_conv_vec_kernel<4>;
-    mi::launch(kernel, dim3((C / 8 + 127) / 128, (T + CONV_TOKENS - 1) / CONV_TOKENS), dim3(128), 0, stream, (__nv_bfloat16*)out, ldo,
-               (const __nv_bfloat16*)x, ldx, w, bias, in_bias, (const float*)state, state_stride, token_item, q_start, seq_slot, T, C, silu);
+    // as many tokens a block, up to 32, as leave four blocks an SM
+    const int across = (C / 2 + 127) / 128;
+    int tokens = 4 * CONV_AHEAD;
+    while (tokens > CONV_AHEAD && (long long)across * ((T + tokens - 1) / tokens) < 4ll * mi::sm_count()) tokens -= CONV_AHEAD;
+    mi::launch(kernel, dim3(across, (T + tokens - 1) / tokens), dim3(128), 0, stream, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)x, ldx, w, bias,
+               in_bias, (const float*)state, state_stride, token_item, q_start, q_len, seq_slot, T, C, silu, tokens);
     mi::launch(conv_state_kernel<__nv_bfloat16>, sgrid, dim3(256), 0, stream, state, state_stride, (const __nv_bfloat16*)x, ldx, in_bias,
                q_start, q_len, seq_slot, C, taps);
   } else if (dtype == MI_BF16) {
@@ -1009,7 +986,7 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
       if (int e = mi::chunked_state_run(c, T, chunks, stream)) return e;                                            \
     }                                                                                                             \
     if (vec)                                                                                                      \
-      mi::launch(mi::head_output_kernel, mi::head_rows_grid((long long)T * heads), dim3(256), 0, stream, (__nv_bfloat16*)out, ldo, (const float*)raw, \
+      mi::launch(vdim > 128 ? mi::head_output_kernel<true> : mi::head_output_kernel<false>, mi::head_rows_grid((long long)T * heads), dim3(256), 0, stream, (__nv_bfloat16*)out, ldo, (const float*)raw, \
                  (const __nv_bfloat16*)gate, ldg, norm_w, T, heads, vdim, eps, gate_silu);                         \
     else                                                                                                          \
       mi::launch(delta_output_kernel<TT>, ogrid, dim3(128), 0, stream, (TT*)out, ldo, (const float*)raw, (const TT*)gate, ldg, norm_w, heads, vdim, eps, gate_silu); \
