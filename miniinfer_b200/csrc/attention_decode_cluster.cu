@@ -100,8 +100,8 @@ __device__ __forceinline__ __nv_bfloat16 finish_value(const ClusterArgs& a, floa
   if (a.sink) {
     const float s2 = a.sink[head] * 1.4426950408889634f;      // base 2, like the scores
     const float Mf = fmaxf(M, s2);
-    const float f = M == -INFINITY ? 0.f : exp2f(M - Mf);
-    L = L * f + exp2f(s2 - Mf);
+    const float f = M == -INFINITY ? 0.f : mi::ex2_fast(M - Mf);
+    L = L * f + mi::ex2_fast(s2 - Mf);
     A = A * f;
   }
   float y = A / L;
@@ -116,16 +116,16 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // the swizzle pattern is a function of the address: the tiles start on a 1024-byte boundary
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  // [stages][K tile, V tile] | recv [RECV_FLOATS] | red [CW][GP][ROW] | barriers | pages [max_tiles] | flag
+  // [stages][K tile, V tile] | recv [RECV_FLOATS] | red [CW][GP][ROW] | barriers | rows [max_tiles] | flag
   unsigned char* stage0 = smem;
   float* recv = reinterpret_cast<float*>(smem + (size_t)a.stages * STAGE_BYTES);   // [block of the cluster][its sums of my slice | max, sum per head]
   float* red = recv + RECV_FLOATS;
   uint64_t* full = reinterpret_cast<uint64_t*>(red + CW * GP * ROW);
   uint64_t* empty = full + CMAX_STAGES;
   uint64_t* patched = empty + CMAX_STAGES;                       // rope: the new token's key and value are in the last tile
-  int* pages = reinterpret_cast<int*>(patched + 1);
-  volatile int* abort = pages + a.max_tiles;
-  __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(pages + ((a.max_tiles + 4 + 3) & ~3));   // [GP][HD]: the query heads, normed and rotated here (rope)
+  int* rows = reinterpret_cast<int*>(patched + 1);               // of a tile's keys in the cache as the tensor map sees it
+  volatile int* abort = rows + a.max_tiles;
+  __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(rows + ((a.max_tiles + 4 + 3) & ~3));   // [GP][HD]: the query heads, normed and rotated here (rope)
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int C = (int)gridDim.x, r = (int)blockIdx.x, kvh = (int)blockIdx.y, e = (int)blockIdx.z;
@@ -155,7 +155,11 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
   const int nb = b1 - b0;
   {
     const int* bt = a.block_table + (size_t)a.seq_slot[item] * a.bt_stride;
-    for (int i = threadIdx.x; i < nb && i < a.max_tiles; i += CTHREADS) pages[i] = bt[(j_first + (b0 + i) * BK) / a.page_size];
+#pragma unroll 1
+    for (int i = threadIdx.x; i < nb && i < a.max_tiles; i += CTHREADS) {
+      const int jb = j_first + (b0 + i) * BK, page = jb / a.page_size;
+      rows[i] = (bt[page] * 2 * a.nkv + kvh) * a.page_size + jb - page * a.page_size;
+    }
   }
   // The kernel that norms and rotates q and k and stores the new token's k and v may be this kernel's work (rope):
   // each computing warp then prepares a query head of this kv head in shared memory, and in the block that holds the
@@ -200,12 +204,11 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
   };
   // this block holds the tile with position p, and the new token's entry is this kernel's to write
   const bool patch = rope && nb > 0 && b1 == tiles && a.slot_mapping != nullptr && a.kv_layer != nullptr;
+  const int slot = patch ? a.slot_mapping[row] : -1;
   auto ask = [&](int b) {                                    // lane 0 of the copying warp
     const int s = b % a.stages;
     mbar_wait(&empty[s], ((b / a.stages) & 1) ^ 1, abort, a.status);
-    const int jb = j_first + (b0 + b) * BK;
-    const int y_k = ((pages[b] * 2) * a.nkv + kvh) * a.page_size + jb % a.page_size;
-    const int y_v = y_k + a.nkv * a.page_size;
+    const int y_k = rows[b], y_v = y_k + a.nkv * a.page_size;
     unsigned char* dst = stage0 + (size_t)s * STAGE_BYTES;
     mbar_expect_tx(&full[s], (uint32_t)STAGE_BYTES);
 #pragma unroll
@@ -220,27 +223,42 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
   // asked for before the wait, while the QKV product still runs; the new token's row is put into its tile afterwards.
   // (Worth 0.4 % of a decode step at batch 8 and 0.3 % at batch 1: a block of this kernel gets onto an SM only when the
   // product's block there has left, so little of the product is left to hide the copies behind.)
-  __syncthreads();                                           // the barriers and the page numbers are in shared memory
-  int asked = 0;
-  if (rope && warp == CW && lane == 0)
-    for (; asked < nb && asked < a.stages; ++asked) ask(asked);       // the ring is empty: no wait in here
-  mi::grid_dependency_sync();
-
-  if (warp == CW) {
-    // ------------------------------------------------------------------ the warp that asks for the copies
-    if (lane == 0)
-      for (; asked < nb && asked < a.stages; ++asked) ask(asked);     // the ring is empty: no wait in here
-    const int slot = patch ? a.slot_mapping[row] : -1;
-    uint32_t ka = 0u, kb = 0u, va = 0u, vb = 0u;               // this lane's pairs of the new key (normed, rotated) and value
-    if (patch && slot >= 0) {
-      const __nv_bfloat16* qkv_row = a.q_base + (size_t)row * a.q_stride;
+  __syncthreads();                                           // the barriers and the tiles' rows are in shared memory
+  // (One place each for the copies and for the norm and rotation, and loops that stay loops: this kernel's instructions are executed once
+  // or a few times, and come from L2 line by line.  Inlined where they were used, 55 KB of them, 8 requests of 16 heads took 7.4 us at 256
+  // tokens and 14.9 at 2048, behind another kernel; so, 30 KB, 5.6 and 13.1.)
+#pragma unroll 1
+  for (int asked = 0, after = rope ? 0 : 1; after < 2; ++after) {      // before the wait what the ring holds, after it the rest
+    if (after) mi::grid_dependency_sync();
+    if (warp == CW && lane == 0)
+#pragma unroll 1
+      for (; asked < nb && (after || asked < a.stages); ++asked) ask(asked);
+  }
+  uint32_t ka = 0u, kb = 0u, va = 0u, vb = 0u;                 // copying warp: this lane's pairs of the new key (normed, rotated) and value
+  if (rope) {                                                // a query head per warp, the new key in the copying warp
+    const __nv_bfloat16* qkv_row = a.q_base + (size_t)row * a.q_stride;
+    const bool key = warp == CW, normed = (key ? a.k_w : a.q_w) != nullptr;
+    if (key && slot >= 0) {
       const __nv_bfloat16* xv = qkv_row + (size_t)(a.nh + a.nkv + kvh) * HD;
       va = *reinterpret_cast<const uint32_t*>(xv + j);
       vb = *reinterpret_cast<const uint32_t*>(xv + HALF + j);
-      norm_rotate(qkv_row + (size_t)(a.nh + kvh) * HD, a.k_w != nullptr, ka, kb);
     }
-    if (lane == 0)
-      for (; asked < nb; ++asked) ask(asked);
+#pragma unroll 1
+    for (int h = key ? 0 : warp; h < (key ? (slot >= 0 ? 1 : 0) : G); h += CW) {
+      uint32_t ua, ub;
+      norm_rotate(qkv_row + (size_t)(key ? a.nh + kvh : kvh * G + h) * HD, normed, ua, ub);
+      if (key) {
+        ka = ua;
+        kb = ub;
+      } else {
+        *reinterpret_cast<uint32_t*>(q_s + h * HD + j) = ua;
+        *reinterpret_cast<uint32_t*>(q_s + h * HD + HALF + j) = ub;
+      }
+    }
+  }
+
+  if (warp == CW) {
+    // ------------------------------------------------------------------ the warp that asks for the copies
     if (patch) {
       // The lanes meet here: a lane that looked at the last tile's barrier before lane 0 had asked for that tile could
       // take an earlier use of the stage - two phases back, the same parity - for it.
@@ -278,13 +296,6 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
     {
       const __nv_bfloat16* qrow = a.q_base + (size_t)row * a.q_stride + (size_t)(kvh * G + g) * HD;
       if (rope) {
-        const __nv_bfloat16* qkv_row = a.q_base + (size_t)row * a.q_stride;
-        for (int h = warp; h < G; h += CW) {                  // a head per warp
-          uint32_t ua, ub;
-          norm_rotate(qkv_row + (size_t)(kvh * G + h) * HD, a.q_w != nullptr, ua, ub);
-          *reinterpret_cast<uint32_t*>(q_s + h * HD + j) = ua;
-          *reinterpret_cast<uint32_t*>(q_s + h * HD + HALF + j) = ub;
-        }
         asm volatile("bar.sync 2, %0;" ::"n"(CW * 32) : "memory");      // the computing warps have left the query heads in shared memory
         qrow = q_s + (g < G ? g : 0) * HD;
       }
@@ -303,6 +314,7 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // heads 2t and 2t + 1
     const TileScores shape = SHAPED ? tile_scores(a.scale, a.softcap, nullptr, a.distance, a.nh, kvh * G + 2 * t4, G - 2 * t4, p)
                                     : plain_scores();
+#pragma unroll 1
     for (int b = warp; b < nb; b += CW) {
       const int s = b % a.stages;
       mbar_wait(&full[s], (b / a.stages) & 1, abort, a.status);
@@ -342,6 +354,7 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
   const int slice = (total + C - 1) / C;
   const int rs = slice + 2 * GP;                           // floats a block receives from one block
   if (C > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");     // every block of the cluster has started
+#pragma unroll 1
   for (int idx = threadIdx.x; idx < total; idx += CTHREADS) {
     const int h = idx / HD, d = idx % HD;
     float M = -INFINITY;
@@ -352,7 +365,7 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
 #pragma unroll
       for (int w = 0; w < CW; ++w) {
         const float* src = red + ((size_t)w * GP + h) * ROW;
-        const float f = src[HD] == -INFINITY ? 0.f : exp2f(src[HD] - M);
+        const float f = src[HD] == -INFINITY ? 0.f : mi::ex2_fast(src[HD] - M);
         L = fmaf(src[HD + 1], f, L);
         A = fmaf(src[d], f, A);
       }
@@ -363,6 +376,7 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
       const int owner = idx / slice;
       cluster.map_shared_rank(recv, owner)[(size_t)r * rs + (idx - owner * slice)] = A;
       if (d == 0) {
+#pragma unroll 1
         for (int rr = 0; rr < C; ++rr) {
           float* to = cluster.map_shared_rank(recv, rr) + (size_t)r * rs + slice;
           to[2 * h] = M;
@@ -376,17 +390,20 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 
   // the blocks of the cluster, in rank order
+#pragma unroll 1
   for (int t = threadIdx.x; t < slice && r * slice + t < total; t += CTHREADS) {
     const int idx = r * slice + t;
     const int h = idx / HD, d = idx % HD;
     float M = -INFINITY;
+#pragma unroll 1
     for (int rr = 0; rr < C; ++rr) M = fmaxf(M, recv[(size_t)rr * rs + slice + 2 * h]);
     float L = 0.f, A = 0.f;
+#pragma unroll 1
     for (int rr = 0; rr < C; ++rr) {
       const float* src = recv + (size_t)rr * rs;
       const float mr = src[slice + 2 * h];
       if (mr == -INFINITY) continue;
-      const float f = exp2f(mr - M);
+      const float f = mi::ex2_fast(mr - M);
       L = fmaf(src[slice + 2 * h + 1], f, L);
       A = fmaf(src[t], f, A);
     }

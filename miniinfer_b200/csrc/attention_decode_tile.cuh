@@ -33,6 +33,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // Bounded wait.  `abort` is a flag in shared memory: once any wait has run out, all waits return.
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort, int* status) {
   const uint32_t addr = smem_u32(bar);
+#pragma unroll 1
   for (int i = 0; i < WAIT_LIMIT; ++i) {
     uint32_t done;
     asm volatile(
@@ -161,7 +162,7 @@ __device__ __forceinline__ void consume_tile(uint32_t kt, uint32_t vt, const uin
     mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 16));
     const float m_new = fmaxf(m_run[h], mx[h]);
     m_use[h] = m_new == -INFINITY ? 0.f : m_new;
-    alpha[h] = exp2f(m_run[h] - m_use[h]);
+    alpha[h] = mi::ex2_fast(m_run[h] - m_use[h]);
     m_run[h] = m_new;
     l_run[h] *= alpha[h];
   }
@@ -169,7 +170,7 @@ __device__ __forceinline__ void consume_tile(uint32_t kt, uint32_t vt, const uin
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const float pe = exp2f(sc[i][c] - m_use[c & 1]);
+      const float pe = mi::ex2_fast(sc[i][c] - m_use[c & 1]);
       sc[i][c] = pe;
       l_run[c & 1] += pe;
     }

@@ -103,6 +103,12 @@ def test_linear_bf16_few_rows(ops, out_dtype, N, K):
       assert (routed.float() - exact).abs().max().item() <= bound, M
 
 
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("N,K", [(2000, 1800), (2056, 1528), (72, 512), (100, 1000)])     # a warp's share of K of 8, 6, 2 and 4 blocks of 32, the last cut off
+def test_linear_bf16_few_rows_without_a_loop(ops, out_dtype, N, K):
+  test_linear_bf16_few_rows(ops, out_dtype, N, K)
+
+
 def test_linear_bf16_many_rows_and_float32_logits(ops):
   x = rnd(200, 136, dtype=torch.bfloat16, seed=1)
   w = rnd(1000, 136, dtype=torch.bfloat16, seed=2, scale=0.05)
