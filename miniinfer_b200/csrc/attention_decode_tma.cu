@@ -115,8 +115,10 @@ __device__ __forceinline__ bool consumer_any(bool flag) {
       : "=r"(out) : "r"((uint32_t)flag), "n"(CONSUMERS * 32) : "memory");
   return out != 0;
 }
-// DISTANCE: the form for a distance bias, compiled apart so that the others carry none of it.
-template <bool DISTANCE>
+// SHAPE: 0 the plain softmax, 1 capped scores and sigmoid weights, 2 a distance bias - compiled apart so that a tile's code has none of
+// what it does not need: with the caps and the sigmoid beside the plain score, sixteen times a tile, 64 requests of 128 to 2303 tokens (32
+// heads over 8) took 78 us instead of 65, 24 of 1000 tokens 31 instead of 28.
+template <int SHAPE>
 __global__ void __launch_bounds__(THREADS, 1)
 decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map, Args a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -235,6 +237,7 @@ decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map, Args a) {
         for (int c0 = from; c0 < to; c0 += 32) {
           const int page = bt[(j0 + min(c0 + lane, nb - 1) * BK) / a.page_size];
           const int run = min(32, to - c0);
+#pragma unroll 1
           for (int u = 0; u < run; ++u, ++blk) {
             const int pg = __shfl_sync(0xffffffffu, page, u);
             if (lane == 0) {
@@ -325,6 +328,7 @@ decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map, Args a) {
           };
           float cur[4][DS], nxt[4][DS];
           // one round trip through L2 for every chunk's max and sum and for the first batch of outputs
+#pragma unroll 1
           for (int idx = lane; idx < G * ns; idx += 32) {
             const int gh = idx / ns, sp = idx % ns;
             const float2 v = __ldcg(reinterpret_cast<const float2*>(ml0 + ((size_t)gh * a.max_splits + sp) * 2));
@@ -333,24 +337,29 @@ decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map, Args a) {
           }
           load_batch(cur, 0, 0);
           __syncwarp();
+#pragma unroll 1
           for (int gh = 0; gh < G; ++gh) {
             float m = -INFINITY;
+#pragma unroll 1
             for (int sp = lane; sp < ns; sp += 32) m = fmaxf(m, merge_s[2 * (gh * ns + sp)]);
             m = mi::warp_max(m);
             const float sink2 = a.sink ? a.sink[d.kvh * G + gh] * 1.4426950408889634f : -INFINITY;   // base 2, like the scores
             m = fmaxf(m, sink2);
             float l = 0.f;
+#pragma unroll 1
             for (int sp = lane; sp < ns; sp += 32) l = fmaf(merge_s[2 * (gh * ns + sp) + 1], exp2f(merge_s[2 * (gh * ns + sp)] - m), l);
             l = mi::warp_sum(l);
             if (a.sink) l += exp2f(sink2 - m);
-            const float inv = a.score_bias ? exp2f(m) : 1.f / l;      // sigmoid weights: the sums hold weight * 2^(-m)
+            const float inv = SHAPE == 1 && a.score_bias ? exp2f(m) : 1.f / l;      // sigmoid weights: the sums hold weight * 2^(-m)
             __syncwarp();
+#pragma unroll 1
             for (int sp = lane; sp < ns; sp += 32) merge_s[2 * (gh * ns + sp)] = exp2f(merge_s[2 * (gh * ns + sp)] - m) * inv;   // the chunk's weight
           }
           __syncwarp();
           // the batches in order (head by head); the next one is on its way while this one is added up
           const int per_head = (ns + 3) / 4;
           float acc[DS];
+#pragma unroll 1
           for (int bi = 0; bi < G * per_head; ++bi) {
             const int gh = bi / per_head, sp0 = (bi % per_head) * 4;
             if (bi + 1 < G * per_head) load_batch(nxt, (bi + 1) / per_head, ((bi + 1) % per_head) * 4);
@@ -421,11 +430,13 @@ decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map, Args a) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) o[i][c] = 0.f;
       float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // heads 2t and 2t + 1
-      const TileScores shape = tile_scores(a.scale, a.softcap, a.score_bias, DISTANCE ? a.distance : nullptr, a.nh, d.kvh * G + g0 + 2 * t4, heads - 2 * t4, d.pos);
+      const TileScores shape = SHAPE == 0 ? plain_scores()
+                                          : tile_scores(a.scale, a.softcap, a.score_bias, SHAPE == 2 ? a.distance : nullptr, a.nh, d.kvh * G + g0 + 2 * t4, heads - 2 * t4, d.pos);
 
       // tile gb of this block's stream goes to warp gb mod 3 (it owns the stages gb mod `stages` can be);
       // `rank` is the warp's place among the item's tiles, which fixes the order of the merge
       const int rank = (warp + CONSUMERS - blk_base % CONSUMERS) % CONSUMERS;
+#pragma unroll 1
       for (int b = rank; b < d.nb; b += CONSUMERS) {
         const int gb = blk_base + b;
         const int s = gb % a.stages;
@@ -464,6 +475,7 @@ decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map, Args a) {
         }
       }
       consumer_sync();
+#pragma unroll 1
       for (int idx = threadIdx.x; idx < heads * HD; idx += CONSUMERS * 32) {
         const int r = idx / HD, dd = idx % HD;
         float m = -INFINITY;
@@ -487,7 +499,7 @@ decode_tma_kernel(const __grid_constant__ CUtensorMap kv_map, Args a) {
             vf = v * f;
             lf = l * f + exp2f(sink2 - mf);
           }
-          const float y = a.score_bias ? (m == -INFINITY ? 0.f : v * exp2f(m)) : vf / lf;
+          const float y = SHAPE == 1 && a.score_bias ? (m == -INFINITY ? 0.f : v * exp2f(m)) : vf / lf;
           a.out[(size_t)d.row * a.nh * HD + (size_t)head * HD + dd] = __float2bfloat16_rn(gated(a, y, d.row, head, dd));
         } else {
           a.part_o[(((size_t)d.e * a.nh + head) * a.max_splits + d.split) * HD + dd] = v;
@@ -592,8 +604,9 @@ MI_API int mi_attention_decode_tma(void* out, const void* q_base, int q_stride, 
   const size_t smem = smem_bytes(stages, a.gp, max_splits, n_dec);
   static size_t configured = 0;
   if (smem > configured) {
-    cudaError_t err = cudaFuncSetAttribute(decode_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(decode_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t err = cudaFuncSetAttribute(decode_tma_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(decode_tma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(decode_tma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (err != cudaSuccess) return mi_fail("attention_decode_tma: cannot get shared memory: %s", cudaGetErrorString(err));
     configured = 227 * 1024;
   }
@@ -601,7 +614,7 @@ MI_API int mi_attention_decode_tma(void* out, const void* q_base, int q_stride, 
   memcpy(&map, kv_map, sizeof(map));
   MI_REQUIRE(n_dec <= 4096, "attention_decode_tma: at most 4096 decode entries per launch (got %d)", n_dec);
   const int grid = num_sms;
-  mi::launch(distance ? decode_tma_kernel<true> : decode_tma_kernel<false>, dim3(grid), dim3(THREADS), smem, stream, map, a);
+  mi::launch(distance ? decode_tma_kernel<2> : softcap > 0.f || score_bias ? decode_tma_kernel<1> : decode_tma_kernel<0>, dim3(grid), dim3(THREADS), smem, stream, map, a);
   MI_LAUNCH_OK("attention_decode_tma");
   return 0;
 }
