@@ -34,6 +34,10 @@
 // tokens, latent 192 + 32: 16 heads 55 us, 232 by the mma.sync kernel; 1000 tokens of 32 heads of 192 + 64 with a window of 1024 35 us,
 // 149 by that.
 //
+// (Pairs of values in one instruction - f32x2, a maximum of three - in the prompt's form: 55.1 -> 52.5 us at 2048 tokens.  The decode form is
+// left at its registers: at 142 instead of 168 a block leaves room for the next kernels beside it, which then find the SMs unevenly
+// taken, and a decode step of 8 tokens of 32 heads took 54 us instead of 48.)
+//
 // Decode tokens run through the same tiles: a work is one request's up to 128 heads and a piece of its keys, counted from key 0, and
 // leaves sums that are not normalised for latent_merge_kernel.  Most of the 128 rows are padding, which costs nothing: a piece is bound
 // by the latency of its one or two tiles and by bytes, and every key row is fetched once for all heads, as key and as value
@@ -384,7 +388,14 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
         }
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int e = 0; e < BN / 2; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], v[e]);
+        for (int e = 0; e < BN / 2; e += 2) {
+          if (DECODE) {
+            mx4[e & 3] = fmaxf(mx4[e & 3], v[e]);
+            mx4[(e & 3) + 1] = fmaxf(mx4[(e & 3) + 1], v[e + 1]);
+          } else {
+            mx4[e >> 1 & 3] = mi::max_of(mx4[e >> 1 & 3], v[e], v[e + 1]);
+          }
+        }
         float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
         float* maxima = row_max + (g & 1) * 2 * BM;
         maxima[half * BM + r] = mx;
@@ -404,7 +415,16 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
               uint32_t x[32];
               tmem_ld(o, t_lane + O_COL + 32 * c);
 #pragma unroll
-              for (int e = 0; e < 32; ++e) x[e] = __float_as_uint(o[e] * alpha);
+              for (int e = 0; e < 32; e += 2) {
+                if (DECODE) {
+                  o[e] *= alpha;
+                  o[e + 1] *= alpha;
+                } else {
+                  mi::mul_pair(o[e], o[e + 1], o[e], o[e + 1], alpha);
+                }
+                x[e] = __float_as_uint(o[e]);
+                x[e + 1] = __float_as_uint(o[e + 1]);
+              }
               tmem_st(t_lane + O_COL + 32 * c, x);
             }
           }
@@ -415,7 +435,10 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
         float part[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t packed[BN / 4];
 #pragma unroll
-        for (int e = 0; e < BN / 2; ++e) v[e] = mi::ex2_fast(fmaf(v[e], a.scale_log2, -m_use));      // nothing where the row may not see the key
+        for (int e = 0; e < BN / 2; e += 2)
+          if (!DECODE) mi::fma_pair(v[e], v[e + 1], v[e], v[e + 1], a.scale_log2, -m_use);
+#pragma unroll
+        for (int e = 0; e < BN / 2; ++e) v[e] = mi::ex2_fast(DECODE ? fmaf(v[e], a.scale_log2, -m_use) : v[e]);      // nothing where the row may not see the key
         if constexpr (DECODE) {      // in two bf16 parts: P V twice
           uint32_t low[BN / 4];
 #pragma unroll
@@ -430,8 +453,7 @@ attention_latent_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
 #pragma unroll
           for (int e = 0; e < BN / 4; ++e) {
             packed[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
-            part[2 * e & 3] += __uint_as_float(packed[e] << 16);
-            part[(2 * e + 1) & 3] += __uint_as_float(packed[e] & 0xffff0000u);
+            mi::add_pair(part[2 * e & 3], part[(2 * e + 1) & 3], __uint_as_float(packed[e] << 16), __uint_as_float(packed[e] & 0xffff0000u));
           }
         }
         tmem_st(s_addr + BN / 4 * half, packed);      // two keys to a column

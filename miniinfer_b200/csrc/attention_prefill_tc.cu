@@ -782,7 +782,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         } else {
           float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int e = 0; e < BN; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], v[e]);
+          for (int e = 0; e < BN; e += 2) mx4[e >> 1 & 3] = mi::max_of(mx4[e >> 1 & 3], v[e], v[e + 1]);
           const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
           const float m_new = fmaxf(m_run, mx * sc);       // the scale is positive
           const bool move = m_new > m_run + 8.f || m_run == -INFINITY;
@@ -798,7 +798,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                 tmem_ld32(op, o_addr + c * 32);
                 uint32_t wv[32];
 #pragma unroll
-                for (int e = 0; e < 32; ++e) wv[e] = __float_as_uint(op[e] * alpha);
+                for (int e = 0; e < 32; e += 2) {
+                  mi::mul_pair(op[e], op[e + 1], op[e], op[e + 1], alpha);
+                  wv[e] = __float_as_uint(op[e]);
+                  wv[e + 1] = __float_as_uint(op[e + 1]);
+                }
                 tmem_st32(o_addr + c * 32, wv);
               }
               asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -812,12 +816,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
           for (int c = 0; c < BN / 32; ++c) {
             uint32_t packed[16];
 #pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              const float x = fmaf(v[32 * c + e], sc, -m_use);     // -inf where the row may not see the key
-              float pe;
-              asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(pe) : "f"(x));
-              v[32 * c + e] = pe;
-              part[e & 3] += pe;
+            for (int e = 0; e < 32; e += 2) {
+              float &p0 = v[32 * c + e], &p1 = v[32 * c + e + 1];
+              mi::fma_pair(p0, p1, p0, p1, sc, -m_use);      // -inf where the row may not see the key
+              p0 = mi::ex2_fast(p0);
+              p1 = mi::ex2_fast(p1);
+              mi::add_pair(part[e & 2], part[(e & 2) + 1], p0, p1);
             }
 #pragma unroll
             for (int e = 0; e < 16; ++e) packed[e] = pack_bf16(v[32 * c + 2 * e], v[32 * c + 2 * e + 1]);

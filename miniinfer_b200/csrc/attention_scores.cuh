@@ -49,6 +49,23 @@ __device__ __forceinline__ float lg2_fast(float x) {
   return y;
 }
 
+// Two float32 operations, or a maximum of three, in one instruction: a row of scores is some hundreds of instructions a thread and tile.
+__device__ __forceinline__ void fma_pair(float& d0, float& d1, float a0, float a1, float b, float c) {      // d = a b + c
+  asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %4};\n mov.b64 c, {%5, %5};\n fma.rn.f32x2 a, a, b, c;\n mov.b64 {%0, %1}, a;\n}\n"
+      : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b), "f"(c));
+}
+__device__ __forceinline__ void add_pair(float& d0, float& d1, float a0, float a1) {      // d += a
+  asm("{\n .reg .b64 a, d;\n mov.b64 d, {%0, %1};\n mov.b64 a, {%2, %3};\n add.rn.f32x2 d, d, a;\n mov.b64 {%0, %1}, d;\n}\n" : "+f"(d0), "+f"(d1) : "f"(a0), "f"(a1));
+}
+__device__ __forceinline__ void mul_pair(float& d0, float& d1, float a0, float a1, float b) {      // d = a b
+  asm("{\n .reg .b64 a, b;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %4};\n mul.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}\n" : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b));
+}
+__device__ __forceinline__ float max_of(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 // raw = q.k; returns the base-2 logit the online softmax takes.  `head_bias` is bias[head] (ignored for softmax).
 __device__ __forceinline__ float shaped_logit2(float raw, float scale, float softcap, bool sigmoid, float head_bias) {
   constexpr float LOG2E = 1.4426950408889634f;
