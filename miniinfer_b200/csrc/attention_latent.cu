@@ -553,6 +553,32 @@ latent_merge_kernel(Args a) {
   mi::grid_dependency_sync();
   const float* ml = a.part_ml + 2 * ((size_t)entry * a.max_splits * a.nh + head);
   const float* po = a.part_o + ((size_t)entry * a.max_splits * a.nh + head) * a.out_hd;
+  // Up to 32 pieces: a lane a piece's maximum and sum, a thread its value of all pieces, all on their way together (8 tokens of 32 heads in 9
+  // pieces, behind another kernel: 5.3 us by the loops below, so 4.8)
+  if (n <= 32) {
+    constexpr int AT_ONCE = 8;
+    const int lane = threadIdx.x & 31;
+    const bool live = threadIdx.x < a.out_hd;
+    float2 mine = make_float2(-INFINITY, 0.f);
+    if (lane < n) mine = *reinterpret_cast<const float2*>(ml + (size_t)2 * lane * a.nh);
+    float f = 0.f, m = sink2, acc = 0.f;
+#pragma unroll 1
+    for (int s0 = 0; s0 < n; s0 += AT_ONCE) {
+      float v[AT_ONCE];
+#pragma unroll
+      for (int s = 0; s < AT_ONCE; ++s) v[s] = live && s0 + s < n ? po[(size_t)(s0 + s) * a.nh * a.out_hd + threadIdx.x] : 0.f;
+      if (s0 == 0) {
+        m = fmaxf(m, mi::warp_max(mine.x));
+        f = lane < n ? exp2f(mine.x - m) : 0.f;
+      }
+#pragma unroll
+      for (int s = 0; s < AT_ONCE; ++s)
+        if (s0 + s < n) acc = fmaf(v[s], __shfl_sync(0xffffffffu, f, s0 + s), acc);
+    }
+    const float l = mi::warp_sum(mine.y * f) + (a.sink ? exp2f(sink2 - m) : 0.f);
+    if (live) a.out[((size_t)a.q_start[item] * a.nh + head) * a.out_hd + threadIdx.x] = __float2bfloat16_rn(n > 0 ? acc * (1.f / l) : 0.f);
+    return;
+  }
   float m = sink2;
   for (int s = threadIdx.x & 31; s < n; s += 32) m = fmaxf(m, ml[(size_t)2 * s * a.nh]);
   m = mi::warp_max(m);

@@ -180,3 +180,27 @@ def test_latent_attention_errs_by_little_more_than_its_last_rounding(items, nh, 
     want[at:at + n] = torch.einsum("hnc,cd->nhd", torch.softmax(s.masked_fill(hidden, float("-inf")), -1), K[:, :ohd])
     at += n
   assert (got.view_as(want).double() - want).norm() <= bound * want.norm()
+
+
+# Rows that go eight values a thread: parts that end in every place of a warp and a block, one value of eight the fewest, zeros behind a key.
+@pytest.mark.parametrize("Q,C,R,hdp,H,D,interleaved", [(64, 48, 16, 80, 3, 8, False), (1536, 192, 64, 256, 2, 128, False), (24, 8, 8, 16, 5, 16, True),
+                                                       (264, 512, 64, 640, 1, 64, True)])
+@pytest.mark.parametrize("T", [1, 37])
+def test_latent_rows_eight_values_a_thread(Q, C, R, hdp, H, D, interleaved, T):
+  import torch_ops
+  from miniinfer_b200.kernels import ops
+  g = torch.Generator().manual_seed(Q + C + T)
+  bf = lambda *s: torch.randn(s, generator=g).to(torch.bfloat16)  # noqa: E731
+  down, q, rope = bf(T, 8 + Q + C + R + 8), bf(T, H * (D + R)), torch.randn((T + 9, R), generator=g)
+  q_w, kv_w, pos = torch.randn(Q, generator=g), torch.randn(C, generator=g), torch.randint(0, T + 9, (T,), generator=g, dtype=torch.int32)
+  slots = torch.randperm(3 * 64, generator=g)[:T].int()
+  runs = []
+  for api, dev in ((torch_ops, "cpu"), (ops, DEV)):
+    d = lambda t: t.to(dev)  # noqa: B023, E731
+    cq, kv = torch.zeros((T, Q), dtype=torch.bfloat16, device=dev), torch.ones((3, 2, 1, 64, hdp), dtype=torch.bfloat16, device=dev)
+    heads = torch.ones((T, H * hdp), dtype=torch.bfloat16, device=dev)
+    api.latent_down(d(down), 8, 8 + Q, Q, C, R, d(q_w), d(kv_w), 1e-6, cq, d(rope), d(pos), interleaved, d(slots), kv)
+    api.latent_query(d(q), heads, H, D, R, C, d(rope), d(pos), interleaved)
+    runs.append([t.float().cpu() for t in (cq, kv, heads)])
+  for want, got in zip(*runs):      # one rounding to bfloat16 of values that float32 sums and products leave: neighbouring bfloat16 values at most
+    assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-5).all()
