@@ -13,9 +13,9 @@
 // the request was cut into steps and whatever else is in the batch.
 //
 // What bounds it: for prompt portions the reads of shared memory (nine of 16 bytes a lane for 16 packed FMAs), for single
-// tokens the instructions of the one warp that walks a segment.  Measured on B200, 16 / 8 heads of 128, microseconds in the
-// generic kernel and here: 300 new tokens 179 -> 88, 400 behind 1600 others 2850 -> 605, one token behind 700 248 -> 37, eight
-// tokens behind 2000 each 1484 -> 78.
+// tokens, whose segments four warps walk together, the latency of a chunk's scores.  Measured on B200, 16 / 8 heads of 128,
+// microseconds in the generic kernel and here: 300 new tokens 179 -> 88, 400 behind 1600 others 2850 -> 605, one token behind
+// 700 248 -> 23, eight tokens behind 2000 each 1484 -> 62.
 #include <cooperative_groups.h>
 
 #include <type_traits>
@@ -243,8 +243,8 @@ attention_f32_kernel(const F32Args a) {
               }
             }
           };
-          if (WARPS == 1 || __all_sync(0xffffffffu, every)) weigh(std::false_type());      // (one token's rows see the same keys, and the others are staged as zeros)
-          else if constexpr (WARPS > 1) weigh(std::true_type());
+          if (__all_sync(0xffffffffu, every)) weigh(std::false_type());
+          else weigh(std::true_type());
         }
         __syncthreads();      // the stage may be filled again
       }
@@ -324,10 +324,247 @@ attention_f32_kernel(const F32Args a) {
   }
 }
 
-template <int WARPS, int RW, int NV>
+// One new token: the same arithmetic, a block's four warps sharing a segment instead of one walking it (a lone warp took 9000 cycles a chunk
+// of 32 keys).  A row's scores of a chunk, its maximum and its sum are one warp's, a key a lane; a thread then weighs the values of an output
+// column, all rows of it, key after key.  While a chunk is weighed the next one's scores are made and the one behind it is copied: a barrier a chunk.
+// RW: rows of a block, the query heads of a key/value head.  16 / 8 heads of 128, microseconds by one warp and by four: two tokens behind 1000
+// 37 -> 23, eight behind 2000 each 77 -> 62, three behind 300 36 -> 23.  The scores' chain of 64 packed FMAs and its reads take two thirds of that.
+// (With bulk copies, two a key, in place of 16-byte ones: 45, 100, 43; with the scores' loop unrolled further the same.)
+template <int RW, int NV>
+struct OneLayout {
+  int hd, ldk;
+  __host__ __device__ explicit OneLayout(int hd) : hd(hd), ldk(hd + 4) {}
+  __host__ __device__ int keys(int stage) const { return stage * CHUNK * ldk; }
+  __host__ __device__ int values(int stage) const { return 3 * CHUNK * ldk + stage * CHUNK * hd; }
+  __host__ __device__ int queries() const { return 3 * CHUNK * (ldk + hd); }
+  __host__ __device__ int weights(int stage) const { return queries() + RW * hd + stage * (CHUNK + 1) * RW; }      // [key][row], then the rows' factors
+  __host__ __device__ int running() const { return queries() + RW * hd + 2 * (CHUNK + 1) * RW; }
+  __host__ __device__ int floats() const { return running() + RW * hd + 4 * RW; }
+};
+
+template <int RW, int NV>
+__global__ void __launch_bounds__(128)
+attention_f32_one_kernel(const F32Args a) {
+  constexpr int WARPS = 4, PER_WARP = (RW + WARPS - 1) / WARPS;
+  extern __shared__ __align__(16) float sm[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const OneLayout<RW, NV> at(a.hd);
+  const int hd = a.hd, ldk = at.ldk, rows = a.nh / a.nkv;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int item = a.items[blockIdx.x / a.cluster], rank = blockIdx.x % a.cluster, kvh = blockIdx.y;
+  const int token = a.q_start[item], p = a.ctx_len[item] - 1;
+  const int* bt = a.block_table + (size_t)a.seq_slot[item] * a.bt_stride;
+  const int lo = mi::first_visible(p, a.window), kept = a.window > 0 ? min(a.keep_first, lo) : 0;
+  const int kept_segs = (kept + SEG - 1) / SEG, seg0 = lo / SEG, segs = kept_segs + p / SEG - seg0 + 1;
+  const size_t page_elems = (size_t)2 * a.nkv * a.page_size * hd, v_off = (size_t)a.nkv * a.page_size * hd;
+  const float* kv = a.kv + (size_t)kvh * a.page_size * hd;
+  float* run_o = sm + at.running();
+  float *run_m = run_o + RW * hd, *run_l = run_m + RW, *part_m = run_l + RW, *part_l = part_m + RW;
+  float* part_o = sm;
+  mi::grid_dependency_sync();
+  for (int i = 4 * tid; i < RW * hd; i += 512) {
+    const int r = i / hd;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < rows) v = *reinterpret_cast<const float4*>(a.q + (size_t)token * a.q_stride + (size_t)(kvh * rows) * hd + i);
+    *reinterpret_cast<float4*>(sm + at.queries() + i) = v;
+    *reinterpret_cast<float4*>(run_o + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (tid < RW) {
+    run_m[tid] = a.sink && tid < rows ? a.sink[kvh * rows + tid] : -INFINITY;
+    run_l[tid] = a.sink ? 1.f : 0.f;
+  }
+  for (int round = 0; round < segs; round += a.cluster) {
+    const int seg = round + rank;
+    float m[PER_WARP], l[PER_WARP], o[RW][NV];
+#pragma unroll
+    for (int i = 0; i < PER_WARP; ++i) {
+      m[i] = -INFINITY;
+      l[i] = 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < RW; ++i)
+#pragma unroll
+      for (int n = 0; n < NV; ++n) o[i][n] = 0.f;
+    if (seg < segs) {
+      const bool first_keys = seg < kept_segs;
+      const int base = first_keys ? seg * SEG : (seg0 + seg - kept_segs) * SEG;
+      const int key_end = first_keys ? min(base + SEG, kept) : min(base + SEG, p + 1), key_lo = first_keys ? 0 : lo;
+      const int c_begin = max(base, key_lo / CHUNK * CHUNK);
+      // four threads a key; keys that are not seen are zeros.  A key's page is looked up a chunk ahead.
+      const int jj = tid >> 2;
+      auto seen_key = [&](int j) { return j >= key_lo && j < key_end; };
+      int page = seen_key(c_begin + jj) ? bt[(c_begin + jj) / a.page_size] : 0;
+      auto stage = [&](int c, int s) {
+        const int j = c + jj;
+        if (c < key_end) {
+          const bool in = seen_key(j);
+          const float* src = in ? kv + (size_t)page * page_elems + (size_t)(j % a.page_size) * hd : kv;
+          const uint32_t kd = (uint32_t)__cvta_generic_to_shared(sm + at.keys(s) + jj * ldk), vd = (uint32_t)__cvta_generic_to_shared(sm + at.values(s) + jj * hd);
+#pragma unroll 4
+          for (int d = (tid & 3) * 4; d < hd; d += 16) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd + 4 * d), "l"(in ? src + d : kv), "r"(in ? 16 : 0) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vd + 4 * d), "l"(in ? src + v_off + d : kv), "r"(in ? 16 : 0) : "memory");
+          }
+          page = seen_key(j + CHUNK) ? bt[(j + CHUNK) / a.page_size] : 0;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      // this warp's rows of a chunk: weights and the factor of what was added up before
+      auto score = [&](int c, int s, int b) {
+        if (c >= key_end || warp >= rows) return;
+        const bool seen = c + lane >= key_lo && c + lane < key_end;
+        uint64_t acc[PER_WARP];
+#pragma unroll
+        for (int i = 0; i < PER_WARP; ++i) acc[i] = 0;
+        const float *kr = sm + at.keys(s) + lane * ldk, *qr = sm + at.queries() + warp * hd;
+#pragma unroll 4
+        for (int d = 0; d < hd; d += 4) {
+          const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kr + d);
+#pragma unroll
+          for (int i = 0; i < PER_WARP; ++i) {
+            const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qr + i * WARPS * hd + d);
+            acc[i] = fma2(q4.y, k4.y, fma2(q4.x, k4.x, acc[i]));
+          }
+        }
+        float* w = sm + at.weights(b);
+#pragma unroll
+        for (int i = 0; i < PER_WARP; ++i) {
+          const int r = warp + i * WARPS;
+          if (r >= rows) break;
+          float x, y;
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(acc[i]));
+          const float sc = seen ? a.scale * (x + y) : -INFINITY, m_new = fmaxf(m[i], mi::warp_max(sc));
+          const bool none = m_new == -INFINITY;      // no key of this segment seen yet, or none whose score weighs anything
+          const float alpha = none ? 1.f : expf(m[i] - m_new), pe = seen ? expf(sc - (none ? 0.f : m_new)) : 0.f;
+          l[i] = l[i] * alpha + mi::warp_sum(pe);
+          m[i] = m_new;
+          w[lane * RW + r] = pe;
+          if (lane == 0) w[CHUNK * RW + r] = alpha;
+        }
+      };
+      auto weigh = [&](int s, int b) {
+        const float *w = sm + at.weights(b), *v = sm + at.values(s) + tid;
+#pragma unroll
+        for (int i = 0; i < RW; ++i)
+#pragma unroll
+          for (int n = 0; n < NV; ++n) o[i][n] *= w[CHUNK * RW + i];
+#pragma unroll 8
+        for (int jj = 0; jj < CHUNK; ++jj) {
+          float x[RW];
+#pragma unroll
+          for (int i = 0; i < RW; i += 2) {
+            const float2 t = *reinterpret_cast<const float2*>(w + jj * RW + i);
+            x[i] = t.x;
+            x[i + 1] = t.y;
+          }
+#pragma unroll
+          for (int n = 0; n < NV; ++n) {
+            const float y = tid + 128 * n < hd ? v[jj * hd + 128 * n] : 0.f;
+#pragma unroll
+            for (int i = 0; i < RW; ++i) o[i][n] = fmaf(x[i], y, o[i][n]);
+          }
+        }
+      };
+      stage(c_begin, 0);
+      stage(c_begin + CHUNK, 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      score(c_begin, 0, 0);
+      int s = 0, b = 0;      // the chunk's stage and buffer of weights
+#pragma unroll 1
+      for (int c = c_begin; c < key_end; c += CHUNK, b ^= 1) {
+        const int s1 = s == 2 ? 0 : s + 1, s2 = s1 == 2 ? 0 : s1 + 1;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();      // the next chunk has landed, this one's weights are there, and the one before is done with
+        stage(c + 2 * CHUNK, s2);
+        score(c + CHUNK, s1, b ^ 1);
+        weigh(s, b);
+        s = s1;
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+    }
+    // this segment's results into shared memory; the owner of a row merges those of the round in the segments' order
+#pragma unroll
+    for (int i = 0; i < RW; ++i)
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+        if (tid + 128 * n < hd) part_o[i * hd + tid + 128 * n] = o[i][n];
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < PER_WARP; ++i)
+        if (warp + i * WARPS < RW) {
+          part_m[warp + i * WARPS] = m[i];
+          part_l[warp + i * WARPS] = l[i];
+        }
+    }
+    cluster.sync();
+    for (int r = rank + a.cluster * warp; r < rows; r += a.cluster * WARPS) {
+      float mm = run_m[r], ll = run_l[r], oo[4 * NV];
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) oo[4 * n + e] = 128 * n + 4 * lane < hd ? run_o[r * hd + 128 * n + 4 * lane + e] : 0.f;
+#pragma unroll 1
+      for (int b = 0; b < a.cluster && round + b < segs; ++b) {
+        const float pm = *cluster.map_shared_rank(part_m + r, b), pl = *cluster.map_shared_rank(part_l + r, b);
+        if (pm == -INFINITY && pl == 0.f) continue;      // no key of that segment is visible (scores that are no numbers leave a sum that is none)
+        const float m_new = fmaxf(mm, pm), fa = expf(mm - m_new), fb = expf(pm - m_new);
+        ll = ll * fa + pl * fb;
+        mm = m_new;
+        const float* po = cluster.map_shared_rank(part_o + r * hd, b);
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          const int d = 128 * n + 4 * lane;
+          if (d < hd) {
+            const float4 v = *reinterpret_cast<const float4*>(po + d);
+            oo[4 * n] = oo[4 * n] * fa + v.x * fb;
+            oo[4 * n + 1] = oo[4 * n + 1] * fa + v.y * fb;
+            oo[4 * n + 2] = oo[4 * n + 2] * fa + v.z * fb;
+            oo[4 * n + 3] = oo[4 * n + 3] * fa + v.w * fb;
+          }
+        }
+      }
+      __syncwarp();
+      if (round + a.cluster < segs) {
+        if (lane == 0) {
+          run_m[r] = mm;
+          run_l[r] = ll;
+        }
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          const int d = 128 * n + 4 * lane;
+          if (d < hd) *reinterpret_cast<float4*>(run_o + r * hd + d) = make_float4(oo[4 * n], oo[4 * n + 1], oo[4 * n + 2], oo[4 * n + 3]);
+        }
+      } else {
+        const int head = kvh * rows + r;
+        const float inv = 1.f / ll;
+        float* dst = a.out + ((size_t)token * a.nh + head) * a.out_hd;
+        const float* gt = a.gate ? a.gate + (size_t)token * a.gate_stride : nullptr;
+#pragma unroll
+        for (int n = 0; n < NV; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int d = 128 * n + 4 * lane + e;
+            if (d < a.out_hd) {
+              float y = oo[4 * n + e] * inv;
+              if (gt) y = y / (1.f + expf(-gt[mi::gate_index(head, d, a.out_hd, a.gate_per_head)]));
+              dst[d] = y;
+            }
+          }
+      }
+    }
+    cluster.sync();      // nobody overwrites what a neighbour still reads, and nobody leaves
+  }
+}
+
+// ONE: one new token's rows, RW of them, by four warps together.
+template <int WARPS, int RW, int NV, bool ONE>
 int launch_form(F32Args a, int units, cudaStream_t stream) {
-  const size_t smem = sizeof(float) * Layout<WARPS, RW, NV>(a.hd).floats();
-  auto kernel = attention_f32_kernel<WARPS, RW, NV>;
+  const size_t smem = sizeof(float) * (ONE ? OneLayout<RW, NV>(a.hd).floats() : Layout<WARPS, RW, NV>(a.hd).floats());
+  void (*kernel)(const F32Args);
+  if constexpr (ONE) kernel = attention_f32_one_kernel<RW, NV>;
+  else kernel = attention_f32_kernel<WARPS, RW, NV>;
   static int ready[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || ready[dev] < (int)smem) {
@@ -355,9 +592,9 @@ int launch_form(F32Args a, int units, cudaStream_t stream) {
   return 0;
 }
 
-template <int WARPS, int RW>
+template <int RW, bool ONE>
 int launch_rows(const F32Args& a, int units, cudaStream_t stream) {
-  return a.hd <= 128 ? launch_form<WARPS, RW, 1>(a, units, stream) : launch_form<WARPS, RW, 2>(a, units, stream);
+  return a.hd <= 128 ? launch_form<4, RW, 1, ONE>(a, units, stream) : launch_form<4, RW, 2, ONE>(a, units, stream);
 }
 
 }  // namespace
@@ -381,11 +618,11 @@ MI_API int mi_attention_f32(float* out, const float* q, int q_stride, const floa
     p.items = tiles;
     p.tokens = 32 / group;
     p.subtiles = (tile_rows + p.tokens - 1) / p.tokens;
-    if (launch_rows<4, 8>(p, num_tiles * p.subtiles, stream)) return 1;
+    if (launch_rows<8, false>(p, num_tiles * p.subtiles, stream)) return 1;
   }
   if (num_decode > 0) {
     a.items = decode_items;
-    if (group <= 2 ? launch_rows<1, 2>(a, num_decode, stream) : group <= 8 ? launch_rows<1, 8>(a, num_decode, stream) : launch_rows<4, 8>(a, num_decode, stream))
+    if (group <= 2 ? launch_rows<2, true>(a, num_decode, stream) : group <= 8 ? launch_rows<8, true>(a, num_decode, stream) : launch_rows<8, false>(a, num_decode, stream))
       return 1;
   }
   return 0;

@@ -144,6 +144,24 @@ def test_attention_float32_segments_of_scores_that_are_no_numbers(score, with_si
   assert torch.allclose(outs[0], outs[1], atol=2e-5, equal_nan=True)
 
 
+# four warps share a segment: fewer rows than warps, a remainder of rows, heads that end inside a group of 128 columns, kept keys that end inside a chunk
+@pytest.mark.parametrize("group,hd,window,keep_first", [(1, 36, None, 0), (2, 256, 290, 33), (3, 132, None, 0), (5, 64, 31, 1), (7, 256, None, 0), (8, 100, 500, 260)])
+def test_attention_float32_one_token_by_four_warps(group, hd, window, keep_first):
+  from gpu_helpers import make_attention_case
+  from miniinfer_b200.kernels import ops
+  nkv, P, contexts = 2, 16, [1, 32, 33, 256, 289, 2311]
+  nh = group * nkv
+  qkv, kv, bt, batch = make_attention_case([(c, 1) for c in contexts], nh, nkv, hd, P, torch.float32, seed=group)
+  out = torch.full((len(contexts), nh * hd), float("nan"), device=DEV)
+  ops.attention(out, qkv, kv, bt, batch, nh, nkv, hd, hd ** -0.5, window, keep_first=keep_first)
+  for b, c in enumerate(contexts):
+    j = torch.tensor([j for j in range(c) if window is None or j >= c - window or j < keep_first], device=DEV)
+    k, v = kv[bt[int(batch.seq_slot[b]), j // P].long(), :, :, j % P].double().permute(1, 2, 0, 3)      # [nkv, keys, hd] each
+    q = qkv[b, :nh * hd].double().view(nkv, group, hd)
+    want = torch.softmax(q @ k.transpose(1, 2) * hd ** -0.5, -1) @ v
+    assert (out[b].double() - want.reshape(-1)).abs().max() < 2e-5, c      # as against the generic kernel
+
+
 @pytest.mark.skipif(DEV == "cpu", reason="a step too long for the general kernel's grid")
 def test_attention_float32_of_more_tokens_than_a_grid_dimension():
   from gpu_helpers import make_attention_case
