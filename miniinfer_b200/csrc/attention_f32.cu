@@ -3,7 +3,7 @@
 // What attention_generic.cu computes, for rows that share their keys: a block takes up to 32 (token, query head) rows of one
 // key/value head, brings the keys and values 32 at a time into shared memory by cp.async (two stages) and uses them for all
 // of its rows, where the generic kernel reads them from L2 again for every token and head.  A warp has eight rows: a lane
-// is a key while the scores are made, and four output columns (or eight) while the values are weighed.
+// is two keys of four of them while the scores are made, and four output columns (or eight) while the values are weighed.
 //
 // The order of the arithmetic of a row depends on its position, the window and keep_first alone.  Its visible keys are cut into segments of
 // 256 keys at multiples of 256 (first those of the kept first keys, then those of the window or of all earlier keys); a
@@ -12,10 +12,10 @@
 // rows in its shared memory for the block that owns a row - and the result is bit-equal whatever the number of blocks, however
 // the request was cut into steps and whatever else is in the batch.
 //
-// What bounds it: for prompt portions the reads of shared memory (nine of 16 bytes a lane for 16 packed FMAs), for single
-// tokens, whose segments four warps walk together, the latency of a chunk's scores.  Measured on B200, 16 / 8 heads of 128,
-// microseconds in the generic kernel and here: 300 new tokens 179 -> 88, 400 behind 1600 others 2850 -> 605, one token behind
-// 700 248 -> 23, eight tokens behind 2000 each 1484 -> 62.
+// What bounds it: for prompt portions the reads of shared memory and two blocks an SM (six reads of 16 bytes a lane for 16 packed
+// FMAs of scores, three for 32 FMAs of values), for single tokens, whose segments four warps walk together, the latency of a chunk's scores.
+// Measured on B200, 16 / 8 heads of 128, microseconds in the generic kernel and here: 300 new tokens 179 -> 75 (85 with a key a
+// lane for all eight rows), 400 behind 1600 others 2850 -> 551 (605), one token behind 700 248 -> 23, eight tokens behind 2000 each 1484 -> 62.
 #include <cooperative_groups.h>
 
 #include <type_traits>
@@ -56,8 +56,8 @@ struct Layout {
   __host__ __device__ int keys(int stage) const { return stage * CHUNK * ldk; }
   __host__ __device__ int values(int stage) const { return 2 * CHUNK * ldk + stage * CHUNK * (ldk - 4); }
   __host__ __device__ int queries() const { return 2 * CHUNK * (2 * ldk - 4); }
-  __host__ __device__ int weights() const { return queries() + ROWS * (ldk - 4); }
-  __host__ __device__ int running() const { return weights() + WARPS * CHUNK * 8; }
+  __host__ __device__ int weights() const { return queries() + ROWS * ldk; }      // of a warp: [key][row], then the rows' factors
+  __host__ __device__ int running() const { return weights() + WARPS * (CHUNK + 1) * 8; }
   __host__ __device__ int floats() const { return running() + ROWS * (ldk - 4) + 4 * ROWS; }
 };
 
@@ -65,7 +65,8 @@ template <int WARPS, int RW, int NV>
 __global__ void __launch_bounds__(32 * WARPS)
 attention_f32_kernel(const F32Args a) {
   using L = Layout<WARPS, RW, NV>;
-  constexpr int ROWS = L::ROWS, THREADS = 32 * WARPS;
+  constexpr int ROWS = L::ROWS, THREADS = 32 * WARPS, HALF = 4;
+  static_assert(RW == 2 * HALF, "");
   extern __shared__ __align__(16) float sm[];
   cg::cluster_group cluster = cg::this_cluster();
   const L at(a.hd);
@@ -96,7 +97,7 @@ attention_f32_kernel(const F32Args a) {
     const int r = i / (hd / 4), d = (i % (hd / 4)) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < rows) v = *reinterpret_cast<const float4*>(a.q + (size_t)(row0 + tok0 + r / group) * a.q_stride + (size_t)(kvh * group + r % group) * hd + d);
-    *reinterpret_cast<float4*>(sm + at.queries() + r * hd + d) = v;
+    *reinterpret_cast<float4*>(sm + at.queries() + r * at.ldk + d) = v;
     *reinterpret_cast<float4*>(run_o + r * hd + d) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   for (int r = threadIdx.x; r < ROWS; r += THREADS) {
@@ -104,12 +105,14 @@ attention_f32_kernel(const F32Args a) {
     run_l[r] = a.sink ? 1.f : 0.f;
   }
 
-  // what this warp's rows see
-  const int wrow = warp * RW;
-  int p[RW], lo[RW], kept[RW];
+  // Of a chunk's scores a lane makes those of four of its warp's rows and two keys, sixteen apart.  Lanes i and i ^ 1 then read the same keys and lanes i and
+  // i ^ 2 the same rows, and a 16-byte read of either takes two cycles of shared memory instead of four (with a key a lane for all eight rows
+  // 16 packed FMAs needed 20 cycles of reads, now 12).
+  const int wrow = warp * RW, half = lane & 1, slot = lane >> 1;
+  int p[HALF], lo[HALF], kept[HALF];      // what its rows see
 #pragma unroll
-  for (int i = 0; i < RW; ++i) {
-    const int r = wrow + i;
+  for (int i = 0; i < HALF; ++i) {
+    const int r = wrow + HALF * half + i;
     p[i] = r < rows ? p0 + r / group : -1;
     lo[i] = r < rows ? mi::first_visible(p[i], a.window) : 0;
     kept[i] = r < rows && a.window > 0 ? min(a.keep_first, lo[i]) : 0;
@@ -125,14 +128,16 @@ attention_f32_kernel(const F32Args a) {
 
   for (int round = 0; round < segs; round += a.cluster) {
     const int seg = round + rank;
-    float m[RW], l[RW], o[RW][4 * NV];
+    float m[HALF], l[HALF], o[RW][4 * NV];
 #pragma unroll
-    for (int i = 0; i < RW; ++i) {
+    for (int i = 0; i < HALF; ++i) {
       m[i] = -INFINITY;
       l[i] = 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < RW; ++i)
 #pragma unroll
       for (int d = 0; d < 4 * NV; ++d) o[i][d] = 0.f;
-    }
     if (seg < segs) {
       const bool first_keys = seg < kept_segs;
       const int base = first_keys ? seg * SEG : (seg0 + seg - kept_segs) * SEG;
@@ -168,61 +173,80 @@ attention_f32_kernel(const F32Args a) {
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
         // a row's key is visible in this stretch; a warp none of whose rows sees any key of the chunk has nothing to do
-        const int j = c + lane;
-        bool seen[RW], any = false, every = true;
+        bool seen[HALF][2], any = false, every = true;
 #pragma unroll
-        for (int i = 0; i < RW; ++i) {
-          seen[i] = first_keys ? j < kept[i] : j >= lo[i] && j <= p[i];
-          any |= seen[i];
-          every &= seen[i] || p[i] < 0;      // (a row that does not exist)
-        }
+        for (int i = 0; i < HALF; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int j = c + slot + 16 * e;
+            seen[i][e] = first_keys ? j < kept[i] : j >= lo[i] && j <= p[i];
+            any |= seen[i][e];
+            every &= seen[i][e] || p[i] < 0;      // (a row that does not exist)
+          }
         if (__any_sync(0xffffffffu, any)) {
-          uint64_t acc[RW];
+          uint64_t acc[HALF][2];
 #pragma unroll
-          for (int i = 0; i < RW; ++i) acc[i] = 0;
-          const float* kr = sm + at.keys(s) + lane * at.ldk;
-          const float* qr = sm + at.queries() + wrow * hd;
+          for (int i = 0; i < HALF; ++i) acc[i][0] = acc[i][1] = 0;
+          const float* kr = sm + at.keys(s) + slot * at.ldk;
+          const float* qr = sm + at.queries() + (wrow + HALF * half) * at.ldk;
 #pragma unroll 4
           for (int d = 0; d < hd; d += 4) {
-            const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kr + d);
+            const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(kr + d), k1 = *reinterpret_cast<const ulonglong2*>(kr + 16 * at.ldk + d);
 #pragma unroll
-            for (int i = 0; i < RW; ++i) {
-              const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qr + i * hd + d);
-              acc[i] = fma2(q4.y, k4.y, fma2(q4.x, k4.x, acc[i]));
+            for (int i = 0; i < HALF; ++i) {
+              const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qr + i * at.ldk + d);
+              acc[i][0] = fma2(q4.y, k0.y, fma2(q4.x, k0.x, acc[i][0]));
+              acc[i][1] = fma2(q4.y, k1.y, fma2(q4.x, k1.x, acc[i][1]));
             }
           }
-          float pe[RW];
+          float pe[2][HALF], alpha[HALF];
 #pragma unroll
-          for (int i = 0; i < RW; ++i) {
-            float x, y;
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(acc[i]));
-            const float sc = seen[i] ? a.scale * (x + y) : -INFINITY;
-            const float m_new = fmaxf(m[i], mi::warp_max(sc));
+          for (int i = 0; i < HALF; ++i) {
+            float sc[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              float x, y;
+              asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(acc[i][e]));
+              sc[e] = seen[i][e] ? a.scale * (x + y) : -INFINITY;
+            }
+            float m_new = fmaxf(sc[0], sc[1]);
+#pragma unroll
+            for (int k = 16; k > 1; k >>= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, k));
+            m_new = fmaxf(m[i], m_new);
             const bool none = m_new == -INFINITY;      // no key of this segment seen yet, or none whose score weighs anything
-            const float alpha = none ? 1.f : expf(m[i] - m_new);
-            pe[i] = seen[i] ? expf(sc - (none ? 0.f : m_new)) : 0.f;
-            l[i] = l[i] * alpha + mi::warp_sum(pe[i]);
+            alpha[i] = none ? 1.f : expf(m[i] - m_new);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) pe[e][i] = seen[i][e] ? expf(sc[e] - (none ? 0.f : m_new)) : 0.f;
+            float sum = pe[0][i] + pe[1][i];      // (as the halves of a warp with a key a lane add up)
+#pragma unroll
+            for (int k = 16; k > 1; k >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
+            l[i] = l[i] * alpha[i] + sum;
             m[i] = m_new;
 #pragma unroll
-            for (int d = 0; d < 4 * NV; ++d) o[i][d] *= alpha;
+            for (int e = 0; e < 2; ++e)
+              if (!seen[i][e]) pe[e][i] = -1.f;      // (no weight is)
           }
-          float* pw = sm + at.weights() + warp * CHUNK * 8;
+          float* pw = sm + at.weights() + warp * (CHUNK + 1) * RW;
 #pragma unroll
-          for (int i = 0; i < RW; i += 2) *reinterpret_cast<float2*>(pw + lane * 8 + i) = make_float2(pe[i], pe[i + 1]);
+          for (int e = 0; e < 2; ++e) *reinterpret_cast<float4*>(pw + (slot + 16 * e) * RW + HALF * half) = make_float4(pe[e][0], pe[e][1], pe[e][2], pe[e][3]);
+          if (slot == 0) *reinterpret_cast<float4*>(pw + CHUNK * RW + HALF * half) = make_float4(alpha[0], alpha[1], alpha[2], alpha[3]);
           __syncwarp();
+#pragma unroll
+          for (int i = 0; i < RW; ++i) {
+            const float f = pw[CHUNK * RW + i];
+#pragma unroll
+            for (int d = 0; d < 4 * NV; ++d) o[i][d] *= f;
+          }
           const float* vr = sm + at.values(s);
           // MASKED: a row takes nothing from a key that it may not see, not even zero times its value, which may be no number
           auto weigh = [&](auto masked) {
             constexpr bool MASKED = decltype(masked)::value;
-            unsigned mask[RW];
-#pragma unroll
-            for (int i = 0; i < RW; ++i) mask[i] = MASKED ? __ballot_sync(0xffffffffu, seen[i]) : 0u;
 #pragma unroll(MASKED ? 1 : 4)
             for (int jj = 0; jj < CHUNK; ++jj) {
               float w[RW];
 #pragma unroll
               for (int i = 0; i < RW; i += 2) {
-                const float2 t = *reinterpret_cast<const float2*>(pw + jj * 8 + i);
+                const float2 t = *reinterpret_cast<const float2*>(pw + jj * RW + i);
                 w[i] = t.x;
                 w[i + 1] = t.y;
               }
@@ -233,7 +257,7 @@ attention_f32_kernel(const F32Args a) {
                   const float4 v = *reinterpret_cast<const float4*>(vr + jj * hd + d);
 #pragma unroll
                   for (int i = 0; i < RW; ++i) {
-                    if (MASKED && !(mask[i] >> jj & 1)) continue;
+                    if (MASKED && w[i] < 0.f) continue;
                     o[i][4 * n] = fmaf(w[i], v.x, o[i][4 * n]);
                     o[i][4 * n + 1] = fmaf(w[i], v.y, o[i][4 * n + 1]);
                     o[i][4 * n + 2] = fmaf(w[i], v.z, o[i][4 * n + 2]);
@@ -260,9 +284,12 @@ attention_f32_kernel(const F32Args a) {
         const int d = 128 * n + 4 * lane;
         if (d < hd) *reinterpret_cast<float4*>(part_o + r * hd + d) = make_float4(o[i][4 * n], o[i][4 * n + 1], o[i][4 * n + 2], o[i][4 * n + 3]);
       }
-      if (lane == 0) {
-        part_m[r] = m[i];
-        part_l[r] = l[i];
+    }
+    if (slot == 0) {
+#pragma unroll
+      for (int i = 0; i < HALF; ++i) {
+        part_m[wrow + HALF * half + i] = m[i];
+        part_l[wrow + HALF * half + i] = l[i];
       }
     }
     cluster.sync();
