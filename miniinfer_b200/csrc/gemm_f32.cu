@@ -9,7 +9,7 @@
 // path gives bit-equal logits however the tokens are cut into steps.  The reference has no 32-bit path (it calls cuBLAS in
 // fp16, miniinfer/layers/linear.py:30-32).
 //
-// What bounds it: reads of shared memory for many rows, latency for few.  A thread computes 8 x 4 elements (fewer for small
+// What bounds it: the packed FMAs' own rate and the clusters' ends for many rows, latency for few.  A thread computes 8 x 4 elements (fewer for small
 // M): rows are staged as they lie in memory, K fastest, so that cp.async brings them without a transposition and a 16-byte
 // read of shared memory gives two packed operands; rows of 36 floats keep the eight rows that a warp reads at a time in
 // different banks.  Two forms, both in three stages of 32 columns:
@@ -19,9 +19,10 @@
 // The groups go to the four blocks of a cluster, whose sums are added up in each other's shared memory, in the order that
 // one block would - for few rows only where the tiles alone leave SMs idle, for many from some hundred columns on.
 // Measured on B200, weights in L2, in microseconds, against one form of 64 x 64 tiles, 4 x 4 elements a thread, staged one
-// step at a time: 8 x 4096 x 1024 74 -> 9.4, 16 x 1024 x 2048 146 -> 6.8, 40 x 6144 x 1024 75 -> 28, 302 x 4096 x 1024 174 -> 86,
-// 302 x 1024 x 2048 149 -> 52, 2048 x 4096 x 1024 583 -> 484 (35 of the 70 TFLOP/s that a loop of FMAs alone reaches),
-// 8 x 151936 x 1024 727 -> 120 (5.2 TB/s).  Sixteen partial sums also err less: 1.2e-7 against 5.7e-7 of the norm at K = 1024.
+// step at a time: 8 x 4096 x 1024 74 -> 9.1, 16 x 1024 x 2048 146 -> 8.9, 40 x 6144 x 1024 75 -> 27, 302 x 4096 x 1024 174 -> 78,
+// 302 x 1024 x 2048 149 -> 48, 2048 x 4096 x 1024 583 -> 433 (40 of the 70 TFLOP/s that a loop of FMAs alone reaches),
+// 8 x 151936 x 1024 727 -> 112 (5.6 TB/s).  (With lanes that share neither rows in pairs and copies that check and place each row
+// by itself: 9.8, 9.0, 29, 88, 53, 491, 124.)  Sixteen partial sums also err less: 1.2e-7 against 5.7e-7 of the norm at K = 1024.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -53,17 +54,20 @@ __device__ __forceinline__ float halves(uint64_t v) {
   return lo + hi;
 }
 
-// Rows row0 .. of a matrix with `rows` rows, ld values apart, columns k0 .. k0 + 31, into ROWS staged rows, by THREADS threads
-// of which this one is number `thread`; zeros beyond the matrix and from column K on.
+// Rows row0 .. of a matrix with `rows` rows, ld values apart, columns k0 .. k0 + 31, into ROWS staged rows, by THREADS threads of which this one
+// is number `thread`.  A copy costs a minimum, a multiplication and itself: rows beyond the matrix are its last one again or what lay there, and nobody
+// stores their sums (with a check of each row and an address of its own the copies took a tenth of the kernel's time).  Columns from K on are zeros.
 template <int ROWS, int THREADS, bool VEC>
 __device__ __forceinline__ void stage_rows(float* dst, const float* src, int row0, int rows, int ld, int k0, int K, int thread) {
-  constexpr int W = VEC ? 4 : 1, PER_ROW = BK / W;
-#pragma unroll 4
-  for (int i = thread; i < ROWS * PER_ROW; i += THREADS) {
-    const int r = i / PER_ROW, c = (i % PER_ROW) * W;
-    const bool valid = row0 + r < rows && k0 + c < K;
-    copy_async<VEC>(dst + r * LDS + c, valid ? src + (size_t)(row0 + r) * ld + k0 + c : src, valid);
-  }
+  constexpr int W = VEC ? 4 : 1, PER_ROW = BK / W, AT_ONCE = THREADS / PER_ROW;
+  static_assert(THREADS % PER_ROW == 0 && ROWS % AT_ONCE == 0, "");
+  const int r = row0 + thread / PER_ROW, c = thread % PER_ROW * W;
+  const bool valid = k0 + c < K;
+  const char* column = reinterpret_cast<const char*>(src + (valid ? k0 + c : 0));
+  dst += thread / PER_ROW * LDS + c;
+#pragma unroll VEC ? 8 : 4
+  for (int i = 0; i < ROWS; i += AT_ONCE)
+    if (!VEC || row0 + i < rows) copy_async<VEC>(dst + i * LDS, reinterpret_cast<const float*>(column + (long long)min(r + i, rows - 1) * (4u * ld)), valid);
 }
 
 // TM: rows of a thread (a warp has 4 TM rows x 32 columns).  SHARED: four warps, 2 x 2, share a tile; else a warp has the
@@ -85,7 +89,9 @@ __device__ __forceinline__ void product(float* __restrict__ out, const float* __
   extern __shared__ __align__(16) float sm[];
   const int m0 = m_tile * BM, n0 = n_tile * BN;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, thread = SHARED ? threadIdx.x : lane;
-  const int row = (SHARED ? (warp & 1) * 4 * TM : 0) + (lane & 3), col = (SHARED ? (warp >> 1) * 8 * TN : 0) + (lane >> 2);
+  // A 16-byte read of a warp takes two cycles of shared memory instead of four if the lanes i and i ^ 1, or i and i ^ 2, of all read the same
+  // place: the rows of x are shared by the former and those of w by the latter
+  const int row = (SHARED ? (warp & 1) * 4 * TM : 0) + (lane >> 1 & 1) + (lane >> 4) * 2, col = (SHARED ? (warp >> 1) * 8 * TN : 0) + (lane & 1) + (lane >> 2 & 3) * 2;
   float* stages = sm + (SHARED ? 0 : warp * STAGES * T::STAGE);
   const int len = ((K + GROUPS * PARTS - 1) / (GROUPS * PARTS) + BK - 1) / BK * BK;       // columns of a part
   const int per_part = len / BK;
@@ -213,7 +219,7 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
 }
 
 template <int TM, bool SHARED, bool VEC>
-__global__ void __cluster_dims__(GROUPS, 1, 1) __launch_bounds__(128)
+__global__ void __cluster_dims__(GROUPS, 1, 1) __launch_bounds__(128, SHARED ? 3 : 1)      // (as many as shared memory holds; with two 302 x 4096 x 1024 takes 89 us)
 gemm_f32_groups_kernel(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w, int M, int N, int K, int ldx, int ldo) {
   product<TM, SHARED, true, VEC>(out, x, w, M, N, K, ldx, ldo, blockIdx.y, blockIdx.x / GROUPS, blockIdx.x % GROUPS);
 }
@@ -234,13 +240,13 @@ int launch_tiles(float* out, const float* x, const float* w, int M, int N, int K
     if (dev >= 0 && dev < 64) ready[dev] = true;
   }
   // Few columns: a block walks all parts of a shared tile itself, for a cluster's blocks would wait longer for one another than
-  // they work (`alone`, below).  In microseconds, walked / in clusters: 40 x 1024 x 128 7.6 / 8.8, x 192 10.7 / 8.8; 300 x 1024
-  // x 64 4.6 / 9.7, x 256 14.0 / 15.9, x 384 20.1 / 16.3; 40 x 4096 x 256 13.9 / 15.4; 300 x 4096 x 384 46 / 49, x 512 60 / 50; 2048 x
-  // 1024 x 384 58 / 73, x 512 75 / 73; 2048 x 4096 x 64 41 / 144, x 384 196 / 273.  (64 x 64 tiles before: 300 x 1024 x 64 5.9, 2048 x
-  // 4096 x 64 41.5, x 384 222.)
-  // Few rows: from a tile for every SM on, a block walks a tile's groups itself (24 x 6144 x 1024, 192 tiles: 21.5 us against
-  // 22.4 with clusters; 8 x 151936 x 1024: 120 against 206).  Shared tiles are better off in clusters at any size (2048 x 4096 x
-  // 1024: 484 against 499; 302 x 4096 x 1024: 86 against 121), whose smaller blocks fill the SMs more evenly.
+  // they work (`alone`, below).  In microseconds, walked / in clusters: 40 x 1024 x 128 8.8 / 9.1, x 192 10.0 / 9.0; 300 x 1024
+  // x 64 8.7 / 10.2, x 256 12.8 / 15.7, x 384 18.0 / 16.0; 40 x 4096 x 256 13.0 / 15.6; 300 x 4096 x 384 41 / 45, x 512 54 / 45; 2048 x
+  // 1024 x 384 54 / 66, x 512 70 / 66; 2048 x 4096 x 64 38 / 134, x 384 178 / 243.
+  // Few rows: from a tile for every SM on, a block walks a tile's groups itself (24 x 6144 x 1024, 192 tiles: 17.8 us against
+  // 20.2 with clusters; 8 x 151936 x 1024: 112 against 191).  Shared tiles of many columns are better off in clusters, whose smaller
+  // blocks fill the SMs more evenly (302 x 4096 x 1024: 78 against 96); 2048 x 4096 x 1024 would take 421 instead of 433, but only while
+  // the last round of blocks is nearly full.
   const long long tiles = (long long)m_tiles * n_tiles;
   const bool alone = K <= 128 || (K <= 256 && tiles >= 64) || (K <= 384 && tiles >= 320);
   if (SHARED ? alone : n_tiles >= mi::sm_count())
