@@ -610,10 +610,10 @@ DELTA_SEGMENTED_MAX_ITEMS = 4      # the same bound for the delta rule, whose sc
 # 16 heads (128 blocks) 7.23 -> 8.11 ms
 DELTA_SEGMENTED_MAX_BLOCKS = 96
 # New tokens a request from which a bfloat16 delta rule goes a chunk at a time (csrc/chunked_state.cu).  Measured on B200, the operation
-# for 8 / 16 / 32 heads of 128 x 128, chunks against the walk in order, in microseconds.  One decay a key channel: 96 tokens 64, 69, 75
-# against 62, 63, 65; 112 tokens 65, 69, 75 against 71, 73, 75; 128 tokens 65, 70, 75 against 80, 82, 85; 256 tokens 73, 78, 90 against 153,
-# 156, 162.  One decay a head: 96 tokens 65, 69, 75 against 60, 61, 63; 112 tokens 65, 69, 68 against 68, 70, 73; 128 tokens 66, 69, 75
-# against 77, 79, 82; 256 tokens 72, 78, 89 against 145, 149, 153
+# for 8 / 16 / 32 heads of 128 x 128, chunks against the walk in order, in microseconds.  One decay a key channel: 80 tokens 53, 60, 66
+# against 52, 55, 57; 96 tokens 53, 60, 67 against 61, 64, 67; 112 tokens 53, 60, 67 against 70, 73, 76; 256 tokens 62, 68, 82 against 107, 155,
+# 163.  One decay a head: 80 tokens 52, 58, 64 against 49, 31, 54; 96 tokens 52, 58, 64 against 59, 43, 63; 112 tokens 52, 59, 65 against 66, 49,
+# 73; 128 tokens 54, 58, 65 against 74, 75, 82; 256 tokens 60, 66, 77 against 83, 123, 151
 DELTA_CHUNK_MIN_TOKENS = 112
 
 
@@ -703,9 +703,9 @@ def gated_delta(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Te
                                  DELTA_CHUNK_MIN_TOKENS, _stream()), kernels=launches)
 
 
-# The same for linear attention.  Decays a key channel: 48 tokens 36, 44, 47 against 38, 41, 41; 64 tokens 36, 42, 48 against 45, 49,
-# 50; 128 tokens 39, 47, 51 against 81, 84, 87.  A constant a head: 48 tokens 35, 43, 45 against 36, 37, 37; 64 tokens 34, 40, 45 against 42,
-# 44, 46; 128 tokens 36, 44, 49 against 76, 77, 80
+# The same for linear attention.  Decays a key channel: 48 tokens 35, 49, 50 against 39, 42, 43; 64 tokens 35, 45, 49 against 43, 46,
+# 47; 80 tokens 36, 47, 52 against 47, 55, 58; 128 tokens 45, 49, 52 against 78, 83, 87.  A constant a head: 48 tokens 36, 48, 49 against 37, 38, 38;
+# 64 tokens 37, 43, 47 against 40, 42, 43; 80 tokens 36, 46, 49 against 46, 49, 52; 128 tokens 43, 46, 50 against 74, 75, 78
 LINEAR_CHUNK_MIN_TOKENS = 64
 LINEAR_SEGMENTED_MAX_ITEMS = 8     # steps of at most this many requests run long bfloat16 portions in stretches side by side
 # ... and only while the walk in order would leave SMs idle (blocks in order, all requests; an SM holds three, and
