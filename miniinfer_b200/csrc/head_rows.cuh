@@ -39,14 +39,13 @@ inline dim3 head_rows_grid(long long units) {
   return dim3((unsigned)(blocks < most ? blocks : most));
 }
 
-// 1 / (1 + exp(-z)) and z times it by the hardware's exponential and reciprocal, for what is rounded to bfloat16 next (the reciprocal keeps
+// 1 / (1 + exp(-z)) by the hardware's exponential and reciprocal, for what is rounded to bfloat16 next (the reciprocal keeps
 // results below 2^-126): a handful of instructions where the exact ones are fifty, of which a kernel this short mostly waits for the fetching.
 __device__ __forceinline__ float near_sigmoid(float z) {
   float r;
   asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-z)));
   return r;
 }
-__device__ __forceinline__ float near_silu(float z) { return z * near_sigmoid(z); }
 
 // out[t, h] = o / sqrt(mean(o^2) + eps) * norm_w * act(gate[t, h]), o = raw[t, h]: norm_w [vdim] and gate optional.  A warp
 // asks for the rows of UNITS (token, head) pairs before it works on the first; heads of more than 128 values take its lanes several times.

@@ -53,10 +53,14 @@ causal_conv_kernel(T* __restrict__ out, int ldo, const T* __restrict__ x, int ld
   out[(size_t)t * ldo + c] = mi::from_float<T>(acc);
 }
 
+// A call, and not one copy of an exponential and a division for every value that a thread makes.
+__device__ __noinline__ float2 silu_pair(float x, float y) { return make_float2(silu_f(x), silu_f(y)); }
+
 // The same for bfloat16 rows that can be read four bytes at a time: a thread has two channels of a block's tokens, the inputs of CONV_AHEAD of them
 // on their way at a time, the last taps - 1 in registers.  Stretches of one request are walked one after the other.  (2048 tokens of
-// 2048 channels, four taps: a value a thread 32 us; eight channels and four tokens a thread 17.8, of which most was the way of 32 KB of
-// instructions from L2 - 32 exact activations -; so 8.7; 1000 tokens of 8192 channels 31.2 and 14.)
+// 2048 channels, four taps, with the pass that keeps the state: a value a thread 32 us; eight channels and four tokens a thread 18.5, of which
+// most was the way of 32 KB of instructions from L2 - 32 copies of an activation -; so 10.7; 1000 tokens of 8192 channels 33 and 18.4.  The
+// hardware's exponential and reciprocal in place of the call would take 8.5 and 13.8, and round some results to the other neighbour.)
 constexpr int CONV_AHEAD = 8;
 
 template <int TAPS>
@@ -109,7 +113,7 @@ causal_conv_vec_kernel(__nv_bfloat16* __restrict__ out, int ldo, const __nv_bflo
           acc.x = fmaf(wt[0][TAPS - 1 - k], in[k].x, acc.x);
           acc.y = fmaf(wt[1][TAPS - 1 - k], in[k].y, acc.y);
         }
-        if (silu) acc = make_float2(mi::near_silu(acc.x), mi::near_silu(acc.y));
+        if (silu) acc = silu_pair(acc.x, acc.y);
         if (t + n < end) *reinterpret_cast<__nv_bfloat162*>(out + (size_t)(t + n) * ldo + c) = __floats2bfloat162_rn(acc.x, acc.y);
       }
     }
@@ -784,8 +788,8 @@ MI_API int mi_causal_conv(void* out, int ldo, const void* x, int ldx, int dtype,
   if (T == 0) return 0;
   dim3 grid((C + 255) / 256, T), sgrid((C + 255) / 256, items);
   // two channels and a stretch of tokens a thread where there are more than 2^17 values, rows start on 16-byte boundaries
-  // and hold whole 16 bytes.  Four taps, this way / a value a thread, in microseconds: 32 x 2048 4.0 / 3.8,
-  // 64 x 2048 4.1 / 4.1, 128 x 2048 4.1 / 4.9, 256 x 2048 4.3 / 6.5, 64 x 8192 4.3 / 6.6, 2048 x 2048 8.7 / 29.8
+  // and hold whole 16 bytes.  Four taps, tokens of one request, this way / a value a thread, in microseconds: 128 x 2048 4.6 / 4.8,
+  // 256 x 2048 4.9 / 6.6, 64 x 8192 4.9 / 6.6, 2048 x 2048 10.7 / 29.8
   const bool vec = dtype == MI_BF16 && (long long)T * C > 1 << 17 && taps >= 2 && taps <= 4 && C % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 &&
                    ((uintptr_t)x % 16) == 0 && ((uintptr_t)out % 16) == 0 && ((uintptr_t)w % 8) == 0;
   if (vec) {

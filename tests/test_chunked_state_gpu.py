@@ -317,6 +317,21 @@ def test_causal_convolution_of_short_stretches(lengths):
   test_causal_convolution_eight_channels_a_thread(4, lengths, 2048, 8)
 
 
+def test_causal_convolution_rounds_the_same_values_in_steps_of_few_and_of_many_tokens():
+  """Two kernels share bfloat16 steps by their size; a row's result does not tell which one it was: same sums, same activation."""
+  from miniinfer_b200.kernels import ops
+  T, C, r = 64, 8192, torch.Generator().manual_seed(15)
+  x = (4 * torch.randn((T, C), generator=r)).to(torch.bfloat16).to(DEV)
+  w, bias, start = torch.randn((C, 4), generator=r).to(DEV), torch.randn(C, generator=r).to(DEV), torch.randn((2, 3 * C), generator=r).to(DEV)
+  runs = []
+  for n in (T, 8):      # tokens a step
+    out, state = torch.empty_like(x), start.clone()
+    for t in range(0, T, n):
+      ops.causal_conv(out[t:t + n], x[t:t + n], w, bias, state, _ctx((n,)))
+    runs.append((out, state))
+  assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
+
+
 @pytest.mark.parametrize("D", [50, 136])      # channels that the chunks do not take: rows of no whole 16 bytes, more than 128
 @pytest.mark.parametrize("kind,per_head", [("delta", False), ("linear", False), ("linear", True)])
 def test_long_portions_of_heads_that_chunks_do_not_take(kind, per_head, D):
