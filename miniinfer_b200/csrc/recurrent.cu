@@ -56,22 +56,31 @@ causal_conv_kernel(T* __restrict__ out, int ldo, const T* __restrict__ x, int ld
 // A call, and not one copy of an exponential and a division for every value that a thread makes.
 __device__ __noinline__ float2 silu_pair(float x, float y) { return make_float2(silu_f(x), silu_f(y)); }
 
-// The same for bfloat16 rows that can be read four bytes at a time: a thread has two channels of a block's tokens, the inputs of CONV_AHEAD of them
-// on their way at a time, the last taps - 1 in registers.  Stretches of one request are walked one after the other.  (2048 tokens of
-// 2048 channels, four taps, with the pass that keeps the state: a value a thread 32 us; eight channels and four tokens a thread 18.5, of which
-// most was the way of 32 KB of instructions from L2 - 32 copies of an activation -; so 10.7; 1000 tokens of 8192 channels 33 and 18.4.  The
-// hardware's exponential and reciprocal in place of the call would take 8.5 and 13.8, and round some results to the other neighbour.)
-constexpr int CONV_AHEAD = 8;
+// The same for bfloat16 rows that can be read four bytes at a time: a thread has two channels of a block's tokens.  Where they are one request's,
+// the inputs of CONV_AHEAD of them are on their way at a time, the last taps - 1 in registers; where several requests share the block, CONV_MIXED
+// tokens at a time fetch all of their inputs, each from the rows or from its request's state, whose places were looked up before the wait.
+// (2048 tokens of 2048 channels, four taps, with the pass that keeps the state: a value a thread 32 us; eight channels and four tokens a thread
+// 18.5, of which most was the way of 32 KB of instructions from L2 - 32 copies of an activation -; so 10.7; 1000 tokens of 8192 channels 33 and
+// 17.3.  The hardware's exponential and reciprocal in place of the call would take 8.5 and 13.8, and round some results to the other neighbour.
+// 256 requests of one token, 8192 channels: walked one after the other, each with its look-ups, 38 us, so 20.9; with eight tokens at a
+// time there, and their registers, 19.7, but 2048 tokens of one request of 4096 channels 21.2 instead of 17.2.)
+constexpr int CONV_AHEAD = 8, CONV_MIXED = 4, CONV_MOST = 4 * CONV_AHEAD;
 
 template <int TAPS>
 __global__ void __launch_bounds__(128)
 causal_conv_vec_kernel(__nv_bfloat16* __restrict__ out, int ldo, const __nv_bfloat16* __restrict__ x, int ldx, const float* __restrict__ w,
                        const float* __restrict__ bias, const float* __restrict__ in_bias, const float* __restrict__ state, long long state_stride,
-                       const int* __restrict__ token_item, const int* __restrict__ q_start, const int* __restrict__ q_len,
-                       const int* __restrict__ seq_slot, int T, int C, int silu, int tokens) {
-  const int c = 2 * (blockIdx.x * blockDim.x + threadIdx.x), t_end = min(T, (int)(blockIdx.y + 1) * tokens);
+                       const int* __restrict__ token_item, const int* __restrict__ q_start, const int* __restrict__ seq_slot,
+                       int T, int C, int silu, int tokens) {
+  __shared__ int place[CONV_MOST], slot[CONV_MOST];      // of the block's tokens: the number among the request's new tokens, the state's row
+  const int c = 2 * (blockIdx.x * blockDim.x + threadIdx.x), t0 = blockIdx.y * tokens, n_tokens = min(tokens, T - t0);
   const bool live = c < C;
   const int cc = live ? c : 0;
+  if (threadIdx.x < n_tokens) {
+    const int item = token_item[t0 + threadIdx.x];
+    place[threadIdx.x] = t0 + (int)threadIdx.x - q_start[item];
+    slot[threadIdx.x] = seq_slot[item];
+  }
   float wt[2][TAPS], b[2], ib[2];
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
@@ -80,44 +89,61 @@ causal_conv_vec_kernel(__nv_bfloat16* __restrict__ out, int ldo, const __nv_bflo
     b[e] = bias ? bias[cc + e] : 0.f;
     ib[e] = in_bias ? in_bias[cc + e] : 0.f;
   }
+  __syncthreads();
   mi::grid_dependency_sync();
   if (!live) return;
-  const __nv_bfloat16* xc = x + c;
+  const __nv_bfloat16* xc = x + (size_t)t0 * ldx + c;      // of the block's first token
+  __nv_bfloat16* oc = out + (size_t)t0 * ldo + c;
   auto input = [&](__nv_bfloat162 v) {
     const float2 f = __bfloat1622float2(v);
     return make_float2(f.x + ib[0], f.y + ib[1]);
   };
-#pragma unroll 1
-  for (int t = blockIdx.y * tokens; t < t_end;) {
-    const int item = token_item[t], start = q_start[item], j = t - start, end = min(t_end, start + q_len[item]);
-    const float* st = state + (size_t)seq_slot[item] * state_stride + c;
-    float2 in[TAPS];      // in[k]: the input k tokens back
+  auto before = [&](int t, int k) {      // the input k > 0 tokens before token t of the block: a row's, or the state's
+    if (place[t] >= k) return input(*reinterpret_cast<const __nv_bfloat162*>(xc + (long long)(t - k) * ldx));
+    const float* st = state + (size_t)slot[t] * state_stride + (size_t)(TAPS - 1 + place[t] - k) * C + c;
+    return make_float2(st[0], st[1]);
+  };
+  auto finish = [&](int t, const float2 (&in)[TAPS]) {      // in[k]: the input k tokens back
+    float2 acc = make_float2(b[0], b[1]);
 #pragma unroll
-    for (int k = 1; k < TAPS; ++k) {      // (those before the item's new tokens are the state's)
-      if (j >= k) in[k - 1] = input(*reinterpret_cast<const __nv_bfloat162*>(xc + (size_t)(t - k) * ldx));
-      else in[k - 1] = make_float2(st[(size_t)(TAPS - 1 + j - k) * C], st[(size_t)(TAPS - 1 + j - k) * C + 1]);
+    for (int k = TAPS - 1; k >= 0; --k) {      // oldest input first
+      acc.x = fmaf(wt[0][TAPS - 1 - k], in[k].x, acc.x);
+      acc.y = fmaf(wt[1][TAPS - 1 - k], in[k].y, acc.y);
     }
+    if (silu) acc = silu_pair(acc.x, acc.y);
+    if (t < n_tokens) *reinterpret_cast<__nv_bfloat162*>(oc + (size_t)t * ldo) = __floats2bfloat162_rn(acc.x, acc.y);
+  };
+  if (place[n_tokens - 1] - place[0] == n_tokens - 1) {      // one request's (a new one starts again from 0)
+    float2 in[TAPS];
+#pragma unroll
+    for (int k = 1; k < TAPS; ++k) in[k - 1] = before(0, k);
 #pragma unroll 1
-    for (; t < end; t += CONV_AHEAD) {
+    for (int t = 0; t < n_tokens; t += CONV_AHEAD) {
       __nv_bfloat162 raw[CONV_AHEAD];
 #pragma unroll
-      for (int n = 0; n < CONV_AHEAD; ++n) raw[n] = *reinterpret_cast<const __nv_bfloat162*>(xc + (size_t)min(t + n, end - 1) * ldx);
+      for (int n = 0; n < CONV_AHEAD; ++n) raw[n] = *reinterpret_cast<const __nv_bfloat162*>(xc + (size_t)min(t + n, n_tokens - 1) * ldx);
 #pragma unroll
       for (int n = 0; n < CONV_AHEAD; ++n) {
 #pragma unroll
         for (int k = TAPS - 1; k > 0; --k) in[k] = in[k - 1];
         in[0] = input(raw[n]);
-        float2 acc = make_float2(b[0], b[1]);
-#pragma unroll
-        for (int k = TAPS - 1; k >= 0; --k) {      // oldest input first
-          acc.x = fmaf(wt[0][TAPS - 1 - k], in[k].x, acc.x);
-          acc.y = fmaf(wt[1][TAPS - 1 - k], in[k].y, acc.y);
-        }
-        if (silu) acc = silu_pair(acc.x, acc.y);
-        if (t + n < end) *reinterpret_cast<__nv_bfloat162*>(out + (size_t)(t + n) * ldo + c) = __floats2bfloat162_rn(acc.x, acc.y);
+        finish(t + n, in);
       }
     }
-    t = end;
+    return;
+  }
+#pragma unroll 1
+  for (int t = 0; t < n_tokens; t += CONV_MIXED) {
+    float2 in[CONV_MIXED][TAPS];
+#pragma unroll
+    for (int n = 0; n < CONV_MIXED; ++n) {
+      const int tt = min(t + n, n_tokens - 1);
+      in[n][0] = input(*reinterpret_cast<const __nv_bfloat162*>(xc + (size_t)tt * ldx));
+#pragma unroll
+      for (int k = 1; k < TAPS; ++k) in[n][k] = before(tt, k);
+    }
+#pragma unroll
+    for (int n = 0; n < CONV_MIXED; ++n) finish(t + n, in[n]);
   }
 }
 
@@ -787,19 +813,22 @@ MI_API int mi_causal_conv(void* out, int ldo, const void* x, int ldx, int dtype,
   MI_REQUIRE(state_stride >= (long long)(taps - 1) * C, "causal_conv: the state rows are too short");
   if (T == 0) return 0;
   dim3 grid((C + 255) / 256, T), sgrid((C + 255) / 256, items);
-  // two channels and a stretch of tokens a thread where there are more than 2^17 values, rows start on 16-byte boundaries
-  // and hold whole 16 bytes.  Four taps, tokens of one request, this way / a value a thread, in microseconds: 128 x 2048 4.6 / 4.8,
-  // 256 x 2048 4.9 / 6.6, 64 x 8192 4.9 / 6.6, 2048 x 2048 10.7 / 29.8
-  const bool vec = dtype == MI_BF16 && (long long)T * C > 1 << 17 && taps >= 2 && taps <= 4 && C % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 &&
+  // Two channels and a stretch of tokens a thread for steps of many values whose rows start on 16-byte boundaries and hold whole 16 bytes: the
+  // more requests share a block's tokens the later, for they don't share inputs.  Four taps, this way / a value a thread, in microseconds:
+  // one request, 70 x 2048 4.2 / 4.0, 128 x 2048 4.3 / 4.8, 64 x 8192 4.5 / 6.6, 2048 x 2048 10.7 / 29.8; some, 127 + 1 x 2048 5.9 / 4.9,
+  // 253 + 3 x 1 x 2048 5.9 / 6.6, 4 x 64 x 2048 4.5 / 6.5; one token each, 32 x 8192 8.2 / 6.2, 64 x 8192 10.0 / 9.2, 72 x 8192 10.3 / 13.9,
+  // 256 x 8192 20.9 / 25; 32 x 1 + 224 x 2048 7.4 / 6.9
+  const long long values = (long long)T * C, most = items == 1 ? 3 << 16 : T >= 64 * items ? 1 << 18 : 1 << 19;
+  const bool vec = dtype == MI_BF16 && values > most && taps >= 2 && taps <= 4 && C % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 &&
                    ((uintptr_t)x % 16) == 0 && ((uintptr_t)out % 16) == 0 && ((uintptr_t)w % 8) == 0;
   if (vec) {
     auto kernel = taps == 2 ? causal_conv_vec_kernel<2> : taps == 3 ? causal_conv_vec_kernel<3> : causal_conv_vec_kernel<4>;
     // as many tokens a block, up to 32, as leave four blocks an SM
     const int across = (C / 2 + 127) / 128;
-    int tokens = 4 * CONV_AHEAD;
+    int tokens = CONV_MOST;
     while (tokens > CONV_AHEAD && (long long)across * ((T + tokens - 1) / tokens) < 4ll * mi::sm_count()) tokens -= CONV_AHEAD;
     mi::launch(kernel, dim3(across, (T + tokens - 1) / tokens), dim3(128), 0, stream, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)x, ldx, w, bias,
-               in_bias, (const float*)state, state_stride, token_item, q_start, q_len, seq_slot, T, C, silu, tokens);
+               in_bias, (const float*)state, state_stride, token_item, q_start, seq_slot, T, C, silu, tokens);
     mi::launch(conv_state_kernel<__nv_bfloat16>, sgrid, dim3(256), 0, stream, state, state_stride, (const __nv_bfloat16*)x, ldx, in_bias,
                q_start, q_len, seq_slot, C, taps);
   } else if (dtype == MI_BF16) {

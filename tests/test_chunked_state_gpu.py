@@ -118,8 +118,8 @@ def test_linear_attention_by_chunks(case, per_head):
 
 
 @pytest.mark.parametrize("taps", [2, 3, 4])
-@pytest.mark.parametrize("lengths,C,lead", [((1025,), 1024, 0), ((1, 2, 700, 3, 1), 1496, 8), ((9, 1018), 1032, 16)])      # items end inside the four tokens of a thread
-def test_causal_convolution_eight_channels_a_thread(taps, lengths, C, lead):
+@pytest.mark.parametrize("lengths,C,lead", [((1025,), 1024, 0), ((1, 2, 700, 3, 1), 1496, 8), ((9, 1018), 1032, 16)])      # items end inside a block's tokens
+def test_causal_convolution_two_channels_a_thread(taps, lengths, C, lead):
   from miniinfer_b200.kernels import ops
   T = sum(lengths)
   r = torch.Generator().manual_seed(taps * T + C)
@@ -312,9 +312,17 @@ def test_linear_attention_in_more_than_one_slab(per_head):
     assert ((out - want).abs() <= 2.0 ** -8 * want.abs().clamp(min=1.0) + 1e-4).all(), i
 
 
-@pytest.mark.parametrize("lengths", [(70,), (1, 2, 31, 33, 4)])      # a stretch of eight tokens a block, and items that end inside it
-def test_causal_convolution_of_short_stretches(lengths):
-  test_causal_convolution_eight_channels_a_thread(4, lengths, 2048, 8)
+@pytest.mark.parametrize("lengths", [(70,), (1, 2, 31, 33, 4), (1,) * 70])      # blocks of eight tokens, and items that end inside them
+@pytest.mark.parametrize("C", [2048, 8192])
+def test_causal_convolution_of_short_stretches(lengths, C):
+  test_causal_convolution_two_channels_a_thread(4, lengths, C, 8)
+
+
+# Blocks of 16, 24 and 32 tokens on 148 SMs: inputs carried from one round of eight tokens to the next, in blocks of one request and of several
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("lengths,C", [((1, 2, 1157, 9, 31), 2048), ((3, 16, 24, 8, 1949, 1, 47), 2048), ((1, 2, 601, 9, 3), 8192), ((32, 64, 1, 520), 8192)])
+def test_causal_convolution_of_long_stretches(taps, lengths, C):
+  test_causal_convolution_two_channels_a_thread(taps, lengths, C, 8)
 
 
 def test_causal_convolution_rounds_the_same_values_in_steps_of_few_and_of_many_tokens():
