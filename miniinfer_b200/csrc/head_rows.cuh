@@ -3,7 +3,8 @@
 // a block a token and four heads spent its time starting and ending
 // (2048 tokens of 8 heads of 128, one value a lane and read against four: the delta rule's inputs 15.0 and 13.1 us; linear attention's
 // inputs with decays, 1800 tokens of 16 heads, 28.5 and 19.9 - the logarithms and exponentials of the decays are most of it).  Read-outs,
-// behind another kernel, with exact activations, unrolled, and as below: 1800 tokens of 16 heads 13.1 and 9.7 us, 2048 of 32 28.6 and 18.2.
+// behind another kernel, unrolled with a copy of the activation a value, and as below: 1800 tokens of 16 heads 13.1 and 11.5 us, 2048 of 32 28.6
+// and 21.6 (9.7 and 18.2 by the hardware's exponential and reciprocal, which round some results to the other neighbour).
 #pragma once
 
 #include "common.cuh"
@@ -39,12 +40,9 @@ inline dim3 head_rows_grid(long long units) {
   return dim3((unsigned)(blocks < most ? blocks : most));
 }
 
-// 1 / (1 + exp(-z)) by the hardware's exponential and reciprocal, for what is rounded to bfloat16 next (the reciprocal keeps
-// results below 2^-126): a handful of instructions where the exact ones are fifty, of which a kernel this short mostly waits for the fetching.
-__device__ __forceinline__ float near_sigmoid(float z) {
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-z)));
-  return r;
+// 1 / (1 + exp(-z)).  A call, and not a copy for every value of a lane, of which a kernel this short would mostly wait for the fetching.
+static __device__ __noinline__ float4 sigmoid4(float4 z) {
+  return make_float4(1.f / (1.f + expf(-z.x)), 1.f / (1.f + expf(-z.y)), 1.f / (1.f + expf(-z.z)), 1.f / (1.f + expf(-z.w)));
 }
 
 // out[t, h] = o / sqrt(mean(o^2) + eps) * norm_w * act(gate[t, h]), o = raw[t, h]: norm_w [vdim] and gate optional.  A warp
@@ -73,7 +71,7 @@ head_output_kernel(__nv_bfloat16* __restrict__ out, int ldo, const float* __rest
       float4 y = scaled4(v, rstd);
       y.x *= w.x; y.y *= w.y; y.z *= w.z; y.w *= w.w;
       if (gate) {
-        const float4 s = make_float4(near_sigmoid(z.x), near_sigmoid(z.y), near_sigmoid(z.z), near_sigmoid(z.w));
+        const float4 s = sigmoid4(z);
         y.x *= gate_silu ? z.x * s.x : s.x;
         y.y *= gate_silu ? z.y * s.y : s.y;
         y.z *= gate_silu ? z.z * s.z : s.z;

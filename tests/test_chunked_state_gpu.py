@@ -351,3 +351,27 @@ def test_long_portions_of_heads_that_chunks_do_not_take(kind, per_head, D):
     assert ((out - want).abs() <= 2.0 ** -8 * want.abs().clamp(min=1.0) + 1e-4).all(), i
   names = {name for name, _ in ws._bufs}
   assert ("gated_delta_segments" if kind == "delta" else "linear_attention_segments") in names and "state_chunks" not in names
+
+
+@pytest.mark.parametrize("silu", [False, True])
+@pytest.mark.parametrize("kind,Dv", [("delta", 128), ("linear", 128), ("linear", 200)])      # up to 128 values a head, and more
+def test_gates_of_read_outs_are_exact_to_float32(kind, Dv, silu):
+  """A read-out that is the same value in all columns is 1 behind its norm, so what is rounded to bfloat16 is weight times activation, of
+  gates whose exponential is finite.  The exponential (2 ulp of float32), the sum, the division, the product with the gate, the norm's sum of
+  squares in halves (up to 9 roundings) and its three roundings, the weight: 12 ulp of 2^-24 or less, 2^-20."""
+  from miniinfer_b200.kernels import ops
+  T, H, D, r = 80, 2, 8, torch.Generator().manual_seed(Dv)
+  gate = (-40 + 20 * torch.randn((T, H * Dv), generator=r)).clamp(-86, 20).to(torch.bfloat16)
+  norm = 1 + torch.rand(Dv, generator=r)
+  one, state, out = torch.ones((T, H * D), dtype=torch.bfloat16), torch.zeros((T + 1, H * D * Dv), device=DEV), torch.empty((T, H * Dv), dtype=torch.bfloat16, device=DEV)
+  v, ctx, dev = torch.ones((T, H * Dv), dtype=torch.bfloat16), _ctx((1,) * T), lambda t: t.to(DEV)
+  if kind == "linear":
+    ops.linear_attention(out, dev(one), dev(one), dev(v), dev(gate), state, ctx, H, D, Dv, 1e-12, head_decay=torch.ones(H, device=DEV), norm_weight=dev(norm), gate_silu=silu)
+  else:
+    ops.gated_delta(out, dev(one), dev(one), dev(v), dev(one), dev(one[:, :H].contiguous()), dev(gate), torch.zeros(H * D, device=DEV), torch.zeros(H, device=DEV),
+                    dev(norm), 1e-12, state, ctx, H, H, D, Dv, gate_silu=silu)
+  z = gate.double().view(T, H, Dv)
+  want = (norm.double() * torch.sigmoid(z) * (z if silu else 1)).view(T, H * Dv)
+  low, high = ((want * (1 + s * 2.0 ** -20)).float().to(torch.bfloat16).double() for s in (-1, 1))
+  got = out.double().cpu()
+  assert ((got == low) | (got == high)).all()
