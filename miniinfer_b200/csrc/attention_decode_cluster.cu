@@ -100,8 +100,8 @@ __device__ __forceinline__ __nv_bfloat16 finish_value(const ClusterArgs& a, floa
   if (a.sink) {
     const float s2 = a.sink[head] * 1.4426950408889634f;      // base 2, like the scores
     const float Mf = fmaxf(M, s2);
-    const float f = M == -INFINITY ? 0.f : mi::ex2_fast(M - Mf);
-    L = L * f + mi::ex2_fast(s2 - Mf);
+    const float f = M == -INFINITY ? 0.f : exp2f(M - Mf);
+    L = L * f + exp2f(s2 - Mf);
     A = A * f;
   }
   float y = A / L;
@@ -225,8 +225,8 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
   // product's block there has left, so little of the product is left to hide the copies behind.)
   __syncthreads();                                           // the barriers and the tiles' rows are in shared memory
   // (One place each for the copies and for the norm and rotation, and loops that stay loops: this kernel's instructions are executed once
-  // or a few times, and come from L2 line by line.  Inlined where they were used, 55 KB of them, 8 requests of 16 heads took 7.4 us at 256
-  // tokens and 14.9 at 2048, behind another kernel; so, 30 KB, 5.6 and 13.1.)
+  // or a few times, and come from L2 line by line.  Inlined where they were used, 55 KB of them, 8 requests of 16 heads took 5.7 us at 256
+  // tokens and 14.6 at 2048, launched one after the other; so, 30 KB, 5.4 and 13.3.)
 #pragma unroll 1
   for (int asked = 0, after = rope ? 0 : 1; after < 2; ++after) {      // before the wait what the ring holds, after it the rest
     if (after) mi::grid_dependency_sync();
@@ -365,7 +365,7 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
 #pragma unroll
       for (int w = 0; w < CW; ++w) {
         const float* src = red + ((size_t)w * GP + h) * ROW;
-        const float f = src[HD] == -INFINITY ? 0.f : mi::ex2_fast(src[HD] - M);
+        const float f = src[HD] == -INFINITY ? 0.f : exp2f(src[HD] - M);
         L = fmaf(src[HD + 1], f, L);
         A = fmaf(src[d], f, A);
       }
@@ -403,7 +403,7 @@ decode_cluster_kernel(const __grid_constant__ CUtensorMap kv_map, ClusterArgs a)
       const float* src = recv + (size_t)rr * rs;
       const float mr = src[slice + 2 * h];
       if (mr == -INFINITY) continue;
-      const float f = mi::ex2_fast(mr - M);
+      const float f = exp2f(mr - M);
       L = fmaf(src[slice + 2 * h + 1], f, L);
       A = fmaf(src[t], f, A);
     }

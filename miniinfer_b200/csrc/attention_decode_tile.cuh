@@ -162,7 +162,7 @@ __device__ __forceinline__ void consume_tile(uint32_t kt, uint32_t vt, const uin
     mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 16));
     const float m_new = fmaxf(m_run[h], mx[h]);
     m_use[h] = m_new == -INFINITY ? 0.f : m_new;
-    alpha[h] = mi::ex2_fast(m_run[h] - m_use[h]);
+    alpha[h] = exp2f(m_run[h] - m_use[h]);
     m_run[h] = m_new;
     l_run[h] *= alpha[h];
   }
@@ -170,7 +170,7 @@ __device__ __forceinline__ void consume_tile(uint32_t kt, uint32_t vt, const uin
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const float pe = mi::ex2_fast(sc[i][c] - m_use[c & 1]);
+      const float pe = exp2f(sc[i][c] - m_use[c & 1]);
       sc[i][c] = pe;
       l_run[c & 1] += pe;
     }

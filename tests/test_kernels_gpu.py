@@ -235,6 +235,30 @@ def test_decode_attention_in_clusters(ops, monkeypatch, cluster, nh, nkv, hd, wi
   assert (out.float() - want.float()).abs().max() < 2e-2
 
 
+# in one tile, in tiles of different warps and blocks, the greater score first and last
+@pytest.mark.parametrize("cluster", [0, 1, 4])      # 0: the persistent kernel
+@pytest.mark.parametrize("top,low", [(5, 6), (5, 100), (100, 5), (690, 3), (3, 690)])
+def test_decode_attention_weights_below_the_smallest_normal_number(ops, monkeypatch, cluster, top, low):
+  """A score 90 below another's weighs e^-90 = 8.2e-40, which float32 still holds, and a value of 3.2e38 makes that a quarter.  The weight of
+  a key as bfloat16, 8.9 of its smallest steps, errs by half a step in 8.9."""
+  monkeypatch.setenv("MINIINFER_B200_DECODE_CLUSTER", str(cluster))
+  nh, nkv, hd = 4, 2, 64
+  qkv, kv, bt, batch = make_attention_case([(700, 1)], nh, nkv, hd, 64, torch.bfloat16, seed=1)
+  qkv.zero_()
+  qkv[:, 0:nh * hd:hd] = 1.0
+  kv.zero_()
+  kv[:, 0, :, :, 0] = -10000.0
+  big = 1.875 * 2.0 ** 127
+  for j, score, value in ((top, 0.0, 1.0), (low, -90.0, big)):
+    page = int(bt[int(batch.seq_slot[0]), j // 64])
+    kv[page, 0, :, j % 64, 0] = score
+    kv[page, 1, :, j % 64] = value
+  out = torch.empty((1, nh * hd), dtype=torch.bfloat16, device=DEV)
+  ops.attention(out, qkv, kv, bt, batch, nh, nkv, hd, 1.0, None)
+  rest = big * math.exp(-90.0)
+  assert ((out.float() - (1 + rest)).abs() <= rest * 0.5 / 8.9 + 2.0 ** -8 * (1 + rest)).all()
+
+
 @pytest.mark.parametrize("cluster", [1, 2, 4, 8, 16])
 @pytest.mark.parametrize("nh,nkv,window,with_norm,with_table,writes,P", [(16, 8, None, True, True, True, 64), (6, 2, 700, True, True, True, 64),
                                                                          (8, 8, None, False, True, True, 128), (4, 2, None, True, False, True, 64),
