@@ -93,7 +93,8 @@ __device__ __forceinline__ void bulk_copy(float* to, const float* from, int floa
 }
 // before a barrier behind which bulk copies go where this thread has read or written
 __device__ __forceinline__ void bulk_may_follow() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// False if the block's own copies, the only thing ever waited for, have not come: what depends on them is then made NaN.
+// False if the block's own copies, the only thing ever waited for, have not come: what depends on them - the chunk's read-outs, the state and
+// all later read-outs of the head - is then made NaN, and the status word is set.
 constexpr int WAIT_LIMIT = 1 << 22;
 __device__ __forceinline__ bool bar_wait(uint64_t* bar, int parity) {
   unsigned done = 0;
@@ -101,6 +102,10 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, int parity) {
   for (int i = 0; i < WAIT_LIMIT && !done; ++i)
     asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(shared_at(bar)), "r"(parity) : "memory");
   return done;
+}
+
+__device__ __forceinline__ void say_late(bool late, int* status) {
+  if (late && status != nullptr) atomicExch(status, CHUNK_STATUS_LATE);
 }
 
 // ------------------------------------------------------------------------------------------------------------ products
@@ -327,8 +332,7 @@ chunk_build_kernel(Args a) {
       }
     }
   }
-  bool late = !bar_wait(bars, 0);
-  __syncthreads();
+  bool late = __syncthreads_or(!bar_wait(bars, 0));
   // Inside the blocks, a warp a block of eight tokens, a lane two key channels at a time: products number p (p + 1) / 2 + s of q_p and
   // k_s for s <= p, then 36 + p (p - 1) / 2 + s of k_p and k_s for s < p, the decays between s and p walked.  A key that has
   // walked to the block's end is E k; F q and F k are left beside it, each in the place of what it was made from.
@@ -397,8 +401,8 @@ chunk_build_kernel(Args a) {
       for (int c = tid < n ? columns : 0; c < VT; c += 4) st4(row + c, make_float4(0.f, 0.f, 0.f, 0.f));
     }
   };
-  auto values_there = [&]() {
-    late |= !bar_wait(bars + 1, values_round & 1);
+  auto values_there = [&]() {      // for all threads
+    late |= (bool)__syncthreads_or(!bar_wait(bars + 1, values_round & 1));
     ++values_round;
   };
   if (!DELTA) fetch_values(gs, 0);
@@ -493,7 +497,7 @@ chunk_build_kernel(Args a) {
     });
   }
   if (!DELTA) values_there();
-  __syncthreads();
+  else __syncthreads();
   // A, a row a token: zeros behind the diagonal; and L^T, the part before the diagonal
   {
     const int t = 8 * warp + g;
@@ -522,7 +526,7 @@ chunk_build_kernel(Args a) {
           if (2 * t4 + 1 < g) lt[(8 * warp + 2 * t4 + 1) * C + t] = b * dk[2 * t4 + 1];
         }
       }
-      st2(out + 8 * j, x, y);
+      st2(out + 8 * j, late ? NAN : x, late ? NAN : y);
     }
   }
   if (!DELTA) {      // K^^T V: a warp 16 key channels - a lane those numbered 2 g and 2 g + 1 -, 32 value columns at a time
@@ -532,7 +536,6 @@ chunk_build_kernel(Args a) {
         __syncthreads();
         fetch_values(gs, v0);
         values_there();
-        __syncthreads();
       }
       if (16 * warp >= dp) continue;
 #pragma unroll 1
@@ -555,6 +558,7 @@ chunk_build_kernel(Args a) {
             st2(a.s0 + (unit * dp + 16 * warp + 2 * g + h) * a.vp + v0 + c + 8 * j + 2 * t4, late ? NAN : more[j].at(2 * h), late ? NAN : more[j].at(2 * h + 1));
       }
     }
+    if (tid == 0) say_late(late, a.status);
     return;
   }
   __syncthreads();
@@ -649,7 +653,6 @@ chunk_build_kernel(Args a) {
     st2(block, -x[0], -x[1]);
     st2(block + 8 * LDT, -x[2], -x[3]);
   }
-  __syncthreads();
   values_there();
   // W and U0, the inverse times diag(beta) times K~ and times V side by side: a warp two tiles of 16 rows, one of the upper and one
   // of the lower half so that all have as much of the inverse before the diagonal, in 32 columns
@@ -659,7 +662,6 @@ chunk_build_kernel(Args a) {
       __syncthreads();
       fetch_values(ks, v0);
       values_there();
-      __syncthreads();
     }
     const int columns = dp + min(VT, a.vp - v0);
 #pragma unroll 1
@@ -696,8 +698,8 @@ chunk_build_kernel(Args a) {
         for (int j = 0; j < 4; ++j) {
           const float c[4] = {sum[j].at(0), sum[j].at(1), sum[j].at(2), sum[j].at(3)};
           st2(o + j * next, late ? NAN : c[0], late ? NAN : c[1]);
-          st2(o + j * next + 8 * ldo, c[2], c[3]);
-          bad |= any_not_finite(c) ? 15u << 4 * j : 0;
+          st2(o + j * next + 8 * ldo, late ? NAN : c[2], late ? NAN : c[3]);
+          bad |= any_not_finite(c) && !late ? 15u << 4 * j : 0;
         }
 #pragma unroll 1
         for (; bad; bad &= bad - 1) {      // element by element, and only up to the diagonal
@@ -710,6 +712,7 @@ chunk_build_kernel(Args a) {
       }
     }
   }
+  if (tid == 0) say_late(late, a.status);
 }
 
 // -------------------------------------------------------------------------------------------------------------- state
@@ -855,7 +858,7 @@ chunk_state_kernel(Args a) {
     }
   if (holds) keep();
   __syncthreads();
-  bool late = false;      // a wait for this block's own copies ran out: the state becomes NaN
+  bool late = false;      // a wait for this block's own copies ran out: U becomes NaN, and with it the state and what is read from it
   for (int c = from; c < to; ++c) {
     const int stage = (c - from) & 1;
     const float* cur = sm + stage * at.stage;
@@ -890,14 +893,14 @@ chunk_state_kernel(Args a) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) st2(a.s0 + (unit * dp + d0 + h) * a.vp + v0 + 8 * (j0 + j) + 2 * t4, S[j][2 * h], S[j][2 * h + 1]);
     }
-    __syncthreads();
+    late = __syncthreads_or(late);
 #pragma unroll
     for (int i = tid; i < C * CB; i += STATE_THREADS) {      // U = U0 - W S_0, element i of [NT][C][8]
       const int t = (i >> 3) & (C - 1), col = (i / (8 * C)) * 8 + (i & 7);
       float x = parts[t * LDX + col];
 #pragma unroll
       for (int q = 1; q < PARTS; ++q) x += parts[(q * C + t) * LDX + col];
-      const float y = cur[at.u + i] - x;
+      const float y = late ? NAN : cur[at.u + i] - x;
       a.u[unit * C * a.vp + (size_t)v0 * C + i] = y;
       us[t * LDU + col] = y;
     }
@@ -949,6 +952,7 @@ chunk_state_kernel(Args a) {
         if (d < a.dim && c < a.vdim) st[(size_t)d * a.vdim + c] = late ? NAN : S[j][e];
       }
   }
+  if (tid == 0) say_late(late, a.status);
 }
 
 // -------------------------------------------------------------------------------------------------------------- out
@@ -1043,6 +1047,7 @@ chunk_out_kernel(Args a) {
   late |= !bar_wait(bars + 2, 0);
   __syncthreads();      // (the zeros behind the last token)
   multiply(sm, m0 + 32, DELTA ? 8 : LDV, DELTA ? 8 * C : 8, std::integral_constant<bool, !DELTA>());      // A U: nothing behind the diagonal; linear attention's U are the values
+  late = __any_sync(0xffffffffu, late);
   float* o = a.raw + (size_t)row0 * (a.heads * a.vdim) + head * a.vdim + v0;
   unsigned bad = 0;
 #pragma unroll
@@ -1055,7 +1060,7 @@ chunk_out_kernel(Args a) {
         const int t = m0 + 16 * i + g + 8 * h, c = n0 + 8 * j + 2 * t4;
         if (t < n && v0 + c < a.vdim) st2(o + (size_t)t * (a.heads * a.vdim) + c, late ? NAN : x[2 * h], late ? NAN : x[2 * h + 1]);
       }
-      bad |= any_not_finite(x) ? 15u << 4 * (4 * i + j) : 0;
+      bad |= any_not_finite(x) && !late ? 15u << 4 * (4 * i + j) : 0;
     }
   const float *aa = sm, *us = sm + C * LDL;
 #pragma unroll 1
@@ -1069,6 +1074,7 @@ chunk_out_kernel(Args a) {
     for (int s = 0; s <= t; ++s) z = fmaf(aa[t * LDL + s], DELTA ? us[(c / 8 * C + s) * 8 + (c & 7)] : us[s * LDV + c], z);
     o[(size_t)t * (a.heads * a.vdim) + c] = fabsf(z) <= 3.402823466e38f ? y + z : NAN;      // an infinite value: the recurrence adds it up over channels of both signs
   }
+  if (lane == 0) say_late(late, a.status);
 }
 
 int most_chunks(int T, int items) { return T / C + items; }      // every item's last chunk may be a short one

@@ -7,6 +7,7 @@ namespace mi {
 
 constexpr int CHUNK_TOKENS = 64;
 constexpr int CHUNK_MAX_DIM = 128;            // key channels a head
+constexpr int CHUNK_STATUS_LATE = 32;
 
 enum ChunkDecay { CHUNK_DECAY_CHANNEL = 0, CHUNK_DECAY_HEAD = 1, CHUNK_DECAY_CONSTANT = 2 };
 
@@ -20,6 +21,7 @@ struct ChunkedStateArgs {
   const int* q_start; const int* q_len; const int* seq_slot;
   int items, heads, qk_heads, dim, vdim;
   int min_tokens;                             // items of fewer new tokens are left alone
+  int* status;                                // null, or a word that is set to CHUNK_STATUS_LATE if a bounded wait for a block's own copies ran out
 };
 
 // Whether the sizes are taken: up to CHUNK_MAX_DIM key channels, rows of whole 16 bytes.

@@ -468,9 +468,9 @@ MI_API int mi_linear_attention(void* out, int ldo, const void* q, int ldq, const
                                const float* head_decay, const float* rope, const int* positions, int rot_dims, float q_scale,
                                float k_scale, const float* norm_w, float eps, int gate_silu, float* state, long long state_stride,
                                const int* q_start, const int* q_len, const int* seq_slot, int T, int items, int heads, int dim,
-                               int vdim, float* scratch, float* segments, float* chunks, int chunk_min, cudaStream_t stream) {
+                               int vdim, float* scratch, float* segments, float* chunks, int chunk_min, int* chunk_status, cudaStream_t stream) {
   // chunks: null, or mi_chunked_state_floats of scratch - then items of at least chunk_min new tokens are walked a chunk of tokens at
-  // a time (bfloat16 only; excludes segments), the others token by token
+  // a time (bfloat16 only; excludes segments), the others token by token.  chunk_status: null, or a word set to 32 if a wait runs out there
   MI_REQUIRE(chunks == nullptr || (dtype == MI_BF16 && segments == nullptr && chunk_min > 1), "linear_attention: chunks are for bfloat16 activations");
   MI_REQUIRE(T >= 0 && items >= 0 && items <= 65535 && heads > 0 && heads <= 65535, "linear_attention: bad counts T=%d items=%d heads=%d", T, items, heads);
   MI_REQUIRE(dim > 0 && vdim > 0 && dim <= 4096, "linear_attention: bad sizes dim=%d vdim=%d", dim, vdim);
@@ -554,7 +554,7 @@ MI_API int mi_linear_attention(void* out, int ldo, const void* q, int ldq, const
     else MI_LIN_DK(false);                                                                                           \
     if (chunks) {                                                                                                    \
       mi::ChunkedStateArgs c{qn, kn, channel ? g : head_decay, channel ? mi::CHUNK_DECAY_CHANNEL : mi::CHUNK_DECAY_CONSTANT, nullptr, raw, state, \
-                             state_stride, q_start, q_len, seq_slot, items, heads, heads, dim, vdim, chunk_min};      \
+                             state_stride, q_start, q_len, seq_slot, items, heads, heads, dim, vdim, chunk_min, chunk_status};      \
       if (int e = mi::chunked_state_run(c, T, chunks, stream)) return e;                                             \
     }                                                                                                                \
     if (vec)                                                                                                         \

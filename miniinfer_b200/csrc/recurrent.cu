@@ -924,9 +924,9 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
                           const void* b_in, int ldb, const void* gate, int ldg, int dtype, const float* dt_bias, const float* A_log,
                           const float* norm_w, float eps, float* state, long long state_stride, const int* q_start, const int* q_len,
                           const int* seq_slot, int T, int items, int heads, int kv_heads, int dim, int vdim, float* scratch,
-                          float* segments, int head_decay, int gate_silu, float* chunks, int chunk_min, cudaStream_t stream) {
+                          float* segments, int head_decay, int gate_silu, float* chunks, int chunk_min, int* chunk_status, cudaStream_t stream) {
   // chunks: null, or mi_chunked_state_floats of scratch - then items of at least chunk_min new tokens are walked a chunk of
-  // tokens at a time (bfloat16 only; excludes segments), the others token by token
+  // tokens at a time (bfloat16 only; excludes segments), the others token by token.  chunk_status: null, or a word set to 32 if a wait runs out there
   MI_REQUIRE(chunks == nullptr || (dtype == MI_BF16 && segments == nullptr && chunk_min > 1), "gated_delta: chunks are for bfloat16 activations");
   // head_decay: a_in [T, heads] and dt_bias [heads], one decay a head, instead of [T, heads * dim] and [heads * dim]
   // segments: null, or items * DELTA_SEGMENTS * heads * dim * (vdim + dim) floats of scratch - then the items' tokens run
@@ -1015,7 +1015,7 @@ MI_API int mi_gated_delta(void* out, int ldo, const void* q, const void* k, int 
     else MI_DELTA(TT, 128);                                                                                       \
     if (chunks) {                                                                                                 \
       mi::ChunkedStateArgs c{qn, kn, head_decay ? lg : g, head_decay ? mi::CHUNK_DECAY_HEAD : mi::CHUNK_DECAY_CHANNEL, beta, raw, state, state_stride, q_start, q_len, \
-                             seq_slot, items, heads, kv_heads, dim, vdim, chunk_min};                              \
+                             seq_slot, items, heads, kv_heads, dim, vdim, chunk_min, chunk_status};                              \
       if (int e = mi::chunked_state_run(c, T, chunks, stream)) return e;                                            \
     }                                                                                                             \
     if (vec)                                                                                                      \

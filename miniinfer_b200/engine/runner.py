@@ -630,7 +630,8 @@ class ModelRunner:
       code = ops.device_status(ws)
       if code:
         raise ops.KernelError(f"a bounded wait inside a kernel ran out (status bits {code}: 1 decode attention, "
-                              f"2 prefill attention, 4 the tcgen05 matrix product)")
+                              f"2 prefill attention, 4 the tcgen05 matrix product, 8 its form for few rows, 16 that form's place in "
+                              f"shared memory, 32 recurrences by chunks)")
 
   def num_graphs(self) -> int:
     return sum(1 for g in list(self._graphs.values()) + list(self._step_graphs.values()) if g.graph is not None)

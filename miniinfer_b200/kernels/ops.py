@@ -684,7 +684,7 @@ def gated_delta(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Te
   # long prompt portions in bfloat16: a chunk of tokens at a time (csrc/chunked_state.cu); with heads too wide for that each
   # request's tokens in up to 16 stretches side by side (five launches instead of three)
   segments, launches = None, 3
-  chunks, more = _state_chunks(lib, v, ctx, heads, dim, vdim, workspace, DELTA_CHUNK_MIN_TOKENS, True)
+  chunks, more, chunk_status = _state_chunks(lib, v, ctx, heads, dim, vdim, workspace, DELTA_CHUNK_MIN_TOKENS, True)
   if chunks is not None:
     launches = (3 if ctx.num_items > 1 else 2) + more
   if (chunks is None and v.dtype == torch.bfloat16 and ctx.num_items <= DELTA_SEGMENTED_MAX_ITEMS and T >= SCAN_SEGMENTED_MIN_TOKENS * ctx.num_items
@@ -700,7 +700,7 @@ def gated_delta(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Te
                                  _ptr(ctx.q_len, torch.int32), _ptr(ctx.seq_slot, torch.int32), T, ctx.num_items, heads, kv_heads, dim, vdim,
                                  _ptr(scratch, torch.float32), _ptr(segments, torch.float32) if segments is not None else _ptr(None),
                                  int(head_decay), int(gate_silu), _ptr(chunks, torch.float32) if chunks is not None else _ptr(None),
-                                 DELTA_CHUNK_MIN_TOKENS, _stream()), kernels=launches)
+                                 DELTA_CHUNK_MIN_TOKENS, _ptr(chunk_status), _stream()), kernels=launches)
 
 
 # The same for linear attention.  Decays a key channel: 48 tokens 35, 49, 50 against 39, 42, 43; 64 tokens 35, 45, 49 against 43, 46,
@@ -724,19 +724,21 @@ def longest_portion_class(longest: int) -> int:
 
 
 def _state_chunks(lib, v: torch.Tensor, ctx, heads: int, dim: int, vdim: int, workspace, min_tokens: int, delta: bool):
-  """(scratch, launches) of the walk by chunks of tokens of a step that brings a request ``min_tokens`` new tokens - or may bring
-  them, where the step's keys do not tell -, or (None, 0): a float32 step, a step of short portions, sizes that the chunks do not take."""
+  """(scratch, launches, status word) of the walk by chunks of tokens of a step that brings a request ``min_tokens`` new tokens - or may
+  bring them, where the step's keys do not tell -, or (None, 0, None): a float32 step, a step of short portions, sizes that the chunks do
+  not take.  A wait that runs out in there leaves NaN, and 32 in the status word, which a workspace keeps (``device_status``)."""
   known = getattr(ctx, "work_key", {}).get(LONGEST_PORTION)
   longest = known[0] if known else v.shape[0] - ctx.num_items + 1
   if v.dtype != torch.bfloat16 or longest < min_tokens or os.environ.get("MINIINFER_B200_DELTA_CHUNKS", "1") == "0":
-    return None, 0
+    return None, 0, None
   lib.mi_chunked_state_floats.restype = ctypes.c_longlong
   m = int(lib.mi_chunked_state_floats(v.shape[0], ctx.num_items, heads, dim, vdim, int(delta)))
   if m == 0:
-    return None, 0
+    return None, 0, None
   chunks = workspace.buffer("state_chunks", (m,), torch.float32) if workspace is not None else \
     torch.empty(m, dtype=torch.float32, device=v.device)
-  return chunks, 3 * int(lib.mi_chunked_state_slabs(v.shape[0], ctx.num_items, heads, dim, vdim, int(delta)))
+  status = workspace.zeros("chunked_state_status", 1, torch.int32) if workspace is not None else None
+  return chunks, 3 * int(lib.mi_chunked_state_slabs(v.shape[0], ctx.num_items, heads, dim, vdim, int(delta))), status
 
 
 def linear_attention(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Tensor, state: torch.Tensor, ctx,
@@ -777,7 +779,7 @@ def linear_attention(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: tor
   scratch = workspace.buffer("linear_attention_scratch", (n,), torch.float32) if workspace is not None else \
     torch.empty(n, dtype=torch.float32, device=v.device)
   segments, launches = None, 3
-  chunks, more = _state_chunks(lib, v, ctx, heads, dim, vdim, workspace, LINEAR_CHUNK_MIN_TOKENS, False)
+  chunks, more, chunk_status = _state_chunks(lib, v, ctx, heads, dim, vdim, workspace, LINEAR_CHUNK_MIN_TOKENS, False)
   if chunks is not None:
     launches = (3 if ctx.num_items > 1 else 2) + more
   if (chunks is None and v.dtype == torch.bfloat16 and ctx.num_items <= LINEAR_SEGMENTED_MAX_ITEMS and T >= SCAN_SEGMENTED_MIN_TOKENS * ctx.num_items
@@ -798,7 +800,7 @@ def linear_attention(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: tor
     ctypes.c_void_p(state.data_ptr()), ctypes.c_longlong(state.stride(0)), _ptr(ctx.q_start, torch.int32), _ptr(ctx.q_len, torch.int32),
     _ptr(ctx.seq_slot, torch.int32), T, ctx.num_items, heads, dim, vdim, _ptr(scratch, torch.float32),
     _ptr(segments, torch.float32) if segments is not None else none, _ptr(chunks, torch.float32) if chunks is not None else none,
-    LINEAR_CHUNK_MIN_TOKENS, _stream()), kernels=launches)
+    LINEAR_CHUNK_MIN_TOKENS, _ptr(chunk_status), _stream()), kernels=launches)
 
 
 def token_shift(out: torch.Tensor, resid: torch.Tensor, shift: Optional[torch.Tensor], state: Optional[torch.Tensor], ctx) -> None:
@@ -1792,7 +1794,7 @@ def forget_tensors() -> None:
 def device_status(ws) -> int:
   """The status words that kernels with bounded waits set when a wait ran out (0: all well)."""
   code = 0
-  for name in ("attention_decode_counters", "attention_prefill_status", "gemm_tc_status"):
+  for name in ("attention_decode_counters", "attention_prefill_status", "gemm_tc_status", "chunked_state_status"):
     buf = ws._bufs.get((name, torch.int32))
     if buf is not None:
       code |= int(buf[0])

@@ -318,6 +318,15 @@ def test_causal_convolution_of_short_stretches(lengths, C):
   test_causal_convolution_two_channels_a_thread(4, lengths, C, 8)
 
 
+@pytest.mark.parametrize("kind", ["delta", "linear"])
+def test_chunks_have_a_status_word_in_the_workspace(kind):
+  from miniinfer_b200.engine.context import Workspace
+  from miniinfer_b200.kernels import ops
+  ws = Workspace(torch.device(DEV))
+  list(_run(kind, True, (130,), 2, 40, 88, 16, ws))
+  assert ("state_chunks", torch.float32) in ws._bufs and ("chunked_state_status", torch.int32) in ws._bufs and ops.device_status(ws) == 0
+
+
 # Blocks of 16, 24 and 32 tokens on 148 SMs: inputs carried from one round of eight tokens to the next, in blocks of one request and of several
 @pytest.mark.parametrize("taps", [2, 3, 4])
 @pytest.mark.parametrize("lengths,C", [((1, 2, 1157, 9, 31), 2048), ((3, 16, 24, 8, 1949, 1, 47), 2048), ((1, 2, 601, 9, 3), 8192), ((32, 64, 1, 520), 8192)])

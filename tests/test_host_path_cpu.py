@@ -284,3 +284,19 @@ def test_a_step_of_short_portions_is_told_from_one_with_a_long_portion():
   for portions, want in (([20] * 30, 0), ([1, low - 1], 0), ([1, low], low), ([high - 1] * 9, low), ([high, 3], high), ([5000], high)):
     step = HostStep(np.array(portions, dtype=np.int32), np.zeros(len(portions), dtype=np.int32), 8192)
     assert LongestPortion().key(step) == (want,) and len(LongestPortion().build(step)) == 0, portions
+
+
+@pytest.mark.parametrize("name,code", [("attention_decode_counters", 1), ("attention_prefill_status", 2), ("gemm_tc_status", 4), ("chunked_state_status", 32)])
+def test_a_wait_that_ran_out_in_a_kernel_is_reported(name, code):
+  from types import SimpleNamespace
+
+  from miniinfer_b200.engine.context import Workspace
+  from miniinfer_b200.engine.runner import ModelRunner
+  from miniinfer_b200.kernels import ops
+  ws = Workspace(torch.device("cpu"))
+  runner = SimpleNamespace(ws=ws, _graphs={}, _step_graphs={})
+  word = ws.zeros(name, 1, torch.int32)
+  ModelRunner.check_status(runner)
+  word[0] = code      # as the kernel leaves it
+  with pytest.raises(ops.KernelError, match=f"status bits {code}:"):
+    ModelRunner.check_status(runner)
