@@ -609,11 +609,15 @@ DELTA_SEGMENTED_MAX_ITEMS = 4      # the same bound for the delta rule, whose sc
 # B200, 2048 tokens of one request, heads of 128 x 128: 8 heads (64 blocks in order) 5.18 -> 4.57 ms a step of six layers,
 # 16 heads (128 blocks) 7.23 -> 8.11 ms
 DELTA_SEGMENTED_MAX_BLOCKS = 96
-# New tokens a request from which a bfloat16 delta rule goes a chunk at a time (csrc/chunked_state.cu).  Measured on B200, the operation
-# for 8 / 16 / 32 heads of 128 x 128, chunks against the walk in order, in microseconds.  One decay a key channel: 80 tokens 53, 60, 66
-# against 52, 55, 57; 96 tokens 53, 60, 67 against 61, 64, 67; 112 tokens 53, 60, 67 against 70, 73, 76; 256 tokens 62, 68, 82 against 107, 155,
-# 163.  One decay a head: 80 tokens 52, 58, 64 against 49, 31, 54; 96 tokens 52, 58, 64 against 59, 43, 63; 112 tokens 52, 59, 65 against 66, 49,
-# 73; 128 tokens 54, 58, 65 against 74, 75, 82; 256 tokens 60, 66, 77 against 83, 123, 151
+# New tokens a request from which a bfloat16 delta rule goes a chunk at a time (csrc/chunked_state.cu).  Measured on B200, the operation of one
+# request, 8 / 16 / 32 heads of 128 x 128, chunks against the walk in order, in microseconds, medians of five repeats that differ by 0.3 or less (0.7
+# at 32 heads).  One decay a key channel: 56 tokens 40, 42, 45 against 40, 41, 42; 64 tokens 39, 41, 45 against 44, 44, 47; 80 tokens 41, 44, 50
+# against 53, 54, 57; 112 tokens 41, 45, 51 against 71, 73, 75; 256 tokens 46, 58, 80 against 153, 156, 162.  One decay a head: 64 tokens 38, 40, 43
+# against 42, 43, 45; 112 tokens 40, 43, 49 against 68, 69, 72; 256 tokens 44, 56, 75 against 144, 149, 152.  Requests side by side, 8 / 32 heads:
+# 16 of 96 tokens 121, 429 against 182, 599 (a decay a head 116, 397 against 121, 427), 32 of 96 230, 898 against 309, 1146 (217, 849 against 226, 844).
+# That the bound lies above all of this is for the state's sake: of a portion that fades fast (decays stronger than 1 / 2 a token) the walk in
+# order leaves it with an error of 0.8e-7 of its norm, the chunks with 1.4e-7; of one that lasts (1 / 1000 a token) 11.6e-7 and 1.5e-7.  From 112
+# tokens on the walk costs half as much again and more
 DELTA_CHUNK_MIN_TOKENS = 112
 
 
@@ -703,9 +707,10 @@ def gated_delta(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Te
                                  DELTA_CHUNK_MIN_TOKENS, _ptr(chunk_status), _stream()), kernels=launches)
 
 
-# The same for linear attention.  Decays a key channel: 48 tokens 35, 49, 50 against 39, 42, 43; 64 tokens 35, 45, 49 against 43, 46,
-# 47; 80 tokens 36, 47, 52 against 47, 55, 58; 128 tokens 45, 49, 52 against 78, 83, 87.  A constant a head: 48 tokens 36, 48, 49 against 37, 38, 38;
-# 64 tokens 37, 43, 47 against 40, 42, 43; 80 tokens 36, 46, 49 against 46, 49, 52; 128 tokens 43, 46, 50 against 74, 75, 78
+# The same for linear attention.  Decays a key channel: 40 tokens 32, 33, 34 against 33, 37, 37; 48 tokens 32, 33, 34 against 38, 41, 41; 64 tokens 31,
+# 31, 33 against 40 .. 43, 45, 47; 128 tokens 32, 33, 41 against 77, 81, 85.  A constant a head: 48 tokens 32, 33, 34 against 36, 37, 38; 64 tokens 30,
+# 31, 32 against 38 .. 40, 41, 43; 128 tokens 31, 32, 40 against 72, 74, 78.  Several requests fill the SMs either way: 16 of 64 tokens, 8 / 32 heads, 60,
+# 162 against 53, 198 (a constant a head 59, 150 against 48, 173), 16 of 96 73, 251 against 76, 284 (69, 233 against 66, 246)
 LINEAR_CHUNK_MIN_TOKENS = 64
 LINEAR_SEGMENTED_MAX_ITEMS = 8     # steps of at most this many requests run long bfloat16 portions in stretches side by side
 # ... and only while the walk in order would leave SMs idle (blocks in order, all requests; an SM holds three, and
