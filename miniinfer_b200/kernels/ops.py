@@ -500,13 +500,14 @@ def _cols(t: torch.Tensor, what: str):
 
 
 def linear_batched(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, softplus: bool = False,
-                   row_gate: Optional[torch.Tensor] = None, value_gate: Optional[torch.Tensor] = None) -> None:
+                   row_gate: Optional[torch.Tensor] = None, value_gate: Optional[torch.Tensor] = None, fixed_weights: bool = False) -> None:
   """out[:, b, :] = x[:, b, :] @ w[b]^T for ``x [M, batch, K]``, ``w [batch, N, K]``, ``out [M, batch, N]`` - views whose
   strides may be anything as long as the last axis is contiguous (the heads of a token's row, a column range of a
   row); float32 sums, k ascending except on the tensor cores (bfloat16 rows that can be read 16 bytes at a time).  bfloat16 with more
   than 16 rows and nothing but a gate a value behind the product: one strided batched library product, the gate in a kernel behind it.
   ``bias [N]`` float32 is added, ``softplus`` applied, and with ``row_gate [M, >= batch]``
-  (one logit per row and batch) or ``value_gate [M, batch * N]`` (one per output value) the result is multiplied with its sigmoid."""
+  (one logit per row and batch) or ``value_gate [M, batch * N]`` (one per output value) the result is multiplied with its sigmoid.  ``fixed_weights``: ``w`` is
+  a model's and not what a kernel of the step writes, so it may be fetched while the kernel before still runs."""
   lib = common_lib()
   M, B, K = x.shape
   N = w.shape[1]
@@ -548,7 +549,7 @@ def linear_batched(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, bias: Op
     int(x.stride(0)), ctypes.c_longlong(x.stride(1)), int(w.stride(1)), ctypes.c_longlong(w.stride(0)),
     int(out.stride(0)), ctypes.c_longlong(out.stride(1)), _ptr(bias, torch.float32) if bias is not None else _ptr(None),
     int(bool(softplus)), ctypes.c_void_p(row_gate.data_ptr()) if row_gate is not None else _ptr(None), gate_stride,
-    ctypes.c_void_p(value_gate.data_ptr()) if value_gate is not None else _ptr(None), _stream()))
+    ctypes.c_void_p(value_gate.data_ptr()) if value_gate is not None else _ptr(None), *((int(bool(fixed_weights)),) if few else ()), _stream()))
 
 
 def linear_parts(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor) -> None:

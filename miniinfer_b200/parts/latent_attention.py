@@ -121,14 +121,14 @@ class LatentAttentionMixer(AttentionMixer):
     ops.linear(q, cq, self.uq)
     q_heads = ctx.ws.buffer("q_heads", (T, H * hdp), ctx.dtype)
     ops.latent_query(q, q_heads, H, D, R, C, table, ctx.positions, self.rotary_interleaved)
-    ops.linear_batched(q_heads.view(T, H, hdp)[:, :, :C], q.view(T, H, D + R)[:, :, :D], self.uk_t)
+    ops.linear_batched(q_heads.view(T, H, hdp)[:, :, :C], q.view(T, H, D + R)[:, :, :D], self.uk_t, fixed_weights=True)
     attn = ctx.ws.buffer("attn_out", (T, H * C), ctx.dtype)
     ops.latent_attention(attn, q_heads, cache.tensor, ctx.block_tables[cache.group], self._batch(ctx), H, hdp, self.scale, self.window,
                          self.sink if self.sinks else None, C)
     heads = ctx.ws.buffer("latent_heads", (T, H * Dv), ctx.dtype)
     gate = down[:, self.g_off:self.g_off + self.gate_width] if self.gated else None
     ops.linear_batched(heads.view(T, H, Dv), attn.view(T, H, C), self.uv_heads, row_gate=gate if self.gate_per_head else None,
-                       value_gate=gate if not self.gate_per_head else None)
+                       value_gate=gate if not self.gate_per_head else None, fixed_weights=True)
     out = ctx.ws.buffer(self.out_buffer, (T, self.hidden_size), ctx.dtype)
     ops.linear(out, heads, self.o)
     return out

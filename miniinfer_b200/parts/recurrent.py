@@ -292,7 +292,7 @@ class RglruMixer(Mixer):
       ops.linear_parts(gates, u, self.gates.view(B, 2 * P, P))
     else:
       gates = ctx.ws.buffer("rglru_gates", (T, 2 * C), torch.float32)
-      ops.linear_batched(gates.view(T, B, 2 * P), u.view(T, B, P), self.gates.view(B, 2 * P, P))
+      ops.linear_batched(gates.view(T, B, 2 * P), u.view(T, B, P), self.gates.view(B, 2 * P, P), fixed_weights=True)
     s = ctx.ws.buffer("rglru_s", (T, C), ctx.dtype)
     ops.rglru_recurrence(s, u, gates, proj[:, C:], self.ra_b, self.ri_b, self.y_b, self.lam, state[:, self.conv_floats:], ctx, B, workspace=ctx.ws)
     out = ctx.ws.buffer(self.out_buffer, (T, self.hidden_size), ctx.dtype)

@@ -88,6 +88,22 @@ def test_per_head_products_into_float32_add_in_order(M, N, K, B):
   assert (outs[0].double() - want).norm() <= K ** 0.5 * 2.0 ** -24 * want.norm()
 
 
+def test_per_head_products_of_what_the_kernel_before_wrote():
+  """Both operands of a product may be results of the step; what is fixed may be fetched early, with the same result."""
+  from miniinfer_b200.kernels import ops
+  M, N, K, B, R = 8, 64, 256, 4, 512
+  g = torch.Generator().manual_seed(9)
+  r = lambda *s: torch.randn(s, generator=g).to(torch.bfloat16).to(DEV)  # noqa: E731
+  x, w, out = r(M, B, K), torch.empty((B, N, K), dtype=torch.bfloat16, device=DEV), torch.empty((M, B, N), device=DEV)
+  for _ in range(20):
+    a, b, fixed = r(B * N, R), r(K, R), torch.empty_like(out)
+    ops.linear(w.view(B * N, K), a, b)
+    ops.linear_batched(out, x, w)
+    ops.linear_batched(fixed, x, w.clone(), fixed_weights=True)
+    want = torch.einsum("mbk,bnk->mbn", x.double(), w.double())
+    assert (out.double() - want).norm() <= K * 2.0 ** -23 * want.norm() and torch.equal(out, fixed)
+
+
 def test_float32_norms_do_not_depend_on_how_many_tokens_share_the_step():
   from miniinfer_b200.kernels import ops
   T, Q, C, R, P = 1500, 700, 192, 32, 64

@@ -362,7 +362,7 @@ def rms_pair_sum(out, a, b, w1, w2, eps, scale):
   out.copy_((scale * (w1 * unit(a) + w2 * unit(b))).to(out.dtype))
 
 
-def linear_batched(out, x, w, bias=None, softplus=False, row_gate=None, value_gate=None):
+def linear_batched(out, x, w, bias=None, softplus=False, row_gate=None, value_gate=None, fixed_weights=False):
   y = torch.einsum("mbk,bnk->mbn", x.float(), w.float())
   if bias is not None:
     y = y + bias
