@@ -553,8 +553,8 @@ latent_merge_kernel(Args a) {
   mi::grid_dependency_sync();
   const float* ml = a.part_ml + 2 * ((size_t)entry * a.max_splits * a.nh + head);
   const float* po = a.part_o + ((size_t)entry * a.max_splits * a.nh + head) * a.out_hd;
-  // Up to 32 pieces: a lane a piece's maximum and sum, a thread its value of all pieces, all on their way together (8 tokens of 32 heads in 9
-  // pieces, behind another kernel: 5.3 us by the loops below, so 4.8)
+  // Up to 32 pieces: a lane a piece's maximum and sum, a thread its value of eight pieces at a time, the first eight on their way with the
+  // maxima (8 tokens of 32 heads in 9 pieces, behind another kernel: 5.3 us by the loops below, so 4.8)
   if (n <= 32) {
     constexpr int AT_ONCE = 8;
     const int lane = threadIdx.x & 31;

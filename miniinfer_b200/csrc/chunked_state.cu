@@ -31,10 +31,10 @@
 // FMAs): delta rule, decays a channel about 1 / 50 a token 1.9e-7 (3.5e-7), 1 / 3000 3.2e-7 (3.4e-6), stronger than 1 / 2 1.2e-7
 // (0.7e-7); a head 1.6e-7 (2.4e-7), 2.3e-7 (4.2e-7), 1.2e-7 (0.9e-7); linear attention 1.4e-7 (1.7e-7), 4.7e-7 (1.3e-5), 0.65e-7 (0.3e-7).
 // Measured on B200, one request of 2048 tokens, 8 / 16 / 32 heads of 128 x 128, the whole operation in microseconds: delta rule with
-// one decay a key channel 129, 227, 412 (in stretches 1017, 1204, 1254), one a head 121, 208, 375, linear attention 82, 139, 248
-// (in stretches 173, 281, 476).  What bounds them: build and out run through some 50 and 20 KB of instructions once, which come from L2,
-// and their products at a third of the tensor cores' rate - splitting the operands takes as many issue slots as the products -; the walk
-// takes 2700 cycles a chunk with 8 columns a block, of which its two products' tensor cycles are 800.
+// one decay a key channel 130, 229, 416 (without chunks 1034, 1203, 1261), one a head 123, 210, 379 (692, 1105, 1151), linear attention
+// 82, 139, 249 (171, 270, 451), with a constant a head 75, 125, 226 (157, 231, 392).  What bounds them: build and out run through 60 to 80 and
+// 20 KB of instructions once, which come from L2, and their products at a third of the tensor cores' rate - splitting the operands takes as many
+// issue slots as the products -; the walk takes 2700 cycles a chunk with 8 columns a block, of which its two products' tensor cycles are 800.
 #include "chunked_state.cuh"
 
 #include <algorithm>

@@ -219,7 +219,7 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
 }
 
 template <int TM, bool SHARED, bool VEC>
-__global__ void __cluster_dims__(GROUPS, 1, 1) __launch_bounds__(128, SHARED ? 3 : 1)      // (as many as shared memory holds; with two 302 x 4096 x 1024 takes 89 us)
+__global__ void __cluster_dims__(GROUPS, 1, 1) __launch_bounds__(128, SHARED ? 3 : 1)      // (three, 168 registers a thread, of the four that shared memory holds; with two 302 x 4096 x 1024 takes 89 us)
 gemm_f32_groups_kernel(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w, int M, int N, int K, int ldx, int ldo) {
   product<TM, SHARED, true, VEC>(out, x, w, M, N, K, ldx, ldo, blockIdx.y, blockIdx.x / GROUPS, blockIdx.x % GROUPS);
 }

@@ -506,8 +506,8 @@ delta_prepare_rows_kernel(DeltaPrepArgs<__nv_bfloat16> a) {
           a.g[(size_t)t * a.heads + h] = expf(lg);
         }
       } else {
-  #pragma unroll 1
-      for (int i = 4 * lane; i < a.dim; i += 128) {
+#pragma unroll 1
+        for (int i = 4 * lane; i < a.dim; i += 128) {
           const float4 z = mi::load_row4(a.a + (size_t)t * a.lda + (size_t)h * a.dim + i), b = mi::load_row4(a.dt_bias + h * a.dim + i);
           *reinterpret_cast<float4*>(a.g + ((size_t)t * a.heads + h) * a.dim + i) =
             make_float4(delta_decay(z.x + b.x, neg_rate), delta_decay(z.y + b.y, neg_rate), delta_decay(z.z + b.z, neg_rate), delta_decay(z.w + b.w, neg_rate));
